@@ -27,6 +27,11 @@ __device__ __forceinline__ void ld_fresh4(const float* p, float (&f)[4]) {
   const float4 v = __ldcg(reinterpret_cast<const float4*>(p));
   f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
 }
+__device__ __forceinline__ void ld_fresh4(const uint16_t* p, float (&f)[4]) {
+  const uint2 v = __ldcg(reinterpret_cast<const uint2*>(p));
+  f[0] = __uint_as_float(v.x << 16); f[1] = __uint_as_float(v.x & 0xFFFF0000u);
+  f[2] = __uint_as_float(v.y << 16); f[3] = __uint_as_float(v.y & 0xFFFF0000u);
+}
 __device__ __forceinline__ float ld_fresh(const float* p) { return __ldcg(p); }
 __device__ __forceinline__ int ld_fresh(const int32_t* p) { return __ldcg(p); }
 
