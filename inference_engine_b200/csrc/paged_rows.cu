@@ -1,6 +1,8 @@
 // The paged cache of unquantised rows: rotary positions + unit norm + write of keys and values (one kernel; a second one
 // norms whole projections first and rotates neighbouring channels), and the
 // general attention over it (any sizes, bf16 or fp32, prompt portions and decoding alike) on the CUDA cores.
+#include <type_traits>
+
 #include "dec_common.cuh"
 
 namespace b200kv {
@@ -363,6 +365,240 @@ attn_rows_kernel(const T* __restrict__ q, DecCache c, b200dec_rows rows, int hea
   }
 }
 
+
+// ---------------------------------------------------------------- attention, one block per (tile of rows, kv head)
+// The rows of a tile are neighbours of one entry, and with the query heads of their kv head they make up to kAtSlots query
+// rows that share every key and value: kAtKeys keys and values at a time come to shared memory in whole lines, a thread
+// computes one key's scores with eight query rows, and a warp keeps four query rows' softmax and output, a lane's channels
+// 4 lane + 128 i + (0..3).  A score is the same chain of multiply-adds as in attn_rows_kernel, where every thread reads a key
+// row of its own from L1, a line per 16 bytes: that, not the arithmetic, bounded it.  Here it is the shared-memory reads (a key
+// against eight query rows, a value against four) and, with few entries, one block's chain of steps.
+// fp32, us, attn_rows_kernel -> this: 200 rows, 16 heads of 112 and 96, 183 -> 43; 8 entries of 550 decoding, 16 heads of 128, 420 -> 67.
+constexpr int kAtThreads = 128;
+constexpr int kAtSlots = 16;
+constexpr int kAtKeys = 64;
+constexpr int kAtPitch = 20;  // of the scores of one key: 16 and 4 that spread the banks
+
+// 16 bytes of which the first `bytes` are copied and the others zero
+__device__ __forceinline__ void at_copy16(float* dst, const float* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(max(bytes, 0))
+               : "memory");
+}
+__device__ __forceinline__ void at_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void at_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+__host__ __device__ constexpr size_t at_floats(int k_row, int v_row) {
+  return (size_t)kAtSlots * k_row + (size_t)kAtKeys * (k_row + 4) + (size_t)kAtKeys * v_row + kAtKeys * kAtPitch;
+}
+
+template <typename T, int kPieces>  // kPieces: output channels, in pieces of 128
+__global__ void __launch_bounds__(kAtThreads, 3)
+attn_tile_kernel(const T* __restrict__ q, DecCache c, b200dec_rows rows, int heads, int slice_heads, float scale, DecAttnOpt opt,
+                 T* __restrict__ out, int32_t* status) {
+  extern __shared__ __align__(16) float at_smem[];
+  const int kp = c.k_row + 4;  // an odd number of 16-byte words: neighbouring keys lie in different banks
+  float* qs = at_smem;                  // [kAtSlots][k_row]
+  float* ks = qs + kAtSlots * c.k_row;  // [kAtKeys][kp]
+  float* vs = ks + kAtKeys * kp;        // [kAtKeys][v_row]
+  float* ps = vs + kAtKeys * c.v_row;   // [kAtKeys][kAtPitch]
+  __shared__ long long at[2][kAtKeys];  // a key's row in the cache, -1: none; of this step and the next
+  constexpr int kWarps = kAtThreads / 32;
+  pdl_enter();
+  const int r0 = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int G = heads / c.heads, slices = (G + kAtSlots - 1) / kAtSlots;
+  const int hk = blockIdx.x / slices, g0 = blockIdx.x % slices * slice_heads, gs = min(slice_heads, G - g0);
+  const int most = kAtSlots / slice_heads;  // rows of a tile
+  // a tile starts at the first row of an entry and at the positions that are multiples of its size
+  int seq = r0, pos, n = 1;
+  if (rows.seq_ids) {
+    seq = rows.seq_ids[r0];
+    pos = rows.positions[r0];
+    if (r0 > 0 && pos >= 0 && pos % most != 0 && rows.seq_ids[r0 - 1] == seq && rows.positions[r0 - 1] == pos - 1) return;
+    while (pos >= 0 && n < most && r0 + n < rows.num_rows && (pos + n) % most != 0 && rows.seq_ids[r0 + n] == seq &&
+           rows.positions[r0 + n] == pos + n)
+      ++n;
+  } else {
+    pos = r0 < *rows.num_decoding ? rows.cached_lens[r0] : -1;
+  }
+  pdl_wait();
+  const int slots = n * gs;
+  if (pos < 0) {  // idle row
+    T* dst = out + r0 * opt.out_stride + (hk * G + g0) * c.v_dim;
+    for (int i = tid; i < gs * c.v_dim; i += kAtThreads) st_elem(dst + i, 0.f);
+    return;
+  }
+  for (int s = warp; s < kAtSlots; s += kWarps) {
+    const T* src = q + ((long long)(r0 + s / gs) * heads + hk * G + g0 + s % gs) * c.k_row;
+    for (int ch = lane; ch < c.k_row; ch += 32) qs[s * c.k_row + ch] = s < slots && ch < c.k_dim ? ld_elem(src + ch) * scale : 0.f;
+  }
+  // what this warp keeps: query rows 4 warp + (0..3)
+  float m[4], l[4], o[4][kPieces][4];
+  int last[4], low[4];  // the keys each of them sees
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int s = 4 * warp + i, h = hk * G + g0 + s % gs;
+    last[i] = s < slots ? pos + s / gs : -1;
+    low[i] = s < slots && opt.window > 0 ? max(0, last[i] - opt.window + 1) : 0;
+    m[i] = opt.sink && s < slots ? opt.sink[h] : -INFINITY;
+    l[i] = opt.sink ? 1.f : 0.f;
+#pragma unroll
+    for (int j = 0; j < kPieces; ++j)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) o[i][j][k] = 0.f;
+  }
+  const bool mine = 4 * warp < slots;
+  // Keys [all_low, all_last] are seen by every query row of the tile; the others are looked at one by one, so that what a row
+  // does not see (a later token, perhaps not a number) never meets it.
+  const int all_last = pos, all_low = opt.window > 0 ? max(0, pos + n - opt.window) : 0, end = pos + n;
+  const int first = opt.window > 0 ? max(0, pos - opt.window + 1) : 0;
+  // the rows of the keys from j0 on
+  auto look_up = [&](int j0, long long* at_rows) {
+    if (tid < kAtKeys) {
+      const int page = j0 + tid < end ? dec_page(c, seq, j0 + tid, status) : -1;
+      at_rows[tid] = page < 0 ? -1 : dec_row(c, page, hk, (j0 + tid) % c.P);
+    }
+  };
+  // their keys or values to shared memory, zero where there is none and behind `dim`
+  auto fetch = [&](const long long* at_rows, const void* cache, int row, int dim, float* to, int pitch) {
+    for (int k0 = warp; k0 < kAtKeys; k0 += 4 * kWarps) {
+      long long src[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) src[u] = at_rows[k0 + u * kWarps] * row;
+      for (int ch = 4 * lane; ch < row; ch += 128) {
+        float* d = to + k0 * pitch + ch;
+        if constexpr (sizeof(T) == 4) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            at_copy16(d + u * kWarps * pitch, (const float*)cache + max(src[u], 0ll) + ch, src[u] < 0 ? 0 : min(16, 4 * (dim - ch)));
+        } else {
+          float f[4][4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) ld_elem4((const T*)cache + max(src[u], 0ll) + ch, f[u]);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (src[u] < 0 || ch + e >= dim) f[u][e] = 0.f;
+            st_elem4(d + u * kWarps * pitch, f[u]);
+          }
+        }
+      }
+    }
+    at_commit();
+  };
+  // The keys of a step are fetched while the values of the one before are used, its values while its scores are made.
+  look_up(first, at[0]);
+  __syncthreads();
+  fetch(at[0], c.k, c.k_row, c.k_dim, ks, kp);
+  fetch(at[0], c.v, c.v_row, c.v_dim, vs, c.v_row);
+  for (int j0 = first, turn = 0; j0 < end; j0 += kAtKeys, turn ^= 1) {
+    const int count = min(kAtKeys, end - j0);
+    const bool more = j0 + kAtKeys < end;
+    look_up(j0 + kAtKeys, at[turn ^ 1]);
+    at_wait<1>();
+    __syncthreads();  // the keys are there, the scores of the step before are used
+    const int key = tid & (kAtKeys - 1), s0 = tid / kAtKeys * 8;
+    if (s0 < slots) {
+      const float *kr = ks + key * kp, *qr = qs + s0 * c.k_row;
+      float acc[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+      auto dots = [&](auto rows_at_once) {
+        constexpr int kN = decltype(rows_at_once)::value;
+#pragma unroll 2
+        for (int ch = 0; ch < c.k_row; ch += 4) {
+          const float4 kv = *reinterpret_cast<const float4*>(kr + ch);
+#pragma unroll
+          for (int i = 0; i < kN; ++i) {
+            const float4 x = *reinterpret_cast<const float4*>(qr + i * c.k_row + ch);
+            acc[i] = fmaf(x.w, kv.w, fmaf(x.z, kv.z, fmaf(x.y, kv.y, fmaf(x.x, kv.x, acc[i]))));
+          }
+        }
+      };
+      if (slots - s0 <= 2) dots(std::integral_constant<int, 2>{}); else dots(std::integral_constant<int, 8>{});
+      *reinterpret_cast<float4*>(ps + key * kAtPitch + s0) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+      *reinterpret_cast<float4*>(ps + key * kAtPitch + s0 + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
+    }
+    __syncthreads();  // the keys are used
+    if (more) fetch(at[turn ^ 1], c.k, c.k_row, c.k_dim, ks, kp); else at_commit();
+    at_wait<1>();
+    __syncthreads();  // every thread's part of the values is there
+    if (mine) {
+      // softmax of the warp's four query rows, keys lane and lane + 32
+      float p[2][4];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int k = lane + 32 * u, j = j0 + k;
+        const float4 x = *reinterpret_cast<const float4*>(ps + k * kAtPitch + 4 * warp);
+        const bool some = at[turn][k] >= 0;
+        p[u][0] = x.x; p[u][1] = x.y; p[u][2] = x.z; p[u][3] = x.w;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (!some || j > last[i] || j < low[i]) p[u][i] = -INFINITY;
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float mx = fmaxf(p[0][i], p[1][i]);
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+        const float mn = fmaxf(m[i], mx), base = mn == -INFINITY ? 0.f : mn, alpha = expf(m[i] - base);
+        m[i] = mn;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) p[u][i] = expf(p[u][i] - base);
+        l[i] = l[i] * alpha + warp_sum(p[0][i] + p[1][i]);
+#pragma unroll
+        for (int a = 0; a < kPieces; ++a)
+#pragma unroll
+          for (int b = 0; b < 4; ++b) o[i][a][b] *= alpha;
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) st_elem4(ps + (lane + 32 * u) * kAtPitch + 4 * warp, p[u]);
+      __syncwarp();
+      auto add = [&](int k, bool every) {
+        const float4 w4 = *reinterpret_cast<const float4*>(ps + k * kAtPitch + 4 * warp);
+        const float w[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+        for (int a = 0; a < kPieces; ++a) {
+          const int ch = 4 * lane + 128 * a;
+          if (ch >= c.v_row) break;
+          const float4 v = *reinterpret_cast<const float4*>(vs + k * c.v_row + ch);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if (!every && (j0 + k > last[i] || j0 + k < low[i])) continue;
+            o[i][a][0] = fmaf(w[i], v.x, o[i][a][0]);
+            o[i][a][1] = fmaf(w[i], v.y, o[i][a][1]);
+            o[i][a][2] = fmaf(w[i], v.z, o[i][a][2]);
+            o[i][a][3] = fmaf(w[i], v.w, o[i][a][3]);
+          }
+        }
+      };
+      // (a key without a page has a weight and a value of zero)
+      const int e0 = min(max(all_low - j0, 0), count), e1 = max(e0, min(all_last + 1 - j0, count));
+      for (int k = 0; k < e0; ++k) add(k, false);
+#pragma unroll 4
+      for (int k = e0; k < e1; ++k) add(k, true);
+      for (int k = e1; k < count; ++k) add(k, false);
+    }
+    __syncthreads();  // the values are used
+    if (more) fetch(at[turn ^ 1], c.v, c.v_row, c.v_dim, vs, c.v_row); else at_commit();
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int s = 4 * warp + i;
+    if (s >= slots) break;
+    const int r = r0 + s / gs, h = hk * G + g0 + s % gs;
+    const float inv = (l[i] > 0.f ? 1.f / l[i] : 0.f) * opt.factor<T>(r, h);
+#pragma unroll
+    for (int a = 0; a < kPieces; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const int ch = 4 * lane + 128 * a + b;
+        if (ch < c.v_dim) st_elem(out + r * opt.out_stride + (long long)h * c.v_dim + ch, o[i][a][b] * inv);
+      }
+  }
+}
+
 }  // namespace b200kv
 
 using namespace b200kv;
@@ -456,9 +692,23 @@ extern "C" int b200dec_attn_rows_opt(const void* q, const b200dec_cache* cache, 
   if (rc != B200KV_OK) return rc;
   if (heads < 1 || heads % cache->kv_heads || cache->v_dim > kArThreads * kArPieces || cache->k_dim > 1024) return B200KV_E_SHAPE;
   if ((long long)cache->num_pages * cache->page_size > 0x7FFFFFFFll || rows->num_rows > 65535) return B200KV_E_RANGE;
-  const size_t smem = (size_t)((cache->k_dim + 3) / 4 * 4 + 2 * kArKeys) * 4;
   const DecCache c = dec_view(cache, table);
   cudaStream_t s = (cudaStream_t)stream;
+  // The line is two blocks of the tile kernel per multiprocessor: heads beyond about 190 channels (of key and value on average)
+  // keep the block per row and head, whose shared memory does not grow with them.
+  const size_t tile_smem = at_floats(cache->k_row, cache->v_row) * 4;
+  if (tile_smem <= 112 * 1024 && cache->v_row <= 256) {
+    const int G = heads / cache->kv_heads, slices = (G + kAtSlots - 1) / kAtSlots, slice_heads = (G + slices - 1) / slices;
+    auto tiles = [&](auto* kernel, auto* in, auto* o) -> int {
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem) != cudaSuccess) return B200KV_E_LAUNCH;
+      return launch_result(launch_chained(kernel, dim3(cache->kv_heads * slices, rows->num_rows), dim3(kAtThreads), tile_smem, s, in, c, *rows,
+                                          heads, slice_heads, scale, opt, o, status));
+    };
+    if (cache->elem == 2)
+      return tiles(cache->v_row <= 128 ? attn_tile_kernel<uint16_t, 1> : attn_tile_kernel<uint16_t, 2>, (const uint16_t*)q, (uint16_t*)out);
+    return tiles(cache->v_row <= 128 ? attn_tile_kernel<float, 1> : attn_tile_kernel<float, 2>, (const float*)q, (float*)out);
+  }
+  const size_t smem = (size_t)((cache->k_dim + 3) / 4 * 4 + 2 * kArKeys) * 4;
   if (cache->elem == 2)
     return launch_result(launch_chained(attn_rows_kernel<uint16_t>, dim3(heads, rows->num_rows), dim3(kArThreads), smem, s,
                                         (const uint16_t*)q, c, *rows, heads, scale, opt, (uint16_t*)out, status));

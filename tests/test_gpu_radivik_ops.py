@@ -159,6 +159,38 @@ def test_attention_single_key_stands_out(heads, kv, dim, vdim, page):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads,kv,dim,vdim", [(2, 2, 24, 40), (16, 1, 32, 132), (5, 1, 36, 256), (34, 2, 16, 8), (4, 2, 184, 184), (4, 2, 192, 192)])
+def test_attention_rows_in_tiles(heads, kv, dim, vdim, dtype):
+    """Tiles of neighbouring rows at their edges: groups of 1 to 17 query heads, entries that begin and end within a tile or
+    one key around a step of 64, the largest sizes of the tiles and the first beyond; a row's result does not depend on what
+    a later token's key and value are."""
+    from inference_engine_b200 import ops
+
+    g = np.random.default_rng(dim)
+    entries = [(63, 1), (500, 1), (0, 66), (61, 7), (64, 64), (125, 5), (7, 1)]
+    rows, table, pages, _ = make_rows(entries, 8)
+    cache = ops.make_paged_kv(pages, kv, 8, dim, vdim, dtype, DEV)
+    q, want, at = H.bf16(g.standard_normal((rows.num_rows, heads, dim))), np.zeros((rows.num_rows, heads, vdim)), 0
+    ends = []
+    for b, (c, x) in enumerate(entries):
+        k, v = H.bf16(g.standard_normal((c + x, kv, dim))), H.bf16(g.standard_normal((c + x, kv, vdim)))
+        fill(cache, table, b, t(k, dtype), t(v, dtype))
+        want[at : at + x] = R.causal_attention(q[at : at + x], k, v, dim ** -0.5, c)
+        at += x
+        ends.append((at - 1, int(table[b, (c + x - 1) // 8]), (c + x - 1) % 8))
+    qd = torch.zeros(rows.num_rows, heads, cache.k.shape[3], device=DEV, dtype=dtype)
+    qd[..., :dim] = t(q, dtype)
+    out = ops.attention_rows(qd, cache, rows, dim ** -0.5)
+    close(out, want, dtype)
+    for _, page, slot in ends:
+        cache.k[page, :, slot], cache.v[page, :, slot] = float("nan"), float("inf")
+    again = ops.attention_rows(qd, cache, rows, dim ** -0.5)
+    others = [r for r in range(rows.num_rows) if r not in [e[0] for e in ends]]
+    assert torch.equal(out[others], again[others])
+    H.status_clear()
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 def test_attention_beyond_the_tensor_core_sizes(dtype):
     from inference_engine_b200 import ops
 
