@@ -61,6 +61,28 @@ __device__ __forceinline__ float sum_squares_ordered(const float (&x)[4], float*
   return __fadd_rn(first, second);
 }
 
+// The same of two head rows at once: lanes 0-15 add up the first and lanes 16-31 the second, whose sum they get.  A segment
+// of 64 starts 8 banks further than the one in front of it; `sq` is this warp's scratch of kSqPair floats.
+constexpr int kSqPair = 4 * (kHalfD + 8);
+__device__ __forceinline__ float sum_squares_ordered2(const float (&x)[4], const float (&y)[4], float* sq, int lane) {
+  float* at = sq + 4 * lane + 8 * (lane >> 4);
+  __syncwarp();
+  *reinterpret_cast<float4*>(at) = make_float4(__fmul_rn(x[0], x[0]), __fmul_rn(x[1], x[1]), __fmul_rn(x[2], x[2]), __fmul_rn(x[3], x[3]));
+  *reinterpret_cast<float4*>(at + kSqPair / 2) =
+      make_float4(__fmul_rn(y[0], y[0]), __fmul_rn(y[1], y[1]), __fmul_rn(y[2], y[2]), __fmul_rn(y[3], y[3]));
+  __syncwarp();
+  const float* a = sq + (lane >> 3) * (kHalfD + 8) + (lane & 7);
+  float r = a[0];
+#pragma unroll
+  for (int i = 1; i < 8; ++i) r = __fadd_rn(r, a[8 * i]);
+  r = __fadd_rn(r, __shfl_xor_sync(0xffffffffu, r, 1));
+  r = __fadd_rn(r, __shfl_xor_sync(0xffffffffu, r, 2));
+  r = __fadd_rn(r, __shfl_xor_sync(0xffffffffu, r, 4));
+  const float first = __shfl_sync(0xffffffffu, r, lane & 16);
+  const float second = __shfl_sync(0xffffffffu, r, (lane & 16) + 8);
+  return __fadd_rn(first, second);
+}
+
 // RMSNorm + half-split rotation of one head row; result elements d = 4*lane + c.
 // kernels.py:414-436 / 583-633.  The operands are already in registers, so that a caller can put all of its
 // loads (this row, the page table, the calibration) in flight before the first arithmetic instruction needs one.
@@ -310,7 +332,13 @@ __device__ __forceinline__ int page_of(const CacheView& c, int b, int pos, int32
 // kFusedNorm = true: q, k are the raw projections; the kernel norms and ropes every row of them into q_out / k_out
 // (what fused_norm_rope_prefill does, kernels.py:547-670) and quantizes from the bf16-rounded k it just produced.
 // kFusedNorm = false: k is already normed + roped bf16 (the argument of quantize_kv_prefill), q is not touched.
-// grid (N, ceil(jobs / 8)); warp job: [0, Hq) q heads (fused only), then Hkv k heads, then Hkv v heads.
+// grid (N, ceil(jobs / warps of a block)); warp job: kRowHeads heads of one kind, q (fused only), then k, then v.
+// Instructions bound it, so a warp does everything that heads of a row share once (the row's entry, page, angles, norm weight)
+// and sums, roots and divisions of two heads at a time: 1011 rows
+// of 32 heads in first portions 12.1 us with one head per warp, now 9.0; 992 on 3072 beside 32 decoding entries 15.0, 13.9.
+constexpr int kRowHeads = 4;
+__host__ __device__ constexpr int row_jobs(int heads) { return (heads + kRowHeads - 1) / kRowHeads; }
+
 template <bool kFusedNorm>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 prefill_rows_kernel(const uint16_t* __restrict__ q, long long q_sn, long long q_sh,
@@ -322,15 +350,15 @@ prefill_rows_kernel(const uint16_t* __restrict__ q, long long q_sn, long long q_
                     uint16_t* __restrict__ k_out, long long ko_sn, long long ko_sh,
                     CacheView c, const int32_t* __restrict__ cu, int num_entries, const int32_t* __restrict__ cached_lens,
                     const int32_t* __restrict__ num_decoding, int Hq, float eps, int32_t* status) {
-  __shared__ __align__(16) float sq_all[kFusedNorm ? kWarpsPerBlock : 1][kD];
+  __shared__ __align__(16) float sq_all[kFusedNorm ? kWarpsPerBlock : 1][kSqPair];
   pdl_enter();
   const int r = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int job = blockIdx.y * kWarpsPerBlock + warp;
-  const int Hkv = c.Hkv, nq = kFusedNorm ? Hq : 0;
-  if (job >= nq + 2 * Hkv) return;
-  const bool is_q = job < nq, is_k = !is_q && job < nq + Hkv;
-  const int j = is_q ? job : (is_k ? job - nq : job - nq - Hkv);
+  const int job = blockIdx.y * (blockDim.x >> 5) + warp;
+  const int Hkv = c.Hkv, q_jobs = kFusedNorm ? row_jobs(Hq) : 0, kv_jobs = row_jobs(Hkv);
+  if (job >= q_jobs + 2 * kv_jobs) return;
+  const bool is_q = job < q_jobs, is_k = !is_q && job < q_jobs + kv_jobs;
+  const int j0 = kRowHeads * (is_q ? job : (is_k ? job - q_jobs : job - q_jobs - kv_jobs)), heads = min(kRowHeads, (is_q ? Hq : Hkv) - j0);
   // round one (metadata, readable before the wait): the row's entry
   const int nd = *num_decoding;
   const RowEntry re = find_row_entry(cu, num_entries, cached_lens, c, r, lane);
@@ -339,48 +367,78 @@ prefill_rows_kernel(const uint16_t* __restrict__ q, long long q_sn, long long q_
   if (!kFusedNorm && (!prefilling || (is_k && first_chunk))) return;  // nothing to quantize here
   if (kFusedNorm && !is_q && !is_k && !prefilling) return;
   pdl_wait();  // q, k, v come from the kernel before this one
-  HeadRow row;
-  if (kFusedNorm && is_q) row = load_head_row(q + act_offset(r, q_sn, j, q_sh), qw, cosp + (long long)r * (int)cos_sn, sinp + (long long)r * (int)sin_sn, lane);
-  else if (kFusedNorm && is_k) row = load_head_row(k + act_offset(r, k_sn, j, k_sh), kw, cosp + (long long)r * (int)cos_sn, sinp + (long long)r * (int)sin_sn, lane);
-  else row.x = *reinterpret_cast<const uint2*>((is_k ? k + act_offset(r, k_sn, j, k_sh) : v + act_offset(r, v_sn, j, v_sh)) + 4 * lane);
-  // round two: the page of this row's token and the entry's calibration
+  const bool normed = kFusedNorm && (is_q || is_k);
+  const uint16_t* src = is_q ? q : (is_k ? k : v);
+  const long long src_sn = is_q ? q_sn : (is_k ? k_sn : v_sn), src_sh = is_q ? q_sh : (is_k ? k_sh : v_sh);
+  uint2 raw[kRowHeads], w_raw, c_raw, s_raw;
+#pragma unroll
+  for (int i = 0; i < kRowHeads; ++i)  // (a head that is not there repeats the last one)
+    raw[i] = *reinterpret_cast<const uint2*>(src + act_offset(r, src_sn, j0 + min(i, heads - 1), src_sh) + 4 * lane);
+  if (normed) {
+    w_raw = *reinterpret_cast<const uint2*>((is_q ? qw : kw) + 4 * lane);
+    c_raw = *reinterpret_cast<const uint2*>(cosp + (long long)r * (int)cos_sn + 4 * (lane & 15));
+    s_raw = *reinterpret_cast<const uint2*>(sinp + (long long)r * (int)sin_sn + 4 * (lane & 15));
+  }
+  // round two: the page of this row's token
   const bool quantizes = prefilling && !is_q && !(is_k && first_chunk);
   const int pos = re.cached + (r - re.start);
   int page = -1;
-  float cal[4] = {1.f, 1.f, 1.f, 1.f};
   if (quantizes) {
     page = page_of(c, re.b, pos, status, lane);
-    if (is_k) {
-      if (re.page0 < 0 || re.page0 >= c.num_pages) {
-        if (lane == 0 && status) atomicOr(status, B200KV_S_BAD_PAGE);
-        page = -1;
-      } else {
-        load4_f32(c.k_cal + cal_offset(c, re.page0, j), lane, cal);
-      }
+    if (is_k && (re.page0 < 0 || re.page0 >= c.num_pages)) {
+      if (lane == 0 && status) atomicOr(status, B200KV_S_BAD_PAGE);
+      page = -1;
     }
   }
-  float x[4];
-  if (kFusedNorm && (is_q || is_k)) {
-    norm_rope_regs(row, eps, sq_all[kFusedNorm ? warp : 0], lane, x);
-    if (is_q) {
-      store4_bf16(q_out + act_offset(r, qo_sn, j, qo_sh), lane, x);
-      return;
-    }
-    store4_bf16(k_out + act_offset(r, ko_sn, j, ko_sh), lane, x);
+  float x[kRowHeads][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) x[i] = bf16_bits_to_float(float_to_bf16_bits(x[i]));  // the quantizer reads the stored bf16
-  } else {
-    unpack4(row.x, x);
+  for (int i = 0; i < kRowHeads; ++i) unpack4(raw[i], x[i]);
+  if (normed) {
+    float wv[4], cs[4], sn[4];
+    unpack4(w_raw, wv);
+    unpack4(c_raw, cs);
+    unpack4(s_raw, sn);
+    const bool first_half = lane < 16;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sn[i] = first_half ? -sn[i] : sn[i];
+#pragma unroll
+    for (int i = 0; i < kRowHeads; i += 2) {  // the arithmetic of norm_rope_regs
+      const float ss = sum_squares_ordered2(x[i], x[i + 1], sq_all[kFusedNorm ? warp : 0], lane);
+      const float rstd = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fmul_rn(ss, 0.0078125f), eps)));
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const float mine = __shfl_sync(0xffffffffu, rstd, 16 * u);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float y = __fmul_rn(__fmul_rn(x[i + u][e], mine), wv[e]);
+          const float other = __shfl_xor_sync(0xffffffffu, y, 16);
+          x[i + u][e] = __fadd_rn(__fmul_rn(y, cs[e]), __fmul_rn(other, sn[e]));
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kRowHeads; ++i) {
+      if (i >= heads) break;
+      store4_bf16((is_q ? q_out + act_offset(r, qo_sn, j0 + i, qo_sh) : k_out + act_offset(r, ko_sn, j0 + i, ko_sh)), lane, x[i]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[i][e] = bf16_bits_to_float(float_to_bf16_bits(x[i][e]));  // the quantizer reads the stored bf16
+    }
   }
   if (!quantizes || page < 0) return;
   int slot_unused, prow;
   split_pos(c, pos, slot_unused, prow);
-  if (is_k) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) x[i] = __fdiv_rn(x[i], cal[i]);
-    quantize_store(x, c.k + code_offset(c, page, j, prow), c.k_scale + scale_offset(c, page, j, prow), lane);
-  } else {
-    quantize_store(x, c.v + code_offset(c, page, j, prow), c.v_scale + scale_offset(c, page, j, prow), lane);
+  for (int i = 0; i < kRowHeads; ++i) {
+    if (i >= heads) break;
+    if (is_k) {
+      float cal[4];
+      load4_f32(c.k_cal + cal_offset(c, re.page0, j0 + i), lane, cal);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[i][e] = __fdiv_rn(x[i][e], cal[e]);
+      quantize_store(x[i], c.k + code_offset(c, page, j0 + i, prow), c.k_scale + scale_offset(c, page, j0 + i, prow), lane);
+    } else {
+      quantize_store(x[i], c.v + code_offset(c, page, j0 + i, prow), c.v_scale + scale_offset(c, page, j0 + i, prow), lane);
+    }
   }
 }
 
@@ -672,7 +730,8 @@ extern "C" int b200kv_quantize_prefill(const void* k, int64_t k_sn, int64_t k_sh
   const int Hkv = cache->num_kv_heads;
   CacheView view = make_view(cache, table);
   cudaStream_t s = (cudaStream_t)stream;
-  launch_chained(prefill_rows_kernel<false>, dim3(N, (2 * Hkv + kWarpsPerBlock - 1) / kWarpsPerBlock), dim3(kWarpsPerBlock * 32), 0, s,
+  const int jobs = 2 * row_jobs(Hkv), warps = jobs < kWarpsPerBlock ? jobs : kWarpsPerBlock;
+  launch_chained(prefill_rows_kernel<false>, dim3(N, (jobs + warps - 1) / warps), dim3(warps * 32), 0, s,
                  (const uint16_t*)nullptr, 0LL, 0LL, (const uint16_t*)k, (long long)k_sn, (long long)k_sh, (const uint16_t*)v,
                  (long long)v_sn, (long long)v_sh, (const uint16_t*)nullptr, (const uint16_t*)nullptr, (const uint16_t*)nullptr,
                  0LL, (const uint16_t*)nullptr, 0LL, (uint16_t*)nullptr, 0LL, 0LL, (uint16_t*)nullptr, 0LL, 0LL, view,
@@ -707,8 +766,8 @@ extern "C" int b200kv_write_prefill(const void* q, int64_t q_sn, int64_t q_sh, c
     return B200KV_E_ALIGN;
   CacheView view = make_view(cache, table);
   cudaStream_t s = (cudaStream_t)stream;
-  launch_chained(prefill_rows_kernel<true>, dim3(N, (Hq + 2 * Hkv + kWarpsPerBlock - 1) / kWarpsPerBlock),
-                 dim3(kWarpsPerBlock * 32), 0, s, (const uint16_t*)q, (long long)q_sn, (long long)q_sh, (const uint16_t*)k,
+  const int jobs = row_jobs(Hq) + 2 * row_jobs(Hkv), warps = jobs < kWarpsPerBlock ? jobs : kWarpsPerBlock;
+  launch_chained(prefill_rows_kernel<true>, dim3(N, (jobs + warps - 1) / warps), dim3(warps * 32), 0, s, (const uint16_t*)q, (long long)q_sn, (long long)q_sh, (const uint16_t*)k,
                  (long long)k_sn, (long long)k_sh, (const uint16_t*)v, (long long)v_sn, (long long)v_sh, (const uint16_t*)qw,
                  (const uint16_t*)kw, (const uint16_t*)cosp, (long long)cos_sn, (const uint16_t*)sinp, (long long)sin_sn,
                  (uint16_t*)q_out, (long long)qo_sn, (long long)qo_sh, (uint16_t*)k_out, (long long)ko_sn, (long long)ko_sh, view,
