@@ -10,7 +10,10 @@
 // A single long portion does not fill the machine.  It is then cut into up to kSsSegments pieces: a first launch carries each
 // piece but the last from zero (the first one from the request's state), a second one starts every piece from the pieces in
 // front of it, decayed.  How many pieces there are is settled on the device, from the step's entries.
-// Chunks arrive by asynchronous copies into a ring shared by a block's warps.
+// Chunks arrive by asynchronous copies into a ring shared by a block's warps.  Bound by the chain of one chunk, with two warps per
+// scheduler to hide it.  What depends on the tokens alone (steps, decays and their exponentials) is found for 128 of them
+// at a time, a token per thread, instead of by every warp for every chunk: one portion of 1024, 64 heads of 128 x 64,
+// both launches 70.2 -> 54.2 us; five portions of 1000 rows, 48 heads of 64 x 64, 35.6 -> 28.2.
 #include "recurrence.cuh"
 
 namespace b200kv {
@@ -20,6 +23,7 @@ constexpr int kSsWarps = 4;   // 64 columns per block
 constexpr int kSsStages = 4;
 constexpr int kSsSegments = 4;
 constexpr int kSsMinSegment = 64;  // tokens
+constexpr int kSsAhead = 2 * kSsWarps;  // chunks whose steps a block finds at a time, a token per thread
 constexpr int kSsXRow = 16 * kSsWarps + 8;  // bf16 per row of x in shared memory (the padding spreads rows over the banks)
 
 __device__ __forceinline__ void ss_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -55,6 +59,11 @@ __device__ __forceinline__ void ss_split(float a, float b, uint32_t& t0, uint32_
   t1 = ss_pack(a, b);
   t2 = ss_pack(a - ss_lo(t1), b - ss_hi(t1));
 }
+// p[0], p[1], p[8], p[9]
+__device__ __forceinline__ void ss_pairs(const float* p, float (&f)[4]) {
+  const float2 a = *reinterpret_cast<const float2*>(p), b = *reinterpret_cast<const float2*>(p + 8);
+  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
+}
 __device__ __forceinline__ void ss_cp16(uint32_t dst, const void* src, int bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
@@ -83,15 +92,22 @@ __device__ __forceinline__ SsCut ss_cut(const b200dec_entries& ent, int nd, int 
   return c;
 }
 
+// Floats of one head's state in a place, padded to what the blocks hold.
+__host__ __device__ constexpr long long ss_place_floats(int kn, int vdim) {
+  return (long long)kn * ((vdim + 16 * kSsWarps - 1) / (16 * kSsWarps) * 16 * kSsWarps);
+}
+
 // kN16: 16-channel pieces of the state's rows (padding is zero).  kLocal: the first launch.
-// Workspace: 2 * kSsSegments places of [head][state channel][round4(vdim)], then [kSsSegments][head] sums of log-decays.
+// Workspace: 2 * kSsSegments places of [head][16 columns][8 channels][lane][4], then [kSsSegments][head] sums of log-decays.
 template <int kN16, bool kLocal>
-__global__ void __launch_bounds__(32 * kSsWarps)
+__global__ void __launch_bounds__(32 * kSsWarps, 2)
 ssd_scan_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, const uint16_t* __restrict__ conv, int conv_stride,
                 const b200dec_entries ent, float* __restrict__ out, int slabs, int max_segments, float* ws, int32_t* status) {
   constexpr int kN = 16 * kN16, kRow = kN + 8;  // bf16 per row of b and c in shared memory
   constexpr uint32_t kStage = kSsTok * (2 * kRow + kSsXRow) * 2;
   extern __shared__ __align__(16) uint8_t ss_smem[];
+  // of the tokens of kSsAhead chunks: dt, the log-decays' sum L in the chunk (units of log 2), exp(L), dt exp(L_16 - L)
+  __shared__ __align__(16) float dts[kSsAhead * kSsTok], logd[kSsAhead * kSsTok], grown[kSsAhead * kSsTok], weight[kSsAhead * kSsTok];
   pdl_enter();
   const int e = blockIdx.y, h = blockIdx.x / slabs, slab = blockIdx.x - h * slabs, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int seg = blockIdx.z, nd = *ent.num_decoding;
@@ -146,8 +162,10 @@ ssd_scan_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, co
   const int p0 = col0 + warp * 16 + g;  // this lane's rows of S^T: p0 and p0 + 8
   const long long head_floats = (long long)N * P4;
   float* state = rec.state + ((long long)x.slot * rec.heads + h) * head_floats;
-  auto place = [&](int i) { return ws + ((long long)i * rec.heads + h) * head_floats; };
-  float* logs = ws + 2 * kSsSegments * rec.heads * head_floats;
+  // a place holds the states as the lanes do, so that a lane moves 16 bytes and a warp whole lines
+  const long long place_floats = ss_place_floats(16 * kN16, P);
+  auto place = [&](int i) { return ws + ((long long)i * rec.heads + h) * place_floats + (slab * kSsWarps + warp) * (2 * kN16 * 128) + 4 * lane; };
+  float* logs = ws + 2 * kSsSegments * rec.heads * place_floats;
   float S[2 * kN16][4];
   auto each = [&](auto f) {  // over the state entries this lane holds
 #pragma unroll
@@ -161,54 +179,67 @@ ssd_scan_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, co
   auto put = [&](float* dst) {
     each([&](float& s, int d, int p) { if (d < N && p < P4) dst[(long long)d * P4 + p] = p < P ? s : 0.f; });
   };
+  auto put_place = [&](float* dst) {
+#pragma unroll
+    for (int n = 0; n < 2 * kN16; ++n) st_elem4(dst + 128 * n, S[n]);
+  };
   each([&](float& s, int, int) { s = 0.f; });
   if (kLocal) {
     if (seg == 0) {
       if (x.pos > 0) take(state);
-      put(place(cut.front));
+      put_place(place(cut.front));
     }
   } else if (cut.count == 1) {
     if (x.pos > 0) take(state);
   } else if (seg == 0) {
-    take(place(cut.front));
+    const float* src = place(cut.front);
+#pragma unroll
+    for (int n = 0; n < 2 * kN16; ++n) ld_fresh4(src + 128 * n, S[n]);
   } else {
-    take(place(cut.first));
-    for (int r = 1; r < seg; ++r) {
-      const float f = exp2f(__ldcg(logs + (long long)(cut.first + r) * rec.heads + h));
+    for (int r = 0; r < seg; ++r) {
+      const float f = r == 0 ? 0.f : exp2f(__ldcg(logs + (long long)(cut.first + r) * rec.heads + h));
       const float* src = place(cut.first + r);
-      each([&](float& s, int d, int p) { s = fmaf(s, f, d < N && p < P ? __ldcg(src + (long long)d * P4 + p) : 0.f); });
+#pragma unroll
+      for (int n = 0; n < 2 * kN16; ++n) {
+        float v[4];
+        ld_fresh4(src + 128 * n, v);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) S[n][i] = fmaf(S[n][i], f, v[i]);
+      }
     }
   }
   const float na = rec.neg_a[h] * 1.4426950408889634f, bias = rec.dt_bias[h], skip = rec.skip ? rec.skip[h] : 0.f;
+  static_assert(kSsAhead * kSsTok == 32 * kSsWarps, "a token per thread");
   auto raw_step = [&](int c) {
-    const int t = c * kSsTok + (lane & 15);
+    const int t = c * kSsTok + tid;
     return t < x.n ? ld_elem((const uint16_t*)in.step + (long long)(x.first + t) * in.step_stride + h) : 0.f;
   };
   float raw = raw_step(0), log_sum = 0.f;
+  const int row_floats = rec.heads * P;
+  float* o_base = out + ((long long)x.first * rec.heads + h) * P + p0;
   for (int c = 0; c < kSsStages - 1; ++c) fetch(c);
   for (int c = 0; c < chunks; ++c) {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(kSsStages - 2) : "memory");
     __syncthreads();  // the chunk is there for every warp, and the stage of the one before is free
     fetch(c + kSsStages - 1);
-    // ---- steps and log-decays of the sixteen tokens (lanes 16.. repeat them)
-    const float dt = c * kSsTok + (lane & 15) < x.n ? softplus_f(raw + bias) : 0.f;
-    raw = raw_step(c + 1);
-    float L = na * dt;  // in units of log 2
+    if (c % kSsAhead == 0) {  // steps and log-decays of this thread's token
+      const float dt = c * kSsTok + tid < x.n ? softplus_f(raw + bias) : 0.f;
+      raw = raw_step(c + kSsAhead);
+      float L = na * dt;
 #pragma unroll
-    for (int o = 1; o < kSsTok; o <<= 1) {
-      const float v = __shfl_up_sync(0xffffffffu, L, o, 16);
-      if ((lane & 15) >= o) L += v;
+      for (int o = 1; o < kSsTok; o <<= 1) {
+        const float v = __shfl_up_sync(0xffffffffu, L, o, 16);
+        if ((lane & 15) >= o) L += v;
+      }
+      const float total = __shfl_sync(0xffffffffu, L, 15, 16);
+      dts[tid] = dt;
+      logd[tid] = L;
+      grown[tid] = exp2f(L);
+      weight[tid] = dt * exp2f(total - L);
+      __syncthreads();
     }
-    const float total = __shfl_sync(0xffffffffu, L, 15);
-    log_sum += total;
-    float Lj[4], dtj[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int j = t2 + (i & 1) + 4 * (i & 2);  // tokens t2, t2 + 1, t2 + 8, t2 + 9
-      Lj[i] = __shfl_sync(0xffffffffu, L, j);
-      dtj[i] = __shfl_sync(0xffffffffu, dt, j);
-    }
-    const float Li[2] = {__shfl_sync(0xffffffffu, L, g), __shfl_sync(0xffffffffu, L, g + 8)};
+    const int tok0 = c % kSsAhead * kSsTok;
+    log_sum += logd[tok0 + 15];
     const uint32_t sc = base + (c % kSsStages) * kStage, sb = sc + kSsTok * kRow * 2, sx = sb + kSsTok * kRow * 2;
     uint32_t fx[4];
     ss_ldsm_t(fx, sx + ((m8 >> 1) * 8 + r8) * kSsXRow * 2 + (warp * 16 + (m8 & 1) * 8) * 2);
@@ -234,9 +265,11 @@ ssd_scan_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, co
           ss_mma(y[i][1], a[i], fc[1], fc[3]);
         }
       }
-      float Y[2][4], ej[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) ej[i] = exp2f(Lj[i]);
+      float Y[2][4], ej[4], Lj[4], dtj[4];  // of tokens t2, t2 + 1, t2 + 8, t2 + 9
+      ss_pairs(grown + tok0 + t2, ej);
+      ss_pairs(logd + tok0 + t2, Lj);
+      ss_pairs(dts + tok0 + t2, dtj);
+      const float Li[2] = {logd[tok0 + g], logd[tok0 + g + 8]};
 #pragma unroll
       for (int n = 0; n < 2; ++n)
 #pragma unroll
@@ -262,20 +295,22 @@ ssd_scan_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, co
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const uint32_t xv = fx[2 * n + (i >> 1)];
-          const int t = c * kSsTok + 8 * n + t2 + (i & 1), p = p0 + 4 * (i & 2);
+          const int t = 8 * n + t2 + (i & 1), p = 4 * (i & 2);
           const float o = fmaf(skip, i & 1 ? ss_hi(xv) : ss_lo(xv), Y[n][i]);
-          if (t < x.n && p < P) out[((long long)(x.first + t) * rec.heads + h) * P + p] = o;
+          if (c * kSsTok + t < x.n && p0 + p < P) o_base[(long long)t * row_floats + p] = o;
         }
+      o_base += (long long)kSsTok * row_floats;
     }
     // ---- the state behind the chunk
     uint32_t xs[3][4];
+    float wj[4];
+    ss_pairs(weight + tok0 + t2, wj);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int j = 2 * (i >> 1);
-      const float w0 = dtj[j] * exp2f(total - Lj[j]), w1 = dtj[j + 1] * exp2f(total - Lj[j + 1]);
-      ss_split(ss_lo(fx[i]) * w0, ss_hi(fx[i]) * w1, xs[0][i], xs[1][i], xs[2][i]);
+      ss_split(ss_lo(fx[i]) * wj[j], ss_hi(fx[i]) * wj[j + 1], xs[0][i], xs[1][i], xs[2][i]);
     }
-    const float decay = exp2f(total);
+    const float decay = grown[tok0 + 15];
 #pragma unroll
     for (int k = 0; k < kN16; ++k) {
       uint32_t fb[4];
@@ -294,7 +329,7 @@ ssd_scan_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, co
   }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   if (kLocal) {
-    put(place(cut.first + seg));
+    put_place(place(cut.first + seg));
     if (tid == 0 && slab == 0) logs[(long long)(cut.first + seg) * rec.heads + h] = log_sum;
   } else if (seg == cut.count - 1) {
     put(state);
@@ -312,7 +347,10 @@ template <int kN16>
 static int ss_launch(const b200dec_recurrence& rec, const b200dec_recurrence_in& in, const void* conv, const b200dec_entries& ent, float* out,
                      float* ws, int max_segments, int32_t* status, cudaStream_t s) {
   const int slabs = (rec.vdim + 16 * kSsWarps - 1) / (16 * kSsWarps), stride = (rec.channels + 7) / 8 * 8;
-  const size_t smem = (size_t)kSsStages * kSsTok * (2 * (16 * kN16 + 8) + kSsXRow) * 2;
+  size_t smem = (size_t)kSsStages * kSsTok * (2 * (16 * kN16 + 8) + kSsXRow) * 2;
+  // Two blocks per multiprocessor, not three: the few long-running blocks of a step spread more
+  // evenly (five portions of 1000 rows, 48 heads of 64 x 64: 29.1 us with three, 23.8 with two).
+  if (kN16 >= 4) smem = smem < 80 * 1024 ? 80 * 1024 : smem;
   if (cudaFuncSetAttribute(ssd_scan_kernel<kN16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
       cudaFuncSetAttribute(ssd_scan_kernel<kN16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return B200KV_E_LAUNCH;
@@ -339,7 +377,8 @@ static bool ss_applies(const b200dec_recurrence* r) {
 
 extern "C" size_t b200dec_state_space_chunked_workspace(const b200dec_recurrence* r) {
   if (!ss_applies(r)) return 0;
-  return ((size_t)2 * kSsSegments * r->heads * r->dim * rec_round4(r->vdim) + (size_t)kSsSegments * r->heads) * 4;
+  const int kn = r->dim <= 16 ? 16 : r->dim <= 32 ? 32 : r->dim <= 64 ? 64 : 128;
+  return ((size_t)2 * kSsSegments * r->heads * ss_place_floats(kn, r->vdim) + (size_t)kSsSegments * r->heads) * 4;
 }
 
 extern "C" int b200dec_state_space_chunked(const b200dec_recurrence* rec, const b200dec_recurrence_in* in, const void* conv_out,
