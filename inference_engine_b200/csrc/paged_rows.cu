@@ -369,14 +369,17 @@ attn_rows_kernel(const T* __restrict__ q, DecCache c, b200dec_rows rows, int hea
 // ---------------------------------------------------------------- attention, one block per (tile of rows, kv head)
 // The rows of a tile are neighbours of one entry, and with the query heads of their kv head they make up to kAtSlots query
 // rows that share every key and value: kAtKeys keys and values at a time come to shared memory in whole lines, a thread
-// computes one key's scores with eight query rows, and a warp keeps four query rows' softmax and output, a lane's channels
+// computes one key's scores with four query rows, and a warp keeps two query rows' softmax and output, a lane's channels
 // 4 lane + 128 i + (0..3).  A score is the same chain of multiply-adds as in attn_rows_kernel, where every thread reads a key
 // row of its own from L1, a line per 16 bytes: that, not the arithmetic, bounded it.  Here it is the shared-memory reads (a key
-// against eight query rows, a value against four) and, with few entries, one block's chain of steps.
-// fp32, us, attn_rows_kernel -> this: 200 rows, 16 heads of 112 and 96, 183 -> 43; 8 entries of 550 decoding, 16 heads of 128, 420 -> 67.
-constexpr int kAtThreads = 128;
+// against four query rows, a value against two) and, with few entries, one block's chain of steps.
+// fp32, us, attn_rows_kernel -> this: 200 rows, 16 heads of 112 and 96, 183 -> 43; 8 entries of 550 decoding, 16 heads of 128, 420 -> 51 (with half
+// the threads 67).
+constexpr int kAtThreads = 256;
 constexpr int kAtSlots = 16;
 constexpr int kAtKeys = 64;
+constexpr int kAtDots = kAtSlots * kAtKeys / kAtThreads;  // query rows of a thread's scores
+constexpr int kAtOwn = kAtSlots * 32 / kAtThreads;         // query rows a warp keeps
 constexpr int kAtPitch = 20;  // of the scores of one key: 16 and 4 that spread the banks
 
 // 16 bytes of which the first `bytes` are copied and the others zero
@@ -388,12 +391,21 @@ __device__ __forceinline__ void at_commit() { asm volatile("cp.async.commit_grou
 template <int N>
 __device__ __forceinline__ void at_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
+template <int N>
+__device__ __forceinline__ void at_read(const float* p, float (&f)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; i += 2) {
+    const float2 v = *reinterpret_cast<const float2*>(p + i);
+    f[i] = v.x; f[i + 1] = v.y;
+  }
+}
+
 __host__ __device__ constexpr size_t at_floats(int k_row, int v_row) {
   return (size_t)kAtSlots * k_row + (size_t)kAtKeys * (k_row + 4) + (size_t)kAtKeys * v_row + kAtKeys * kAtPitch;
 }
 
 template <typename T, int kPieces>  // kPieces: output channels, in pieces of 128
-__global__ void __launch_bounds__(kAtThreads, 3)
+__global__ void __launch_bounds__(kAtThreads, 2)
 attn_tile_kernel(const T* __restrict__ q, DecCache c, b200dec_rows rows, int heads, int slice_heads, float scale, DecAttnOpt opt,
                  T* __restrict__ out, int32_t* status) {
   extern __shared__ __align__(16) float at_smem[];
@@ -432,12 +444,12 @@ attn_tile_kernel(const T* __restrict__ q, DecCache c, b200dec_rows rows, int hea
     const T* src = q + ((long long)(r0 + s / gs) * heads + hk * G + g0 + s % gs) * c.k_row;
     for (int ch = lane; ch < c.k_row; ch += 32) qs[s * c.k_row + ch] = s < slots && ch < c.k_dim ? ld_elem(src + ch) * scale : 0.f;
   }
-  // what this warp keeps: query rows 4 warp + (0..3)
-  float m[4], l[4], o[4][kPieces][4];
-  int last[4], low[4];  // the keys each of them sees
+  // what this warp keeps: query rows kAtOwn warp + i
+  float m[kAtOwn], l[kAtOwn], o[kAtOwn][kPieces][4];
+  int last[kAtOwn], low[kAtOwn];  // the keys each of them sees
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int s = 4 * warp + i, h = hk * G + g0 + s % gs;
+  for (int i = 0; i < kAtOwn; ++i) {
+    const int s = kAtOwn * warp + i, h = hk * G + g0 + s % gs;
     last[i] = s < slots ? pos + s / gs : -1;
     low[i] = s < slots && opt.window > 0 ? max(0, last[i] - opt.window + 1) : 0;
     m[i] = opt.sink && s < slots ? opt.sink[h] : -INFINITY;
@@ -447,7 +459,7 @@ attn_tile_kernel(const T* __restrict__ q, DecCache c, b200dec_rows rows, int hea
 #pragma unroll
       for (int k = 0; k < 4; ++k) o[i][j][k] = 0.f;
   }
-  const bool mine = 4 * warp < slots;
+  const bool mine = kAtOwn * warp < slots;
   // Keys [all_low, all_last] are seen by every query row of the tile; the others are looked at one by one, so that what a row
   // does not see (a later token, perhaps not a number) never meets it.
   const int all_last = pos, all_low = opt.window > 0 ? max(0, pos + n - opt.window) : 0, end = pos + n;
@@ -498,12 +510,12 @@ attn_tile_kernel(const T* __restrict__ q, DecCache c, b200dec_rows rows, int hea
     look_up(j0 + kAtKeys, at[turn ^ 1]);
     at_wait<1>();
     __syncthreads();  // the keys are there, the scores of the step before are used
-    const int key = tid & (kAtKeys - 1), s0 = tid / kAtKeys * 8;
+    const int key = tid & (kAtKeys - 1), s0 = tid / kAtKeys * kAtDots;
     if (s0 < slots) {
       const float *kr = ks + key * kp, *qr = qs + s0 * c.k_row;
-      float acc[8];
+      float acc[kAtDots];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+      for (int i = 0; i < kAtDots; ++i) acc[i] = 0.f;
       auto dots = [&](auto rows_at_once) {
         constexpr int kN = decltype(rows_at_once)::value;
 #pragma unroll 2
@@ -516,29 +528,29 @@ attn_tile_kernel(const T* __restrict__ q, DecCache c, b200dec_rows rows, int hea
           }
         }
       };
-      if (slots - s0 <= 2) dots(std::integral_constant<int, 2>{}); else dots(std::integral_constant<int, 8>{});
-      *reinterpret_cast<float4*>(ps + key * kAtPitch + s0) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-      *reinterpret_cast<float4*>(ps + key * kAtPitch + s0 + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
+      if (slots - s0 <= 2) dots(std::integral_constant<int, 2>{}); else dots(std::integral_constant<int, kAtDots>{});
+#pragma unroll
+      for (int i = 0; i < kAtDots; i += 4)
+        *reinterpret_cast<float4*>(ps + key * kAtPitch + s0 + i) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
     }
     __syncthreads();  // the keys are used
     if (more) fetch(at[turn ^ 1], c.k, c.k_row, c.k_dim, ks, kp); else at_commit();
     at_wait<1>();
     __syncthreads();  // every thread's part of the values is there
     if (mine) {
-      // softmax of the warp's four query rows, keys lane and lane + 32
-      float p[2][4];
+      // softmax of the warp's query rows, keys lane and lane + 32
+      float p[2][kAtOwn];
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         const int k = lane + 32 * u, j = j0 + k;
-        const float4 x = *reinterpret_cast<const float4*>(ps + k * kAtPitch + 4 * warp);
+        at_read(ps + k * kAtPitch + kAtOwn * warp, p[u]);
         const bool some = at[turn][k] >= 0;
-        p[u][0] = x.x; p[u][1] = x.y; p[u][2] = x.z; p[u][3] = x.w;
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < kAtOwn; ++i)
           if (!some || j > last[i] || j < low[i]) p[u][i] = -INFINITY;
       }
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < kAtOwn; ++i) {
         float mx = fmaxf(p[0][i], p[1][i]);
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
@@ -553,18 +565,21 @@ attn_tile_kernel(const T* __restrict__ q, DecCache c, b200dec_rows rows, int hea
           for (int b = 0; b < 4; ++b) o[i][a][b] *= alpha;
       }
 #pragma unroll
-      for (int u = 0; u < 2; ++u) st_elem4(ps + (lane + 32 * u) * kAtPitch + 4 * warp, p[u]);
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int i = 0; i < kAtOwn; i += 2)
+          *reinterpret_cast<float2*>(ps + (lane + 32 * u) * kAtPitch + kAtOwn * warp + i) = make_float2(p[u][i], p[u][i + 1]);
       __syncwarp();
       auto add = [&](int k, bool every) {
-        const float4 w4 = *reinterpret_cast<const float4*>(ps + k * kAtPitch + 4 * warp);
-        const float w[4] = {w4.x, w4.y, w4.z, w4.w};
+        float w[kAtOwn];
+        at_read(ps + k * kAtPitch + kAtOwn * warp, w);
 #pragma unroll
         for (int a = 0; a < kPieces; ++a) {
           const int ch = 4 * lane + 128 * a;
           if (ch >= c.v_row) break;
           const float4 v = *reinterpret_cast<const float4*>(vs + k * c.v_row + ch);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
+          for (int i = 0; i < kAtOwn; ++i) {
             if (!every && (j0 + k > last[i] || j0 + k < low[i])) continue;
             o[i][a][0] = fmaf(w[i], v.x, o[i][a][0]);
             o[i][a][1] = fmaf(w[i], v.y, o[i][a][1]);
@@ -584,8 +599,8 @@ attn_tile_kernel(const T* __restrict__ q, DecCache c, b200dec_rows rows, int hea
     if (more) fetch(at[turn ^ 1], c.v, c.v_row, c.v_dim, vs, c.v_row); else at_commit();
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int s = 4 * warp + i;
+  for (int i = 0; i < kAtOwn; ++i) {
+    const int s = kAtOwn * warp + i;
     if (s >= slots) break;
     const int r = r0 + s / gs, h = hk * G + g0 + s % gs;
     const float inv = (l[i] > 0.f ? 1.f / l[i] : 0.f) * opt.factor<T>(r, h);
