@@ -7,7 +7,7 @@
 // contracted into FMA), IEEE sqrt and divide, and a fixed order for the sum of squares.
 // This translation unit is additionally compiled with -fmad=false.
 //
-// Mapping: one warp per (token, head).  Lane l holds elements d = 4l..4l+3 of the 128-wide
+// Mapping: one warp per (token, head), or per four heads of a token (prefill_rows_kernel).  Lane l holds elements d = 4l..4l+3 of the 128-wide
 // head, so lanes 0-15 own the first rotary half and lanes 16-31 the second; the rotation
 // partner of a lane is lane ^ 16.  A warp reads one 256-byte bf16 head row with 8-byte loads
 // (fully coalesced) and writes one 128-byte int8 row with 4-byte stores.
@@ -277,7 +277,7 @@ __device__ __forceinline__ bool is_first_chunk(int b, int nd, const int32_t* cu,
 // ------------------------------------------------------------------ prefill write
 // Two kernels that do not depend on one another replace the reference's serial loop over a chunk (8 programs per
 // chunk, kernels.py:717-823):
-//   rows kernel        one warp per (packed row, head): V of every prefilling row, and K of the rows whose entry
+//   rows kernel        one warp per (packed row, four heads): V of every prefilling row, and K of the rows whose entry
 //                      already has a calibration (not its first chunk): k / calibration -> codes + scale;
 //   first-chunk kernel K of entries on their first chunk, which need the column maxima of the WHOLE chunk before
 //                      any row can be quantized (kernels.py:764-780): a cluster of kFirstCtas CTAs per kv head
