@@ -13,8 +13,11 @@ constexpr int kRtWarps = 8;
 constexpr int kRtExperts = 4;
 constexpr int kRtMaxExperts = 1024;
 
+// The loads of the weights are its chain: with four rows a block two blocks a multiprocessor are enough (256 blocks for 1024 rows),
+// and their registers hold eight steps of weights in flight; with one row more blocks do better than more steps (1024 rows of
+// 2048, 32 experts: 14.0 -> 12.5 us; 600 rows 13.1 -> 11.0; 1000 rows, 8 experts 8.8 as before).
 template <int kR>
-__global__ void __launch_bounds__(kRtWarps * 32, 4)
+__global__ void __launch_bounds__(kRtWarps * 32, kR == 4 ? 2 : 4)
 router_kernel(const float* __restrict__ x, const uint16_t* __restrict__ w, int N, int width, int E, int top, int slices,
               int32_t* __restrict__ ids, float* __restrict__ scores, int32_t* __restrict__ ranks, int32_t* __restrict__ counts) {
   extern __shared__ __align__(16) float rt_smem[];
@@ -52,7 +55,7 @@ router_kernel(const float* __restrict__ x, const uint16_t* __restrict__ w, int N
     for (int i = 0; i < kRtExperts; ++i) wp[i] = w + (long long)min(e0 + i, E - 1) * width;
     if (width % 4 == 0) {
       const int per = (width / 4 + slices - 1) / slices * 4, hi = min(width, (slice + 1) * per);
-#pragma unroll 2
+#pragma unroll(kR == 4 ? 8 : 2)
       for (int c = slice * per + 4 * lane; c < hi; c += 128) {
         float wv[kRtExperts][4];
 #pragma unroll
