@@ -79,6 +79,14 @@ inline cudaError_t launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 bloc
   return launch_kernel(chained_launch_enabled(), kernel, grid, block, smem, stream, args...);
 }
 
+// Opts a kernel in to `most` bytes of dynamic shared memory (per function and device, so on every call): the most that any
+// call of it may ask for, not what the call at hand asks for.  With the latter, host threads that launch one kernel for
+// different sizes lower each other's limit between this and the launch, which then fails.
+template <typename... KArgs>
+inline bool allow_smem(void (*kernel)(KArgs...), size_t most) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) == cudaSuccess;
+}
+
 inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 
 // Host-side validation shared by the entry points.  Returns B200KV_OK or an error code.

@@ -381,6 +381,7 @@ constexpr int kAtKeys = 64;
 constexpr int kAtDots = kAtSlots * kAtKeys / kAtThreads;  // query rows of a thread's scores
 constexpr int kAtOwn = kAtSlots * 32 / kAtThreads;         // query rows a warp keeps
 constexpr int kAtPitch = 20;  // of the scores of one key: 16 and 4 that spread the banks
+constexpr size_t kAtMostSmem = 112 * 1024;  // two blocks per multiprocessor
 
 // 16 bytes of which the first `bytes` are copied and the others zero
 __device__ __forceinline__ void at_copy16(float* dst, const float* src, int bytes) {
@@ -712,10 +713,10 @@ extern "C" int b200dec_attn_rows_opt(const void* q, const b200dec_cache* cache, 
   // The line is two blocks of the tile kernel per multiprocessor: heads beyond about 190 channels (of key and value on average)
   // keep the block per row and head, whose shared memory does not grow with them.
   const size_t tile_smem = at_floats(cache->k_row, cache->v_row) * 4;
-  if (tile_smem <= 112 * 1024 && cache->v_row <= 256) {
+  if (tile_smem <= kAtMostSmem && cache->v_row <= 256) {
     const int G = heads / cache->kv_heads, slices = (G + kAtSlots - 1) / kAtSlots, slice_heads = (G + slices - 1) / slices;
     auto tiles = [&](auto* kernel, auto* in, auto* o) -> int {
-      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem) != cudaSuccess) return B200KV_E_LAUNCH;
+      if (!allow_smem(kernel, kAtMostSmem)) return B200KV_E_LAUNCH;
       return launch_result(launch_chained(kernel, dim3(cache->kv_heads * slices, rows->num_rows), dim3(kAtThreads), tile_smem, s, in, c, *rows,
                                           heads, slice_heads, scale, opt, o, status));
     };
