@@ -13,11 +13,9 @@ constexpr int kRtWarps = 8;
 constexpr int kRtExperts = 4;
 constexpr int kRtMaxExperts = 1024;
 
-// The loads of the weights are its chain: with four rows a block two blocks a multiprocessor are enough (256 blocks for 1024 rows),
-// and their registers hold eight steps of weights in flight; with one row more blocks do better than more steps (1024 rows of
-// 2048, 32 experts: 14.0 -> 12.5 us; 600 rows 13.1 -> 11.0; 1000 rows, 8 experts 8.8 as before).
-template <int kR>
-__global__ void __launch_bounds__(kRtWarps * 32, kR == 4 ? 2 : 4)
+// kSteps: steps of weights in flight, which are its chain; eight take the registers of half the blocks.
+template <int kR, int kSteps>
+__global__ void __launch_bounds__(kRtWarps * 32, kSteps > 2 ? 2 : 4)
 router_kernel(const float* __restrict__ x, const uint16_t* __restrict__ w, int N, int width, int E, int top, int slices,
               int32_t* __restrict__ ids, float* __restrict__ scores, int32_t* __restrict__ ranks, int32_t* __restrict__ counts) {
   extern __shared__ __align__(16) float rt_smem[];
@@ -55,7 +53,7 @@ router_kernel(const float* __restrict__ x, const uint16_t* __restrict__ w, int N
     for (int i = 0; i < kRtExperts; ++i) wp[i] = w + (long long)min(e0 + i, E - 1) * width;
     if (width % 4 == 0) {
       const int per = (width / 4 + slices - 1) / slices * 4, hi = min(width, (slice + 1) * per);
-#pragma unroll(kR == 4 ? 8 : 2)
+#pragma unroll(kSteps)
       for (int c = slice * per + 4 * lane; c < hi; c += 128) {
         float wv[kRtExperts][4];
 #pragma unroll
@@ -286,12 +284,19 @@ extern "C" int b200dec_router(const float* x, const void* router_w, int32_t num_
   const size_t smem1 = (size_t)((width + 3) / 4 * 4 + (1 + extra) * experts) * 4, smem4 = 4 * smem1;
   if (smem1 > 220 * 1024) return B200KV_E_RANGE;
   if (num_rows >= 512 && smem4 <= 72 * 1024) {
-    if (cudaFuncSetAttribute(router_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem4) != cudaSuccess) return B200KV_E_LAUNCH;
-    return launch_result(launch_chained(router_kernel<4>, dim3((num_rows + 3) / 4), dim3(kRtWarps * 32), smem4, s, x, (const uint16_t*)router_w,
+    // Eight steps hold two blocks per multiprocessor, two steps four (three of the widest rows).  A round of the former takes 0.6 to 0.65
+    // of a round of the latter, if a slice has eight steps at all, so rounds decide.  Two -> eight steps, us: 1024 rows of 2048, 32 experts
+    // 16.5 -> 14.7; 4096 channels, 128 experts 65 -> 49; 2048 rows of that 141 -> 94.  Beyond the line: 2048 rows of 2048,
+    // 32 experts 22.6 -> 27.8; 1500 rows, 8 experts 12.1 -> 19.0; short slices: 512 rows of 2048, 8 experts 9.8 -> 10.5.
+    const int blocks = (num_rows + 3) / 4, fit = smem4 <= 56 * 1024 ? 4 : 3, steps = width / (128 * slices);
+    const int rounds = (blocks + 148 * fit - 1) / (148 * fit), deep_rounds = (blocks + 148 * 2 - 1) / (148 * 2);
+    auto* kernel = (slices == 1 || steps >= 8) && 2 * deep_rounds < 3 * rounds + (fit < 4) ? router_kernel<4, 8> : router_kernel<4, 2>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem4) != cudaSuccess) return B200KV_E_LAUNCH;
+    return launch_result(launch_chained(kernel, dim3((num_rows + 3) / 4), dim3(kRtWarps * 32), smem4, s, x, (const uint16_t*)router_w,
                                         num_rows, width, experts, top, slices, ids, scores, ranks, counts));
   }
-  if (cudaFuncSetAttribute(router_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1) != cudaSuccess) return B200KV_E_LAUNCH;
-  return launch_result(launch_chained(router_kernel<1>, dim3(num_rows), dim3(kRtWarps * 32), smem1, s, x, (const uint16_t*)router_w, num_rows,
+  if (cudaFuncSetAttribute(router_kernel<1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1) != cudaSuccess) return B200KV_E_LAUNCH;
+  return launch_result(launch_chained(router_kernel<1, 2>, dim3(num_rows), dim3(kRtWarps * 32), smem1, s, x, (const uint16_t*)router_w, num_rows,
                                       width, experts, top, slices, ids, scores, ranks, counts));
 }
 

@@ -272,6 +272,13 @@ def test_mixture(dtype, rows, width, ff, experts, top, limit):
     H.status_clear()
 
 
+@pytest.mark.parametrize("rows,width,experts,top", [(600, 2052, 33, 3), (515, 4100, 5, 2), (700, 2052, 5, 2), (1190, 2052, 33, 4), (2060, 1028, 40, 2)])
+def test_router_of_prompt_steps(rows, width, experts, top):
+    """The router's forms for many rows: eight steps of weights in flight with a remainder behind them, few experts whose
+    channels are cut into slices, and more rows than two blocks per multiprocessor hold."""
+    test_mixture(torch.bfloat16, rows, width, 16, experts, top, 1.0)
+
+
 def test_router_takes_rows_that_are_not_numbers():
     """Idle rows of a padded step may hold anything; they must not disturb the others or leave the expert range."""
     from inference_engine_b200 import ops
