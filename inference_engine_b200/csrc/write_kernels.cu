@@ -7,7 +7,7 @@
 // contracted into FMA), IEEE sqrt and divide, and a fixed order for the sum of squares.
 // This translation unit is additionally compiled with -fmad=false.
 //
-// Mapping: one warp per (token, head), or per four heads of a token (prefill_rows_kernel).  Lane l holds elements d = 4l..4l+3 of the 128-wide
+// Mapping: one warp per (token, head), or per one to four heads of a token (prefill_rows_kernel).  Lane l holds elements d = 4l..4l+3 of the 128-wide
 // head, so lanes 0-15 own the first rotary half and lanes 16-31 the second; the rotation
 // partner of a lane is lane ^ 16.  A warp reads one 256-byte bf16 head row with 8-byte loads
 // (fully coalesced) and writes one 128-byte int8 row with 4-byte stores.
@@ -277,7 +277,7 @@ __device__ __forceinline__ bool is_first_chunk(int b, int nd, const int32_t* cu,
 // ------------------------------------------------------------------ prefill write
 // Two kernels that do not depend on one another replace the reference's serial loop over a chunk (8 programs per
 // chunk, kernels.py:717-823):
-//   rows kernel        one warp per (packed row, four heads): V of every prefilling row, and K of the rows whose entry
+//   rows kernel        one warp per (packed row, one to four heads): V of every prefilling row, and K of the rows whose entry
 //                      already has a calibration (not its first chunk): k / calibration -> codes + scale;
 //   first-chunk kernel K of entries on their first chunk, which need the column maxima of the WHOLE chunk before
 //                      any row can be quantized (kernels.py:764-780): a cluster of kFirstCtas CTAs per kv head
@@ -332,15 +332,14 @@ __device__ __forceinline__ int page_of(const CacheView& c, int b, int pos, int32
 // kFusedNorm = true: q, k are the raw projections; the kernel norms and ropes every row of them into q_out / k_out
 // (what fused_norm_rope_prefill does, kernels.py:547-670) and quantizes from the bf16-rounded k it just produced.
 // kFusedNorm = false: k is already normed + roped bf16 (the argument of quantize_kv_prefill), q is not touched.
-// grid (N, ceil(jobs / warps of a block)); warp job: kRowHeads heads of one kind, q (fused only), then k, then v.
-// Instructions bound it, so a warp does everything that heads of a row share once (the row's entry, page, angles, norm weight)
-// and sums, roots and divisions of two heads at a time: 1011 rows
-// of 32 heads in first portions 12.1 us with one head per warp, now 9.0; 992 on 3072 beside 32 decoding entries 15.0, 13.9.
-constexpr int kRowHeads = 4;
-__host__ __device__ constexpr int row_jobs(int heads) { return (heads + kRowHeads - 1) / kRowHeads; }
+// grid (N, ceil(jobs / warps of a block)); warp job: kHeads heads of one kind, q (fused only), then k, then v.
+// With many rows instructions bound it, so a warp does everything that heads of a row share once (the row's entry, page, angles, norm
+// weight) and sums, roots and divisions of two heads at a time: 1011 rows of 32 heads in first portions 12.1 us with one head per
+// warp, 9.0 with four; 992 on 3072 beside 32 decoding entries 15.0, 13.9.  With few rows one warp's chain does (row_heads).
+__host__ __device__ constexpr int row_jobs(int heads, int per_warp) { return (heads + per_warp - 1) / per_warp; }
 
-template <bool kFusedNorm>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
+template <bool kFusedNorm, int kHeads>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, kHeads == 1 ? 6 : 1)
 prefill_rows_kernel(const uint16_t* __restrict__ q, long long q_sn, long long q_sh,
                     const uint16_t* __restrict__ k, long long k_sn, long long k_sh,
                     const uint16_t* __restrict__ v, long long v_sn, long long v_sh,
@@ -350,15 +349,15 @@ prefill_rows_kernel(const uint16_t* __restrict__ q, long long q_sn, long long q_
                     uint16_t* __restrict__ k_out, long long ko_sn, long long ko_sh,
                     CacheView c, const int32_t* __restrict__ cu, int num_entries, const int32_t* __restrict__ cached_lens,
                     const int32_t* __restrict__ num_decoding, int Hq, float eps, int32_t* status) {
-  __shared__ __align__(16) float sq_all[kFusedNorm ? kWarpsPerBlock : 1][kSqPair];
+  __shared__ __align__(16) float sq_all[kFusedNorm ? kWarpsPerBlock : 1][kHeads > 1 ? kSqPair : kD];
   pdl_enter();
   const int r = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int job = blockIdx.y * (blockDim.x >> 5) + warp;
-  const int Hkv = c.Hkv, q_jobs = kFusedNorm ? row_jobs(Hq) : 0, kv_jobs = row_jobs(Hkv);
+  const int Hkv = c.Hkv, q_jobs = kFusedNorm ? row_jobs(Hq, kHeads) : 0, kv_jobs = row_jobs(Hkv, kHeads);
   if (job >= q_jobs + 2 * kv_jobs) return;
   const bool is_q = job < q_jobs, is_k = !is_q && job < q_jobs + kv_jobs;
-  const int j0 = kRowHeads * (is_q ? job : (is_k ? job - q_jobs : job - q_jobs - kv_jobs)), heads = min(kRowHeads, (is_q ? Hq : Hkv) - j0);
+  const int j0 = kHeads * (is_q ? job : (is_k ? job - q_jobs : job - q_jobs - kv_jobs)), heads = kHeads == 1 ? 1 : min(kHeads, (is_q ? Hq : Hkv) - j0);
   // round one (metadata, readable before the wait): the row's entry
   const int nd = *num_decoding;
   const RowEntry re = find_row_entry(cu, num_entries, cached_lens, c, r, lane);
@@ -368,56 +367,73 @@ prefill_rows_kernel(const uint16_t* __restrict__ q, long long q_sn, long long q_
   if (kFusedNorm && !is_q && !is_k && !prefilling) return;
   pdl_wait();  // q, k, v come from the kernel before this one
   const bool normed = kFusedNorm && (is_q || is_k);
-  const uint16_t* src = is_q ? q : (is_k ? k : v);
-  const long long src_sn = is_q ? q_sn : (is_k ? k_sn : v_sn), src_sh = is_q ? q_sh : (is_k ? k_sh : v_sh);
-  uint2 raw[kRowHeads], w_raw, c_raw, s_raw;
+  uint2 raw[kHeads];
+  HeadRow first;  // the first head's row, and what the heads share
+  if constexpr (kHeads == 1) {
+    if (kFusedNorm && is_q) first = load_head_row(q + act_offset(r, q_sn, j0, q_sh), qw, cosp + (long long)r * (int)cos_sn, sinp + (long long)r * (int)sin_sn, lane);
+    else if (kFusedNorm && is_k) first = load_head_row(k + act_offset(r, k_sn, j0, k_sh), kw, cosp + (long long)r * (int)cos_sn, sinp + (long long)r * (int)sin_sn, lane);
+    else first.x = *reinterpret_cast<const uint2*>((is_k ? k + act_offset(r, k_sn, j0, k_sh) : v + act_offset(r, v_sn, j0, v_sh)) + 4 * lane);
+    raw[0] = first.x;
+  } else {
+    const uint16_t* src = is_q ? q : (is_k ? k : v);
+    const long long src_sn = is_q ? q_sn : (is_k ? k_sn : v_sn), src_sh = is_q ? q_sh : (is_k ? k_sh : v_sh);
 #pragma unroll
-  for (int i = 0; i < kRowHeads; ++i)  // (a head that is not there repeats the last one)
-    raw[i] = *reinterpret_cast<const uint2*>(src + act_offset(r, src_sn, j0 + min(i, heads - 1), src_sh) + 4 * lane);
-  if (normed) {
-    w_raw = *reinterpret_cast<const uint2*>((is_q ? qw : kw) + 4 * lane);
-    c_raw = *reinterpret_cast<const uint2*>(cosp + (long long)r * (int)cos_sn + 4 * (lane & 15));
-    s_raw = *reinterpret_cast<const uint2*>(sinp + (long long)r * (int)sin_sn + 4 * (lane & 15));
+    for (int i = 0; i < kHeads; ++i)  // (a head that is not there repeats the last one)
+      raw[i] = *reinterpret_cast<const uint2*>(src + act_offset(r, src_sn, j0 + min(i, heads - 1), src_sh) + 4 * lane);
+    if (normed) {
+      first.w = *reinterpret_cast<const uint2*>((is_q ? qw : kw) + 4 * lane);
+      first.c = *reinterpret_cast<const uint2*>(cosp + (long long)r * (int)cos_sn + 4 * (lane & 15));
+      first.s = *reinterpret_cast<const uint2*>(sinp + (long long)r * (int)sin_sn + 4 * (lane & 15));
+    }
   }
-  // round two: the page of this row's token
+  // round two: the page of this row's token (and a single head's calibration; more would cost registers)
   const bool quantizes = prefilling && !is_q && !(is_k && first_chunk);
   const int pos = re.cached + (r - re.start);
   int page = -1;
+  float cal[4] = {1.f, 1.f, 1.f, 1.f};
   if (quantizes) {
     page = page_of(c, re.b, pos, status, lane);
     if (is_k && (re.page0 < 0 || re.page0 >= c.num_pages)) {
       if (lane == 0 && status) atomicOr(status, B200KV_S_BAD_PAGE);
       page = -1;
+    } else if (is_k && kHeads == 1) {
+      load4_f32(c.k_cal + cal_offset(c, re.page0, j0), lane, cal);
     }
   }
-  float x[kRowHeads][4];
+  float x[kHeads][4];
 #pragma unroll
-  for (int i = 0; i < kRowHeads; ++i) unpack4(raw[i], x[i]);
+  for (int i = 0; i < kHeads; ++i) unpack4(raw[i], x[i]);
   if (normed) {
-    float wv[4], cs[4], sn[4];
-    unpack4(w_raw, wv);
-    unpack4(c_raw, cs);
-    unpack4(s_raw, sn);
-    const bool first_half = lane < 16;
+    float* sq = sq_all[kFusedNorm ? warp : 0];
+    if constexpr (kHeads == 1) {
+      norm_rope_regs(first, eps, sq, lane, x[0]);
+    } else {
+      float wv[4], cs[4], sn[4];
+      unpack4(first.w, wv);
+      unpack4(first.c, cs);
+      unpack4(first.s, sn);
+      const bool first_half = lane < 16;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) sn[i] = first_half ? -sn[i] : sn[i];
+      for (int i = 0; i < 4; ++i) sn[i] = first_half ? -sn[i] : sn[i];
 #pragma unroll
-    for (int i = 0; i < kRowHeads; i += 2) {  // the arithmetic of norm_rope_regs
-      const float ss = sum_squares_ordered2(x[i], x[i + 1], sq_all[kFusedNorm ? warp : 0], lane);
-      const float rstd = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fmul_rn(ss, 0.0078125f), eps)));
+      for (int i = 0; i < kHeads; i += 2) {  // the arithmetic of norm_rope_regs
+        if (i >= heads) break;
+        const float ss = sum_squares_ordered2(x[i], x[i + 1], sq, lane);
+        const float rstd = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fmul_rn(ss, 0.0078125f), eps)));
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const float mine = __shfl_sync(0xffffffffu, rstd, 16 * u);
+        for (int u = 0; u < 2; ++u) {
+          const float mine = __shfl_sync(0xffffffffu, rstd, 16 * u);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float y = __fmul_rn(__fmul_rn(x[i + u][e], mine), wv[e]);
-          const float other = __shfl_xor_sync(0xffffffffu, y, 16);
-          x[i + u][e] = __fadd_rn(__fmul_rn(y, cs[e]), __fmul_rn(other, sn[e]));
+          for (int e = 0; e < 4; ++e) {
+            const float y = __fmul_rn(__fmul_rn(x[i + u][e], mine), wv[e]);
+            const float other = __shfl_xor_sync(0xffffffffu, y, 16);
+            x[i + u][e] = __fadd_rn(__fmul_rn(y, cs[e]), __fmul_rn(other, sn[e]));
+          }
         }
       }
     }
 #pragma unroll
-    for (int i = 0; i < kRowHeads; ++i) {
+    for (int i = 0; i < kHeads; ++i) {
       if (i >= heads) break;
       store4_bf16((is_q ? q_out + act_offset(r, qo_sn, j0 + i, qo_sh) : k_out + act_offset(r, ko_sn, j0 + i, ko_sh)), lane, x[i]);
 #pragma unroll
@@ -428,11 +444,10 @@ prefill_rows_kernel(const uint16_t* __restrict__ q, long long q_sn, long long q_
   int slot_unused, prow;
   split_pos(c, pos, slot_unused, prow);
 #pragma unroll
-  for (int i = 0; i < kRowHeads; ++i) {
+  for (int i = 0; i < kHeads; ++i) {
     if (i >= heads) break;
     if (is_k) {
-      float cal[4];
-      load4_f32(c.k_cal + cal_offset(c, re.page0, j0 + i), lane, cal);
+      if (kHeads > 1) load4_f32(c.k_cal + cal_offset(c, re.page0, j0 + i), lane, cal);
 #pragma unroll
       for (int e = 0; e < 4; ++e) x[i][e] = __fdiv_rn(x[i][e], cal[e]);
       quantize_store(x[i], c.k + code_offset(c, page, j0 + i, prow), c.k_scale + scale_offset(c, page, j0 + i, prow), lane);
@@ -693,6 +708,31 @@ extern "C" int b200kv_norm_rope_prefill(const void* q, int64_t q_sn, int64_t q_s
   return launch_status();
 }
 
+// Heads per warp of prefill_rows_kernel.  As long as one per warp is a single round of warps (9,472 fit the GPU), a call takes as long
+// as one warp's chain; with more, fewer instructions count, and four heads pay behind about three rounds (without the norms,
+// whose registers they share, behind one and a half).  Groups that are no multiple of four would compute heads that are not there.
+// us with 1 / 2 / 4 heads: 100 rows of 16 + 2 x 8 heads on 64 tokens 3.7 / 4.9 / 6.8, 300 rows 6.1 / 5.7 / 7.3, 1011 rows in first
+// portions 12.1 / 10.0 / 9.0, 4096 rows of 32 + 2 x 8 67.9 / 52.9 / 48.9, of 10 + 2 x 5 32.4 / 29.6 / 37.3; keys and values alone,
+// 2 x 8 heads, 300 rows 3.7 / 4.3 / 5.9, 800 in first portions 5.2 / 4.1 / 4.7, 1000 rows 7.3 / 7.6 / 6.8.
+static int row_heads(bool fused, int N, int Hq, int Hkv) {
+  const long long all = (long long)N * (Hq + 2 * Hkv);
+  if (all <= 9 * 1024) return 1;
+  return Hq % 4 || Hkv % 4 || all < (fused ? 28 : 14) * 1024 ? 2 : 4;
+}
+
+template <bool kFusedNorm, typename... Args>
+static void launch_rows(int N, int Hq, int Hkv, cudaStream_t s, Args... args) {
+  auto run = [&](auto* kernel, int per_warp) {
+    const int jobs = row_jobs(Hq, per_warp) + 2 * row_jobs(Hkv, per_warp), warps = jobs < kWarpsPerBlock ? jobs : kWarpsPerBlock;
+    launch_chained(kernel, dim3(N, (jobs + warps - 1) / warps), dim3(warps * 32), 0, s, args...);
+  };
+  switch (row_heads(kFusedNorm, N, Hq, Hkv)) {
+    case 1: return run(prefill_rows_kernel<kFusedNorm, 1>, 1);
+    case 2: return run(prefill_rows_kernel<kFusedNorm, 2>, 2);
+    default: return run(prefill_rows_kernel<kFusedNorm, 4>, 4);
+  }
+}
+
 // The first-chunk kernel: a cluster of kFirstCtas CTAs per (kv head, entry lane), chained like the others.
 static cudaError_t launch_first_chunk(const uint16_t* k, long long k_sn, long long k_sh, const CacheView& view,
                                       const int32_t* cu, int num_entries, const int32_t* cached_lens,
@@ -730,12 +770,10 @@ extern "C" int b200kv_quantize_prefill(const void* k, int64_t k_sn, int64_t k_sh
   const int Hkv = cache->num_kv_heads;
   CacheView view = make_view(cache, table);
   cudaStream_t s = (cudaStream_t)stream;
-  const int jobs = 2 * row_jobs(Hkv), warps = jobs < kWarpsPerBlock ? jobs : kWarpsPerBlock;
-  launch_chained(prefill_rows_kernel<false>, dim3(N, (jobs + warps - 1) / warps), dim3(warps * 32), 0, s,
-                 (const uint16_t*)nullptr, 0LL, 0LL, (const uint16_t*)k, (long long)k_sn, (long long)k_sh, (const uint16_t*)v,
-                 (long long)v_sn, (long long)v_sh, (const uint16_t*)nullptr, (const uint16_t*)nullptr, (const uint16_t*)nullptr,
-                 0LL, (const uint16_t*)nullptr, 0LL, (uint16_t*)nullptr, 0LL, 0LL, (uint16_t*)nullptr, 0LL, 0LL, view,
-                 cu_seqlens, (int)num_entries, cached_lens, num_decoding, 0, 0.f, status);
+  launch_rows<false>(N, 0, Hkv, s, (const uint16_t*)nullptr, 0LL, 0LL, (const uint16_t*)k, (long long)k_sn, (long long)k_sh,
+                     (const uint16_t*)v, (long long)v_sn, (long long)v_sh, (const uint16_t*)nullptr, (const uint16_t*)nullptr,
+                     (const uint16_t*)nullptr, 0LL, (const uint16_t*)nullptr, 0LL, (uint16_t*)nullptr, 0LL, 0LL,
+                     (uint16_t*)nullptr, 0LL, 0LL, view, cu_seqlens, (int)num_entries, cached_lens, num_decoding, 0, 0.f, status);
   if (cudaGetLastError() != cudaSuccess) return B200KV_E_LAUNCH;
   if (launch_first_chunk((const uint16_t*)k, k_sn, k_sh, view, cu_seqlens, num_entries, cached_lens, num_decoding, N, status,
                          s) != cudaSuccess)
@@ -766,12 +804,11 @@ extern "C" int b200kv_write_prefill(const void* q, int64_t q_sn, int64_t q_sh, c
     return B200KV_E_ALIGN;
   CacheView view = make_view(cache, table);
   cudaStream_t s = (cudaStream_t)stream;
-  const int jobs = row_jobs(Hq) + 2 * row_jobs(Hkv), warps = jobs < kWarpsPerBlock ? jobs : kWarpsPerBlock;
-  launch_chained(prefill_rows_kernel<true>, dim3(N, (jobs + warps - 1) / warps), dim3(warps * 32), 0, s, (const uint16_t*)q, (long long)q_sn, (long long)q_sh, (const uint16_t*)k,
-                 (long long)k_sn, (long long)k_sh, (const uint16_t*)v, (long long)v_sn, (long long)v_sh, (const uint16_t*)qw,
-                 (const uint16_t*)kw, (const uint16_t*)cosp, (long long)cos_sn, (const uint16_t*)sinp, (long long)sin_sn,
-                 (uint16_t*)q_out, (long long)qo_sn, (long long)qo_sh, (uint16_t*)k_out, (long long)ko_sn, (long long)ko_sh, view,
-                 cu_seqlens, (int)num_entries, cached_lens, num_decoding, (int)Hq, eps, status);
+  launch_rows<true>(N, Hq, cache->num_kv_heads, s, (const uint16_t*)q, (long long)q_sn, (long long)q_sh, (const uint16_t*)k, (long long)k_sn,
+                    (long long)k_sh, (const uint16_t*)v, (long long)v_sn, (long long)v_sh, (const uint16_t*)qw, (const uint16_t*)kw,
+                    (const uint16_t*)cosp, (long long)cos_sn, (const uint16_t*)sinp, (long long)sin_sn, (uint16_t*)q_out,
+                    (long long)qo_sn, (long long)qo_sh, (uint16_t*)k_out, (long long)ko_sn, (long long)ko_sh, view, cu_seqlens,
+                    (int)num_entries, cached_lens, num_decoding, (int)Hq, eps, status);
   if (cudaGetLastError() != cudaSuccess) return B200KV_E_LAUNCH;
   if (launch_first_chunk((const uint16_t*)k_out, ko_sn, ko_sh, view, cu_seqlens, num_entries, cached_lens, num_decoding, N,
                          status, s) != cudaSuccess)

@@ -165,6 +165,50 @@ def test_prefill_write_paged_random(K, T, first_chunk, fused):
     assert K.check_status() == 0
 
 
+@pytest.mark.parametrize("fused", [False, True])
+@pytest.mark.parametrize("per_warp", [1, 2, 4])
+@pytest.mark.parametrize("hq,hkv", [(1, 1), (3, 1), (6, 3), (10, 5), (14, 7), (12, 4)])
+def test_prefill_write_groups_of_heads(K, hq, hkv, per_warp, fused):
+    """Warps of one, two and four heads, with fewer heads than that in the last warp of a kind: a first portion and one behind 48
+    tokens beside a decoding entry.  Outputs and the whole cache are compared, so a head that is missed, written twice or
+    written to another's place shows."""
+    if per_warp == 4 and (hq % 4 or hkv % 4):
+        pytest.skip("head counts that are no multiple of four are cut into twos")
+    rng = np.random.default_rng(100 * hq + hkv)
+    P, heads = 16, (hq if fused else 0) + 2 * hkv
+    N = {1: 37, 2: 9 * 1024 // heads + 4, 4: (28 if fused else 14) * 1024 // heads + 5}[per_warp]
+    chunk = [1, N // 3, N - 1 - N // 3, 0]
+    cached = np.array([7, 0, 48, 0], np.int32)
+    cu = np.concatenate([[0], np.cumsum(chunk)]).astype(np.int32)
+    q, k, v = (H.randn_bf16(rng, N, h, D) for h in (hq, hkv, hkv))
+    qw, kw = (O.bf16_round((1 + 0.02 * rng.standard_normal(D)).astype(np.float32)) for _ in range(2))
+    pos = np.concatenate([np.arange(c, c + L) for c, L in zip(cached, chunk)]).astype(np.int32)
+    cos, sin = O.rope_tables(pos)
+    lens = [int(c + L) for c, L in zip(cached, chunk)]
+    num_pages = sum((n + P - 1) // P for n in lens) + 3
+    table = H.random_block_table(rng, lens, P, num_pages)
+    table[3, 0] = table[2, 0]
+    cache = O.make_cache(num_pages, hkv, P, D)
+    for name in ("k", "v"):
+        getattr(cache, name)[...] = rng.integers(-127, 128, cache.k.shape)
+        getattr(cache, name + "_scale")[...] = rng.random(cache.k_scale.shape)
+    cache.k_calibration[...] = (0.5 + 2 * rng.random(cache.k_calibration.shape)).astype(np.float32)
+    dev_cache = H.cache_to_torch(cache)
+    want_qp, want_kp = O.norm_rope_prefill(q, k, qw, kw, cos, sin, 1e-6)
+    O.quantize_prefill(want_kp, v, cu, table, cached, 1, cache)
+    tv = H.bf16_tensor(v)
+    if fused:
+        got_qp, got_kp = K.write_prefill(H.bf16_tensor(q), H.bf16_tensor(k), tv, H.bf16_tensor(qw), H.bf16_tensor(kw),
+                                         H.bf16_tensor(cos)[:, None, :], H.bf16_tensor(sin)[:, None, :], H.i32(cu), H.i32(table),
+                                         H.i32(cached), H.i32([1]), dev_cache, 1e-6)
+        assert np.array_equal(H.to_bits(got_qp), O.bf16_bits(want_qp))
+        assert np.array_equal(H.to_bits(got_kp), O.bf16_bits(want_kp))
+    else:
+        K.quantize_kv_prefill(H.bf16_tensor(want_kp), tv, H.i32(cu), H.i32(table), H.i32(cached), H.i32([1]), dev_cache)
+    H.assert_cache_equal(H.cache_to_numpy(dev_cache), cache, f"{hq}/{hkv} ")
+    assert K.check_status() == 0
+
+
 def test_quantizer_known_answers(K):
     """Hand-made rows through the decode write's V branch (no norm/rope): all zeros -> scale
     1e-6/127 and zero codes; +-absmax -> +-127 (never -128); exact .5 ties round to even."""
