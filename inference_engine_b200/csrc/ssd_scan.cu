@@ -13,7 +13,7 @@
 // Chunks arrive by asynchronous copies into a ring shared by a block's warps.  Bound by the chain of one chunk, with two warps per
 // scheduler to hide it.  What depends on the tokens alone (steps, decays and their exponentials) is found for 128 of them
 // at a time, a token per thread, instead of by every warp for every chunk: one portion of 1024, 64 heads of 128 x 64,
-// both launches 70.2 -> 54.2 us; five portions of 1000 rows, 48 heads of 64 x 64, 35.6 -> 28.2.
+// both launches 70.2 -> 54.2 us; five portions of 1000 rows in all, 48 heads of 64 x 64, 32.5 -> 25.4.
 #include "recurrence.cuh"
 
 namespace b200kv {
@@ -97,10 +97,18 @@ __host__ __device__ constexpr long long ss_place_floats(int kn, int vdim) {
   return (long long)kn * ((vdim + 16 * kSsWarps - 1) / (16 * kSsWarps) * 16 * kSsWarps);
 }
 
-// kN16: 16-channel pieces of the state's rows (padding is zero).  kLocal: the first launch.
+// Blocks per multiprocessor that a kernel gets registers for.  Few long-running blocks want short chains; many (kCrowd), and the
+// blocks of decoding entries and of pieces that are not there, which only come and go, want places.
+constexpr int kSsMostResident = 6;
+__host__ __device__ constexpr int ss_blocks(int kn16, bool local, bool crowd) {
+  if (!crowd) return 2;
+  return local ? (kn16 == 8 ? 3 : 6) : (kn16 == 8 ? 2 : 4);
+}
+
+// kN16: 16-channel pieces of the state's rows (padding is zero).  kLocal: the first launch.  kCrowd: ss_blocks.
 // Workspace: 2 * kSsSegments places of [head][16 columns][8 channels][lane][4], then [kSsSegments][head] sums of log-decays.
-template <int kN16, bool kLocal>
-__global__ void __launch_bounds__(32 * kSsWarps, 2)
+template <int kN16, bool kLocal, bool kCrowd>
+__global__ void __launch_bounds__(32 * kSsWarps, ss_blocks(kN16, kLocal, kCrowd))
 ssd_scan_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, const uint16_t* __restrict__ conv, int conv_stride,
                 const b200dec_entries ent, float* __restrict__ out, int slabs, int max_segments, float* ws, int32_t* status) {
   constexpr int kN = 16 * kN16, kRow = kN + 8;  // bf16 per row of b and c in shared memory
@@ -343,27 +351,48 @@ static int ss_segments(const b200dec_recurrence& rec, int sm_count) {
   return fit < 2 ? 1 : (fit < kSsSegments ? fit : kSsSegments);
 }
 
-template <int kN16>
+// Shared memory with which no more than `resident` blocks fit a multiprocessor (228 KB, of which a block takes 1 KB and at least
+// 1.5 KB of its own arrays).
+static size_t ss_padded(size_t need, int resident) {
+  const size_t pad = 228 * 1024 / (resident + 1) - 2560 + 64;
+  return resident < kSsMostResident && need < pad ? pad : need;
+}
+
+template <int kN16, bool kCrowd>
 static int ss_launch(const b200dec_recurrence& rec, const b200dec_recurrence_in& in, const void* conv, const b200dec_entries& ent, float* out,
-                     float* ws, int max_segments, int32_t* status, cudaStream_t s) {
+                     float* ws, int max_segments, int resident, int32_t* status, cudaStream_t s) {
+  constexpr size_t kNeed = (size_t)kSsStages * kSsTok * (2 * (16 * kN16 + 8) + kSsXRow) * 2, kMost = 80 * 1024;
+  static_assert(kNeed <= kMost, "");
+  auto *local = ssd_scan_kernel<kN16, true, kCrowd>, *scan = ssd_scan_kernel<kN16, false, kCrowd>;
   const int slabs = (rec.vdim + 16 * kSsWarps - 1) / (16 * kSsWarps), stride = (rec.channels + 7) / 8 * 8;
-  size_t smem = (size_t)kSsStages * kSsTok * (2 * (16 * kN16 + 8) + kSsXRow) * 2;
-  // Two blocks per multiprocessor, not three: the few long-running blocks of a step spread more
-  // evenly (five portions of 1000 rows, 48 heads of 64 x 64: 29.1 us with three, 23.8 with two).
-  if (kN16 >= 4) smem = smem < 80 * 1024 ? 80 * 1024 : smem;
-  if (cudaFuncSetAttribute(ssd_scan_kernel<kN16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-      cudaFuncSetAttribute(ssd_scan_kernel<kN16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return B200KV_E_LAUNCH;
+  if (!allow_smem(local, kMost) || !allow_smem(scan, kMost)) return B200KV_E_LAUNCH;
   if (max_segments > 1 && ent.num_rows >= 2 * kSsMinSegment) {
-    const int rc = launch_result(launch_chained(ssd_scan_kernel<kN16, true>, dim3(rec.heads * slabs, ent.num_entries, max_segments - 1),
-                                                dim3(32 * kSsWarps), smem, s, rec, in, (const uint16_t*)conv, stride, ent, out, slabs,
-                                                max_segments, ws, status));
+    // (pieces are carried only if at most half as many portions as pieces are there)
+    const size_t smem = ss_padded(kNeed, 2 * (ent.num_entries - 1) <= max_segments ? resident : kSsMostResident);
+    const int rc = launch_result(launch_chained(local, dim3(rec.heads * slabs, ent.num_entries, max_segments - 1), dim3(32 * kSsWarps), smem, s, rec,
+                                                in, (const uint16_t*)conv, stride, ent, out, slabs, max_segments, ws, status));
     if (rc != B200KV_OK) return rc;
   } else {
     max_segments = 1;
   }
-  return launch_result(launch_chained(ssd_scan_kernel<kN16, false>, dim3(rec.heads * slabs, ent.num_entries, max_segments), dim3(32 * kSsWarps),
-                                      smem, s, rec, in, (const uint16_t*)conv, stride, ent, out, slabs, max_segments, ws, status));
+  return launch_result(launch_chained(scan, dim3(rec.heads * slabs, ent.num_entries, max_segments), dim3(32 * kSsWarps), ss_padded(kNeed, resident), s,
+                                      rec, in, (const uint16_t*)conv, stride, ent, out, slabs, max_segments, ws, status));
+}
+
+template <int kN16>
+static int ss_run(const b200dec_recurrence& rec, const b200dec_recurrence_in& in, const void* conv, const b200dec_entries& ent, float* out, float* ws,
+                  int sm_count, int32_t* status, cudaStream_t s) {
+  // A step's blocks spread evenly when a multiprocessor takes no more of them than its share of one round, and with less
+  // than a round nothing is gained by more: shared memory is padded to that.  Beyond three the kernels with more places take over.
+  // Entries are all that is known here (the last one pads a step), so decoding ones count too; a portion beside many of them finds the places
+  // that their blocks come and go through.  Both launches, us, two blocks whatever the step / all that fit / this rule: heads x channels x
+  // columns 48 x 64 x 64, 5 portions of 1000 rows 81.7 / 103 / 81.0, 7 of 1000 133 / 108 / 108, 24 of 300 131 / 108 / 102, 40 of 20
+  // 90 / 63 / 53, 900 rows beside 200 decoding entries 135 / 103 / 101; 64 x 64 x 64, 1 of 1000 38.1 / 46.6 / 38.4, 5 of 200 38.6 / 30.2 / 30.6.
+  const long long portions = ent.num_entries > 1 ? ent.num_entries - 1 : 1;
+  const long long blocks = portions * rec.heads * ((rec.vdim + 16 * kSsWarps - 1) / (16 * kSsWarps)), share = (blocks + sm_count - 1) / sm_count;
+  const int resident = share < 2 ? 2 : (share < kSsMostResident ? (int)share : kSsMostResident), m = ss_segments(rec, sm_count);
+  return resident > 3 ? ss_launch<kN16, true>(rec, in, conv, ent, out, ws, m, resident, status, s)
+                      : ss_launch<kN16, false>(rec, in, conv, ent, out, ws, m, resident, status, s);
 }
 
 }  // namespace b200kv
@@ -395,9 +424,8 @@ extern "C" int b200dec_state_space_chunked(const b200dec_recurrence* rec, const 
   if (ent->num_entries == 0 || ent->num_rows == 0) return B200KV_OK;
   cudaStream_t s = (cudaStream_t)stream;
   float* ws = (float*)workspace;
-  const int m = ss_segments(*rec, sm_count);
-  if (rec->dim <= 16) return ss_launch<1>(*rec, *in, conv_out, *ent, out, ws, m, status, s);
-  if (rec->dim <= 32) return ss_launch<2>(*rec, *in, conv_out, *ent, out, ws, m, status, s);
-  if (rec->dim <= 64) return ss_launch<4>(*rec, *in, conv_out, *ent, out, ws, m, status, s);
-  return ss_launch<8>(*rec, *in, conv_out, *ent, out, ws, m, status, s);
+  if (rec->dim <= 16) return ss_run<1>(*rec, *in, conv_out, *ent, out, ws, sm_count, status, s);
+  if (rec->dim <= 32) return ss_run<2>(*rec, *in, conv_out, *ent, out, ws, sm_count, status, s);
+  if (rec->dim <= 64) return ss_run<4>(*rec, *in, conv_out, *ent, out, ws, sm_count, status, s);
+  return ss_run<8>(*rec, *in, conv_out, *ent, out, ws, sm_count, status, s);
 }

@@ -312,6 +312,33 @@ def test_long_portions_beside_others(kind, heads, groups, dim, vdim):
     status_clear()
 
 
+@pytest.mark.parametrize("heads,groups,dim,vdim", [(40, 8, 16, 16), (40, 4, 24, 8), (38, 2, 64, 64), (26, 2, 128, 72)])
+@pytest.mark.parametrize("decoding,chunks", [(0, [33] * 5), (0, [33, 140] + [31] * 7), (0, [20] * 13 + [1, 70]), (14, [330]), (13, [129, 200])])
+def test_state_space_of_many_portions(heads, groups, dim, vdim, decoding, chunks):
+    """Steps of two, three and more blocks per multiprocessor: many portions, and a few that are cut beside decoding entries, whose
+    states stay as they are."""
+    from inference_engine_b200 import ops
+
+    g = np.random.default_rng(dim + len(chunks))
+    dtype = torch.bfloat16
+    rec, a_log = make_rec(g, "state_space", heads, groups, dim, vdim, 4)
+    st = ops.make_recurrent_state(rec, decoding + len(chunks), dtype, DEV)
+    st.state.normal_()
+    st.ring.normal_()
+    before = st.state.clone()
+    seqs = [rec_inputs(g, rec, n, dtype) for n in [1] * decoding + chunks]
+    rows, _ = step_rows([5] * decoding + [0] * len(chunks), [1] * decoding + chunks, decoding)
+    x, step = (torch.cat([s[i] for s in seqs]) for i in range(2))
+    out = torch.full((rows.num_rows, heads * vdim), float("nan"), device=DEV)
+    ops.recurrence_prefill(rec, st, x, step, None, rows, out, "chunked")
+    at = decoding
+    for s, n in zip(seqs[decoding:], chunks):
+        close(out[at : at + n].view(-1, heads, vdim), rec_want(rec, a_log, *s), dtype, b16=3e-2)
+        at += n
+    assert torch.equal(st.state[:decoding], before[:decoding]) and torch.isnan(out[:decoding]).all()
+    status_clear()
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_decode_with_the_gated_norm_inside(dtype):
     from inference_engine_b200 import ops
