@@ -190,6 +190,38 @@ def test_attention_rows_in_tiles(heads, kv, dim, vdim, dtype):
     H.status_clear()
 
 
+@pytest.mark.parametrize("heads,kv,dim,vdim", [(2, 1, 64, 48), (4, 2, 128, 128)])
+@pytest.mark.parametrize("page,prior,new,window", [(16, 950, 70, 0), (16, 970, 70, 0), (16, 2041, 70, 0), (48, 1000, 133, 0), (32, 2000, 101, 0), (64, 4015, 70, 0),
+                                                   (64, 4090, 70, 0), (16, 2500, 70, 1200), (32, 4500, 33, 2100), (64, 5000, 200, 4200)])
+def test_prompt_attention_over_many_keys(heads, kv, dim, vdim, page, prior, new, window):
+    """Keys around 1024, 2048 and 4096: the fetching warps find the places of 32 boxes of 16, 32 or 64 rows at a time, half of a
+    tile's blocks each, and here need them more than once; with a window the first block is not the first.  Rows of the last page
+    that no token was written to are not numbers."""
+    from inference_engine_b200 import ops
+
+    gen = torch.Generator(device=DEV).manual_seed(prior)
+    rows, table, pages, _ = make_rows([(3, 1), (prior, new)], page)
+    cache = ops.make_paged_kv(pages, kv, page, dim, vdim, torch.bfloat16, DEV)
+    cache.k.fill_(float("nan"))
+    cache.v.fill_(float("nan"))
+    seqs = []
+    for b, n in enumerate((4, prior + new)):
+        k, v = (torch.randn(n, kv, d, generator=gen, device=DEV).to(torch.bfloat16) for d in (dim, vdim))
+        p = torch.arange(n, device=DEV)
+        at = torch.as_tensor(table[b], device=DEV)[p // page].long()
+        cache.k[at, :, p % page], cache.v[at, :, p % page] = k, v
+        seqs.append((k.double(), v.double()))
+    q = torch.randn(1 + new, heads, dim, generator=gen, device=DEV).to(torch.bfloat16)
+    out = ops.paged_attention(q, cache, rows, 3.0 / dim ** 0.5, ops.AttnOptions(window))
+    k, v = (x.repeat_interleave(heads // kv, 1) for x in seqs[1])
+    s = torch.einsum("nhd,khd->hnk", q[1:].double(), k) * (3.0 / dim ** 0.5)
+    pos, key = prior + torch.arange(new, device=DEV)[:, None], torch.arange(prior + new, device=DEV)
+    seen = (key <= pos) & ((key > pos - window) if window else True)
+    want = torch.einsum("hnk,khd->nhd", s.masked_fill(~seen, -torch.inf).softmax(-1), v)
+    close(out[1:], want.cpu().numpy(), torch.bfloat16)
+    H.status_clear()
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_attention_beyond_the_tensor_core_sizes(dtype):
     from inference_engine_b200 import ops
