@@ -282,8 +282,9 @@ extern "C" int b200dec_router(const float* x, const void* router_w, int32_t num_
   const int slices = groups >= kRtWarps ? 1 : kRtWarps / groups;
   const int extra = slices > 1 ? slices : 0;
   const size_t smem1 = (size_t)((width + 3) / 4 * 4 + (1 + extra) * experts) * 4, smem4 = 4 * smem1;
-  if (smem1 > 220 * 1024) return B200KV_E_RANGE;
-  if (num_rows >= 512 && smem4 <= 72 * 1024) {
+  constexpr size_t kMost1 = 220 * 1024, kMost4 = 72 * 1024;
+  if (smem1 > kMost1) return B200KV_E_RANGE;
+  if (num_rows >= 512 && smem4 <= kMost4) {
     // Eight steps hold two blocks per multiprocessor, two steps four (three of the widest rows).  A round of the former takes 0.6 to 0.65
     // of a round of the latter, if a slice has eight steps at all, so rounds decide.  Two -> eight steps, us: 1024 rows of 2048, 32 experts
     // 16.5 -> 14.7; 4096 channels, 128 experts 65 -> 49; 2048 rows of that 141 -> 94.  Beyond the line: 2048 rows of 2048,
@@ -291,11 +292,11 @@ extern "C" int b200dec_router(const float* x, const void* router_w, int32_t num_
     const int blocks = (num_rows + 3) / 4, fit = smem4 <= 56 * 1024 ? 4 : 3, steps = width / (128 * slices);
     const int rounds = (blocks + 148 * fit - 1) / (148 * fit), deep_rounds = (blocks + 148 * 2 - 1) / (148 * 2);
     auto* kernel = (slices == 1 || steps >= 8) && 2 * deep_rounds < 3 * rounds + (fit < 4) ? router_kernel<4, 8> : router_kernel<4, 2>;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem4) != cudaSuccess) return B200KV_E_LAUNCH;
+    if (!allow_smem(kernel, kMost4)) return B200KV_E_LAUNCH;
     return launch_result(launch_chained(kernel, dim3((num_rows + 3) / 4), dim3(kRtWarps * 32), smem4, s, x, (const uint16_t*)router_w,
                                         num_rows, width, experts, top, slices, ids, scores, ranks, counts));
   }
-  if (cudaFuncSetAttribute(router_kernel<1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1) != cudaSuccess) return B200KV_E_LAUNCH;
+  if (!allow_smem(router_kernel<1, 2>, kMost1)) return B200KV_E_LAUNCH;
   return launch_result(launch_chained(router_kernel<1, 2>, dim3(num_rows), dim3(kRtWarps * 32), smem1, s, x, (const uint16_t*)router_w, num_rows,
                                       width, experts, top, slices, ids, scores, ranks, counts));
 }

@@ -452,9 +452,9 @@ template <int KB, int VB, bool kWide>
 static int pd_launch(const void* q, const DecCache& c, const int32_t* cached_lens, const int32_t* num_decoding, int B, int heads, int groups,
                      float scale_log2, const DecAttnOpt& opt, void* out, int zero_idle, int* counters, float* parts, int grid, int box_rows, int32_t* status,
                      const CUtensorMap& tm_k, const CUtensorMap& tm_v, cudaStream_t stream) {
-  const size_t smem = (size_t)pd_stages(KB, VB) * (KB + VB) * kPdBlockBytes + 1024 + (size_t)(B + 1) * 4;
-  if (cudaFuncSetAttribute(paged_decode_kernel<KB, VB, kWide>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return B200KV_E_LAUNCH;
+  constexpr size_t kRings = (size_t)pd_stages(KB, VB) * (KB + VB) * kPdBlockBytes + 1024;
+  const size_t smem = kRings + (size_t)(B + 1) * 4;
+  if (!allow_smem(paged_decode_kernel<KB, VB, kWide>, kRings + (size_t)(kPdMaxB + 1) * 4)) return B200KV_E_LAUNCH;
   return launch_result(launch_chained(paged_decode_kernel<KB, VB, kWide>, dim3(grid), dim3(kPdThreads), smem, stream, (const uint16_t*)q, c,
                                       cached_lens, num_decoding, B, heads, groups, scale_log2, opt, (uint16_t*)out, zero_idle, counters, parts,
                                       box_rows, status, tm_k, tm_v));

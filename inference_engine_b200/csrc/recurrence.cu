@@ -471,9 +471,9 @@ static int rd_run(const b200dec_recurrence& rec, const b200dec_recurrence_in& in
                   int32_t* status, cudaStream_t s) {
   const int quads = rec_round4(rec.vdim) / 4, cg = quads < kRdThreads ? quads : kRdThreads, rg = kRdThreads / cg;
   const size_t smem = (size_t)(3 * rec_round4(rec.dim) + 3 * rec_round4(rec.vdim) + 8 * rg * cg) * 4;
-  if (smem > 200 * 1024) return B200KV_E_RANGE;
-  if (cudaFuncSetAttribute(recurrence_decode_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return B200KV_E_LAUNCH;
+  constexpr size_t kMost = 200 * 1024;
+  if (smem > kMost) return B200KV_E_RANGE;
+  if (!allow_smem(recurrence_decode_kernel<T>, kMost)) return B200KV_E_LAUNCH;
   return launch_result(launch_chained(recurrence_decode_kernel<T>, dim3(rec.heads, ent.num_entries), dim3(kRdThreads), smem, s, rec, in, ent, norm,
                                       out, cg, rg, status));
 }

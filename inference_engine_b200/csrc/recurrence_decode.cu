@@ -309,6 +309,7 @@ recurrence_step_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in
   if (copier) asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");
 }
 
+constexpr size_t kRpdMostSmem = 225 * 1024;
 struct RpdShape {
   int threads, cg, rg, rows, blocks_per_sm;
   size_t smem;
@@ -322,7 +323,7 @@ static bool rpd_shape(const b200dec_recurrence& r, RpdShape* s) {
   s->rg = s->threads / quads;
   s->rows = (r.dim + s->rg - 1) / s->rg;
   s->smem = (kRpdStages * floats + 3 * rec_round4(r.dim) + 3 * 4 * quads + (size_t)8 * s->rg * quads) * 4;
-  if (s->rows > (s->threads == 256 ? 16 : 8) || s->smem > 225 * 1024) return false;
+  if (s->rows > (s->threads == 256 ? 16 : 8) || s->smem > kRpdMostSmem) return false;
   const int fit = (int)(227 * 1024 / (s->smem + 1024 + 512)), regs = s->rows > 8 ? 1 : 512 / s->threads;
   s->blocks_per_sm = fit < regs ? fit : regs;
   return true;
@@ -332,7 +333,7 @@ template <typename T, int kRows, int kThreads>
 static int rpd_launch(const b200dec_recurrence& rec, const b200dec_recurrence_in& in, const b200dec_entries& ent, const RecNorm& norm, void* out,
                       const RpdShape& sh, int sm_count, int32_t* status, cudaStream_t s) {
   auto* kernel = recurrence_step_kernel<T, kRows, kThreads>;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem) != cudaSuccess) return B200KV_E_LAUNCH;
+  if (!allow_smem(kernel, kRpdMostSmem)) return B200KV_E_LAUNCH;
   const long long items = (long long)ent.num_entries * rec.heads, most = (long long)sm_count * sh.blocks_per_sm;
   return launch_result(launch_chained(kernel, dim3((unsigned)(items < most ? items : most)), dim3(kThreads), sh.smem, s, rec, in, ent, norm, out,
                                       sh.cg, sh.rg, status));

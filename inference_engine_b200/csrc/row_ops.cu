@@ -302,9 +302,9 @@ static int run_scaled_add_norm(const float* x, const void* delta, const int32_t*
     return launch_result(launch_chained(scaled_add_norm_kernel<T, kRowChunks>, dim3(rows), dim3(kRowThreads), 0, stream, x, (const T*)delta, index,
                                         top, weight, alpha, eps, x_out, (T*)xb_out, width, zero, num_zero));
   const size_t smem = (size_t)width * 4;
-  if (smem > 200 * 1024) return B200KV_E_RANGE;
-  if (cudaFuncSetAttribute(scaled_add_norm_any_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return B200KV_E_LAUNCH;
+  constexpr size_t kMost = 200 * 1024;
+  if (smem > kMost) return B200KV_E_RANGE;
+  if (!allow_smem(scaled_add_norm_any_kernel<T>, kMost)) return B200KV_E_LAUNCH;
   return launch_result(launch_chained(scaled_add_norm_any_kernel<T>, dim3(rows), dim3(kRowThreads), smem, stream, x, (const T*)delta,
                                       index, top, weight, alpha, eps, x_out, (T*)xb_out, width, zero, num_zero));
 }

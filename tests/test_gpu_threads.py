@@ -42,6 +42,7 @@ def side_by_side(monkeypatch, makers, times=20000):
     start, codes = threading.Barrier(len(work)), []
 
     def repeat(fn, args):
+        torch.cuda.synchronize()  # the thread has a context
         start.wait()
         codes.append({fn(*args) for _ in range(times)})
 
@@ -79,6 +80,89 @@ def attention_rows(dim):
     return make
 
 
-@pytest.mark.parametrize("makers", [(attention_rows(16), attention_rows(128))], ids=["attention_rows"])
-def test_sizes_side_by_side(makers, monkeypatch):
-    side_by_side(monkeypatch, makers)
+def router(rows, width):
+    from inference_engine_b200 import kernels as K
+    from inference_engine_b200 import ops
+
+    def make():
+        x, w = torch.randn(rows, width, device=DEV), torch.randn(5, width, device=DEV, dtype=torch.bfloat16)
+        ids, ranks, counts = (torch.zeros(n, dtype=torch.int32, device=DEV) for n in (2 * rows, 2 * rows, 5))
+        scores = torch.zeros(2 * rows, device=DEV)
+
+        def call():
+            args = [t.data_ptr() for t in (ids, scores, ranks, counts)]
+            assert ops._lib_dec().b200dec_router(x.data_ptr(), w.data_ptr(), rows, width, 5, 2, *args, K._stream()) == 0
+            return (x, w, ids, ranks, counts), scores
+
+        return call
+
+    return make
+
+
+def norm(width):
+    from inference_engine_b200 import ops
+
+    def make():
+        x, w = torch.randn(2, width, device=DEV), torch.rand(width, device=DEV)
+
+        def call():
+            return (x, w), ops.scaled_add_norm(x, None, w, 1.0, 1e-6, torch.bfloat16, keep=False)[1]
+
+        return call
+
+    return make
+
+
+def decode_attention(entries):
+    from inference_engine_b200 import ops
+
+    def make():
+        cache = ops.make_paged_kv(4, 2, 16, 64, 64, torch.bfloat16, DEV)
+        cache.k.normal_()
+        cache.v.normal_()
+        q = torch.randn(entries, 4, 64, device=DEV).to(torch.bfloat16)
+        rows = ops.Rows(entries, i32([15] * entries), i32([entries]), i32([[e % 4] for e in range(entries)]))
+
+        def call():
+            return (cache, q, rows), ops.paged_attention(q, cache, rows, 0.125)
+
+        return call
+
+    return make
+
+
+def recurrent_step(dim, vdim, variant):
+    """No entry decodes, so that the states stay as they are."""
+    from inference_engine_b200 import ops
+
+    def make():
+        rec = ops.Recurrence(2, 1, dim, vdim, torch.randn(4, 2 * dim + 2 * vdim, device=DEV), None, -torch.ones(2, device=DEV),
+                             torch.zeros(2, device=DEV), torch.ones(2, device=DEV), 2 * vdim + dim, 2 * vdim, 0)
+        st = ops.make_recurrent_state(rec, 1, torch.bfloat16, DEV)
+        x, step = torch.randn(1, rec.channels, device=DEV).to(torch.bfloat16), torch.randn(1, 2, device=DEV).to(torch.bfloat16)
+        rows = ops.Rows(1, i32([3]), i32([0]), i32([[0]]), slots=i32([0]))
+        out = torch.zeros(1, 2 * vdim, device=DEV)
+
+        def call():
+            ops.recurrence_decode(rec, st, x, step, None, rows, out, variant=variant)
+            return (rec, st, x, step, rows), out
+
+        return call
+
+    return make
+
+
+PAIRS = {
+    "attention_rows": (attention_rows(16), attention_rows(128)),
+    "router": (router(3, 64), router(3, 20000)),
+    "router_of_many_rows": (router(600, 64), router(600, 4096)),
+    "norm_of_any_width": (norm(33), norm(45001)),
+    "decode_attention": (decode_attention(1), decode_attention(1500)),
+    "recurrent_step": (recurrent_step(48, 64, 0), recurrent_step(64, 64, 0)),
+    "recurrent_step_of_any_size": (recurrent_step(8, 8, 1), recurrent_step(4000, 8, 1)),
+}
+
+
+@pytest.mark.parametrize("name", PAIRS)
+def test_sizes_side_by_side(name, monkeypatch):
+    side_by_side(monkeypatch, PAIRS[name])
