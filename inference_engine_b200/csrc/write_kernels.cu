@@ -708,16 +708,19 @@ extern "C" int b200kv_norm_rope_prefill(const void* q, int64_t q_sn, int64_t q_s
   return launch_status();
 }
 
-// Heads per warp of prefill_rows_kernel.  As long as one per warp is a single round of warps (9,472 fit the GPU), a call takes as long
-// as one warp's chain; with more, fewer instructions count, and four heads pay behind about three rounds (without the norms,
-// whose registers they share, behind one and a half).  Groups that are no multiple of four would compute heads that are not there.
-// us with 1 / 2 / 4 heads: 100 rows of 16 + 2 x 8 heads on 64 tokens 3.7 / 4.9 / 6.8, 300 rows 6.1 / 5.7 / 7.3, 1011 rows in first
-// portions 12.1 / 10.0 / 9.0, 4096 rows of 32 + 2 x 8 67.9 / 52.9 / 48.9, of 10 + 2 x 5 32.4 / 29.6 / 37.3; keys and values alone,
-// 2 x 8 heads, 300 rows 3.7 / 4.3 / 5.9, 800 in first portions 5.2 / 4.1 / 4.7, 1000 rows 7.3 / 7.6 / 6.8.
+// Heads per warp of prefill_rows_kernel: the fewest with which all warps are one round (6, 5 and 4 blocks of 8 fit a multiprocessor
+// by the registers of the fused forms, 8 and 6 of the others), because a call then takes as long as one warp's chain.  With more rows fewer
+// instructions count: two heads first, since a tail of four-head warps is long, four from about 900 rows of 32 heads on (the forms
+// without the norms: at once).  Head counts that are no multiple of four would make warps compute heads that are not there.
+// us with 1 / 2 / 4 heads, 16 + 2 x 8 of them: 100 rows on 64 cached ones 3.7 / 4.9 / 6.8, 343 rows 6.9 / 5.8 / 7.3, 425 rows in first
+// portions 6.8 / 6.2 / 5.3, 625 rows on 64 9.9 / 8.5 / 13.2, 1000 in first portions 12.4 / 9.9 / 9.0; 4096 rows of 32 + 2 x 8 67.9 / 52.9 /
+// 48.9, of 10 + 2 x 5 32.4 / 29.6 / 37.3; keys and values alone, 2 x 8 heads, 300 rows 3.7 / 4.4 / 6.0, 750 6.0 / 5.6 / 6.4, 1000 7.4 / 7.7 / 6.8.
 static int row_heads(bool fused, int N, int Hq, int Hkv) {
-  const long long all = (long long)N * (Hq + 2 * Hkv);
-  if (all <= 9 * 1024) return 1;
-  return Hq % 4 || Hkv % 4 || all < (fused ? 28 : 14) * 1024 ? 2 : 4;
+  auto warps = [&](int per_warp) { return (long long)N * (row_jobs(Hq, per_warp) + 2 * row_jobs(Hkv, per_warp)); };
+  constexpr int kSms = 148;
+  if (warps(1) <= kSms * (fused ? 48 : 64)) return 1;
+  if (Hq % 4 || Hkv % 4 || warps(2) <= kSms * (fused ? 40 : 48)) return 2;
+  return fused && warps(4) > kSms * 32 && warps(1) < 28 * 1024 ? 2 : 4;
 }
 
 template <bool kFusedNorm, typename... Args>

@@ -176,7 +176,7 @@ def test_prefill_write_groups_of_heads(K, hq, hkv, per_warp, fused):
         pytest.skip("head counts that are no multiple of four are cut into twos")
     rng = np.random.default_rng(100 * hq + hkv)
     P, heads = 16, (hq if fused else 0) + 2 * hkv
-    N = {1: 37, 2: 9 * 1024 // heads + 4, 4: (28 if fused else 14) * 1024 // heads + 5}[per_warp]
+    N = {1: 37, 2: 148 * (48 if fused else 64) // heads + 4, 4: (28 * 1024 if fused else 148 * 96) // heads + 5}[per_warp]
     chunk = [1, N // 3, N - 1 - N // 3, 0]
     cached = np.array([7, 0, 48, 0], np.int32)
     cu = np.concatenate([[0], np.cumsum(chunk)]).astype(np.int32)
