@@ -889,6 +889,7 @@ decode_plan_kernel(const int32_t* __restrict__ cached_lens, const int32_t* __res
       e2[0] = make_int2(b0, h0);
       e2[1] = make_int2(tile0, T0);
       e2[2] = make_int2(n0, base0);
+      static_assert(kStages == 4, "three pages in an entry's places 6 to 8");
       e2[3] = make_int2(page[0], page[1]);
       e[8] = page[2];
     }
