@@ -332,13 +332,13 @@ __device__ __forceinline__ int page_of(const CacheView& c, int b, int pos, int32
 // kFusedNorm = true: q, k are the raw projections; the kernel norms and ropes every row of them into q_out / k_out
 // (what fused_norm_rope_prefill does, kernels.py:547-670) and quantizes from the bf16-rounded k it just produced.
 // kFusedNorm = false: k is already normed + roped bf16 (the argument of quantize_kv_prefill), q is not touched.
-// grid (N, ceil(jobs / warps of a block)); warp job: kHeads heads of one kind, q (fused only), then k, then v.
+// grid (N, ceil(jobs / warps of a block)); warp job: kHeads q heads (fused only), or kKv heads of k, or of v.
 // With many rows instructions bound it, so a warp does everything that heads of a row share once (the row's entry, page, angles, norm
 // weight) and sums, roots and divisions of two heads at a time: 1011 rows of 32 heads in first portions 12.1 us with one head per
 // warp, 9.0 with four; 992 on 3072 beside 32 decoding entries 15.0, 13.9.  With few rows one warp's chain does (row_heads).
 __host__ __device__ constexpr int row_jobs(int heads, int per_warp) { return (heads + per_warp - 1) / per_warp; }
 
-template <bool kFusedNorm, int kHeads>
+template <bool kFusedNorm, int kHeads, int kKv>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, kHeads == 1 ? 6 : 1)
 prefill_rows_kernel(const uint16_t* __restrict__ q, long long q_sn, long long q_sh,
                     const uint16_t* __restrict__ k, long long k_sn, long long k_sh,
@@ -354,10 +354,11 @@ prefill_rows_kernel(const uint16_t* __restrict__ q, long long q_sn, long long q_
   const int r = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int job = blockIdx.y * (blockDim.x >> 5) + warp;
-  const int Hkv = c.Hkv, q_jobs = kFusedNorm ? row_jobs(Hq, kHeads) : 0, kv_jobs = row_jobs(Hkv, kHeads);
+  const int Hkv = c.Hkv, q_jobs = kFusedNorm ? row_jobs(Hq, kHeads) : 0, kv_jobs = row_jobs(Hkv, kKv);
   if (job >= q_jobs + 2 * kv_jobs) return;
   const bool is_q = job < q_jobs, is_k = !is_q && job < q_jobs + kv_jobs;
-  const int j0 = kHeads * (is_q ? job : (is_k ? job - q_jobs : job - q_jobs - kv_jobs)), heads = kHeads == 1 ? 1 : min(kHeads, (is_q ? Hq : Hkv) - j0);
+  const int j0 = is_q ? kHeads * job : kKv * (is_k ? job - q_jobs : job - q_jobs - kv_jobs);
+  const int heads = kHeads == 1 ? 1 : min(is_q ? kHeads : kKv, (is_q ? Hq : Hkv) - j0);
   // round one (metadata, readable before the wait): the row's entry
   const int nd = *num_decoding;
   const RowEntry re = find_row_entry(cu, num_entries, cached_lens, c, r, lane);
@@ -708,32 +709,36 @@ extern "C" int b200kv_norm_rope_prefill(const void* q, int64_t q_sn, int64_t q_s
   return launch_status();
 }
 
-// Heads per warp of prefill_rows_kernel: the fewest with which all warps are one round (6, 5 and 4 blocks of 8 fit a multiprocessor
-// by the registers of the fused forms, 8 and 6 of the others), because a call then takes as long as one warp's chain.  With more rows fewer
-// instructions count: two heads first, since a tail of four-head warps is long, four from about 900 rows of 32 heads on (the forms
-// without the norms: at once).  Head counts that are no multiple of four would make warps compute heads that are not there.
-// us with 1 / 2 / 4 heads, 16 + 2 x 8 of them: 100 rows on 64 cached ones 3.7 / 4.9 / 6.8, 343 rows 6.9 / 5.8 / 7.3, 425 rows in first
-// portions 6.8 / 6.2 / 5.3, 625 rows on 64 9.9 / 8.5 / 13.2, 1000 in first portions 12.4 / 9.9 / 9.0; 4096 rows of 32 + 2 x 8 67.9 / 52.9 /
-// 48.9, of 10 + 2 x 5 32.4 / 29.6 / 37.3; keys and values alone, 2 x 8 heads, 300 rows 3.7 / 4.4 / 6.0, 750 6.0 / 5.6 / 6.4, 1000 7.4 / 7.7 / 6.8.
-static int row_heads(bool fused, int N, int Hq, int Hkv) {
+// Heads per warp of prefill_rows_kernel, queries and keys or values: the fewest with which all warps are one round (6, 5 and 4 blocks
+// of 8 fit a multiprocessor by the registers of the fused forms, 8 and 6 of the others), because a call then takes as long as one
+// warp's chain.  With more rows fewer instructions count.  Four keys that are normed and quantized are the longest chain, whose tail shows
+// up to about 900 rows of 32 heads: until then two of them beside four queries where these are most of the heads, else two of
+// each.  Head counts that are no multiple of four would make warps compute heads that are not there.
+// us with 1 / 2 / 4 + 2 / 4 heads, 16 + 2 x 8 of them: 100 rows on 64 cached ones 3.7 / 4.9 / 4.9 / 6.8, 343 rows 6.9 / 5.8 / 6.4 / 7.3, 425 rows
+// in first portions 6.8 / 6.1 / 6.2 / 5.3, 625 rows on 64 9.9 / 8.4 / 9.1 / 12.8, 1000 in first portions 12.4 / 9.9 / 10.1 / 9.1; 32 + 2 x 8:
+// 283 rows on 64 7.1 / 7.2 / 6.1 / 7.7, 500 11.0 / 9.4 / 8.8 / 9.9, 4096 68 / 53 / 50 / 49; 4096 of 10 + 2 x 5 32.4 / 29.6 / 32.8 / 37.5; keys and
+// values alone, 2 x 8 heads, 1 / 2 / 4: 300 rows 3.7 / 4.4 / 6.0, 750 6.0 / 5.6 / 6.4, 1000 7.4 / 7.7 / 6.8.
+struct RowHeads {
+  int q, kv;
+};
+static RowHeads row_heads(bool fused, int N, int Hq, int Hkv) {
   auto warps = [&](int per_warp) { return (long long)N * (row_jobs(Hq, per_warp) + 2 * row_jobs(Hkv, per_warp)); };
   constexpr int kSms = 148;
-  if (warps(1) <= kSms * (fused ? 48 : 64)) return 1;
-  if (Hq % 4 || Hkv % 4 || warps(2) <= kSms * (fused ? 40 : 48)) return 2;
-  return fused && warps(4) > kSms * 32 && warps(1) < 28 * 1024 ? 2 : 4;
+  if (warps(1) <= kSms * (fused ? 48 : 64)) return {1, 1};
+  if (Hq % 4 || Hkv % 4 || warps(2) <= kSms * (fused ? 40 : 48)) return {2, 2};
+  if (!fused || warps(1) >= 28 * 1024) return {4, 4};
+  if (Hq >= 4 * Hkv) return {4, 2};
+  return warps(4) <= kSms * 32 ? RowHeads{4, 4} : RowHeads{2, 2};
 }
 
 template <bool kFusedNorm, typename... Args>
 static void launch_rows(int N, int Hq, int Hkv, cudaStream_t s, Args... args) {
-  auto run = [&](auto* kernel, int per_warp) {
-    const int jobs = row_jobs(Hq, per_warp) + 2 * row_jobs(Hkv, per_warp), warps = jobs < kWarpsPerBlock ? jobs : kWarpsPerBlock;
-    launch_chained(kernel, dim3(N, (jobs + warps - 1) / warps), dim3(warps * 32), 0, s, args...);
-  };
-  switch (row_heads(kFusedNorm, N, Hq, Hkv)) {
-    case 1: return run(prefill_rows_kernel<kFusedNorm, 1>, 1);
-    case 2: return run(prefill_rows_kernel<kFusedNorm, 2>, 2);
-    default: return run(prefill_rows_kernel<kFusedNorm, 4>, 4);
-  }
+  const RowHeads n = row_heads(kFusedNorm, N, Hq, Hkv);
+  const int jobs = row_jobs(Hq, n.q) + 2 * row_jobs(Hkv, n.kv), warps = jobs < kWarpsPerBlock ? jobs : kWarpsPerBlock;
+  auto* kernel = n.kv == 1   ? prefill_rows_kernel<kFusedNorm, 1, 1>
+                 : n.kv == 4 ? prefill_rows_kernel<kFusedNorm, 4, 4>
+                 : n.q == 2  ? prefill_rows_kernel<kFusedNorm, 2, 2> : prefill_rows_kernel<kFusedNorm, kFusedNorm ? 4 : 2, 2>;
+  launch_chained(kernel, dim3(N, (jobs + warps - 1) / warps), dim3(warps * 32), 0, s, args...);
 }
 
 // The first-chunk kernel: a cluster of kFirstCtas CTAs per (kv head, entry lane), chained like the others.

@@ -167,16 +167,16 @@ def test_prefill_write_paged_random(K, T, first_chunk, fused):
 
 @pytest.mark.parametrize("fused", [False, True])
 @pytest.mark.parametrize("per_warp", [1, 2, 4])
-@pytest.mark.parametrize("hq,hkv", [(1, 1), (3, 1), (6, 3), (10, 5), (14, 7), (12, 4)])
+@pytest.mark.parametrize("hq,hkv", [(1, 1), (3, 1), (6, 3), (10, 5), (14, 7), (12, 4), (16, 4)])
 def test_prefill_write_groups_of_heads(K, hq, hkv, per_warp, fused):
-    """Warps of one, two and four heads, with fewer heads than that in the last warp of a kind: a first portion and one behind 48
-    tokens beside a decoding entry.  Outputs and the whole cache are compared, so a head that is missed, written twice or
+    """Warps of one, two and four heads (16 and 4: of four queries, two keys or two values instead of two), with fewer heads than that
+    in the last warp of a kind: a first portion and one behind 48 tokens beside a decoding entry.  Outputs and the whole cache are compared, so a head that is missed, written twice or
     written to another's place shows."""
     if per_warp == 4 and (hq % 4 or hkv % 4):
         pytest.skip("head counts that are no multiple of four are cut into twos")
     rng = np.random.default_rng(100 * hq + hkv)
     P, heads = 16, (hq if fused else 0) + 2 * hkv
-    N = {1: 37, 2: 148 * (48 if fused else 64) // heads + 4, 4: (28 * 1024 if fused else 148 * 96) // heads + 5}[per_warp]
+    N = {1: 37, 2: 148 * (96 if fused and hq == 4 * hkv else 48 if fused else 64) // heads + 4, 4: (28 * 1024 if fused else 148 * 96) // heads + 5}[per_warp]
     chunk = [1, N // 3, N - 1 - N // 3, 0]
     cached = np.array([7, 0, 48, 0], np.int32)
     cu = np.concatenate([[0], np.cumsum(chunk)]).astype(np.int32)
