@@ -466,10 +466,9 @@ prefill_rows_kernel(const uint16_t* __restrict__ q, long long q_sn, long long q_
 // max(1e-3, column max) (exact and order-independent, kernels.py:764-780) is stored by CTA 0, and every warp
 // quantizes its rows as k / calibration (kernels.py:786-811).
 constexpr int kFirstCtas = 8, kFirstWarps = 16, kFirstLanes = 4, kKeepRows = 8;
-// kPerSm: blocks per multiprocessor that there are registers for.  With two the clusters of four entries are one round of blocks (five
-// prompts of 1011 rows, 8 heads: 14.7 -> 10.0 us), at 64 registers of which 16 bytes are spilled.
-template <int kPerSm>
-__global__ void __launch_bounds__(kFirstWarps * 32, kPerSm)
+// Registers for two blocks per multiprocessor, so that the clusters of four entries are one round of blocks (five prompts of
+// 1011 rows, 8 heads: 14.7 -> 10.0 us).
+__global__ void __launch_bounds__(kFirstWarps * 32, 2)
 first_chunk_k_kernel(const uint16_t* __restrict__ k, long long k_sn, long long k_sh, CacheView c,
                      const int32_t* __restrict__ cu, int num_entries, const int32_t* __restrict__ cached_lens,
                      const int32_t* __restrict__ num_decoding, int N, int32_t* status) {
@@ -760,11 +759,7 @@ static cudaError_t launch_first_chunk(const uint16_t* k, long long k_sn, long lo
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = chained_launch_enabled() ? 2 : 1;
-  // Fifteen clusters with a block per multiprocessor are resident at a time.  Up to there its registers are worth 2 to 3 % (one portion of 16 / 300 /
-  // 1000 rows, 8 heads: 4.6 / 6.0 / 9.3 us against 4.8 / 6.3 / 9.7), beyond it they cost a round (two of 300 rows 10.4 against 8.0).  How many
-  // entries are on their first portion is known on the device only; the last entry pads the step.
-  const int lanes = num_entries - 1 < 1 ? 1 : (num_entries - 1 < kFirstLanes ? num_entries - 1 : kFirstLanes);
-  return cudaLaunchKernelEx(&cfg, view.Hkv * lanes <= 15 ? first_chunk_k_kernel<1> : first_chunk_k_kernel<2>, k, k_sn, k_sh, view, cu, num_entries, cached_lens, num_decoding, N,
+  return cudaLaunchKernelEx(&cfg, first_chunk_k_kernel, k, k_sn, k_sh, view, cu, num_entries, cached_lens, num_decoding, N,
                             status);
 }
 
