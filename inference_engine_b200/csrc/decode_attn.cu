@@ -181,9 +181,9 @@ __device__ void scan_tiles(const int32_t* __restrict__ cached_lens, int B, const
 // hand-offs: a piece that goes through the workspace costs about as much as 8 tiles of work, but the four pieces
 // of a CTA that covers exactly one (entry, head) meet in shared memory and cost nothing of the kind.  So short
 // sequences (32 tiles or fewer on average) are cut into quarters of the average length (2..8 tiles) when the grid
-// has warps to spare for that: in a batch of equal lengths every CTA then owns exactly one (entry, head), and its
-// four warps fetch the few tiles side by side instead of one warp streaming all of them (5.8 instead of 10.3 us
-// for one 128-token sequence).  When the quarters would not fit the grid, short sequences use pieces of 8 tiles
+// has warps to spare for that: in a batch of equal lengths of a multiple of four tiles every CTA then owns exactly one
+// (entry, head), and its four warps fetch the few tiles side by side instead of one warp streaming all of them (5.8
+// instead of 10.3 us for one 128-token sequence).  With other lengths the heads straddle CTAs and their pieces go through the workspace.  When the quarters would not fit the grid, short sequences use pieces of 8 tiles
 // (a whole sequence per warp, or exactly a CTA of 4 x 8); longer ones pieces of 4 (64 tokens, the reference's
 // MIN_PIECE, kernels.py:295).
 __host__ __device__ __forceinline__ Partition make_partition(int total_tiles_one_head, int Hkv, int W, int num_entries) {
