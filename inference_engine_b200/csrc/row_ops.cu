@@ -49,48 +49,76 @@ embed_kernel(const T* __restrict__ table, const int32_t* __restrict__ ids, float
   }
 }
 
-// The registers path: width % 4 == 0 and width <= 8192.
-template <typename T, int kChunks>
+template <typename T>
+struct __align__(4 * sizeof(T)) Raw4 {
+  T v[4];
+};
+
+// The registers path: width % 4 == 0 and width <= 8192.  Bound by the chain of its loads, so kAtOnce rows of delta (all of one token's
+// experts, as a rule) are in flight together, behind one load of their places, and the weights come ahead of all.  Rows x channels (rows of
+// delta each), us: 64 x 2048 (2) 6.1 -> 3.9, (1) 4.0 -> 2.6; 1024 x 2048 (4) 10.5 -> 9.1, (1) 7.5 -> 4.6.
+template <typename T, int kChunks, int kAtOnce>
 __global__ void __launch_bounds__(kRowThreads)
 scaled_add_norm_kernel(const float* x, const T* __restrict__ delta, const int32_t* __restrict__ index, int top,
                        const float* __restrict__ weight, float alpha, float eps, float* x_out, T* __restrict__ xb_out,
                        int width, int32_t* __restrict__ zero, int num_zero) {
   pdl_enter();
+  float w[kChunks][4];
+#pragma unroll
+  for (int c = 0; c < kChunks; ++c) {
+    const int col = (c * kRowThreads + threadIdx.x) * 4;
+    if (col < width) ld_elem4(weight + col, w[c]);
+  }
   pdl_wait();
   const long long r = blockIdx.x;
   if (zero && blockIdx.x == 0)
     for (int i = threadIdx.x; i < num_zero; i += kRowThreads) zero[i] = 0;
   float s[kChunks][4];
-  float ss = 0.f;
 #pragma unroll
   for (int c = 0; c < kChunks; ++c) {
     const int col = (c * kRowThreads + threadIdx.x) * 4;
-    if (col < width) {
-      ld_fresh4(x + r * width + col, s[c]);
+    if (col < width) ld_fresh4(x + r * width + col, s[c]);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) s[c][i] *= alpha;
-      if (delta) {
-        for (int j = 0; j < top; ++j) {
-          const long long row = index ? ld_fresh(index + r * top + j) : r;
-          float d[4];
-          ld_elem4(delta + row * width + col, d);
+    for (int i = 0; i < 4; ++i) s[c][i] *= alpha;
+  }
+  if (delta) {
+    for (int j0 = 0; j0 < top; j0 += kAtOnce) {
+      long long row[kAtOnce];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) s[c][i] += d[i];
+      for (int j = 0; j < kAtOnce; ++j) row[j] = index ? (j0 + j < top ? ld_fresh(index + r * top + j0 + j) : 0) : r;
+      Raw4<T> d[kAtOnce][kChunks];  // as they lie in memory, for registers' sake
+#pragma unroll
+      for (int j = 0; j < kAtOnce; ++j)
+#pragma unroll
+        for (int c = 0; c < kChunks; ++c) {
+          const int col = (c * kRowThreads + threadIdx.x) * 4;
+          if (j0 + j < top && col < width) d[j][c] = *reinterpret_cast<const Raw4<T>*>(delta + row[j] * width + col);
         }
-      }
 #pragma unroll
-      for (int i = 0; i < 4; ++i) ss = fmaf(s[c][i], s[c][i], ss);
+      for (int j = 0; j < kAtOnce; ++j)
+#pragma unroll
+        for (int c = 0; c < kChunks; ++c) {
+          if (j0 + j >= top || (c * kRowThreads + threadIdx.x) * 4 >= width) continue;
+          float f[4];
+          ld_elem4(reinterpret_cast<const T*>(&d[j][c]), f);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) s[c][i] += f[i];
+        }
     }
   }
+  float ss = 0.f;
+#pragma unroll
+  for (int c = 0; c < kChunks; ++c)
+    if ((c * kRowThreads + threadIdx.x) * 4 < width)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) ss = fmaf(s[c][i], s[c][i], ss);
   const float inv = 1.0f / sqrtf(row_sum(ss) / (float)width + eps);
 #pragma unroll
   for (int c = 0; c < kChunks; ++c) {
     const int col = (c * kRowThreads + threadIdx.x) * 4;
     if (col < width) {
-      float w[4];
-      ld_elem4(weight + col, w);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) s[c][i] = s[c][i] * inv * w[i];
+      for (int i = 0; i < 4; ++i) s[c][i] = s[c][i] * inv * w[c][i];
       if (x_out) st_elem4(x_out + r * width + col, s[c]);
       if (xb_out) st_elem4(xb_out + r * width + col, s[c]);
     }
@@ -196,8 +224,8 @@ silu_mul_rows_kernel(const T* __restrict__ gu, long long stride, T* __restrict__
 template <typename T, int kThreads, int kVec, int kKeep>
 __global__ void __launch_bounds__(kRowThreads)
 gated_norm_kernel(const float* __restrict__ o, const T* __restrict__ gate, long long gate_stride, int gate_first,
-                  const float* __restrict__ weight, int weight_len, float eps, float out_scale, T* __restrict__ out, long long out_stride,
-                  int rows, int len, int parts) {
+                  const float* __restrict__ weight, int weight_len, int weight_vec, float eps, float out_scale, T* __restrict__ out,
+                  long long out_stride, int rows, int len, int parts) {
   pdl_enter();
   const int part = len / parts;
   const long long item = (long long)blockIdx.x * (kRowThreads / kThreads) + threadIdx.x / kThreads;
@@ -220,21 +248,30 @@ gated_norm_kernel(const float* __restrict__ o, const T* __restrict__ gate, long 
       if (gate_first) v[i] *= z[i] * s;
     }
   };
-  auto put = [&](int c, float inv, float (&v)[kVec], const float (&f)[kVec]) {
+  // weight_vec: its length is a multiple of kVec, so that one remainder and one load serve all of them (1000 rows of 16 parts of 128, whose
+  // weights are shared: 7.6 -> 6.9 us)
+  auto weights = [&](int c, float (&w)[kVec]) {
+    const int at = p * part + c, first = weight_len == len ? at : at % weight_len;
+    if (weight_vec) {
+      ld_vec(weight + first, w);
+    } else {
 #pragma unroll
-    for (int i = 0; i < kVec; ++i) {
-      const int at = p * part + c + i;
-      v[i] = v[i] * inv * weight[weight_len == len ? at : at % weight_len] * f[i] * out_scale;
+      for (int i = 0; i < kVec; ++i) w[i] = weight[(first + i) % weight_len];
     }
+  };
+  auto put = [&](int c, float inv, float (&v)[kVec], const float (&f)[kVec], const float (&w)[kVec]) {
+#pragma unroll
+    for (int i = 0; i < kVec; ++i) v[i] = v[i] * inv * w[i] * f[i] * out_scale;
     st_vec(dst + c, v);
   };
-  float v[kKeep > 0 ? kKeep : 1][kVec], f[kKeep > 0 ? kKeep : 1][kVec], ss = 0.f;
+  float v[kKeep > 0 ? kKeep : 1][kVec], f[kKeep > 0 ? kKeep : 1][kVec], w[kKeep > 0 ? kKeep : 1][kVec], ss = 0.f;
   if (live) {
     if (kKeep > 0) {
 #pragma unroll
       for (int i = 0; i < kKeep; ++i) {
         const int c = (t + i * kThreads) * kVec;
         if (c < part) {
+          weights(c, w[i]);
           load(c, v[i], f[i]);
 #pragma unroll
           for (int k = 0; k < kVec; ++k) ss = fmaf(v[i][k], v[i][k], ss);
@@ -254,11 +291,12 @@ gated_norm_kernel(const float* __restrict__ o, const T* __restrict__ gate, long 
   if (kKeep > 0) {
 #pragma unroll
     for (int i = 0; i < kKeep; ++i)
-      if ((t + i * kThreads) * kVec < part) put((t + i * kThreads) * kVec, inv, v[i], f[i]);
+      if ((t + i * kThreads) * kVec < part) put((t + i * kThreads) * kVec, inv, v[i], f[i], w[i]);
   } else {
     for (int c = t * kVec; c < part; c += kThreads * kVec) {
       load(c, v[0], f[0]);
-      put(c, inv, v[0], f[0]);
+      weights(c, w[0]);
+      put(c, inv, v[0], f[0], w[0]);
     }
   }
 }
@@ -288,7 +326,8 @@ static int run_gated_norm(const float* o, const void* gate, int64_t gate_stride,
   const long long items = (long long)rows * parts, per = warp ? kRowThreads / 32 : 1, blocks = (items + per - 1) / per;
   if (blocks > 0x7FFFFFF0ll) return B200KV_E_RANGE;
   return launch_result(launch_chained(kernel, dim3((unsigned)blocks), dim3(kRowThreads), 0, s, o, (const T*)gate, (long long)gate_stride,
-                                      gate_first, weight, weight_len, eps, out_scale, (T*)out, (long long)out_stride, rows, len, parts));
+                                      gate_first, weight, weight_len, !vec || (weight_len % 4 == 0 && aligned(weight, 16)), eps, out_scale, (T*)out,
+                                      (long long)out_stride, rows, len, parts));
 }
 
 template <typename T>
@@ -296,10 +335,10 @@ static int run_scaled_add_norm(const float* x, const void* delta, const int32_t*
                                float eps, float* x_out, void* xb_out, int rows, int width, int32_t* zero, int num_zero,
                                cudaStream_t stream) {
   if (width % 4 == 0 && width <= kRowThreads * 4 * 2)
-    return launch_result(launch_chained(scaled_add_norm_kernel<T, 2>, dim3(rows), dim3(kRowThreads), 0, stream, x, (const T*)delta, index,
+    return launch_result(launch_chained(delta && top > 1 ? scaled_add_norm_kernel<T, 2, 4> : scaled_add_norm_kernel<T, 2, 1>, dim3(rows), dim3(kRowThreads), 0, stream, x, (const T*)delta, index,
                                         top, weight, alpha, eps, x_out, (T*)xb_out, width, zero, num_zero));
   if (width % 4 == 0 && width <= kRowThreads * 4 * kRowChunks)
-    return launch_result(launch_chained(scaled_add_norm_kernel<T, kRowChunks>, dim3(rows), dim3(kRowThreads), 0, stream, x, (const T*)delta, index,
+    return launch_result(launch_chained(scaled_add_norm_kernel<T, kRowChunks, 1>, dim3(rows), dim3(kRowThreads), 0, stream, x, (const T*)delta, index,
                                         top, weight, alpha, eps, x_out, (T*)xb_out, width, zero, num_zero));
   const size_t smem = (size_t)width * 4;
   constexpr size_t kMost = 200 * 1024;

@@ -78,6 +78,13 @@ def test_scaled_add_norm(dtype, width, top):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("width,top", [(2048, 4), (1028, 5), (64, 9), (4096, 3)])
+def test_scaled_add_norm_of_several_experts(dtype, width, top):
+    """Rows of a token's experts that are fetched together, and more of them than are."""
+    test_scaled_add_norm(dtype, width, top)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("scaling", [None, H.YARN])
 @pytest.mark.parametrize("dim,vdim,rot", [(48, 40, 16), (20, 36, 20), (7, 130, 2)])
 def test_rotation_unit_norm_and_write(dtype, scaling, dim, vdim, rot):
