@@ -11,7 +11,7 @@
 namespace b200kv {
 
 constexpr int kRpdTaps = 4;   // more taps: the other form
-constexpr int kRpdStages = 3;
+constexpr int kRpdMostStages = 3;
 
 __device__ __forceinline__ void rpd_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
@@ -54,8 +54,9 @@ struct RpdItem {
   int row, head, slot;  // row: also the entry, since decoding entries come first with one row each
 };
 
-template <typename T, int kRows, int kRpdThreads>  // kRows: rows of the state per thread
-__global__ void __launch_bounds__(kRpdThreads, kRows > 8 ? 1 : 512 / kRpdThreads)
+// kRows: rows of the state per thread.  kRpdStages: states in the ring of a block (rpd_shape).
+template <typename T, int kRows, int kRpdThreads, int kRpdStages>
+__global__ void __launch_bounds__(kRpdThreads, kRows > 8 && kRpdStages == 3 ? 1 : 512 / kRpdThreads)
 recurrence_step_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, const b200dec_entries ent, const RecNorm norm,
                        void* __restrict__ out, int cg, int rg, int32_t* status) {
   extern __shared__ __align__(128) float rpd_smem[];
@@ -223,23 +224,28 @@ recurrence_step_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in
     }
     if (!dt_mbar_wait(dt_smem(bars + i % kRpdStages), (i / kRpdStages) & 1)) dead = true;
     float* st = stage(i);
-    ulonglong2 S[kRows];
+    // Many rows of two blocks' threads do not fit the registers: they are read and decayed a second time for the write.
+    constexpr bool kKeep = kRows <= 8 || kRpdStages == 3;
+    ulonglong2 S[kKeep ? kRows : 1];
+    auto decayed = [&](int d) {
+      ulonglong2 s = make_ulonglong2(0ull, 0ull);
+      if (!fresh) s = *reinterpret_cast<const ulonglong2*>(st + d * P4 + 4 * c4);
+      const rpd_pair g = rpd_both(gs[d]);
+      return make_ulonglong2(rpd_mul(s.x, g), rpd_mul(s.y, g));
+    };
     if (ok && !dead && mine) {
       ulonglong2 ak = make_ulonglong2(0ull, 0ull), aq = ak;
 #pragma unroll
       for (int j = 0; j < kRows; ++j) {
         const int d = r0 + j * rg;
         if (d >= D) break;
-        ulonglong2 s = make_ulonglong2(0ull, 0ull);
-        if (!fresh) s = *reinterpret_cast<const ulonglong2*>(st + d * P4 + 4 * c4);
-        const rpd_pair g = rpd_both(gs[d]), k = rpd_both(ks[d]), q = rpd_both(qs[d]);
-        s.x = rpd_mul(s.x, g);
-        s.y = rpd_mul(s.y, g);
+        const ulonglong2 s = decayed(d);
+        const rpd_pair k = rpd_both(ks[d]), q = rpd_both(qs[d]);
         ak.x = rpd_fma(s.x, k, ak.x);
         ak.y = rpd_fma(s.y, k, ak.y);
         aq.x = rpd_fma(s.x, q, aq.x);
         aq.y = rpd_fma(s.y, q, aq.y);
-        S[j] = s;
+        if (kKeep) S[j] = s;
       }
       *reinterpret_cast<ulonglong2*>(red + r0 * 4 * cg + 4 * c4) = ak;
       *reinterpret_cast<ulonglong2*>(red + (rg + r0) * 4 * cg + 4 * c4) = aq;
@@ -281,7 +287,8 @@ recurrence_step_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in
         const int d = r0 + j * rg;
         if (d >= D) break;
         const rpd_pair k = rpd_both(ks[d]);
-        *reinterpret_cast<ulonglong2*>(st + d * P4 + 4 * c4) = make_ulonglong2(rpd_fma(k, u.x, S[j].x), rpd_fma(k, u.y, S[j].y));
+        const ulonglong2 s = kKeep ? S[j] : decayed(d);
+        *reinterpret_cast<ulonglong2*>(st + d * P4 + 4 * c4) = make_ulonglong2(rpd_fma(k, u.x, s.x), rpd_fma(k, u.y, s.y));
       }
     }
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // the new state, for the copy out
@@ -311,7 +318,7 @@ recurrence_step_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in
 
 constexpr size_t kRpdMostSmem = 225 * 1024;
 struct RpdShape {
-  int threads, cg, rg, rows, blocks_per_sm;
+  int threads, cg, rg, rows, stages, blocks_per_sm;
   size_t smem;
 };
 static bool rpd_shape(const b200dec_recurrence& r, RpdShape* s) {
@@ -322,17 +329,29 @@ static bool rpd_shape(const b200dec_recurrence& r, RpdShape* s) {
   s->cg = quads;
   s->rg = s->threads / quads;
   s->rows = (r.dim + s->rg - 1) / s->rg;
-  s->smem = (kRpdStages * floats + 3 * rec_round4(r.dim) + 3 * 4 * quads + (size_t)8 * s->rg * quads) * 4;
-  if (s->rows > (s->threads == 256 ? 16 : 8) || s->smem > kRpdMostSmem) return false;
-  const int fit = (int)(227 * 1024 / (s->smem + 1024 + 512)), regs = s->rows > 8 ? 1 : 512 / s->threads;
-  s->blocks_per_sm = fit < regs ? fit : regs;
+  if (s->rows > (s->threads == 256 ? 16 : 8)) return false;
+  // A ring of three states, unless a ring of two is what lets two blocks share a multiprocessor: an item is a chain of phases, in
+  // which another block's copies and phases then run (64 entries of 16 heads, states of 128 x 128: 28.3 -> 21.1 us).
+  s->blocks_per_sm = 0;
+  for (int stages = kRpdMostStages; stages >= 2; --stages) {
+    const size_t smem = (stages * floats + 3 * rec_round4(r.dim) + 3 * 4 * quads + (size_t)8 * s->rg * quads) * 4;
+    if (smem > kRpdMostSmem) return false;
+    const int fit = (int)(227 * 1024 / (smem + 1024 + 512)), regs = s->rows > 8 && stages == 3 ? 1 : 512 / s->threads;
+    const int blocks = fit < regs ? fit : regs;
+    if (stages < kRpdMostStages && (s->threads < 256 || blocks <= s->blocks_per_sm)) continue;
+    s->blocks_per_sm = blocks;
+    s->stages = stages;
+    s->smem = smem;
+  }
   return true;
 }
 
 template <typename T, int kRows, int kThreads>
 static int rpd_launch(const b200dec_recurrence& rec, const b200dec_recurrence_in& in, const b200dec_entries& ent, const RecNorm& norm, void* out,
                       const RpdShape& sh, int sm_count, int32_t* status, cudaStream_t s) {
-  auto* kernel = recurrence_step_kernel<T, kRows, kThreads>;
+  auto* kernel = recurrence_step_kernel<T, kRows, kThreads, kRpdMostStages>;
+  if constexpr (kThreads == 256)
+    if (sh.stages == 2) kernel = recurrence_step_kernel<T, kRows, kThreads, 2>;
   if (!allow_smem(kernel, kRpdMostSmem)) return B200KV_E_LAUNCH;
   const long long items = (long long)ent.num_entries * rec.heads, most = (long long)sm_count * sh.blocks_per_sm;
   return launch_result(launch_chained(kernel, dim3((unsigned)(items < most ? items : most)), dim3(kThreads), sh.smem, s, rec, in, ent, norm, out,

@@ -284,6 +284,14 @@ def test_recurrence_portions_and_decoding(heads, groups, dim, vdim, taps, kind, 
     status_clear()
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("heads,groups,dim,vdim", [(12, 6, 96, 112), (2, 1, 64, 112), (3, 3, 100, 100), (2, 2, 36, 132)])
+def test_recurrence_with_two_states_in_the_ring(heads, groups, dim, vdim, kind, dtype):
+    """States of which two blocks share a multiprocessor with two each in their rings, with many and few rows a thread."""
+    test_recurrence_portions_and_decoding(heads, groups, dim, vdim, 4, kind, dtype, False, None)
+
+
 @pytest.mark.parametrize("kind", KINDS)
 @pytest.mark.parametrize("heads,groups,dim,vdim", [(2, 1, 64, 64), (16, 4, 128, 72), (40, 8, 16, 16), (100, 4, 32, 8)])
 def test_long_portions_beside_others(kind, heads, groups, dim, vdim):
