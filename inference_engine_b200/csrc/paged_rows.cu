@@ -1,6 +1,7 @@
 // The paged cache of unquantised rows: rotary positions + unit norm + write of keys and values (one kernel; a second one
 // norms whole projections first and rotates neighbouring channels), and the
 // general attention over it (any sizes, bf16 or fp32, prompt portions and decoding alike) on the CUDA cores.
+#include <algorithm>
 #include <type_traits>
 
 #include "dec_common.cuh"
@@ -123,8 +124,260 @@ rope_write_kernel(const T* __restrict__ qkv, long long qkv_stride, b200dec_rows 
   }
 }
 
+// ---------------------------------------------------------------- the same by whole rows
+// Eight channels as they lie in memory, until their arithmetic.
+template <typename T>
+struct Raw8 {
+  uint4 v[sizeof(T) / 2];
+};
+template <typename T>
+__device__ __forceinline__ Raw8<T> ld_raw8(const T* p) {
+  Raw8<T> r;
+#pragma unroll
+  for (int i = 0; i < (int)sizeof(T) / 2; ++i) r.v[i] = reinterpret_cast<const uint4*>(p)[i];
+  return r;
+}
+__device__ __forceinline__ void raw_floats(const Raw8<uint16_t>& r, float (&f)[8]) { unpack8(r.v[0], f); }
+__device__ __forceinline__ void raw_floats(const Raw8<float>& r, float (&f)[8]) {
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    f[4 * i] = __uint_as_float(r.v[i].x); f[4 * i + 1] = __uint_as_float(r.v[i].y);
+    f[4 * i + 2] = __uint_as_float(r.v[i].z); f[4 * i + 3] = __uint_as_float(r.v[i].w);
+  }
+}
+// Four (cos, sin) or eight floats
+__device__ __forceinline__ void ld_floats8(const float* p, float (&f)[8]) { ld_vec(p, f); }
+
+// One block per row, kLanes lanes per head, eight channels a lane: what rope_write_kernel's warps each find for themselves (the
+// row's position and page, divisions, a lane's angles) is found once for all heads, and memory moves in 16 bytes.  For sizes and strides
+// that are multiples of eight channels.  Bound by the chain of a row's loads; its own come before the page is looked at, and two heads
+// of a group of lanes at a time leave room for more blocks than four (1024 rows 7.5 against 10.8 us).  us, rope_write_kernel -> this:
+// 1024 rows of 32 heads of 128 13.4 -> 7.5, 300 rows 6.1 -> 5.2, 60 rows 4.0 -> 4.4; 200 rows in fp32 7.7 -> 6.9.
+template <typename T, int kLanes>
+__global__ void __launch_bounds__(512)
+rope_rows_kernel(const T* __restrict__ qkv, long long qkv_stride, b200dec_rows rows, DecCache c, const float* __restrict__ cos_sin,
+                 int table_len, int half, int heads, int write_kv, int unit_norm, float eps, T* __restrict__ q_out, int32_t* status) {
+  constexpr int kAtOnce = 2;  // heads of a group of lanes whose loads are in flight together
+  pdl_enter();
+  const int r = blockIdx.x, tid = threadIdx.x, gl = tid % kLanes, groups = blockDim.x / kLanes;
+  const int hkv = write_kv ? c.heads : 0, per_row = heads + 2 * hkv;
+  int seq = r, pos;
+  if (rows.seq_ids) {
+    seq = rows.seq_ids[r];
+    pos = rows.positions[r];
+  } else {
+    if (r >= *rows.num_decoding) {  // an idle row: nothing is written to the cache, q reads as zero
+      pdl_wait();
+      for (int i = tid; i < heads * c.k_row; i += blockDim.x) st_elem(q_out + (long long)r * heads * c.k_row + i, 0.f);
+      return;
+    }
+    pos = rows.cached_lens[r];
+  }
+  const bool ok = pos >= 0 && (half == 0 || pos < table_len);
+  if (!ok) {
+    if (tid == 0 && status) atomicOr(status, B200KV_S_BAD_POSITION);
+    pos = 0;
+  }
+  const int col = pos / c.P, prow = pos - col * c.P;  // the page, asked for here and looked at behind the row's loads
+  const bool listed = ok && hkv > 0 && col < c.max_pages;
+  const int id = listed ? c.table[(long long)seq * c.table_stride + col] : -1;
+  const int ch = 8 * gl;
+  const bool turned = ch < 2 * half, low = ch < half;
+  const int partner = (tid & 31) + (turned ? (low ? half / 8 : -(half / 8)) : 0);
+  float cs[8], sn[8];
+  if (turned) {
+    const float* a = cos_sin + 2 * ((long long)pos * half + (low ? ch : ch - half));
+    float x[2][8];
+    ld_floats8(a, x[0]);
+    ld_floats8(a + 8, x[1]);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      cs[i] = x[i / 4][2 * (i % 4)];
+      const float v = x[i / 4][2 * (i % 4) + 1];
+      sn[i] = low ? -v : v;
+    }
+  }
+  const unsigned lanes = kLanes == 32 ? 0xffffffffu : ((1u << kLanes) - 1) << ((tid & 31) / kLanes * kLanes);
+  pdl_wait();
+  const T* src = qkv + r * qkv_stride;
+  long long at0 = 0;
+  bool stored = false;
+  for (int j0 = tid / kLanes; j0 < per_row; j0 += kAtOnce * groups) {
+    Raw8<T> own[kAtOnce];
+#pragma unroll
+    for (int u = 0; u < kAtOnce; ++u) {
+      const int j = j0 + u * groups;
+      if (j >= per_row) break;
+      const bool is_v = j >= heads + hkv;
+      const T* from = src + (is_v ? (heads + hkv) * c.k_dim + (j - heads - hkv) * c.v_dim : j * c.k_dim) + ch;
+      if (ch < (is_v ? c.v_dim : c.k_dim)) own[u] = ld_raw8(from);
+    }
+    stored = listed && id >= 0 && id < c.num_pages;
+    at0 = stored ? dec_row(c, id, 0, prow) : 0;
+#pragma unroll
+    for (int u = 0; u < kAtOnce; ++u) {
+      const int j = j0 + u * groups;
+      if (j >= per_row) break;
+      const bool is_v = j >= heads + hkv, some = ch < (is_v ? c.v_dim : c.k_dim);
+      float y[8];
+      raw_floats(own[u], y);
+      if (!is_v) {
+        float ss = 0.f;
+        if (half > 0) {
+          Raw8<T> other;  // the partner's channels
+#pragma unroll
+          for (int i = 0; i < (int)sizeof(T) / 2; ++i) {
+            other.v[i].x = __shfl_sync(lanes, own[u].v[i].x, partner);
+            other.v[i].y = __shfl_sync(lanes, own[u].v[i].y, partner);
+            other.v[i].z = __shfl_sync(lanes, own[u].v[i].z, partner);
+            other.v[i].w = __shfl_sync(lanes, own[u].v[i].w, partner);
+          }
+          if (turned) {
+            float o[8];
+            raw_floats(other, o);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) y[i] = y[i] * cs[i] + o[i] * sn[i];
+          }
+        }
+        if (some) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) ss = fmaf(y[i], y[i], ss);
+        }
+        if (unit_norm) {
+#pragma unroll
+          for (int o = kLanes / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(lanes, ss, o);
+          const float inv = 1.0f / sqrtf(ss / (float)c.k_dim + eps);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) y[i] *= inv;
+        }
+      }
+      if (!some || (j >= heads && !stored)) continue;
+      T* dst = j < heads ? q_out + ((long long)r * heads + j) * c.k_row
+               : is_v    ? (T*)c.v + (at0 + (long long)(j - heads - hkv) * c.P) * c.v_row
+                         : (T*)c.k + (at0 + (long long)(j - heads) * c.P) * c.k_row;
+      st_vec(dst + ch, y);
+    }
+  }
+  if (ok && hkv > 0 && tid == 0 && status && !(listed && id >= 0 && id < c.num_pages))
+    atomicOr(status, listed ? B200KV_S_BAD_PAGE : B200KV_S_BAD_POSITION);
+}
+
 // ---------------------------------------------------------------- norm of whole projections, interleaved rotation, write
-// One block per row; a thread owns channel pairs tid, tid + 256, ... of q | k | v.
+// Sizes and strides that are multiples of eight channels: one block per row, kVecs times eight channels a thread.  Against pairs of channels
+// (norm_rope_write_kernel below) a quarter of the loads, and a row's inputs as they lie, so that with many rows twice as many blocks
+// fit a multiprocessor.  1024 rows of 32 heads of 128 16.4 -> 7.1 us; of 48 heads of 64 15.4 -> 6.7, 64 rows of these 6.0 -> 4.1.
+template <typename T, int kVecs>
+__global__ void __launch_bounds__(512)
+norm_rope_rows_kernel(const T* __restrict__ qkv, long long qkv_stride, b200dec_rows rows, DecCache c, const float* __restrict__ q_norm,
+                      const float* __restrict__ k_norm, float eps, const float* __restrict__ cos_sin, int table_len, int half, int heads,
+                      int k_shift, int v_shift, T* __restrict__ q_out, int32_t* status) {
+  __shared__ float part[2][16];
+  pdl_enter();
+  const int r = blockIdx.x, tid = threadIdx.x, threads = blockDim.x;
+  T* qdst = q_out + (long long)r * heads * c.k_row;
+  int seq = r, pos;
+  if (rows.seq_ids) {
+    seq = rows.seq_ids[r];
+    pos = rows.positions[r];
+  } else {
+    if (r >= *rows.num_decoding) {  // an idle row: nothing is written to the cache, q reads as zero
+      pdl_wait();
+      for (int i = tid; i < heads * c.k_row; i += threads) st_elem(qdst + i, 0.f);
+      return;
+    }
+    pos = rows.cached_lens[r];
+  }
+  const bool ok = pos >= 0 && (half == 0 || pos < table_len);
+  if (!ok) {
+    if (tid == 0 && status) atomicOr(status, B200KV_S_BAD_POSITION);
+    pos = 0;
+  }
+  const int col = pos / c.P, prow = pos - col * c.P;  // the page, asked for here and looked at behind the row's loads
+  const bool listed = ok && col < c.max_pages;
+  const int id = listed ? c.table[(long long)seq * c.table_stride + col] : -1;
+  const float* cs = cos_sin + 2 * (long long)pos * half;
+  const int kv8 = c.k_dim / 8, vv8 = c.v_dim / 8, nq = heads * kv8, nqk = nq + c.heads * kv8, all = nqk + c.heads * vv8;  // in eights
+  // head and channel of the i-th eight of this thread (of q | k heads, or of v heads)
+  auto locate = [&](int p, int& h, int& ch) {
+    const bool is_v = p >= nqk;
+    const int m = is_v ? p - nqk : p, per = is_v ? vv8 : kv8, shift = is_v ? v_shift : k_shift;
+    h = shift >= 0 ? m >> shift : m / per;
+    ch = 8 * (m - h * per);
+  };
+  float w[8], t[8];  // of a thread's eight channels: weights, (cos, sin) of their pairs
+  auto constants = [&](int p, int ch) {
+    ld_floats8(p < nq ? q_norm + 8 * p : k_norm + 8 * (p - nq), w);
+    if (ch < 2 * half) ld_floats8(cs + ch, t);
+  };
+  if (kVecs == 1 && tid < nqk) {  // they do not wait for the kernel in front
+    int h, ch;
+    locate(tid, h, ch);
+    constants(tid, ch);
+  }
+  pdl_wait();
+  Raw8<T> raw[kVecs];
+  const T* src = qkv + r * qkv_stride;
+#pragma unroll
+  for (int i = 0; i < kVecs; ++i)
+    if (tid + i * threads < all) raw[i] = ld_raw8(src + 8 * (tid + i * threads));
+  const bool stored = listed && id >= 0 && id < c.num_pages;
+  if (ok && !stored && tid == 0 && status) atomicOr(status, listed ? B200KV_S_BAD_PAGE : B200KV_S_BAD_POSITION);
+  const long long at0 = stored ? dec_row(c, id, 0, prow) : 0;
+  float sq = 0.f, sk = 0.f;
+#pragma unroll
+  for (int i = 0; i < kVecs; ++i) {
+    const int p = tid + i * threads;
+    if (p < nqk) {
+      float x[8], s = 0.f;
+      raw_floats(raw[i], x);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) s = fmaf(x[e], x[e], s);
+      if (p < nq) sq += s; else sk += s;
+    }
+  }
+  sq = warp_sum(sq);
+  sk = warp_sum(sk);
+  if ((tid & 31) == 0) {
+    part[0][tid >> 5] = sq;
+    part[1][tid >> 5] = sk;
+  }
+  __syncthreads();
+  sq = sk = 0.f;
+  for (int i = 0; i < threads / 32; ++i) {
+    sq += part[0][i];
+    sk += part[1][i];
+  }
+  sq = 1.0f / sqrtf(sq / (float)(heads * c.k_dim) + eps);
+  sk = 1.0f / sqrtf(sk / (float)(c.heads * c.k_dim) + eps);
+#pragma unroll
+  for (int i = 0; i < kVecs; ++i) {
+    const int p = tid + i * threads;
+    if (p >= all || (p >= nq && !stored)) continue;
+    int h, ch;
+    locate(p, h, ch);
+    float x[8];
+    raw_floats(raw[i], x);
+    T* dst = (T*)c.v + (at0 + (long long)h * c.P) * c.v_row;
+    if (p < nqk) {
+      if (kVecs > 1) constants(p, ch);
+      const float inv = p < nq ? sq : sk;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[e] = x[e] * inv * w[e];
+      if (ch < 2 * half) {
+#pragma unroll
+        for (int e = 0; e < 8; e += 2) {
+          const float a = x[e], b = x[e + 1];
+          x[e] = a * t[e] - b * t[e + 1];
+          x[e + 1] = b * t[e] + a * t[e + 1];
+        }
+      }
+      dst = p < nq ? qdst + h * c.k_row : (T*)c.k + (at0 + (long long)(h - heads) * c.P) * c.k_row;
+    }
+    st_vec(dst + ch, x);
+  }
+}
+
+// Any sizes: one block per row; a thread owns channel pairs tid, tid + 256, ... of q | k | v.
 constexpr int kNrThreads = 256;
 
 // Pair p of a group of heads of `pairs` pairs each (shift: log2 of it, or -1).
@@ -627,6 +880,16 @@ static int check_rows(const b200dec_rows* r) {
   return B200KV_OK;
 }
 
+// Threads of a block that does one row of `items` threads' shares.  With few rows a share each, so that a row's chain is short; with more, as
+// many shares a thread, up to `most`, as let all blocks be one round (about 1024 threads of these kernels fit a multiprocessor).
+// Rotation, attention and all, us with 64 / 128 / 256 / 512 threads: 1000 rows 30.8 / 28.8 / 30.8 / 34.9, 300 rows 22.6 / 21.2 / 20.6 / 22.6,
+// 64 rows 45.6 / 43.2 / 42.3 / 42.2.
+static int row_threads(int num_rows, int items, int most) {
+  int threads = 512;
+  while (threads > 64 && (threads / 2 >= items || (2 * items <= most * threads && (long long)num_rows * threads > 148ll * 1024))) threads /= 2;
+  return threads;
+}
+
 extern "C" int b200dec_rope_write(const void* qkv, int64_t qkv_stride, const b200dec_rows* rows, const b200dec_cache* cache,
                                   const b200kv_table* table, const float* cos_sin, int32_t table_len, int32_t half, int32_t heads,
                                   int32_t write_kv, int32_t unit_norm, float eps, void* q_out, int32_t* status, void* stream) {
@@ -649,6 +912,19 @@ extern "C" int b200dec_rope_write(const void* qkv, int64_t qkv_stride, const b20
     return launch_result(launch_chained(kernel, dim3((unsigned)blocks), dim3(kRwWarps * 32), 0, s, in, (long long)qkv_stride, *rows, c, cos_sin,
                                         table_len, half, heads, write_kv, unit_norm, eps, q, status));
   };
+  const bool eights = cache->k_dim % 8 == 0 && cache->v_dim % 8 == 0 && half % 8 == 0 && qkv_stride % 8 == 0 && aligned(qkv, 16) &&
+                      aligned(cos_sin, 16) && cache->k_row <= 128 && cache->v_row <= 128;
+  if (eights) {
+    const int lanes = cache->k_row <= 64 && cache->v_row <= 64 ? 8 : 16, per_row = heads + (write_kv ? 2 * cache->kv_heads : 0);
+    const int threads = row_threads(rows->num_rows, per_row * lanes, 4);
+    auto by_rows = [&](auto* kernel, auto* in, auto* q) {
+      return launch_result(launch_chained(kernel, dim3(rows->num_rows), dim3(threads), 0, s, in, (long long)qkv_stride, *rows, c, cos_sin, table_len,
+                                          half, heads, write_kv, unit_norm, eps, q, status));
+    };
+    if (cache->elem == 2)
+      return by_rows(lanes == 8 ? rope_rows_kernel<uint16_t, 8> : rope_rows_kernel<uint16_t, 16>, (const uint16_t*)qkv, (uint16_t*)q_out);
+    return by_rows(lanes == 8 ? rope_rows_kernel<float, 8> : rope_rows_kernel<float, 16>, (const float*)qkv, (float*)q_out);
+  }
   if (cache->elem == 2) {
     if (pairs && cache->k_row <= 128 && cache->v_row <= 128) return run(rope_write_kernel<uint16_t, true, 2>, (const uint16_t*)qkv, (uint16_t*)q_out);
     return run(pairs ? rope_write_kernel<uint16_t, true, kRwMaxPairs> : rope_write_kernel<uint16_t, false, kRwMaxPairs>, (const uint16_t*)qkv,
@@ -684,6 +960,20 @@ extern "C" int b200dec_norm_rope_write(const void* qkv, int64_t qkv_stride, cons
                                         k_norm, eps, cos_sin, table_len, half, heads, log2_of(cache->k_dim / 2), log2_of(cache->v_dim / 2), q,
                                         status));
   };
+  const int items = (int)std::min<long long>(pairs / 4, 1 << 20), threads = row_threads(rows->num_rows, items, 4), vecs = (items + threads - 1) / threads;
+  if (even && cache->k_dim % 8 == 0 && cache->v_dim % 8 == 0 && half % 4 == 0 && qkv_stride % 8 == 0 && aligned(qkv, 16) && aligned(q_norm, 16) &&
+      aligned(k_norm, 16) && aligned(cos_sin, 16) && vecs <= 4) {
+    auto by_rows = [&](auto* kernel, auto* in, auto* q) {
+      return launch_result(launch_chained(kernel, dim3(rows->num_rows), dim3(threads), 0, s, in, (long long)qkv_stride, *rows, c, q_norm, k_norm,
+                                          eps, cos_sin, table_len, half, heads, log2_of(cache->k_dim / 8), log2_of(cache->v_dim / 8), q, status));
+    };
+    if (cache->elem == 2)
+      return by_rows(vecs == 1   ? norm_rope_rows_kernel<uint16_t, 1>
+                     : vecs == 2 ? norm_rope_rows_kernel<uint16_t, 2> : norm_rope_rows_kernel<uint16_t, 4>,
+                     (const uint16_t*)qkv, (uint16_t*)q_out);
+    return by_rows(vecs == 1 ? norm_rope_rows_kernel<float, 1> : vecs == 2 ? norm_rope_rows_kernel<float, 2> : norm_rope_rows_kernel<float, 4>,
+                   (const float*)qkv, (float*)q_out);
+  }
   const int keep = !even ? 0 : pairs <= 4 * kNrThreads ? 4 : pairs <= 8 * kNrThreads ? 8 : pairs <= 16 * kNrThreads ? 16 : 0;
   if (cache->elem == 2)
     return run(keep == 4   ? norm_rope_write_kernel<uint16_t, 4>

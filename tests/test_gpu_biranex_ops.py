@@ -117,6 +117,32 @@ def test_norm_rotation_and_write(heads, kv, dim, vdim, dims, dtype):
     status_clear()
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads,kv,dim,vdim,dims,n", [(8, 4, 64, 64, 64, 7), (8, 4, 64, 48, 8, 700), (16, 8, 128, 128, 128, 1300), (32, 8, 64, 64, 32, 400)])
+def test_norm_rotation_and_write_by_eights(heads, kv, dim, vdim, dims, n, dtype):
+    """One, two and four times eight channels a thread: a decode step of n rows, the last two of them idle."""
+    from inference_engine_b200 import ops
+
+    g = np.random.default_rng(n)
+    cache = ops.make_paged_kv(n, kv, 16, dim, vdim, dtype, DEV)
+    perm = g.permutation(n)
+    ints = lambda x: torch.as_tensor(np.asarray(x, np.int32)).to(DEV)  # noqa: E731
+    pos = g.integers(0, 16, n)
+    rows = ops.Rows(n, ints(pos), ints([n - 2]), ints(perm[:, None]))
+    qkv = rnd(g, n, heads * dim + kv * (dim + vdim), dtype=dtype, gain=2.0)
+    qn, kn = rnd(g, heads * dim), rnd(g, kv * dim)
+    rot = {"dims": dims, "base": 300.0, "scaling": {"factor": 1.5}}
+    q = ops.norm_rope_write(qkv, rows, cache, qn, kn, 1e-5, ops.Rotary(dims, 300.0, stretch=1.5).table(16, DEV), heads)
+    a, m = np64(qkv), n - 2
+    want_q = B.rotate_interleaved(B.rms_norm(a[:, : heads * dim], 1e-5, np64(qn)).reshape(n, heads, dim), pos, rot)
+    want_k = B.rotate_interleaved(B.rms_norm(a[:, heads * dim : (heads + kv) * dim], 1e-5, np64(kn)).reshape(n, kv, dim), pos, rot)
+    close(q[:m, :, :dim], want_q[:m], dtype)
+    assert (q[m:] == 0).all()
+    close(cache.k[perm[:m], :, pos[:m], :dim], want_k[:m], dtype)
+    assert torch.equal(cache.v[perm[:m], :, pos[:m], :vdim].reshape(m, -1), qkv[:m, (heads + kv) * dim :])
+    status_clear()
+
+
 # ------------------------------------------------------------------ attention: window, sink, gate
 def attention_case(g, dtype, cached, chunks, nd, heads, kv, dim, vdim, page):
     """Random keys and values of whole sequences in a cache, and the queries of a step's rows."""

@@ -119,6 +119,30 @@ def test_rotation_unit_norm_and_write(dtype, scaling, dim, vdim, rot):
     H.status_clear()
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("dim,vdim,rot", [(112, 96, 32), (128, 128, 128), (64, 8, 48), (8, 64, 0), (16, 16, 16)])
+def test_rotation_by_whole_rows(dtype, dim, vdim, rot):
+    """Sizes in eights: eight and sixteen lanes a head, heads that leave lanes idle, a rotation of all, some and none of the channels."""
+    if rot:
+        test_rotation_unit_norm_and_write(dtype, None, dim, vdim, rot)
+    from inference_engine_b200 import ops
+
+    g = np.random.default_rng(dim)
+    heads, kv, n = 6, 3, 1300  # enough rows for few threads and several heads each; one page of one row per entry
+    cache = ops.make_paged_kv(n, kv, 16, dim, vdim, dtype, DEV)
+    perm = g.permutation(n)
+    rows = ops.Rows(n, i32(np.zeros(n)), i32([n - 2]), i32(perm[:, None]))  # a decode step with two idle rows
+    qkv = H.bf16(g.standard_normal((n, (heads + kv) * dim + kv * vdim)))
+    table = ops.Rotary(rot, 500.0).table(4, DEV) if rot else None
+    q = ops.rope_write(t(qkv, dtype), rows, cache, table, heads, True, False, 1e-4)
+    live = slice(0, n - 2)
+    close(q[live, :, :dim], qkv[live, : heads * dim].reshape(-1, heads, dim), dtype)
+    assert q[n - 2 :].abs().sum().item() == 0
+    close(cache.k[perm[live], :, 0, :dim], qkv[live, heads * dim : (heads + kv) * dim].reshape(-1, kv, dim), dtype)
+    close(cache.v[perm[live], :, 0, :vdim], qkv[live, (heads + kv) * dim :].reshape(-1, kv, vdim), dtype)
+    H.status_clear()
+
+
 CASES = [  # heads, kv heads, key size, value size
     (4, 2, 48, 40), (3, 1, 128, 64), (8, 8, 64, 128), (12, 1, 104, 88), (40, 2, 16, 24), (2, 1, 36, 12), (2, 2, 10, 7),
 ]
