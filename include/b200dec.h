@@ -123,6 +123,11 @@ typedef struct b200dec_attn_options {
 
 int b200dec_attn_rows_opt(const void* q, const b200dec_cache* cache, const b200kv_table* table, const b200dec_rows* rows, int32_t heads,
                           float scale, const b200dec_attn_options* opt, void* out, int32_t* status, void* stream);
+/* The same with the entries' first rows, cu_seqlens int32 [num_entries + 1]: entry e brings rows cu_seqlens[e] to cu_seqlens[e + 1] - 1 at
+ * consecutive positions, and all rows belong to one.  No more blocks are launched than the rows need then.  NULL: as above. */
+int b200dec_attn_rows_entries(const void* q, const b200dec_cache* cache, const b200kv_table* table, const b200dec_rows* rows,
+                              const int32_t* cu_seqlens, int32_t num_entries, int32_t heads, float scale, const b200dec_attn_options* opt, void* out,
+                              int32_t* status, void* stream);
 int b200dec_decode_attn_opt(const void* q, const b200dec_cache* cache, const b200kv_table* table, const int32_t* cached_lens,
                             const int32_t* num_decoding, int32_t B, int32_t heads, float scale, const b200dec_attn_options* opt, void* out,
                             int32_t zero_idle, void* workspace, size_t workspace_bytes, int32_t sm_count, int32_t* status, void* stream);

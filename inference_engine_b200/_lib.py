@@ -144,6 +144,8 @@ DECODER_SIGNATURES = {
     "b200dec_prefill_attn": (c_int32, [c_void_p, P_DCACHE, P_TABLE, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32,
                                        c_int32, c_float, c_void_p, c_void_p, c_void_p]),
     "b200dec_attn_rows_opt": (c_int32, [c_void_p, P_DCACHE, P_TABLE, P_ROWS, c_int32, c_float, P_OPT, c_void_p, c_void_p, c_void_p]),
+    "b200dec_attn_rows_entries": (c_int32, [c_void_p, P_DCACHE, P_TABLE, P_ROWS, c_void_p, c_int32, c_int32, c_float, P_OPT, c_void_p,
+                                            c_void_p, c_void_p]),
     "b200dec_decode_attn_opt": (c_int32, [c_void_p, P_DCACHE, P_TABLE, c_void_p, c_void_p, c_int32, c_int32, c_float, P_OPT, c_void_p,
                                           c_int32, c_void_p, c_size_t, c_int32, c_void_p, c_void_p]),
     "b200dec_prefill_attn_opt": (c_int32, [c_void_p, P_DCACHE, P_TABLE, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32,

@@ -628,6 +628,7 @@ attn_rows_kernel(const T* __restrict__ q, DecCache c, b200dec_rows rows, int hea
 // against four query rows, a value against two) and, with few entries, one block's chain of steps.
 // fp32, us, attn_rows_kernel -> this: 200 rows, 16 heads of 112 and 96, 183 -> 43; 8 entries of 550 decoding, 16 heads of 128, 420 -> 51 (with half
 // the threads 67).
+// A tile's keys are shared by the blocks of a cluster (at_splits), whose parts meet in its shared memory, in the order of the keys.
 constexpr int kAtThreads = 256;
 constexpr int kAtSlots = 16;
 constexpr int kAtKeys = 64;
@@ -645,6 +646,25 @@ __device__ __forceinline__ void at_commit() { asm volatile("cp.async.commit_grou
 template <int N>
 __device__ __forceinline__ void at_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
+__device__ __forceinline__ void at_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// shared memory of block `rank` of the cluster, at the place where `p` lies in this one's
+__device__ __forceinline__ uint32_t at_peer(const float* p, int rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float2 at_peer2(const float* p, int rank) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(at_peer(p, rank)) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 at_peer4(const float* p, int rank) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at_peer(p, rank)) : "memory");
+  return v;
+}
 template <int N>
 __device__ __forceinline__ void at_read(const float* p, float (&f)[N]) {
 #pragma unroll
@@ -660,9 +680,10 @@ __host__ __device__ constexpr size_t at_floats(int k_row, int v_row) {
 
 template <typename T, int kPieces>  // kPieces: output channels, in pieces of 128
 __global__ void __launch_bounds__(kAtThreads, 2)
-attn_tile_kernel(const T* __restrict__ q, DecCache c, b200dec_rows rows, int heads, int slice_heads, float scale, DecAttnOpt opt,
+attn_tile_kernel(const T* __restrict__ q, DecCache c, b200dec_rows rows, const int32_t* __restrict__ cu_seqlens, int num_entries, int heads, int slice_heads, float scale, DecAttnOpt opt,
                  T* __restrict__ out, int32_t* status) {
   extern __shared__ __align__(16) float at_smem[];
+  const int splits = gridDim.z, part = blockIdx.z;  // of the cluster's blocks
   const int kp = c.k_row + 4;  // an odd number of 16-byte words: neighbouring keys lie in different banks
   float* qs = at_smem;                  // [kAtSlots][k_row]
   float* ks = qs + kAtSlots * c.k_row;  // [kAtKeys][kp]
@@ -671,27 +692,42 @@ attn_tile_kernel(const T* __restrict__ q, DecCache c, b200dec_rows rows, int hea
   __shared__ long long at[2][kAtKeys];  // a key's row in the cache, -1: none; of this step and the next
   constexpr int kWarps = kAtThreads / 32;
   pdl_enter();
-  const int r0 = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int G = heads / c.heads, slices = (G + kAtSlots - 1) / kAtSlots;
   const int hk = blockIdx.x / slices, g0 = blockIdx.x % slices * slice_heads, gs = min(slice_heads, G - g0);
-  const int most = kAtSlots / slice_heads;  // rows of a tile
-  // a tile starts at the first row of an entry and at the positions that are multiples of its size
-  int seq = r0, pos, n = 1;
+  // A tile starts at the first row of an entry and then every `most` rows.  With the entries' first rows a block finds its tile, of a list with
+  // a few places too many; without, there is a block for every row, and those that start nothing leave.
+  const int most = kAtSlots / slice_heads;
+  int r0 = blockIdx.y, seq = r0, pos, n = 1;
   if (rows.seq_ids) {
+    if (cu_seqlens) {
+      int lo = 0, hi = num_entries;  // the last entry whose first place is not behind this block's
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (cu_seqlens[mid] / most + mid <= r0) lo = mid; else hi = mid;
+      }
+      const int first = cu_seqlens[lo], end = min(cu_seqlens[lo + 1], rows.num_rows), tile = r0 - (first / most + lo);
+      r0 = first + tile * most;
+      if (r0 < 0 || r0 >= end) return;
+      n = min(most, end - r0);
+    }
     seq = rows.seq_ids[r0];
     pos = rows.positions[r0];
-    if (r0 > 0 && pos >= 0 && pos % most != 0 && rows.seq_ids[r0 - 1] == seq && rows.positions[r0 - 1] == pos - 1) return;
-    while (pos >= 0 && n < most && r0 + n < rows.num_rows && (pos + n) % most != 0 && rows.seq_ids[r0 + n] == seq &&
-           rows.positions[r0 + n] == pos + n)
-      ++n;
+    if (!cu_seqlens) {
+      if (r0 > 0 && pos >= 0 && pos % most != 0 && rows.seq_ids[r0 - 1] == seq && rows.positions[r0 - 1] == pos - 1) return;
+      while (pos >= 0 && n < most && r0 + n < rows.num_rows && (pos + n) % most != 0 && rows.seq_ids[r0 + n] == seq &&
+             rows.positions[r0 + n] == pos + n)
+        ++n;
+    }
   } else {
     pos = r0 < *rows.num_decoding ? rows.cached_lens[r0] : -1;
   }
   pdl_wait();
   const int slots = n * gs;
   if (pos < 0) {  // idle row
-    T* dst = out + r0 * opt.out_stride + (hk * G + g0) * c.v_dim;
-    for (int i = tid; i < gs * c.v_dim; i += kAtThreads) st_elem(dst + i, 0.f);
+    if (part == 0)
+      for (int r = r0; r < r0 + n; ++r)
+        for (int i = tid; i < gs * c.v_dim; i += kAtThreads) st_elem(out + r * opt.out_stride + (hk * G + g0) * c.v_dim + i, 0.f);
     return;
   }
   for (int s = warp; s < kAtSlots; s += kWarps) {
@@ -706,8 +742,8 @@ attn_tile_kernel(const T* __restrict__ q, DecCache c, b200dec_rows rows, int hea
     const int s = kAtOwn * warp + i, h = hk * G + g0 + s % gs;
     last[i] = s < slots ? pos + s / gs : -1;
     low[i] = s < slots && opt.window > 0 ? max(0, last[i] - opt.window + 1) : 0;
-    m[i] = opt.sink && s < slots ? opt.sink[h] : -INFINITY;
-    l[i] = opt.sink ? 1.f : 0.f;
+    m[i] = opt.sink && s < slots && part == 0 ? opt.sink[h] : -INFINITY;
+    l[i] = opt.sink && part == 0 ? 1.f : 0.f;
 #pragma unroll
     for (int j = 0; j < kPieces; ++j)
 #pragma unroll
@@ -716,8 +752,13 @@ attn_tile_kernel(const T* __restrict__ q, DecCache c, b200dec_rows rows, int hea
   const bool mine = kAtOwn * warp < slots;
   // Keys [all_low, all_last] are seen by every query row of the tile; the others are looked at one by one, so that what a row
   // does not see (a later token, perhaps not a number) never meets it.
-  const int all_last = pos, all_low = opt.window > 0 ? max(0, pos + n - opt.window) : 0, end = pos + n;
-  const int first = opt.window > 0 ? max(0, pos - opt.window + 1) : 0;
+  const int all_last = pos, all_low = opt.window > 0 ? max(0, pos + n - opt.window) : 0;
+  int first = opt.window > 0 ? max(0, pos - opt.window + 1) : 0, end = pos + n;
+  if (splits > 1) {  // this block's steps
+    const int share = ((end - first + kAtKeys - 1) / kAtKeys + splits - 1) / splits * kAtKeys;
+    first += part * share;
+    end = min(end, first + share);
+  }
   // the rows of the keys from j0 on
   auto look_up = [&](int j0, long long* at_rows) {
     if (tid < kAtKeys) {
@@ -754,10 +795,12 @@ attn_tile_kernel(const T* __restrict__ q, DecCache c, b200dec_rows rows, int hea
     at_commit();
   };
   // The keys of a step are fetched while the values of the one before are used, its values while its scores are made.
-  look_up(first, at[0]);
-  __syncthreads();
-  fetch(at[0], c.k, c.k_row, c.k_dim, ks, kp);
-  fetch(at[0], c.v, c.v_row, c.v_dim, vs, c.v_row);
+  if (first < end) {
+    look_up(first, at[0]);
+    __syncthreads();
+    fetch(at[0], c.k, c.k_row, c.k_dim, ks, kp);
+    fetch(at[0], c.v, c.v_row, c.v_dim, vs, c.v_row);
+  }
   for (int j0 = first, turn = 0; j0 < end; j0 += kAtKeys, turn ^= 1) {
     const int count = min(kAtKeys, end - j0);
     const bool more = j0 + kAtKeys < end;
@@ -852,25 +895,91 @@ attn_tile_kernel(const T* __restrict__ q, DecCache c, b200dec_rows rows, int hea
     __syncthreads();  // the values are used
     if (more) fetch(at[turn ^ 1], c.v, c.v_row, c.v_dim, vs, c.v_row); else at_commit();
   }
-#pragma unroll
-  for (int i = 0; i < kAtOwn; ++i) {
-    const int s = kAtOwn * warp + i;
-    if (s >= slots) break;
+  auto store = [&](int s, float sum, const float (&v)[kPieces][4]) {
     const int r = r0 + s / gs, h = hk * G + g0 + s % gs;
-    const float inv = (l[i] > 0.f ? 1.f / l[i] : 0.f) * opt.factor<T>(r, h);
+    const float inv = (sum > 0.f ? 1.f / sum : 0.f) * opt.factor<T>(r, h);
 #pragma unroll
     for (int a = 0; a < kPieces; ++a)
 #pragma unroll
       for (int b = 0; b < 4; ++b) {
         const int ch = 4 * lane + 128 * a + b;
-        if (ch < c.v_dim) st_elem(out + r * opt.out_stride + (long long)h * c.v_dim + ch, o[i][a][b] * inv);
+        if (ch < c.v_dim) st_elem(out + r * opt.out_stride + (long long)h * c.v_dim + ch, v[a][b] * inv);
       }
+  };
+  if (splits == 1) {
+#pragma unroll
+    for (int i = 0; i < kAtOwn; ++i)
+      if (kAtOwn * warp + i < slots) store(kAtOwn * warp + i, l[i], o[i]);
+    return;
   }
+  // the cluster's parts meet in its shared memory: outputs where the values were, maxima and sums where the scores were
+#pragma unroll
+  for (int i = 0; i < kAtOwn; ++i) {
+    const int s = kAtOwn * warp + i;
+    if (lane == 0) *reinterpret_cast<float2*>(ps + 2 * s) = make_float2(m[i], l[i]);
+#pragma unroll
+    for (int a = 0; a < kPieces; ++a)
+      if (4 * lane + 128 * a < c.v_row) st_elem4(vs + s * c.v_row + 4 * lane + 128 * a, o[i][a]);
+  }
+  at_cluster_sync();
+  for (int s = part + splits * warp; s < slots; s += splits * kWarps) {
+    float top = -INFINITY, sum = 0.f, v[kPieces][4] = {};
+    for (int j = 0; j < splits; ++j) top = fmaxf(top, at_peer2(ps + 2 * s, j).x);
+    const float base = top == -INFINITY ? 0.f : top;
+    for (int j = 0; j < splits; ++j) {
+      const float2 ml = at_peer2(ps + 2 * s, j);
+      const float w = expf(ml.x - base);
+      sum = fmaf(ml.y, w, sum);
+#pragma unroll
+      for (int a = 0; a < kPieces; ++a) {
+        if (4 * lane + 128 * a >= c.v_row) break;
+        const float4 x = at_peer4(vs + s * c.v_row + 4 * lane + 128 * a, j);
+        v[a][0] = fmaf(x.x, w, v[a][0]);
+        v[a][1] = fmaf(x.y, w, v[a][1]);
+        v[a][2] = fmaf(x.z, w, v[a][2]);
+        v[a][3] = fmaf(x.w, w, v[a][3]);
+      }
+    }
+    store(s, sum, v);
+  }
+  at_cluster_sync();  // a block's shared memory stays until its peers have read it
 }
 
 }  // namespace b200kv
 
 using namespace b200kv;
+
+// Blocks that share a tile's keys: as many as are resident at a time (two per multiprocessor), but no more than a tile has steps.  A block's
+// fixed cost is about two steps, so that with more than a round of blocks sharing only adds work.  us with 1 / 2 / 4 / 8, 16 heads of
+// 128 over 8: an entry of 550 decoding 51.3 / 34.9 / 24.7 / 20.6, of 4000 314 / 166 / 89 / 51; 8 of 550 55.4 / 34.9 / 26.7 / 37.0, 64 of
+// 550 118 / 133 / 164 / 240; 200 rows of a prompt 41.0 / 41.7 / 49.1 / 90.
+static int at_splits(long long blocks, int tile_rows, long long most_keys, int window) {
+  if (window > 0 && window + tile_rows < most_keys) most_keys = window + tile_rows;
+  int splits = 1;
+  while (splits < 8 && 2 * splits * blocks <= 2 * 148 && splits * kAtKeys < most_keys) splits *= 2;
+  return splits;
+}
+
+// launch_chained with the grid's z extent as clusters
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_clusters(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+  if (grid.z == 1) return launch_chained(kernel, grid, block, smem, stream, args...);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = grid.z;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = chained_launch_enabled() ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
 
 static int check_rows(const b200dec_rows* r) {
   if (!r) return B200KV_E_NULL;
@@ -989,6 +1098,12 @@ extern "C" int b200dec_norm_rope_write(const void* qkv, int64_t qkv_stride, cons
 extern "C" int b200dec_attn_rows_opt(const void* q, const b200dec_cache* cache, const b200kv_table* table, const b200dec_rows* rows,
                                      int32_t heads, float scale, const b200dec_attn_options* options, void* out, int32_t* status,
                                      void* stream) {
+  return b200dec_attn_rows_entries(q, cache, table, rows, nullptr, 0, heads, scale, options, out, status, stream);
+}
+
+extern "C" int b200dec_attn_rows_entries(const void* q, const b200dec_cache* cache, const b200kv_table* table, const b200dec_rows* rows,
+                                         const int32_t* cu_seqlens, int32_t num_entries, int32_t heads, float scale, const b200dec_attn_options* options, void* out,
+                                         int32_t* status, void* stream) {
   if (rows && rows->num_rows == 0) return B200KV_OK;
   if (!q || !out) return B200KV_E_NULL;
   int rc = check_rows(rows);
@@ -996,7 +1111,7 @@ extern "C" int b200dec_attn_rows_opt(const void* q, const b200dec_cache* cache, 
   DecAttnOpt opt;
   if (rc == B200KV_OK) rc = dec_attn_opt(options, heads, cache->v_dim, &opt);
   if (rc != B200KV_OK) return rc;
-  if (heads < 1 || heads % cache->kv_heads || cache->v_dim > kArThreads * kArPieces || cache->k_dim > 1024) return B200KV_E_SHAPE;
+  if (heads < 1 || heads % cache->kv_heads || cache->v_dim > kArThreads * kArPieces || cache->k_dim > 1024 || num_entries < 0) return B200KV_E_SHAPE;
   if ((long long)cache->num_pages * cache->page_size > 0x7FFFFFFFll || rows->num_rows > 65535) return B200KV_E_RANGE;
   const DecCache c = dec_view(cache, table);
   cudaStream_t s = (cudaStream_t)stream;
@@ -1007,10 +1122,14 @@ extern "C" int b200dec_attn_rows_opt(const void* q, const b200dec_cache* cache, 
   const size_t tile_smem = at_floats(cache->k_row, cache->v_row) * 4;
   if (tile_smem <= kAtMostSmem && cache->v_row <= 256) {
     const int G = heads / cache->kv_heads, slices = (G + kAtSlots - 1) / kAtSlots, slice_heads = (G + slices - 1) / slices;
+    const int most = kAtSlots / slice_heads;
+    const bool listed = rows->seq_ids && cu_seqlens && num_entries > 0 && rows->num_rows / most + (long long)num_entries <= 65535;
+    const int blocks = listed ? rows->num_rows / most + num_entries : rows->num_rows;
+    const int splits = at_splits((long long)cache->kv_heads * slices * (listed || !rows->seq_ids ? blocks : blocks / most + 1), most, (long long)table->max_pages * cache->page_size, opt.window);
     auto tiles = [&](auto* kernel, auto* in, auto* o) -> int {
       if (!allow_smem(kernel, kAtMostSmem)) return B200KV_E_LAUNCH;
-      return launch_result(launch_chained(kernel, dim3(cache->kv_heads * slices, rows->num_rows), dim3(kAtThreads), tile_smem, s, in, c, *rows,
-                                          heads, slice_heads, scale, opt, o, status));
+      return launch_result(launch_clusters(kernel, dim3(cache->kv_heads * slices, blocks, splits), dim3(kAtThreads), tile_smem, s, in, c,
+                                           *rows, listed ? cu_seqlens : nullptr, (int)num_entries, heads, slice_heads, scale, opt, o, status));
     };
     if (cache->elem == 2)
       return tiles(cache->v_row <= 128 ? attn_tile_kernel<uint16_t, 1> : attn_tile_kernel<uint16_t, 2>, (const uint16_t*)q, (uint16_t*)out);
