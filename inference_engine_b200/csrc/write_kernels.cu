@@ -459,128 +459,148 @@ prefill_rows_kernel(const uint16_t* __restrict__ q, long long q_sn, long long q_
 }
 
 // K of first-chunk entries.  grid (Hkv, kFirstLanes, kFirstCtas), cluster (1, 1, kFirstCtas), kFirstWarps warps.
-// Cluster (h, y) walks the entries b = y, y + kFirstLanes, ... that are on their first chunk; its CTAs share the
-// chunk's rows round-robin by warp.  Per entry: every warp takes the column maxima of its rows (the first
-// kKeepRows stay in registers), the CTA folds its warps' maxima in shared memory, the cluster's CTAs read one
+// Cluster (h, y) does every kFirstLanes-th of the entries that are on their first chunk; its CTAs share the
+// chunk's rows round-robin by warp.  Where more than one entry falls to it, its warps are cut into up to kFirstTeams teams that
+// do one each, side by side.  Per entry: every warp takes the column maxima of its rows (the first
+// kKeepRows stay in registers), the CTA folds its teams' maxima in shared memory, the cluster's CTAs read one
 // another's 128 maxima through distributed shared memory between two cluster barriers, calibration =
 // max(1e-3, column max) (exact and order-independent, kernels.py:764-780) is stored by CTA 0, and every warp
 // quantizes its rows as k / calibration (kernels.py:786-811).
-constexpr int kFirstCtas = 8, kFirstWarps = 16, kFirstLanes = 4, kKeepRows = 8;
-// Registers for two blocks per multiprocessor (64, of which 16 bytes are spilled), so that the clusters of four entries are one round of
-// blocks: five prompts of 1011 rows, 8 heads: 14.7 -> 10.0 us.  One portion alone would take 2 to 3 % less with more registers (300 rows 6.0 us
-// instead of 6.3), but a call without first portions, whose blocks only come and go, 0.4 us more.
+constexpr int kFirstCtas = 8, kFirstWarps = 16, kFirstLanes = 4, kFirstTeams = 4, kKeepRows = 8;
+// The kept rows lie in shared memory and the quantizing loop is not unrolled: two blocks share a multiprocessor without spills, and the
+// code that every call has to fetch is 27 KB instead of 69.  With the entries of a lane one after the other, 30 portions of 2000 rows in all
+// took 84 us, 59 now; 12 of 2000 65.6 and 60; one portion 7.55 and 7.4; five prompts of 1011 rows, with all else of two layers, 75.8
+// and 70.9.
 __global__ void __launch_bounds__(kFirstWarps * 32, 2)
 first_chunk_k_kernel(const uint16_t* __restrict__ k, long long k_sn, long long k_sh, CacheView c,
                      const int32_t* __restrict__ cu, int num_entries, const int32_t* __restrict__ cached_lens,
                      const int32_t* __restrict__ num_decoding, int N, int32_t* status) {
   __shared__ __align__(16) float part[kFirstWarps][kD];
-  __shared__ float cta_max[kD];
-  __shared__ __align__(16) float cal_s[kD];
+  __shared__ float cta_max[kFirstTeams][kD];
+  __shared__ __align__(16) float cal_s[kFirstTeams][kD];
+  __shared__ uint2 keep[kFirstWarps][kKeepRows][32];  // each warp's first rows
   pdl_enter();
   const int h = blockIdx.x, y = blockIdx.y;
   unsigned crank;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(crank));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nd = *num_decoding;
-  const int wid = (int)crank * kFirstWarps + warp, nw = kFirstCtas * kFirstWarps;  // this warp among the cluster's
-  bool waited = false;
-  for (int e0 = 0; e0 < num_entries; e0 += 32) {
-    // the entries of this cluster's lane that are on their first chunk, 32 candidates per round of loads; every
-    // thread of the cluster sees the same mask, so the barriers below are reached by all or by none
-    const int e = e0 + lane;
-    unsigned mask = __ballot_sync(0xffffffffu, e < num_entries && (e % kFirstLanes) == y && is_first_chunk(e, nd, cu, cached_lens));
-    while (mask) {
-      const int b = e0 + __ffs(mask) - 1;
-      mask &= mask - 1;
-      if (!waited) {
-        pdl_wait();  // k comes from the kernel before this one
-        waited = true;
+  // the n-th entry on its first chunk, or -1 (n: large) and their number; the same in every warp, so the barriers below are reached by all
+  const unsigned first32 = __ballot_sync(0xffffffffu, lane < num_entries && is_first_chunk(lane, nd, cu, cached_lens));
+  auto find = [&](int n, int& count) {
+    count = 0;
+    for (int e0 = 0; e0 < num_entries; e0 += 32) {
+      const int e = e0 + lane;
+      unsigned mask = e0 == 0 ? first32 : __ballot_sync(0xffffffffu, e < num_entries && is_first_chunk(e, nd, cu, cached_lens));
+      const int here = __popc(mask);
+      if (n < count + here) {
+        for (int i = count; i < n; ++i) mask &= mask - 1;
+        return e0 + __ffs(mask) - 1;
       }
-      const int s0 = cu[b], s1 = min(cu[b + 1], N);
-      const uint16_t* kcol = k + h * k_sh + 4 * lane;
-      uint2 keep[kKeepRows];
-      int keep_page[kKeepRows];  // table entries of the kept rows, fetched in the same round as the rows
-      float m[4] = {0.f, 0.f, 0.f, 0.f};
+      count += here;
+    }
+    return -1;
+  };
+  int total, unused;
+  find(1 << 30, total);
+  const int mine = (total - y + kFirstLanes - 1) / kFirstLanes;  // entries of this cluster
+  if (mine <= 0) return;
+  const int lg = mine >= 4 ? 2 : mine > 1 ? 1 : 0, teams = 1 << lg, per_team = kFirstWarps >> lg, team = warp >> (4 - lg);
+  static_assert(kFirstTeams == 4 && kFirstWarps == 16 && kKeepRows <= 32, "");
+  const int wid = (int)crank * per_team + (warp & (per_team - 1)), nw = kFirstCtas * per_team;  // this warp among its team's
+  pdl_wait();  // k comes from the kernel before this one
+  for (int first = 0; first < mine; first += teams) {
+    const int b = first + team < mine ? find(y + kFirstLanes * (first + team), unused) : -1;
+    const int s0 = b < 0 ? 0 : cu[b], s1 = b < 0 ? 0 : min(cu[b + 1], N);
+    const uint16_t* kcol = k + h * k_sh + 4 * lane;
+    uint2 raw[kKeepRows];
 #pragma unroll
-      for (int i = 0; i < kKeepRows; ++i) {  // independent loads: all in flight together
-        const int t = s0 + wid + i * nw;
-        keep[i] = t < s1 ? *reinterpret_cast<const uint2*>(kcol + (long long)t * (int)k_sn) : make_uint2(0u, 0u);
-        int slot, prow_unused;
-        split_pos(c, t - s0, slot, prow_unused);
-        keep_page[i] = (t < s1 && slot < c.max_pages) ? c.table[(long long)b * c.table_stride + slot] : -2;
+    for (int i = 0; i < kKeepRows; ++i) {  // independent loads: all in flight together
+      const int t = s0 + wid + i * nw;
+      raw[i] = t < s1 ? *reinterpret_cast<const uint2*>(kcol + (long long)t * (int)k_sn) : make_uint2(0u, 0u);
+    }
+    // lane i: the page of the i-th kept row, fetched in the same round as the rows
+    int pages = -2;
+    if (lane < kKeepRows && s0 + wid + lane * nw < s1) {
+      int slot, prow_unused;
+      split_pos(c, wid + lane * nw, slot, prow_unused);
+      if (slot < c.max_pages) pages = c.table[(long long)b * c.table_stride + slot];
+    }
+    float m[4] = {0.f, 0.f, 0.f, 0.f};
+    auto take = [&](uint2 r) {
+      float x[4];
+      unpack4(r, x);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) m[j] = fmaxf(m[j], fabsf(x[j]));
+    };
+#pragma unroll
+    for (int i = 0; i < kKeepRows; ++i) {
+      take(raw[i]);
+      keep[warp][i][lane] = raw[i];
+    }
+    for (int t = s0 + wid + kKeepRows * nw; t < s1; t += nw)  // chunks beyond kKeepRows rows a warp
+      take(*reinterpret_cast<const uint2*>(kcol + (long long)t * (int)k_sn));
+    *reinterpret_cast<float4*>(&part[warp][4 * lane]) = make_float4(m[0], m[1], m[2], m[3]);
+    __syncthreads();
+    for (int i = threadIdx.x; i < teams * kD; i += kFirstWarps * 32) {
+      const int tm = i / kD, ch = i % kD;
+      float v = 0.f;
+      for (int w0 = tm * per_team; w0 < (tm + 1) * per_team; w0 += 4)
+#pragma unroll
+        for (int w = 0; w < 4; ++w) v = fmaxf(v, part[w0 + w][ch]);
+      cta_max[tm][ch] = v;
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    for (int i = threadIdx.x; i < teams * kD; i += kFirstWarps * 32) {
+      float v = 1e-3f;
+      const uint32_t at = (uint32_t)__cvta_generic_to_shared(&cta_max[i / kD][i % kD]);
+#pragma unroll
+      for (int p = 0; p < kFirstCtas; ++p) {
+        uint32_t remote;
+        float pv;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(at), "r"(p));
+        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(pv) : "r"(remote) : "memory");
+        v = fmaxf(v, pv);
       }
-#pragma unroll
-      for (int i = 0; i < kKeepRows; ++i) {
-        float x[4];
-        unpack4(keep[i], x);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) m[j] = fmaxf(m[j], fabsf(x[j]));
-      }
-      for (int t = s0 + wid + kKeepRows * nw; t < s1; t += nw) {  // chunks beyond kKeepRows * 128 rows
-        float x[4];
-        unpack4(*reinterpret_cast<const uint2*>(kcol + (long long)t * (int)k_sn), x);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) m[j] = fmaxf(m[j], fabsf(x[j]));
-      }
-      *reinterpret_cast<float4*>(&part[warp][4 * lane]) = make_float4(m[0], m[1], m[2], m[3]);
-      __syncthreads();
-      if (threadIdx.x < kD) {
-        float v = 0.f;
-#pragma unroll
-        for (int w = 0; w < kFirstWarps; ++w) v = fmaxf(v, part[w][threadIdx.x]);
-        cta_max[threadIdx.x] = v;
-      }
-      asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-      if (threadIdx.x < kD) {
-        float v = 1e-3f;
-        const uint32_t mine = (uint32_t)__cvta_generic_to_shared(&cta_max[threadIdx.x]);
-#pragma unroll
-        for (int p = 0; p < kFirstCtas; ++p) {
-          uint32_t remote;
-          float pv;
-          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(mine), "r"(p));
-          asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(pv) : "r"(remote) : "memory");
-          v = fmaxf(v, pv);
-        }
-        cal_s[threadIdx.x] = v;
-      }
-      // nobody may overwrite cta_max (next entry) or leave while a peer still reads it
-      asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-      __syncthreads();
+      cal_s[i / kD][i % kD] = v;
+    }
+    // nobody may overwrite cta_max (next entry) or leave while a peer still reads it
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    __syncthreads();
+    float cal[4];
+    load4_f32(cal_s[team], lane, cal);
+    if (b >= 0 && wid == 0) {
       const int page0 = c.table[(long long)b * c.table_stride];
-      const bool page0_ok = page0 >= 0 && page0 < c.num_pages;
-      if (!page0_ok && crank == 0 && threadIdx.x == 0 && status) atomicOr(status, B200KV_S_BAD_PAGE);
-      if (crank == 0 && threadIdx.x < kD && page0_ok)
-        c.k_cal[cal_offset(c, page0, h) + threadIdx.x] = cal_s[threadIdx.x];
-      float cal[4];
-      load4_f32(cal_s, lane, cal);
-      auto quantize_row = [&](int t, uint2 raw, int page) {
-        float x[4];
-        unpack4(raw, x);
+      if (page0 >= 0 && page0 < c.num_pages)
+        *reinterpret_cast<float4*>(c.k_cal + cal_offset(c, page0, h) + 4 * lane) = make_float4(cal[0], cal[1], cal[2], cal[3]);
+      else if (lane == 0 && status) atomicOr(status, B200KV_S_BAD_PAGE);
+    }
+    auto quantize_row = [&](int t, uint2 r, int page) {
+      float x[4];
+      unpack4(r, x);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) x[j] = __fdiv_rn(x[j], cal[j]);
-        const int pos = t - s0;  // first chunk: the entry's cached length is zero
-        if (page < 0 || page >= c.num_pages) {
-          if (lane == 0 && status) atomicOr(status, page == -2 ? B200KV_S_BAD_POSITION : B200KV_S_BAD_PAGE);
-          return;
-        }
-        int slot_unused, prow;
-        split_pos(c, pos, slot_unused, prow);
-        quantize_store(x, c.k + code_offset(c, page, h, prow), c.k_scale + scale_offset(c, page, h, prow), lane);
-      };
-#pragma unroll
-      for (int i = 0; i < kKeepRows; ++i) {
-        const int t = s0 + wid + i * nw;
-        if (t < s1) quantize_row(t, keep[i], keep_page[i]);
+      for (int j = 0; j < 4; ++j) x[j] = __fdiv_rn(x[j], cal[j]);
+      const int pos = t - s0;  // first chunk: the entry's cached length is zero
+      if (page < 0 || page >= c.num_pages) {
+        if (lane == 0 && status) atomicOr(status, page == -2 ? B200KV_S_BAD_POSITION : B200KV_S_BAD_PAGE);
+        return;
       }
-      for (int t = s0 + wid + kKeepRows * nw; t < s1; t += nw) {
+      int slot_unused, prow;
+      split_pos(c, pos, slot_unused, prow);
+      quantize_store(x, c.k + code_offset(c, page, h, prow), c.k_scale + scale_offset(c, page, h, prow), lane);
+    };
+#pragma unroll 1
+    for (int i = 0, t = s0 + wid; t < s1; ++i, t += nw) {
+      if (i < kKeepRows) {
+        quantize_row(t, keep[warp][i][lane], __shfl_sync(0xffffffffu, pages, i));
+      } else {
         int slot, prow_unused;
         split_pos(c, t - s0, slot, prow_unused);
         quantize_row(t, *reinterpret_cast<const uint2*>(kcol + (long long)t * (int)k_sn),
                      slot < c.max_pages ? c.table[(long long)b * c.table_stride + slot] : -2);
       }
-      __syncthreads();  // part / cal_s are reused by the next entry
     }
+    __syncthreads();  // part / cal_s are reused by the next entries
   }
 }
 

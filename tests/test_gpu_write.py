@@ -209,6 +209,37 @@ def test_prefill_write_groups_of_heads(K, hq, hkv, per_warp, fused):
     assert K.check_status() == 0
 
 
+@pytest.mark.parametrize("portions", [2, 5, 8, 9, 16, 37])
+def test_first_portions_side_by_side(K, portions):
+    """Several first portions per cluster, which its warps then do in two or four teams, some in a second round, beside a decoding
+    entry and portions that continue; with 37 also more entries than one look at their lengths covers."""
+    rng = np.random.default_rng(300 + portions)
+    P = 16
+    chunk, cached = [1], [9]
+    for i in range(portions):
+        chunk.append(int(rng.integers(1, 90)) if i else 600)  # one with more rows than a quarter of a cluster keeps in registers
+        cached.append(0)
+        if i % 3 == 1:
+            chunk.append(int(rng.integers(1, 20)))
+            cached.append(int(rng.integers(1, 40)))
+    chunk.append(0)
+    cached.append(0)
+    N, B = sum(chunk), len(chunk)
+    cached = np.array(cached, np.int32)
+    cu = np.concatenate([[0], np.cumsum(chunk)]).astype(np.int32)
+    k, v = (H.randn_bf16(rng, N, HKV, D) for _ in range(2))
+    lens = [max(int(c + n), 1) for c, n in zip(cached, chunk)]
+    num_pages = sum((n + P - 1) // P for n in lens) + 3
+    table = H.random_block_table(rng, lens, P, num_pages)
+    cache = H.random_filled_cache(rng, num_pages, P)
+    cache.k_calibration[...] = (0.5 + 2 * rng.random(cache.k_calibration.shape)).astype(np.float32)
+    dev_cache = H.cache_to_torch(cache)
+    O.quantize_prefill(k, v, cu, table, cached, 1, cache)
+    K.quantize_kv_prefill(H.bf16_tensor(k), H.bf16_tensor(v), H.i32(cu), H.i32(table), H.i32(cached), H.i32([1]), dev_cache)
+    H.assert_cache_equal(H.cache_to_numpy(dev_cache), cache, f"{portions} portions ")
+    assert K.check_status() == 0
+
+
 def test_quantizer_known_answers(K):
     """Hand-made rows through the decode write's V branch (no norm/rope): all zeros -> scale
     1e-6/127 and zero codes; +-absmax -> +-127 (never -128); exact .5 ties round to even."""
