@@ -144,6 +144,29 @@ __device__ __forceinline__ float t5_exp2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
   return y;
 }
+// Two 32-bit numbers in one register pair.
+typedef unsigned long long t5_pair;
+__device__ __forceinline__ t5_pair t5_two(float a, float b) {
+  t5_pair r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void t5_split(t5_pair p, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p)); }
+__device__ __forceinline__ t5_pair t5_fma2(t5_pair a, t5_pair b, t5_pair c) {
+  t5_pair r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ t5_pair t5_add2(t5_pair a, t5_pair b) {
+  t5_pair r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float t5_max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
 __device__ __forceinline__ uint32_t t5_pack_bf16x2(float lo, float hi) {
   uint32_t r;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(r) : "f"(hi), "f"(lo));
@@ -181,6 +204,15 @@ struct T5Paged {
   DecAttnOpt opt;
 };
 
+// With more CTAs of one head and tile than multiprocessors, the CTAs of tiles with few keys do two heads each, one a warpgroup: what
+// comes in front of and behind a CTA's products (Q, the first tiles, the last P V, the merge of the warpgroups, which falls away)
+// is as long as its products then, and is there once instead of twice.  16 heads in bf16, us per pass with the row writes: five portions
+// of 1000 rows 34.9 -> 25.0, and on 2000 cached keys 53.3 -> 37.0; two portions on 4000 114 -> 90.  With
+// tiles of up to 6 blocks only that second one took 53.4, with 10 41.1 and with 16 as long, and the first 27.9 and 28.7 (before the loops
+// behind the products were rolled up).
+constexpr int kT5Sms = 148;
+constexpr int kT5PairBlocks = 10;
+
 template <bool kPaged, int kKeyBlocks = 2, bool kOptions = false>  // kKeyBlocks: 64-channel blocks of a key (2 covers up to 128 channels)
 __global__ void __launch_bounds__(kT5Threads, 1)
 prefill_attn_tc5_kernel(const uint16_t* __restrict__ q, long long q_sn, long long q_sh, const uint16_t* __restrict__ k,
@@ -203,10 +235,11 @@ prefill_attn_tc5_kernel(const uint16_t* __restrict__ q, long long q_sn, long lon
   if ((blockIdx.x | blockIdx.y) == 0) pdl_wait();
   // heads run fastest in the grid: the caller's real tiles come first in tile_start, so every CTA with work
   // is dispatched before the idle ones behind them
-  const int tile = blockIdx.y / subs, sub = blockIdx.y - tile * subs;
+  const int tile = blockIdx.y / subs, sub = blockIdx.y - tile * subs, Hq = gridDim.x;
+  // the last tile with which every CTA of one head and tile has a multiprocessor of its own (the real tiles come first)
+  const int full = kT5Sms / Hq / subs, past = full * subs < (int)gridDim.y ? tile_start[full] : -1;
   const int tile_row = tile_start[tile];
   if (tile_row < 0 || tile_row >= N) return;
-  const int hq = blockIdx.x, hk = hq / G;
   const int seq = seq_ids[tile_row];
   // a step in which no entry has a cached prefix may pass empty prefix tensors (no storage: NULL pointers)
   const int prefix_start = kPaged ? 0 : cu_cached[seq], prefix_len = (!kPaged && k_prefix && v_prefix) ? cu_cached[seq + 1] - prefix_start : 0;
@@ -222,14 +255,22 @@ prefill_attn_tc5_kernel(const uint16_t* __restrict__ q, long long q_sn, long lon
   // blocks in front of every row's window
   const int skipped = kOptions && pg.opt.window > 0 ? max(0, cached + row0 - seq_start - pg.opt.window + 1) / kT5Keys : 0;
   const int nb = nb_pre + nb_own - skipped;
+  // Each warpgroup a head of its own (pair), or both the keys of one?
+  const bool pair = past >= 0 && past < N && nb <= kT5PairBlocks;
+  if (pair && 2 * (int)blockIdx.x >= Hq) return;
+  auto head = [&](int w) { return pair ? min(2 * (int)blockIdx.x + w, Hq - 1) : (int)blockIdx.x; };
 
   float m_ref_keep = -INFINITY, l_keep = 0.f;
   // roles: warps 0-3 and 4-7 = softmax warpgroups 0 and 1, warps 8 and 9 = issue the products of warpgroup 0
   // and 1, warps 10 and 11 = fetch the K and V tiles of warpgroup 0 and 1
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wg = tid >> 7, wt = tid & 127;
-  const int n_blk[2] = {(nb + 1) >> 1, nb >> 1};  // warpgroup w owns blocks w, w + 2, ...
+  // warpgroup w owns blocks w, w + 2, ..., or all of its own head (one head too few: none)
+  auto n_blk = [&](int w) { return pair ? (2 * (int)blockIdx.x + w < Hq ? nb : 0) : (nb + 1 - w) >> 1; };
+  auto block_of = [&](int w, int h) { return pair ? h : w + 2 * h; };
+  const int ring = pair ? 2 : 3;  // slots of a ring; a pair has a second Q tile where the third ones were
   const uint32_t base = (t5_smem_u32(t5_raw) + 1023u) & ~1023u;
-  const uint32_t sQ = base;
+  auto q_tile = [&](int w) { return base + (pair ? w * kT5QBytes : 0u); };
+  const uint32_t rings = base + (pair ? 2 * kT5QBytes : kT5QBytes);
   const uint32_t bars = base + kT5QBytes + 2 * kT5WgBytes;
   // per warpgroup w, 18 barriers at bars + 144 w:
   //   s_done[2]  S buffer b holds a complete S (arrival = tcgen05.commit)
@@ -239,8 +280,8 @@ prefill_attn_tc5_kernel(const uint16_t* __restrict__ q, long long q_sn, long lon
   //   kfull[3], vfull[3]    ring slot holds its tile (one arrival by the fetching warp, plus the tile's bytes
   //                         when it is a tensor-map copy)
   //   kempty[3], vempty[3]  the product that read the slot is complete (tcgen05.commit)
-  auto ring_k = [&](int w) { return base + kT5QBytes + w * kT5WgBytes; };
-  auto ring_v = [&](int w) { return ring_k(w) + 3 * kT5KvBytes; };
+  auto ring_k = [&](int w) { return rings + w * 2 * ring * kT5KvBytes; };
+  auto ring_v = [&](int w) { return ring_k(w) + ring * kT5KvBytes; };
   auto bar_s = [&](int w, int buf) { return bars + 144 * w + 8 * buf; };
   auto bar_o = [&](int w, int which) { return bars + 144 * w + 16 + 8 * which; };
   auto bar_r = [&](int w, int buf) { return bars + 144 * w + 32 + 8 * buf; };
@@ -273,8 +314,16 @@ prefill_attn_tc5_kernel(const uint16_t* __restrict__ q, long long q_sn, long lon
     // The softmax threads copy the Q tile while the fetching warps already stream K and V.  Q rows past the end
     // of the packed batch are zero-filled; rows of other entries inside the tile are read and computed but
     // never stored.
-    t5_load_tile<256, kT5Tile>(sQ, q + (long long)row0 * q_sn + hq * q_sh, q_sn, min(kT5Tile, N - row0), tid,
-                                   kPaged ? pg.c.k_row / 8 : 16);
+    // a pair's warpgroups bring a tile each, others one half of the same
+    const int half = pair ? 0 : wg * (kT5Tile / 2), rows = min(kT5Tile, N - row0), cols = kPaged ? pg.c.k_row / 8 : 16;
+    const uint16_t* src = q + (long long)row0 * q_sn + head(wg) * q_sh;
+    const int col = wt & 15;
+    const uint32_t to = q_tile(wg) + (col >> 3) * (kT5Tile * 128);
+#pragma unroll 8
+    for (int r = half + (wt >> 4); r < half + (pair ? kT5Tile : kT5Tile / 2); r += 8) {
+      const bool valid = r < rows && col < cols;
+      t5_cp16(to + r * 128 + (((col & 7) ^ (r & 7)) << 4), valid ? src + r * q_sn + col * 8 : src, valid ? 16 : 0);
+    }
     t5_commit_group();
     t5_wait_group<0>();
     t5_fence_async_smem();
@@ -283,12 +332,12 @@ prefill_attn_tc5_kernel(const uint16_t* __restrict__ q, long long q_sn, long lon
 
   if (warp >= 10) {
     // ---- a fetching warp: streams the K and V tiles of warpgroup w into its rings.  Block h of the warpgroup
-    // is block w + 2h of the tile and lives in slot h % 3.  Full tiles come by tensor-map copies started by
+    // is block w + 2h (of a pair: h) of the tile and lives in slot h % ring.  Full tiles come by tensor-map copies started by
     // lane 0 (two boxes of 64 rows x 64 channels, swizzled by the copy engine into the layout described
     // above).  A prefix block that is not full is copied by the warp's 32 lanes with cp.async instead, because
     // the rows behind a prefix may be uninitialised memory and have to be zero in shared memory (0 x NaN would
     // poison O); so is every prefix block when the caller gave no row capacity for the prefix tensors.
-    const int w = warp - 10, n = n_blk[w];
+    const int w = warp - 10, n = n_blk(w), hk = head(w) / G;
     const uint16_t* kpre = k_prefix + hk * p_sh + (long long)prefix_start * p_sn;
     const uint16_t* vpre = v_prefix + hk * p_sh + (long long)prefix_start * p_sn;
     const uint16_t* kown = k + (long long)seq_start * k_sn + hk * k_sh;
@@ -313,7 +362,7 @@ prefill_attn_tc5_kernel(const uint16_t* __restrict__ q, long long q_sn, long lon
         for (int x = 0; x < 4; ++x) { v_ph[x] = k_ph[x]; v_row[x] = k_row[x]; }
         if (step < n) {
           if (((step << lg) & 31) == 0) {
-            const int box = (step << lg) + lane, j = (w + 2 * (box >> lg) + skipped) * kT5Keys + (box & (boxes - 1)) * R;
+            const int box = (step << lg) + lane, j = (block_of(w, box >> lg) + skipped) * kT5Keys + (box & (boxes - 1)) * R;
             const int col = j / pg.c.P;
             int page = 0;
             if (j < own_keys) {
@@ -332,10 +381,10 @@ prefill_attn_tc5_kernel(const uint16_t* __restrict__ q, long long q_sn, long lon
             k_ph[x] = __shfl_sync(0xffffffffu, my_ph, ((step << lg) + x) & 31);
             k_row[x] = __shfl_sync(0xffffffffu, my_row, ((step << lg) + x) & 31);
           }
-          if (step >= 3 && !t5_mbar_wait(bar_ke(w, k_sl), k_par, spin)) { live = false; break; }
+          if (step >= ring && !t5_mbar_wait(bar_ke(w, k_sl), k_par, spin)) { live = false; break; }
           if (lane == 0) {
             // keys behind the last one may be anything: their scores are never looked at
-            const int count = min(kT5Keys, own_keys - (w + 2 * step + skipped) * kT5Keys);
+            const int count = min(kT5Keys, own_keys - (block_of(w, step) + skipped) * kT5Keys);
             const int some = count == kT5Keys ? boxes : (count + R - 1) / R;
             const uint32_t dst = ring_k(w) + k_sl * kT5KvBytes, full = bar_kf(w, k_sl);
             t5_mbar_expect_tx(full, (uint32_t)(some * R * 128 * kKeyBlocks));
@@ -350,9 +399,9 @@ prefill_attn_tc5_kernel(const uint16_t* __restrict__ q, long long q_sn, long lon
           __syncwarp();
         }
         if (step > 0) {
-          const int j0 = (w + 2 * (step - 1) + skipped) * kT5Keys, count = min(kT5Keys, own_keys - j0);
+          const int j0 = (block_of(w, step - 1) + skipped) * kT5Keys, count = min(kT5Keys, own_keys - j0);
           const uint32_t dst = ring_v(w) + v_sl * kT5KvBytes, full = bar_vf(w, v_sl);
-          if (step > 3 && !t5_mbar_wait(bar_ve(w, v_sl), v_par, spin)) { live = false; break; }
+          if (step > ring && !t5_mbar_wait(bar_ve(w, v_sl), v_par, spin)) { live = false; break; }
           if (count == kT5Keys) {
             if (lane == 0) {
               t5_mbar_expect_tx(full, (uint32_t)(kT5Keys * 128 * v_blocks));
@@ -364,15 +413,20 @@ prefill_attn_tc5_kernel(const uint16_t* __restrict__ q, long long q_sn, long lon
               }
             }
           } else {  // values behind the last key must be zero in shared memory (0 x NaN would poison O)
-            const int cols = pg.c.v_row / 8;
-            for (int i = lane; i < kT5Keys * 16; i += 32) {
-              const int r = i >> 4, col = i & 15, x = r / R;
-              const bool valid = r < count && col < cols;
-              const int ph = x == 0 ? v_ph[0] : (x == 1 ? v_ph[1] : (x == 2 ? v_ph[2] : v_ph[3]));
-              const int row = x == 0 ? v_row[0] : (x == 1 ? v_row[1] : (x == 2 ? v_row[2] : v_row[3]));
-              const uint16_t* src = (const uint16_t*)pg.c.v;
-              if (valid) src += ((long long)ph * pg.c.P + row + r - x * R) * pg.c.v_row + col * 8;
-              t5_cp16(dst + (col >> 3) * (kT5Keys * 128) + r * 128 + (((col & 7) ^ (r & 7)) << 4), src, valid ? 16 : 0);
+            // (a lane keeps its 16-byte column and takes every other row; this ends nearly every tile)
+            const int col = lane & 15;
+            const bool some = col < pg.c.v_row / 8;
+            const uint32_t to = dst + (col >> 3) * (kT5Keys * 128);
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+              if (x >= boxes) break;
+              const uint16_t* src = (const uint16_t*)pg.c.v + ((long long)v_ph[x] * pg.c.P + v_row[x] + (lane >> 4)) * pg.c.v_row + (some ? col * 8 : 0);
+#pragma unroll 4
+              for (int r = x * R + (lane >> 4); r < (x + 1) * R; r += 2) {
+                const bool valid = some && r < count;
+                t5_cp16(to + r * 128 + (((col & 7) ^ (r & 7)) << 4), valid ? src : (const uint16_t*)pg.c.v, valid ? 16 : 0);
+                src += 2 * pg.c.v_row;
+              }
             }
             t5_commit_group();
             t5_wait_group<0>();
@@ -384,14 +438,14 @@ prefill_attn_tc5_kernel(const uint16_t* __restrict__ q, long long q_sn, long lon
         }
         v_sl = k_sl;
         v_par = k_par;
-        if (++k_sl == 3) {
+        if (++k_sl == ring) {
           k_sl = 0;
           k_par ^= 1;
         }
       }
     } else {
-      for (int h = 0; h < n && live; ++h) {
-        const int kb = w + 2 * h, sl = h % 3;
+      for (int h = 0, sl = 0, par = 1; h < n && live; ++h) {
+        const int kb = block_of(w, h);
         const bool pre = kb < nb_pre;
         const int j0 = pre ? kb * kT5Keys : (kb - nb_pre) * kT5Keys;
         const int count = min(kT5Keys, (pre ? prefix_len : own_keys) - j0);
@@ -400,8 +454,8 @@ prefill_attn_tc5_kernel(const uint16_t* __restrict__ q, long long q_sn, long lon
         for (int is_v = 0; is_v < 2 && live; ++is_v) {
           const uint32_t dst = (is_v ? ring_v(w) : ring_k(w)) + sl * kT5KvBytes;
           const uint32_t full = is_v ? bar_vf(w, sl) : bar_kf(w, sl), empty = is_v ? bar_ve(w, sl) : bar_ke(w, sl);
-          // the product that read this slot three blocks ago has completed
-          if (h >= 3 && !t5_mbar_wait(empty, (h / 3 - 1) & 1, spin)) { live = false; break; }
+          // the product that read this slot a ring of blocks ago has completed
+          if (h >= ring && !t5_mbar_wait(empty, par, spin)) { live = false; break; }
           if (tma) {
             if (lane == 0) {
               t5_mbar_expect_tx(full, kT5KvBytes);
@@ -420,6 +474,10 @@ prefill_attn_tc5_kernel(const uint16_t* __restrict__ q, long long q_sn, long lon
             if (lane == 0) t5_mbar_arrive(full);
           }
         }
+        if (++sl == ring) {
+          sl = 0;
+          par ^= 1;
+        }
       }
     }
     if (!live && lane == 0) t5_sts_u32(dead_flag, 1);
@@ -429,15 +487,20 @@ prefill_attn_tc5_kernel(const uint16_t* __restrict__ q, long long q_sn, long lon
     // queue is full, and this lane's waits and commits are not hidden behind its own products; with one
     // issuing lane per warpgroup the bookkeeping of one overlaps the products of the other.
     if (lane == 0 && !idle_issuers) {
-      const int w = warp - 8, n = n_blk[w];
-      const uint64_t dq = t5_desc(sQ, 16, 1024), dk = t5_desc(ring_k(w), 16, 1024);
+      const int w = warp - 8, n = n_blk(w);
+      const uint64_t dq = t5_desc(q_tile(w), 16, 1024), dk = t5_desc(ring_k(w), 16, 1024);
       const uint64_t dv = t5_desc(ring_v(w), kT5Keys * 128, 1024);
       const uint32_t tw = tmem + 256 * w;
       const uint32_t idesc_pv = kPaged ? t5_idesc((uint32_t)((vdim + 15) / 16 * 16)) | (1u << 16) : kT5IdescPV;
       bool live = t5_mbar_wait(bar_q, 0, spin);
-      auto issue_s = [&](int h) {  // S(h) = Q K(h)^T into S buffer h & 1, then the arrivals
-        const int sl = h % 3;
-        if (!t5_mbar_wait(bar_kf(w, sl), (h / 3) & 1, spin)) { live = false; return; }
+      int k_sl = 0, k_par = 0;
+      auto issue_s = [&](int h) {  // S(h) = Q K(h)^T into S buffer h & 1, then the arrivals; called for h = 0, 1, ...
+        const int sl = k_sl;
+        if (!t5_mbar_wait(bar_kf(w, sl), k_par, spin)) { live = false; return; }
+        if (++k_sl == ring) {
+          k_sl = 0;
+          k_par ^= 1;
+        }
         const uint64_t kd = dk + (uint64_t)(sl * (kT5KvBytes >> 4));
         const uint32_t d = tw + 64 * (h & 1);
 #pragma unroll
@@ -449,10 +512,9 @@ prefill_attn_tc5_kernel(const uint16_t* __restrict__ q, long long q_sn, long lon
       };
       for (int h = 0; h < 2; ++h)
         if (h < n && live) issue_s(h);
-      for (int h = 0; h < n && live; ++h) {
-        const int sl = h % 3;
+      for (int h = 0, sl = 0, par = 0; h < n && live; ++h) {
         // P(h) is stored and V(h) has landed
-        if (!t5_mbar_wait(bar_r(w, h & 1), (h >> 1) & 1, spin) || !t5_mbar_wait(bar_vf(w, sl), (h / 3) & 1, spin)) {
+        if (!t5_mbar_wait(bar_r(w, h & 1), (h >> 1) & 1, spin) || !t5_mbar_wait(bar_vf(w, sl), par, spin)) {
           live = false;
           break;
         }
@@ -464,11 +526,15 @@ prefill_attn_tc5_kernel(const uint16_t* __restrict__ q, long long q_sn, long lon
         t5_mma_commit(bar_ve(w, sl));
         if (h + 2 < n) issue_s(h + 2);  // executes behind P V(h): it overwrites the columns P(h) is read from
         else t5_mma_commit(bar_o(w, h + 1 < n ? 0 : 1));  // the last-but-one / the last P V of the warpgroup
+        if (++sl == ring) {
+          sl = 0;
+          par ^= 1;
+        }
       }
       if (!live) t5_sts_u32(dead_flag, 1);
     }
   } else {
-    const int n_mine = n_blk[wg];
+    const int n_mine = n_blk(wg);
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t tS = tmem + 256 * wg + lane_base, tO = tS + 128;  // this thread's lane
     const int my_keys = min(own_keys, cached + row0 + wt - seq_start + 1);  // own-chunk keys this row may see
@@ -480,8 +546,8 @@ prefill_attn_tc5_kernel(const uint16_t* __restrict__ q, long long q_sn, long lon
         my_first = cached + row0 + wt - seq_start - pg.opt.window + 1;
         last_first = cached + cta_last - seq_start - pg.opt.window + 1;
       }
-      if (pg.opt.sink && wg == 0) {
-        m_ref = pg.opt.sink[hq] * 1.4426950408889634f;
+      if (pg.opt.sink && (wg == 0 || pair)) {
+        m_ref = pg.opt.sink[head(wg)] * 1.4426950408889634f;
         l = 1.f;
       }
     }
@@ -490,7 +556,7 @@ prefill_attn_tc5_kernel(const uint16_t* __restrict__ q, long long q_sn, long lon
       ok = t5_mbar_wait(bar_s(wg, h & 1), (h >> 1) & 1, spin);  // S(h) is complete
       t5_fence_after();
       // ---- softmax of this thread's row
-      const int kb = wg + 2 * h;
+      const int kb = block_of(wg, h);
       const bool pre = kb < nb_pre;
       const int j0 = pre ? kb * kT5Keys : (kb - nb_pre + skipped) * kT5Keys;
       const int lim = (pre ? prefix_len : my_keys) - j0;                // keys [0, lim) visible to this row
@@ -502,7 +568,7 @@ prefill_attn_tc5_kernel(const uint16_t* __restrict__ q, long long q_sn, long lon
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};  // four chains instead of one of 64
       if (full) {
 #pragma unroll
-        for (int c = 0; c < 64; ++c) mx4[c & 3] = fmaxf(mx4[c & 3], __uint_as_float(u[c]));
+        for (int c = 0; c < 64; c += 2) mx4[(c >> 1) & 3] = t5_max3(mx4[(c >> 1) & 3], __uint_as_float(u[c]), __uint_as_float(u[c + 1]));
       } else {
 #pragma unroll
         for (int c = 0; c < 64; ++c) mx4[c & 3] = fmaxf(mx4[c & 3], c < lim && (!kOptions || c >= low) ? __uint_as_float(u[c]) : -INFINITY);
@@ -518,7 +584,7 @@ prefill_attn_tc5_kernel(const uint16_t* __restrict__ q, long long q_sn, long lon
           // at the top of the next block is harmless.
           ok = ok && (h + 1 < n_mine ? t5_mbar_wait(bar_s(wg, (h + 1) & 1), ((h + 1) >> 1) & 1, spin) : t5_mbar_wait(bar_o(wg, 0), 0, spin));
           t5_fence_after();
-#pragma unroll
+#pragma unroll 1  // here and below: code that runs once or twice has to be fetched, which is what a short tile waits for
           for (int c = 0; c < 4; ++c) {
             if (kPaged && 32 * c >= vdim) break;
             uint32_t w[32];
@@ -532,14 +598,20 @@ prefill_attn_tc5_kernel(const uint16_t* __restrict__ q, long long q_sn, long lon
       const float off = m_ref == -INFINITY ? 0.f : m_ref;  // kernels.py:1062
       float ps4[4] = {0.f, 0.f, 0.f, 0.f};
       uint32_t pk[32];
-      if (full) {
+      if (full) {  // two scores per instruction where there is one for it: what paces a block is its warps' instructions
+        const t5_pair scale2 = t5_two(scale_log2, scale_log2), off2 = t5_two(-off, -off);
+        t5_pair sum2[2] = {t5_two(0.f, 0.f), t5_two(0.f, 0.f)};
 #pragma unroll
         for (int c = 0; c < 32; ++c) {
-          const float p0 = t5_exp2(fmaf(__uint_as_float(u[2 * c]), scale_log2, -off));
-          const float p1 = t5_exp2(fmaf(__uint_as_float(u[2 * c + 1]), scale_log2, -off));
-          ps4[c & 3] += p0 + p1;
+          float p0, p1;
+          t5_split(t5_fma2(t5_two(__uint_as_float(u[2 * c]), __uint_as_float(u[2 * c + 1])), scale2, off2), p0, p1);
+          p0 = t5_exp2(p0);
+          p1 = t5_exp2(p1);
+          sum2[c & 1] = t5_add2(sum2[c & 1], t5_two(p0, p1));
           pk[c] = t5_pack_bf16x2(p0, p1);
         }
+        t5_split(sum2[0], ps4[0], ps4[1]);
+        t5_split(sum2[1], ps4[2], ps4[3]);
       } else {
 #pragma unroll
         for (int c = 0; c < 32; ++c) {
@@ -563,21 +635,21 @@ prefill_attn_tc5_kernel(const uint16_t* __restrict__ q, long long q_sn, long lon
     l_keep = l;
   }
 
-  // ---- merge the two warpgroups: warpgroup 1 hands its (offset, sum, O) over through shared memory
+  // ---- merge the two warpgroups (a pair has nothing to merge): warpgroup 1 hands its (offset, sum, O) over through shared memory
   // (the first 64 KB of its rings, [channel][row] fp32 so that both sides touch consecutive banks)
-  const uint32_t xO = base + kT5QBytes + kT5WgBytes, xML = base + kT5QBytes;  // scalars: start of warpgroup 0's rings
+  const uint32_t xO = base + kT5QBytes + kT5WgBytes, xML = base + kT5QBytes;  // (unless a pair) scalars: start of warpgroup 0's rings
   const uint32_t tO = tmem + 256 * (wg & 1) + 128 + ((uint32_t)(((tid >> 5) & 3) * 32) << 16);
   const int my_row = row0 + wt;
   t5_fence_before();
   __syncthreads();  // every product of the CTA is complete (or given up), nobody uses the rings any more
   t5_fence_after();
   dead = t5_lds_u32(dead_flag) != 0;
-  if (wg == 1) {
-#pragma unroll
+  if (wg == 1 && !pair) {
+#pragma unroll 1
     for (int c = 0; c < 4; ++c) {
       if (kPaged && 32 * c >= vdim) break;
       uint32_t w[32];
-      if (n_blk[1] > 0 && !dead) {
+      if (n_blk(1) > 0 && !dead) {
         t5_ld32(tO + 32 * c, w);
       } else {
 #pragma unroll
@@ -590,9 +662,10 @@ prefill_attn_tc5_kernel(const uint16_t* __restrict__ q, long long q_sn, long lon
     t5_sts_u32(xML + 512 + wt * 4, __float_as_uint(l_keep));
   }
   __syncthreads();
-  if (wg == 0) {
+  if (wg == 0 || (pair && wg == 1 && n_blk(1) > 0)) {
+    const int hq = head(wg);
     const float m0 = m_ref_keep, l0 = l_keep;
-    const float m1 = __uint_as_float(t5_lds_u32(xML + wt * 4)), l1 = __uint_as_float(t5_lds_u32(xML + 512 + wt * 4));
+    const float m1 = pair ? -INFINITY : __uint_as_float(t5_lds_u32(xML + wt * 4)), l1 = pair ? 0.f : __uint_as_float(t5_lds_u32(xML + 512 + wt * 4));
     if (dead && wt == 0 && status) atomicOr(status, B200KV_S_TIMEOUT);
     if (!dead) {
       const float mm = fmaxf(m0, m1);
@@ -602,15 +675,18 @@ prefill_attn_tc5_kernel(const uint16_t* __restrict__ q, long long q_sn, long lon
       if constexpr (kOptions) inv *= my_row < row_end ? pg.opt.factor<uint16_t>(my_row, hq) : 0.f;
       const float f0 = a0 * inv, f1 = a1 * inv;
       uint4* dst = reinterpret_cast<uint4*>(out + (long long)my_row * o_sn + hq * o_sh);
-#pragma unroll
+#pragma unroll 1
       for (int c = 0; c < 4; ++c) {
         if (kPaged && 32 * c >= vdim) break;
         uint32_t w[32];
         t5_ld32(tO + 32 * c, w);
         float o[32];
 #pragma unroll
-        for (int e = 0; e < 32; ++e)
-          o[e] = __uint_as_float(w[e]) * f0 + __uint_as_float(t5_lds_u32(xO + ((32 * c + e) * 128 + wt) * 4)) * f1;
+        for (int e = 0; e < 32; ++e) {
+          uint32_t x = 0u;
+          if (!pair) x = t5_lds_u32(xO + ((32 * c + e) * 128 + wt) * 4);
+          o[e] = __uint_as_float(w[e]) * f0 + __uint_as_float(x) * f1;
+        }
         if (kPaged && vdim % 8 != 0) {
           if (my_row < row_end) {
             uint16_t* p = out + (long long)my_row * o_sn + hq * o_sh + 32 * c;

@@ -221,6 +221,34 @@ def test_attention_rows_in_tiles(heads, kv, dim, vdim, dtype):
     H.status_clear()
 
 
+@pytest.mark.parametrize("heads,kv,dim,vdim,window", [(16, 8, 128, 128, 0), (15, 5, 64, 48, 0), (15, 3, 48, 40, 100)])
+@pytest.mark.parametrize("entries", [[(0, 1), (0, 1200)], [(0, 700), (200, 129), (40, 515)], [(0, 65)] * 20, [(700, 40)] * 12])
+def test_prompt_attention_of_many_tiles(heads, kv, dim, vdim, window, entries):
+    """More tiles and heads than multiprocessors: two heads a block where a tile has few keys, also an odd number of heads, beside tiles with more."""
+    from inference_engine_b200 import ops
+
+    g = np.random.default_rng(heads + len(entries))
+    rows, table, pages, _ = make_rows(entries, 16)
+    cache = ops.make_paged_kv(pages, kv, 16, dim, vdim, torch.bfloat16, DEV)
+    cache.k.fill_(float("nan"))
+    cache.v.fill_(float("nan"))
+    n = rows.num_rows
+    q, want, at = H.bf16(g.standard_normal((n, heads, dim))), np.zeros((n, heads, vdim)), 0
+    for b, (c, x) in enumerate(entries):
+        k, v = H.bf16(g.standard_normal((c + x, kv, dim))), H.bf16(g.standard_normal((c + x, kv, vdim)))
+        fill(cache, table, b, t(k, torch.bfloat16), t(v, torch.bfloat16))
+        for i in range(x):  # keys in the row's window
+            lo = max(0, c + i - window + 1) if window else 0
+            want[at + i : at + i + 1] = R.causal_attention(q[at + i : at + i + 1], k[lo : c + i + 1], v[lo : c + i + 1], dim ** -0.5, c + i - lo)
+        at += x
+    qd = torch.zeros(n, heads, cache.k.shape[3], device=DEV, dtype=torch.bfloat16)
+    qd[..., :dim] = t(q, torch.bfloat16)
+    out = torch.empty(n, heads, vdim, device=DEV, dtype=torch.bfloat16)
+    ops.paged_prefill_attention(qd, cache, rows, dim ** -0.5, out, ops.AttnOptions(window=window) if window else None)
+    close(out, want, torch.bfloat16)
+    H.status_clear()
+
+
 @pytest.mark.parametrize("heads,kv,dim,vdim", [(2, 1, 64, 48), (4, 2, 128, 128)])
 @pytest.mark.parametrize("page,prior,new,window", [(16, 950, 70, 0), (16, 970, 70, 0), (16, 2041, 70, 0), (48, 1000, 133, 0), (32, 2000, 101, 0), (64, 4015, 70, 0),
                                                    (64, 4090, 70, 0), (16, 2500, 70, 1200), (32, 4500, 33, 2100), (64, 5000, 200, 4200)])
