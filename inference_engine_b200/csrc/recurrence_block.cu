@@ -27,18 +27,17 @@ __host__ __device__ constexpr int rb_floats(int Dp) { return 3 * kRbTok * Dp + D
 __device__ __forceinline__ int rb_first(const b200dec_entries& ent, int e) { return ent.cu_seqlens[e] / kRbTok + e; }
 
 // ---------------------------------------------------------------- prepare
-constexpr int kRpThreads = 128;
-constexpr int kRpSums = 96;  // A (28), B (36), squares of q and of k (8 each), padded for the exchange
+constexpr int kRpSums = 80;  // A (28), B (36), squares of q and of k (8 each)
 
 __host__ __device__ constexpr int rp_a(int i, int j) { return i * (i - 1) / 2 + j; }       // j < i
 __host__ __device__ constexpr int rp_b(int i, int j) { return 28 + i * (i + 1) / 2 + j; }  // j <= i
 constexpr int kRpQ = 64, kRpK = 72;
 
-// Sums of 96 values over the warp's lanes; every lane keeps three.
-__device__ __forceinline__ void rp_exchange(float (&v)[kRpSums], int lane) {
-  int n = kRpSums / 2;
+// Sums of 16 values over 16 lanes, of which lane l keeps the l-th.
+__device__ __forceinline__ float rp_exchange(float (&v)[16], int lane) {
+  int n = 8;
 #pragma unroll
-  for (int bit = 16; bit > 0; bit >>= 1) {
+  for (int bit = 8; bit > 0; bit >>= 1) {
     const bool hi = lane & bit;
 #pragma unroll
     for (int i = 0; i < n; ++i) {
@@ -47,16 +46,25 @@ __device__ __forceinline__ void rp_exchange(float (&v)[kRpSums], int lane) {
     }
     n >>= 1;
   }
+  return v[0];
 }
 
-template <typename T, bool kOne>  // kOne: dim <= kRpThreads, a thread's channel stays in registers
-__global__ void __launch_bounds__(kRpThreads)
+// Two mappings of the threads: a key channel of all or half of the eight tokens each (kParts 1, 2), and, for the sums over the channels, 16 or
+// 32 lanes per token j, which find the products of token j with every later one in a handful of registers.  With all 64 sums of its
+// channel in one thread's registers three blocks fitted a multiprocessor, and a warp spent a third of its instructions exchanging them: 1000
+// rows of 16 heads of 128 27.0 -> 20.0 us.  Twice the threads shorten the chain where all blocks are at work at once (50 rows) and are
+// slower where they are not (23.5).
+template <typename T, int Dp, int kParts>
+__global__ void __launch_bounds__(128 * kParts)
 rb_prepare_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, const T* __restrict__ conv, int conv_stride,
-                  const b200dec_entries ent, float* __restrict__ ws, int Dp, int32_t* status) {
-  __shared__ float red[kRpThreads / 32][kRpSums];
+                  const b200dec_entries ent, float* __restrict__ ws, int32_t* status) {
+  constexpr int kChannels = 128, kRpHalf = kRbTok / kParts, kLanes = 16 * kParts;
+  constexpr bool kOne = Dp <= kChannels;  // a thread's channel stays in registers
+  __shared__ float2 kq[kRbTok][Dp];  // k, q
+  __shared__ float decay[kRbTok][Dp];
   __shared__ float sums[kRpSums], beta[kRbTok], fq[kRbTok], fk[kRbTok];
   pdl_enter();
-  const int s = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
+  const int s = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
   int lo = 0, hi = ent.num_entries;
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
@@ -73,13 +81,15 @@ rb_prepare_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, 
   const T* steps = (const T*)in.step + row0 * in.step_stride + h * D;
   const T* src = conv + row0 * conv_stride + hq * D;
   if (tid < kRbTok) beta[tid] = tid < nt ? sigmoid_f(ld_elem((const T*)in.beta + (row0 + tid) * in.beta_stride + h)) : 0.f;
-  float q[kRbTok], k[kRbTok], g[kRbTok];
+  const int half = tid / kChannels, i0 = half * kRpHalf;  // this thread's tokens: kRpHalf from i0 on
+  float q[kRpHalf], k[kRpHalf], g[kRpHalf];
   auto load = [&](int d) {
     const float bias = d < D ? rec.dt_bias[h * D + d] : 0.f;
-    const T *pq = src + rec.off_q + d, *pk = src + rec.off_k + d, *ps = steps + d;
+    const T *pq = src + i0 * (long long)conv_stride + rec.off_q + d, *pk = src + i0 * (long long)conv_stride + rec.off_k + d,
+            *ps = steps + i0 * (long long)in.step_stride + d;
 #pragma unroll
-    for (int i = 0; i < kRbTok; ++i) {
-      const bool some = i < nt && d < D;
+    for (int i = 0; i < kRpHalf; ++i) {
+      const bool some = i0 + i < nt && d < D;
       q[i] = some ? ld_elem(pq) : 0.f;
       k[i] = some ? ld_elem(pk) : 0.f;
       g[i] = some ? ld_elem(ps) + bias : 0.f;
@@ -88,35 +98,59 @@ rb_prepare_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, 
       ps += in.step_stride;
     }
 #pragma unroll
-    for (int i = 0; i < kRbTok; ++i) g[i] = i < nt && d < D ? expf(na * softplus_f(g[i])) : 1.f;
+    for (int i = 0; i < kRpHalf; ++i) g[i] = i0 + i < nt && d < D ? expf(na * softplus_f(g[i])) : 1.f;
   };
-  float v[kRpSums];
-#pragma unroll
-  for (int i = 0; i < kRpSums; ++i) v[i] = 0.f;
-  for (int d = tid; d < Dp; d += kRpThreads) {
+  for (int d = tid % kChannels; d < Dp; d += kChannels) {
     load(d);
 #pragma unroll
-    for (int j = 0; j < kRbTok; ++j) {
-      float f = k[j];  // k_j times the decays since
-      v[rp_b(j, j)] = fmaf(q[j], f, v[rp_b(j, j)]);
-      v[kRpQ + j] = fmaf(q[j], q[j], v[kRpQ + j]);
-      v[kRpK + j] = fmaf(f, f, v[kRpK + j]);
-#pragma unroll
-      for (int i = j + 1; i < kRbTok; ++i) {
-        f *= g[i];
-        v[rp_a(i, j)] = fmaf(k[i], f, v[rp_a(i, j)]);
-        v[rp_b(i, j)] = fmaf(q[i], f, v[rp_b(i, j)]);
-      }
+    for (int i = 0; i < kRpHalf; ++i) {
+      kq[i0 + i][d] = make_float2(k[i], q[i]);
+      decay[i0 + i][d] = g[i];
     }
   }
-  rp_exchange(v, lane);
-  {
-    const int at = ((lane >> 4) & 1) * 48 + ((lane >> 3) & 1) * 24 + ((lane >> 2) & 1) * 12 + ((lane >> 1) & 1) * 6 + (lane & 1) * 3;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) red[tid >> 5][at + i] = v[i];
-  }
   __syncthreads();
-  if (tid < kRpSums) sums[tid] = (red[0][tid] + red[1][tid]) + (red[2][tid] + red[3][tid]);
+  {
+    const int j = tid / kLanes, l = tid % kLanes;
+    float v[16], nk = 0.f, nq = 0.f;  // A of tokens 0 to 7 with j, B
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = 0.f;
+    for (int d = l; d < Dp; d += kLanes) {
+      float2 x[kRbTok];
+      float g8[kRbTok];
+#pragma unroll
+      for (int i = 0; i < kRbTok; ++i) {
+        x[i] = kq[i][d];
+        g8[i] = decay[i][d];
+      }
+      float f = 0.f;  // k_j times the decays since
+#pragma unroll
+      for (int i = 0; i < kRbTok; ++i) {
+        if (i < j) continue;
+        if (i == j) {
+          f = x[i].x;
+          nk = fmaf(x[i].x, x[i].x, nk);
+          nq = fmaf(x[i].y, x[i].y, nq);
+        } else {
+          f *= g8[i];
+          v[i] = fmaf(x[i].x, f, v[i]);
+        }
+        v[8 + i] = fmaf(x[i].y, f, v[8 + i]);
+      }
+    }
+    float mine = rp_exchange(v, l);
+#pragma unroll
+    for (int o = kLanes / 2; o > 0; o >>= 1) {
+      nk += __shfl_xor_sync(0xffffffffu, nk, o);
+      nq += __shfl_xor_sync(0xffffffffu, nq, o);
+    }
+    if (kParts == 2) mine += __shfl_xor_sync(0xffffffffu, mine, 16);
+    const int i = l & 7;
+    if (l < 8 ? i > j : (l < 16 && i >= j)) sums[l < 8 ? rp_a(i, j) : rp_b(i, j)] = mine;
+    if (l == 0) {
+      sums[kRpQ + j] = nq;
+      sums[kRpK + j] = nk;
+    }
+  }
   __syncthreads();
   if (tid < kRbTok) {
     fq[tid] = rec.q_scale * (rec.unit_norm ? 1.0f / sqrtf(sums[kRpQ + tid] + rec.unit_eps) : 1.f);
@@ -125,20 +159,27 @@ rb_prepare_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, 
   __syncthreads();
   float* dst = ws + ((long long)s * rec.heads + h) * rb_floats(Dp);
   float* tb = dst + 3 * kRbTok * Dp + Dp;
-  for (int d = tid; d < Dp; d += kRpThreads) {
+  for (int d = tid % kChannels; d < Dp; d += kChannels) {
     if (!kOne) load(d);
-    float f = 1.f;
+    float f = 1.f, rest = 1.f;  // the decays up to here, and those of the other half's tokens, if they come later
+    if (kParts == 2) {
 #pragma unroll
-    for (int i = 0; i < kRbTok; ++i) {
-      f *= g[i];
-      dst[i * Dp + d] = k[i] * fk[i] * f;
-      dst[(kRbTok + i) * Dp + d] = q[i] * fq[i] * f;
+      for (int i = 0; i < kRpHalf; ++i) {
+        const float other = decay[kRpHalf - i0 + i][d];
+        if (half) f *= other; else rest *= other;
+      }
     }
-    dst[3 * kRbTok * Dp + d] = f;
-    f = 1.f;
 #pragma unroll
-    for (int i = kRbTok - 1; i >= 0; --i) {
-      dst[(2 * kRbTok + i) * Dp + d] = k[i] * fk[i] * f;
+    for (int i = 0; i < kRpHalf; ++i) {
+      f *= g[i];
+      dst[(i0 + i) * Dp + d] = k[i] * fk[i0 + i] * f;
+      dst[(kRbTok + i0 + i) * Dp + d] = q[i] * fq[i0 + i] * f;
+    }
+    if (half == kParts - 1) dst[3 * kRbTok * Dp + d] = f;
+    f = rest;
+#pragma unroll
+    for (int i = kRpHalf - 1; i >= 0; --i) {
+      dst[(2 * kRbTok + i0 + i) * Dp + d] = k[i] * fk[i0 + i] * f;
       f *= g[i];
     }
   }
@@ -152,7 +193,7 @@ rb_prepare_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, 
       c[i] = beta[i] * a;
       tb[i * kRbTok + tid] = c[i];
     }
-  } else if (tid >= 64) {
+  } else if (tid >= 64 && tid < 128) {
     const int i = (tid - 64) / kRbTok, j = tid % kRbTok;
     tb[kRbTok * kRbTok + tid - 64] = j <= i ? sums[28 + i * (i + 1) / 2 + j] * fq[i] * fk[j] : 0.f;
   }
@@ -400,9 +441,9 @@ static int rb_launch(const b200dec_recurrence& rec, const b200dec_recurrence_in&
   constexpr int Dp = kLanes * kR, kCols = kRbWarps * 32 / kLanes * kRbCols;
   const int stride = (rec.channels + 7) / 8 * 8, slabs = (rec.vdim + kCols - 1) / kCols;
   const int list = ent.num_rows / kRbTok + ent.num_entries;
-  auto* prepare = rec.dim <= kRpThreads ? rb_prepare_kernel<T, true> : rb_prepare_kernel<T, false>;
-  const int rc = launch_result(launch_chained(prepare, dim3(list, rec.heads), dim3(kRpThreads), 0, s, rec, in, (const T*)conv, stride, ent, ws, Dp,
-                                              status));
+  const bool few = (long long)list * rec.heads <= 148 * 4;  // blocks of 256 threads in one round
+  const int rc = launch_result(launch_chained(few ? rb_prepare_kernel<T, Dp, 2> : rb_prepare_kernel<T, Dp, 1>, dim3(list, rec.heads),
+                                              dim3(few ? 256 : 128), 0, s, rec, in, (const T*)conv, stride, ent, ws, status));
   if (rc != B200KV_OK) return rc;
   const size_t smem = (size_t)kRbStages * rb_floats(Dp) * 4;
   if (cudaFuncSetAttribute(rb_scan_kernel<T, kLanes, kR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
