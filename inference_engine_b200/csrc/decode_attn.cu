@@ -55,9 +55,15 @@ constexpr int kMaxB = 1 << 20;
 static_assert((kStages & (kStages - 1)) == 0, "ring indices are masked");
 
 struct Partition {
-  int U;        // total tiles over all (entry, head)
+  int U;        // total tiles over all (entry, head), with the padding of an aligned split
   int per;      // tiles per worker
   int W;        // workers (warps in the grid)
+  int aligned;  // every (entry, head) starts at a CTA's first warp: its tiles are padded to whole CTAs, T -> padded(T)
+  __host__ __device__ __forceinline__ int padded(int T) const {
+    const int span = kWarps * per;
+    if (!aligned) return T;
+    return T <= span ? (T > 0 ? span : 0) : (T + span - 1) / span * span;
+  }
 };
 
 // ------------------------------------------------------------------ small PTX wrappers
@@ -128,55 +134,6 @@ struct Lens {
   __device__ __forceinline__ int tiles(int b) const { return (n(b) + kTile - 1) / kTile; }
 };
 
-// Tiles per kv head of entries [0,B), scanned by the whole CTA.  Thread i owns the `chunk`
-// consecutive entries starting at i*chunk; chunk_prefix[i] (shared, blockDim.x+1 ints) is the
-// number of tiles before that chunk, chunk_prefix[blockDim.x] the total; lens_s receives the
-// token counts of the first kSmemLens entries.  The loads of cached_lens do not wait for
-// num_decoding (it only masks them).  When `gprefix` is given (one CTA does this) the per-entry
-// exclusive prefix [B+1] is also written to global memory for the separate reduction kernel.
-__device__ void scan_tiles(const int32_t* __restrict__ cached_lens, int B, const int32_t* __restrict__ num_decoding,
-                           int chunk, int* chunk_prefix, int* lens_s, int* __restrict__ gprefix, int& nd_out) {
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const int lo = min(tid * chunk, B), hi = min(lo + chunk, B);
-  const int nd_raw = *num_decoding;
-  int first = lo < hi ? cached_lens[lo] : 0;  // issued together with the load above
-  const int nd = min(nd_raw, B);
-  int sum = 0;
-  for (int b = lo; b < hi; ++b) {
-    const int cl = b == lo ? first : cached_lens[b];
-    const int n = b < nd ? cl + 1 : 0;
-    if (b < kSmemLens) lens_s[b] = n;
-    sum += (n + kTile - 1) / kTile;
-  }
-  chunk_prefix[tid] = sum;
-  __syncthreads();
-  if (tid < 32) {  // exclusive scan of the nt chunk sums by one warp
-    int carry = 0;
-    for (int base = 0; base < nt; base += 32) {
-      int v = (base + tid < nt) ? chunk_prefix[base + tid] : 0;
-      int incl = v;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        int y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (tid >= o) incl += y;
-      }
-      if (base + tid < nt) chunk_prefix[base + tid] = carry + incl - v;
-      carry += __shfl_sync(0xffffffffu, incl, 31);
-    }
-    if (tid == 0) chunk_prefix[nt] = carry;
-  }
-  __syncthreads();
-  if (gprefix) {
-    int run = chunk_prefix[tid];
-    for (int b = lo; b < hi; ++b) {
-      gprefix[b] = run;
-      run += (b < nd ? (cached_lens[b] + 1 + kTile - 1) / kTile : 0);
-    }
-    if (tid == 0) gprefix[B] = chunk_prefix[nt];
-  }
-  nd_out = nd;
-}
-
 // `per` = tiles per warp.  Never below the even share; the floor below it trades parallelism against
 // hand-offs: a piece that goes through the workspace costs about as much as 8 tiles of work, but the four pieces
 // of a CTA that covers exactly one (entry, head) meet in shared memory and cost nothing of the kind.  So short
@@ -186,10 +143,30 @@ __device__ void scan_tiles(const int32_t* __restrict__ cached_lens, int B, const
 // instead of 10.3 us for one 128-token sequence).  With other lengths the heads straddle CTAs and their pieces go through the workspace.  When the quarters would not fit the grid, short sequences use pieces of 8 tiles
 // (a whole sequence per warp, or exactly a CTA of 4 x 8); longer ones pieces of 4 (64 tokens, the reference's
 // MIN_PIECE, kernels.py:295).
-__host__ __device__ __forceinline__ Partition make_partition(int total_tiles_one_head, int Hkv, int W, int num_entries) {
+//
+// A hand-off through the workspace (counter, merge by the last arriver) is a chain of about kHandOffTiles tiles' length at the
+// end of a call, kHandOffTilesBusy where the multiprocessors hold more than half of the CTAs they can.  Where no (entry, head) is so
+// long that one CTA's share of it outlasts that, each gets whole CTAs (`aligned`): the pieces of one CTA meet in shared memory and
+// nothing is handed off; and where one CTA is too few, all of an (entry, head)'s pieces come from whole CTAs.  U is then settled by the
+// scan of the padded tiles.  Flat and aligned, two layers of 8 kv heads with the row writes, us: one entry of 300 tokens 34.9 and 26.7, of 1500 36.0
+// and 30.7; eight of 100 to 400 36.9 and 28.8; three of 40 to 900 36.0 and 28.7; four of 512 32.8 and 28.8; sixteen of 300 39.0 and 30.8.
+// may_align = 0: the reduction is the separate kernel, which knows the flat split only.
+constexpr int kHandOffTiles = 4, kHandOffTilesBusy = 6;
+constexpr int kMinPiece = 4;
+
+__host__ __device__ __forceinline__ Partition make_partition(int total_tiles_one_head, int most_tiles, int Hkv, int W, int num_entries,
+                                                             int may_align) {
   Partition p;
   p.U = total_tiles_one_head * Hkv;
   p.W = W;
+  const int ctas = W / kWarps, pairs = num_entries * Hkv;
+  const bool fits = may_align && num_entries > 0 && pairs <= ctas;
+  const int alone = (most_tiles + kWarps - 1) / kWarps;  // one CTA per (entry, head)
+  const int hand_off = 2 * pairs * kCtasPerSm <= ctas ? kHandOffTiles : kHandOffTilesBusy;
+  p.per = alone;
+  p.aligned = 1;
+  if (fits && alone <= 2 + hand_off) return p;  // (the others are at least 2)
+  p.aligned = 0;
   const int share = (p.U + W - 1) / W;
   int min_tiles = 4;
   if (num_entries > 0 && total_tiles_one_head <= 32 * num_entries) {
@@ -198,15 +175,122 @@ __host__ __device__ __forceinline__ Partition make_partition(int total_tiles_one
     min_tiles = share <= quarter ? quarter : 8;
   }
   p.per = share > min_tiles ? share : min_tiles;
+  if (!fits) return p;
+  // Several: at most as many for each as leave a CTA for all, or as few tiles a warp as do (their number is at most pairs + all
+  // tiles / the tiles of a CTA); but no more than eight, which are merged in one round of loads, while that is less than kMinPiece.
+  const int each = kWarps * (ctas / pairs), rest = kWarps * (ctas - pairs);
+  int some = (most_tiles + each - 1) / each;
+  if (rest > 0 && (p.U + rest - 1) / rest < some) some = (p.U + rest - 1) / rest;
+  const int round = (most_tiles + 8 * kWarps - 1) / (8 * kWarps);
+  some = max(max(some, 2), min(round, kMinPiece));
+  if (alone <= min(some, p.per) + hand_off) {
+    p.per = alone;
+    p.aligned = 1;
+  } else if (some <= p.per + p.per / 8) {
+    p.per = some;
+    p.aligned = 1;
+  }
   return p;
 }
+
+// At most one (entry, head) per multiprocessor: above that even shares keep the grid busy and hand-offs are hidden behind other
+// CTAs' tiles, while the longer code of an aligned split costs its fetch (nineteen entries of 512: the same either way).
+__host__ __device__ __forceinline__ bool few_pairs(long long B, int Hkv, int sm_count) { return B * Hkv <= sm_count; }
+
+__host__ __device__ constexpr int scan_ints(int threads) { return threads + 1 + 2 * (threads / 32); }  // shared: prefix, warps' sums and maxima
+
+// The split of entries [0,B), found by the whole CTA.  Thread i owns the `chunk` consecutive entries starting at i*chunk;
+// chunk_prefix (shared, scan_ints(blockDim.x) ints) gets the number of tiles per kv head before each of the `nchunks`
+// chunks, padded ones in an aligned split, and their total behind them; lens_s the token counts of the first kSmemLens
+// entries.  The loads of cached_lens do not wait for num_decoding (it only masks them).  When `gprefix` is given (one
+// CTA does this) the per-entry exclusive prefix [B+1] is also written to global memory for the separate reduction kernel.
+template <int kThreads, bool kAlign>
+__device__ __forceinline__ Partition split_batch(const int32_t* __restrict__ cached_lens, int B, const int32_t* __restrict__ num_decoding, int Hkv, int W, int chunk,
+                                                 int nchunks, int* chunk_prefix, int* lens_s, int* __restrict__ gprefix, int& nd_out) {
+  const int tid = threadIdx.x;
+  const int lo = min(tid * chunk, B), hi = min(lo + chunk, B);
+  const int nd_raw = *num_decoding;
+  const int first = lo < hi ? cached_lens[lo] : 0;  // issued together with the load above
+  const int nd = min(nd_raw, B);
+  int sum = 0, most = 0;
+#pragma unroll 1
+  for (int b = lo; b < hi; ++b) {
+    const int cl = b == lo ? first : cached_lens[b];
+    const int n = b < nd ? cl + 1 : 0;
+    if (b < kSmemLens) lens_s[b] = n;
+    const int T = (n + kTile - 1) / kTile;
+    sum += T;
+    most = max(most, T);
+  }
+  Partition part;
+  if constexpr (kAlign) {  // the padding has to be known before anything is added up in order
+    int* totals = chunk_prefix + kThreads + 1;
+    const int all = __reduce_add_sync(0xffffffffu, sum);
+    most = __reduce_max_sync(0xffffffffu, most);
+    if ((tid & 31) == 0) {
+      totals[tid >> 5] = all;
+      totals[kThreads / 32 + (tid >> 5)] = most;
+    }
+    __syncthreads();
+    int total = 0;
+    most = 0;
+#pragma unroll
+    for (int i = 0; i < kThreads / 32; ++i) {
+      total += totals[i];
+      most = max(most, totals[kThreads / 32 + i]);
+    }
+    part = make_partition(total, most, Hkv, W, nd, 1);
+    if (part.aligned) {
+      sum = 0;
+#pragma unroll 1
+      for (int b = lo; b < hi; ++b) sum += part.padded(((b < nd ? (b == lo ? first : cached_lens[b]) + 1 : 0) + kTile - 1) / kTile);
+    }
+  }
+  chunk_prefix[tid] = sum;
+  __syncthreads();
+  if (tid < 32) {  // exclusive scan of the chunks' sums by one warp
+    int carry = 0;
+#pragma unroll 1
+    for (int base = 0; base < nchunks; base += 32) {
+      int v = (base + tid < nchunks) ? chunk_prefix[base + tid] : 0;
+      int incl = v;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (tid >= o) incl += y;
+      }
+      if (base + tid < nchunks) chunk_prefix[base + tid] = carry + incl - v;
+      carry += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (tid == 0) chunk_prefix[nchunks] = carry;
+  }
+  __syncthreads();
+  if (gprefix) {
+    int run = lo < hi ? chunk_prefix[tid] : 0;
+    for (int b = lo; b < hi; ++b) {
+      gprefix[b] = run;
+      run += (b < nd ? (cached_lens[b] + 1 + kTile - 1) / kTile : 0);
+    }
+    if (tid == 0) gprefix[B] = chunk_prefix[nchunks];
+  }
+  if constexpr (!kAlign) {
+    part = make_partition(chunk_prefix[nchunks], 0, Hkv, W, nd, 0);
+    part.aligned = 0;
+  } else if (part.aligned) {
+    part.U = Hkv * chunk_prefix[nchunks];
+  }
+  nd_out = nd;
+  return part;
+}
+// Chunks that hold an entry, at least one.
+__device__ __forceinline__ int chunks_of(int B, int chunk) { return max(1, (B + chunk - 1) / chunk); }
 
 // Position in the flattened (entry, head, tile) list.  (slot, row0) locate the tile in the
 // entry's page table (table column and first row inside that page); they advance incrementally
 // so the hot loop never divides.
 struct Cursor {
-  int b, h, tile, T, n, slot, row0, base;  // base: flat index of (entry b, head 0, tile 0)
-  __device__ __forceinline__ void seek(const int* chunk_prefix, int nchunks, int chunk, const Lens& lens, int Hkv,
+  int b, h, tile, T, n, slot, row0, base;  // base: flat index of (entry b, head 0, tile 0), with the padding of an aligned split
+  __device__ __forceinline__ void seek(const int* chunk_prefix, int nchunks, int chunk, const Lens& lens, const Partition& part, int Hkv,
                                        int page_size, int u) {
     int lo = 0, hi = nchunks;  // largest chunk whose first flat index is <= u
     while (hi - lo > 1) {
@@ -215,17 +299,19 @@ struct Cursor {
     }
     b = lo * chunk;
     int run = chunk_prefix[lo];
+    int Tp;
     while (true) {
       T = lens.tiles(b);
-      if (Hkv * (run + T) > u) break;
-      run += T;
+      Tp = part.padded(T);
+      if (Hkv * (run + Tp) > u) break;
+      run += Tp;
       ++b;
     }
     n = lens.n(b);
     base = Hkv * run;
     int r = u - base;
-    h = r / T;
-    tile = r - h * T;
+    h = r / Tp;
+    tile = r - h * Tp;  // aligned: perhaps behind the last one
     slot = (tile * kTile) / page_size;
     row0 = tile * kTile - slot * page_size;
   }
@@ -711,6 +797,8 @@ struct Pieces {
       n = w_last - w_first + 1;
     }
   }
+  // An aligned split: one piece per CTA.
+  __device__ __forceinline__ Pieces(int first_warp, int ctas) : w_first(first_warp), n_a(0), w_b(first_warp), n_b(ctas), w_c(first_warp), n(ctas), slot_first(0) {}
   // workspace slot index (2 * warp + slot) of piece k
   __device__ __forceinline__ int slot_of(int k) const {
     const int w = k < n_a ? w_first + k : (k < n_a + n_b ? w_b + kWarps * (k - n_a) : w_c + (k - n_a - n_b));
@@ -839,59 +927,62 @@ __host__ __device__ inline size_t ws_ml_bytes(int W, int G) { return (((size_t)W
 // before its first copies are in flight, instead of the length scan, a binary search and a dependent
 // page-table read in each of its CTAs in each layer.
 constexpr int kPlanMagic = 0x6b765031;  // "kvP1"
-constexpr int kPlanHeaderInts = 8;      // magic, B, Hkv, W, U, per, num_decoding, page_size
-constexpr int kPlanEntryInts = 16;      // b, h, tile, T, n, base, page[0..2], reserved
+constexpr int kPlanHeaderInts = 8;      // magic, B, Hkv, W, U, per (negative: aligned), num_decoding, page_size
+constexpr int kPlanEntryInts = 16;      // b, h, tile, T, n, base, page[0..2]; aligned: CTAs of the (entry, head), which of them; reserved
 // One warp of the persistent grid per thread, over several blocks that each repeat the (short) scan: a single block of
 // 1024 threads spent its time in a 32-step scan by one warp and in the issue slots of one multiprocessor (64 entries of
 // 4096: 14.4 us, now 4.3).
 constexpr int kPlanThreads = 256;
 __host__ __device__ inline size_t plan_bytes(int W) { return ((size_t)kPlanHeaderInts + (size_t)W * kPlanEntryInts) * 4; }
 
+template <bool kAlign>
 __global__ void __launch_bounds__(kPlanThreads)
 decode_plan_kernel(const int32_t* __restrict__ cached_lens, const int32_t* __restrict__ num_decoding,
                    const int32_t* __restrict__ table, int table_stride, int max_pages, int page_size, int B, int Hkv,
                    int W, int* __restrict__ plan) {
-  __shared__ int chunk_prefix[kPlanThreads + 1];
+  __shared__ int chunk_prefix[scan_ints(kPlanThreads)];
   __shared__ int lens_s[kSmemLens];
   // No early trigger here: a kernel chained behind this one is only brought up when every thread of this
   // grid has exited, i.e. after the fence below, so it may read the plan before its own wait.
   pdl_wait();
-  const int chunk = (B + kPlanThreads - 1) / kPlanThreads;
+  const int chunk = (B + kPlanThreads - 1) / kPlanThreads, nchunks = chunks_of(B, chunk);
   int nd;
-  scan_tiles(cached_lens, B, num_decoding, chunk, chunk_prefix, lens_s, nullptr, nd);
+  const Partition part = split_batch<kPlanThreads, kAlign>(cached_lens, B, num_decoding, Hkv, W, chunk, nchunks, chunk_prefix, lens_s, nullptr, nd);
   const Lens lens{cached_lens, lens_s, nd};
-  const Partition part = make_partition(chunk_prefix[kPlanThreads], Hkv, W, nd);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     plan[0] = kPlanMagic; plan[1] = B; plan[2] = Hkv; plan[3] = W;
-    plan[4] = part.U; plan[5] = part.per; plan[6] = nd; plan[7] = page_size;
+    plan[4] = part.U; plan[5] = part.aligned ? -part.per : part.per; plan[6] = nd; plan[7] = page_size;
   }
   const int w = blockIdx.x * kPlanThreads + threadIdx.x;
   if (w < W) {
     int* e = plan + kPlanHeaderInts + (size_t)w * kPlanEntryInts;
     const long long u_begin = (long long)w * part.per;
-    if (u_begin >= part.U) {
+    Cursor cur;
+    if (u_begin < part.U) cur.seek(chunk_prefix, nchunks, chunk, lens, part, Hkv, page_size, (int)u_begin);
+    if (u_begin >= part.U || cur.tile >= cur.T) {
       e[0] = -1;
     } else {
-      Cursor cur;
-      cur.seek(chunk_prefix, kPlanThreads, chunk, lens, Hkv, page_size, (int)u_begin);
-      int page[kStages - 1];
-      const int b0 = cur.b, h0 = cur.h, tile0 = cur.tile, T0 = cur.T, n0 = cur.n, base0 = cur.base;
-      int left = min(part.per, part.U - (int)u_begin);
-#pragma unroll
+      int2* e2 = reinterpret_cast<int2*>(e);  // plan is 16-byte aligned, header and entries are multiples of that
+      e2[0] = make_int2(cur.b, cur.h);
+      e2[1] = make_int2(cur.tile, cur.T);
+      e2[2] = make_int2(cur.n, cur.base);
+      const int T0 = cur.T, tile0 = cur.tile;
+      int left = part.aligned ? min(part.per, T0 - tile0) : min(part.per, part.U - (int)u_begin);
+      static_assert(kStages == 4, "three pages in an entry's places 6 to 8");
+#pragma unroll 1
       for (int i = 0; i < kStages - 1; ++i) {
-        page[i] = -1;
+        int page = -1;
         if (left > 0) {
-          page[i] = cur.slot < max_pages ? table[(long long)cur.b * table_stride + cur.slot] : -2;
+          page = cur.slot < max_pages ? table[(long long)cur.b * table_stride + cur.slot] : -2;
           if (--left > 0) cur.next(lens, Hkv, page_size);
         }
+        e[6 + i] = page;
       }
-      int2* e2 = reinterpret_cast<int2*>(e);  // plan is 16-byte aligned, header and entries are multiples of that
-      e2[0] = make_int2(b0, h0);
-      e2[1] = make_int2(tile0, T0);
-      e2[2] = make_int2(n0, base0);
-      static_assert(kStages == 4, "three pages in an entry's places 6 to 8");
-      e2[3] = make_int2(page[0], page[1]);
-      e[8] = page[2];
+      if (part.aligned) {
+        const int span = kWarps * part.per;
+        e[9] = (T0 + span - 1) / span;
+        e[10] = tile0 / span;
+      }
     }
   }
   __threadfence();
@@ -916,7 +1007,9 @@ __device__ __forceinline__ unsigned long long gtime() {
 #define STAMP(i, v) do { } while (0)
 #endif
 
-template <bool kScalar>
+// kAlign: the split may be an aligned one.  kPlanned: it is read from a plan (a kernel by itself, as a short call is bound by the fetch of its code:
+// 73 KB instead of 96; twelve layers of one entry of 128 tokens 110.6 -> 108.6 us).
+template <bool kScalar, bool kAlign, bool kPlanned>
 __global__ void __launch_bounds__(kWarps * 32, kCtasPerSm)
 decode_attn_kernel(const uint16_t* __restrict__ q, long long q_sb, long long q_sh, CacheView c,
                    const int32_t* __restrict__ cached_lens, const int32_t* __restrict__ num_decoding, float scale_log2,
@@ -938,31 +1031,33 @@ decode_attn_kernel(const uint16_t* __restrict__ q, long long q_sb, long long q_s
   // brought up while this kernel still streams sit on the SMs waiting and slow the streaming down (measured:
   // +16 us per call when the trigger was the first statement).
   if (blockIdx.x == 0) pdl_wait();
-  int* lens_s = chunk_prefix + kWarps * 32 + 1;
+  int* lens_s = chunk_prefix + scan_ints(kWarps * 32);
   int* cta_arrive = lens_s + kSmemLens;  // how many of this CTA's warps have parked a piece in shared memory
   if (threadIdx.x == 0) *cta_arrive = 0;  // ordered before any use by the barriers below
   int nd;
   Partition part;
   Cursor pc;  // producer position (runs kStages-1 tiles ahead of the consumer)
+  int peers = 0, mine = 0;  // aligned split: CTAs of this one's (entry, head), and which of them it is
   int first_page = -1;  // planned: lane i < kStages-1 holds the page id of the warp's i-th tile
-  if (plan != nullptr) {
+  if constexpr (kPlanned) {
     // One round of independent loads: the warp's plan entry (lanes 0-15), the header (lanes 16-23),
     // num_decoding and this thread's share of the lengths.
     int pe = 0;
     if (lane < kPlanEntryInts) pe = __ldcg(plan + kPlanHeaderInts + (size_t)w * kPlanEntryInts + lane);
     else if (lane < kPlanEntryInts + kPlanHeaderInts) pe = __ldcg(plan + (lane - kPlanEntryInts));
     const int nd_raw = __ldcg(num_decoding);
-    int cl[kSmemLens / (kWarps * 32)];
+    constexpr int kLensEach = (kSmemLens + kWarps * 32 - 1) / (kWarps * 32);
+    int cl[kLensEach];
 #pragma unroll
-    for (int i = 0; i < kSmemLens / (kWarps * 32); ++i) {
+    for (int i = 0; i < kLensEach; ++i) {
       const int b = threadIdx.x + i * kWarps * 32;
-      cl[i] = b < B ? __ldcg(cached_lens + b) : 0;
+      cl[i] = b < min(B, kSmemLens) ? __ldcg(cached_lens + b) : 0;
     }
     nd = min(nd_raw, B);
 #pragma unroll
-    for (int i = 0; i < kSmemLens / (kWarps * 32); ++i) {
+    for (int i = 0; i < kLensEach; ++i) {
       const int b = threadIdx.x + i * kWarps * 32;
-      if (b < B) lens_s[b] = b < nd ? cl[i] + 1 : 0;
+      if (b < min(B, kSmemLens)) lens_s[b] = b < nd ? cl[i] + 1 : 0;
     }
     __syncthreads();
     const bool hdr_ok = __shfl_sync(0xffffffffu, pe, 16) == kPlanMagic && __shfl_sync(0xffffffffu, pe, 17) == B &&
@@ -971,6 +1066,8 @@ decode_attn_kernel(const uint16_t* __restrict__ q, long long q_sb, long long q_s
     part.U = __shfl_sync(0xffffffffu, pe, 20);
     part.per = __shfl_sync(0xffffffffu, pe, 21);
     part.W = W;
+    part.aligned = kAlign && part.per < 0;
+    part.per = abs(part.per);
     pc.b = __shfl_sync(0xffffffffu, pe, 0);
     pc.h = __shfl_sync(0xffffffffu, pe, 1);
     pc.tile = __shfl_sync(0xffffffffu, pe, 2);
@@ -989,21 +1086,35 @@ decode_attn_kernel(const uint16_t* __restrict__ q, long long q_sb, long long q_s
       if (lane == 0 && status) atomicOr(status, B200KV_S_BAD_PLAN);
       return;
     }
+    if (kAlign && part.aligned) {
+      const int span = kWarps * part.per;
+      peers = __shfl_sync(0xffffffffu, pe, 9);
+      mine = __shfl_sync(0xffffffffu, pe, 10);
+      if (mine < 0 || mine > (int)blockIdx.x || pc.tile != mine * span + warp * part.per || (peers - 1) * span >= pc.T || pc.T > peers * span) {
+        if (lane == 0 && status) atomicOr(status, B200KV_S_BAD_PLAN);
+        return;
+      }
+    }
     pc.slot = (pc.tile * kTile) / c.page_size;
     pc.row0 = pc.tile * kTile - pc.slot * c.page_size;
   } else {
-    const int nchunks = blockDim.x, chunk = (B + nchunks - 1) / nchunks;
-    scan_tiles(cached_lens, B, num_decoding, chunk, chunk_prefix, lens_s,
-               (blockIdx.x == 0 && !fused) ? reinterpret_cast<int*>(workspace) : nullptr, nd);
-    part = make_partition(chunk_prefix[nchunks], c.Hkv, W, nd);
-    if ((long long)w * part.per >= part.U) return;
+    const int chunk = (B + kWarps * 32 - 1) / (kWarps * 32), nchunks = chunks_of(B, chunk);
+    part = split_batch<kWarps * 32, kAlign>(cached_lens, B, num_decoding, c.Hkv, W, chunk, nchunks, chunk_prefix, lens_s,
+                                    (blockIdx.x == 0 && !fused) ? reinterpret_cast<int*>(workspace) : nullptr, nd);
     const Lens probe{cached_lens, lens_s, nd};
-    pc.seek(chunk_prefix, nchunks, chunk, probe, c.Hkv, c.page_size, w * part.per);
+    if ((long long)w * part.per >= part.U) return;
+    pc.seek(chunk_prefix, nchunks, chunk, probe, part, c.Hkv, c.page_size, w * part.per);
+    if (pc.tile >= pc.T) return;  // in the padding
+    if (kAlign && part.aligned) {
+      const int span = kWarps * part.per;
+      peers = (pc.T + span - 1) / span;
+      mine = pc.tile / span;
+    }
   }
   STAMP(8, dclk());
   const Lens lens{cached_lens, lens_s, nd};
   const int u0 = w * part.per;
-  const int ntiles = min(part.per, part.U - u0);
+  const int ntiles = part.aligned ? min(part.per, pc.T - pc.tile) : min(part.per, part.U - u0);
 
   int* ws_count = reinterpret_cast<int*>(workspace + ws_prefix_bytes(B));
   float* ws_ml = reinterpret_cast<float*>(workspace + ws_head_bytes(B, c.Hkv));
@@ -1022,14 +1133,14 @@ decode_attn_kernel(const uint16_t* __restrict__ q, long long q_sb, long long q_s
   // not touched by it and are fetched right away, hiding the first burst behind that kernel.
   bool must_wait = early != 0;
   int p_left = ntiles;  // tiles not yet issued
-#pragma unroll
+#pragma unroll 1  // (code that runs once has to be fetched)
   for (int i = 0; i < kStages - 1; ++i) {
     if (p_left > 0) {
       if (must_wait && pc.tile == pc.T - 1) {
         asm volatile("griddepcontrol.wait;" ::: "memory");
         must_wait = false;
       }
-      const int page = plan != nullptr ? __shfl_sync(0xffffffffu, first_page, i) : window_page(c, pc, win, lane);
+      const int page = kPlanned ? __shfl_sync(0xffffffffu, first_page, i) : window_page(c, pc, win, lane);
       issue_tile(c, pc, page, lc, my_ring_s + i * kTileBytes, lane, status);
       if (--p_left > 0) pc.next(lens, c.Hkv, c.page_size);
     }
@@ -1037,7 +1148,7 @@ decode_attn_kernel(const uint16_t* __restrict__ q, long long q_sb, long long q_s
   }
   STAMP(2, dclk());
   // planned: the table row of the next tile is requested now and is there when the main loop wants it
-  if (plan != nullptr && p_left > 0) load_window(c, pc.b, pc.slot, win, lane);
+  if (kPlanned && p_left > 0) load_window(c, pc.b, pc.slot, win, lane);
   if (must_wait) asm volatile("griddepcontrol.wait;" ::: "memory");
 
   typename std::conditional<kScalar, ScalarState, MmaState>::type st;
@@ -1091,12 +1202,16 @@ decode_attn_kernel(const uint16_t* __restrict__ q, long long q_sb, long long q_s
     // whole iff the segment began at the sequence's first tile and reached its last one
     const bool whole = cc.tile == 0 && seg == cc.T;
     const int slot = done == 0 ? 0 : 1;
-    const int s0 = cc.base + cc.h * cc.T;  // flat tile range of this (entry, head): [s0, s0 + T)
     uint16_t* out_row = out + cc.b * o_sb + (long long)(cc.h * G) * o_sh;
-    // Do all four warps of this CTA hold pieces of this same (entry, head)?  Then the pieces meet
+    // Do all warps of this CTA that have tiles hold pieces of this same (entry, head)?  Then the pieces meet
     // in shared memory and one warp forwards their sum (no global round trip for three of them).
+    const bool aligned = kAlign && part.aligned;
+    const int s0 = aligned ? (blockIdx.x - mine) * kWarps * part.per : cc.base + cc.h * cc.T;  // flat tile range of this (entry, head): [s0, s0 + T)
     const int cta_u0 = blockIdx.x * kWarps * part.per, cta_u1 = cta_u0 + kWarps * part.per;
-    const bool cta_inside = !whole && s0 <= cta_u0 && cta_u1 <= s0 + cc.T && cta_u1 <= part.U;
+    const bool cta_inside = !whole && (aligned || (s0 <= cta_u0 && cta_u1 <= s0 + cc.T && cta_u1 <= part.U));
+    int met = kWarps;  // (in the last CTA of an aligned split only the first warps have tiles)
+    if (aligned)
+      while (s0 + cc.T <= cta_u0 + (met - 1) * part.per) --met;
     bool deliver = !whole;                       // a piece of mine (or my CTA's sum) goes to the workspace
     float* po = ws_o + ((size_t)w * 2 + slot) * G * kD;
     float* pml = ws_ml + ((size_t)w * 2 + slot) * G * 2;
@@ -1111,23 +1226,24 @@ decode_attn_kernel(const uint16_t* __restrict__ q, long long q_sb, long long q_s
       int t = 0;
       if (lane == 0) t = atomicAdd(cta_arrive, 1);
       t = __shfl_sync(0xffffffffu, t, 0);
-      deliver = t == kWarps - 1;
-      if (deliver) {  // last of the four: sum them; lane l owns channels 4l..4l+3
+      deliver = t == met - 1;
+      if (deliver) {  // last of them: sum them; lane l owns channels 4l..4l+3
         __threadfence_block();
-        const bool exact = s0 == cta_u0 && s0 + cc.T == cta_u1;  // the CTA saw the whole sequence
+        const bool exact = aligned ? peers == 1 : s0 == cta_u0 && s0 + cc.T == cta_u1;  // the CTA saw the whole sequence
         po = ws_o + ((size_t)(blockIdx.x * kWarps) * 2) * G * kD;  // slot 0 of the CTA's first warp
         pml = ws_ml + ((size_t)(blockIdx.x * kWarps) * 2) * G * 2;
         for (int col = 0; col < G; ++col) {
           float m4[kWarps], M = -INFINITY;
 #pragma unroll
           for (int i = 0; i < kWarps; ++i) {
-            m4[i] = reinterpret_cast<const float*>(ring + i * kStages * kTileBytes)[kMaxG * kD + col * 2];
+            m4[i] = i < met ? reinterpret_cast<const float*>(ring + i * kStages * kTileBytes)[kMaxG * kD + col * 2] : -INFINITY;
             M = fmaxf(M, m4[i]);
           }
           float L = 0.f;
           float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
           for (int i = 0; i < kWarps; ++i) {
+            if (i >= met) break;
             const float* sp = reinterpret_cast<const float*>(ring + i * kStages * kTileBytes);
             const float wg = fast_exp2(m4[i] - M);
             L = fmaf(sp[kMaxG * kD + col * 2 + 1], wg, L);
@@ -1157,7 +1273,7 @@ decode_attn_kernel(const uint16_t* __restrict__ q, long long q_sb, long long q_s
     if (fused && deliver) {
       // Fused cross-split reduction: the warp that delivers the last piece of (entry, head) merges
       // all of them.  Release: partial stores -> warp barrier -> counter; acquire: counter -> warp barrier -> loads.
-      const Pieces pieces(part, s0, s0 + cc.T);
+      const Pieces pieces = aligned ? Pieces(kWarps * (int)(blockIdx.x - mine), peers) : Pieces(part, s0, s0 + cc.T);
       __syncwarp();  // the lanes' partial stores are ordered before lane 0's release below
       int arrived = 0;
       if (lane == 0) arrived = atom_add_acq_rel(ws_count + cc.b * c.Hkv + cc.h, 1) + 1;
@@ -1209,7 +1325,7 @@ decode_combine_kernel(const uint8_t* __restrict__ workspace, const int32_t* __re
   const int* prefix = reinterpret_cast<const int*>(workspace);
   const int T = prefix[b + 1] - prefix[b];
   if (T == 0) return;
-  const Partition part = make_partition(prefix[B], Hkv, W, min(*num_decoding, B));
+  const Partition part = make_partition(prefix[B], 0, Hkv, W, min(*num_decoding, B), 0);
   const int s = Hkv * prefix[b] + h * T, e = s + T;
   const int w_first = s / part.per, w_last = (e - 1) / part.per;
   if (w_first == w_last) return;  // one warp saw the whole sequence and wrote the output itself
@@ -1266,11 +1382,10 @@ decode_combine_kernel(const uint8_t* __restrict__ workspace, const int32_t* __re
   }
 }
 
-static size_t main_smem_bytes(int B, bool scalar) {
+static size_t main_smem_bytes(bool scalar) {
   size_t s = (size_t)kWarps * kStages * kTileBytes;
   if (scalar) s += (size_t)kWarps * (kMaxG * kD + kMaxG * kTile) * 4;
-  s += (size_t)(kWarps * 32 + 1 + kSmemLens + 1) * 4;
-  (void)B;
+  s += (size_t)(scan_ints(kWarps * 32) + kSmemLens + 1) * 4;
   return s;
 }
 
@@ -1319,21 +1434,28 @@ static int launch_decode(const void* q, int64_t q_sb, int64_t q_sh, const b200kv
   // Only CTAs that can have work are launched.  No entry has more tiles than its table row can address; a warp takes
   // at least 4 tiles, except in a batch of short sequences (32 tiles or fewer on average, make_partition), where it
   // takes at least 2 - and such a batch has at most 32 B Hkv tiles, i.e. 4 B Hkv CTAs.
-  const long long max_tiles = (long long)B * Hkv * (((long long)table->max_pages * cache->page_size + kTile - 1) / kTile);
+  // An aligned split uses one CTA per (entry, head), or several with at least 2 tiles a warp.
+  const bool scalar = (variant & 1) != 0;
+  const int fused = (variant & 2) ? 0 : 1;
+  const bool few = fused && few_pairs(B, Hkv, sm_count);
+  const long long entry_tiles = ((long long)table->max_pages * cache->page_size + kTile - 1) / kTile, max_tiles = (long long)B * Hkv * entry_tiles;
+  const long long want_aligned = (long long)B * Hkv * ((entry_tiles + 2 * kWarps - 1) / (2 * kWarps));
   const long long want_long = (max_tiles + 4 * kWarps - 1) / (4 * kWarps);
   const long long want_short = std::min<long long>((max_tiles + 2 * kWarps - 1) / (2 * kWarps), 4LL * B * Hkv);
-  const long long want = std::max(want_long, want_short);
+  const long long want = std::max(std::max(want_long, want_short), want_aligned);
   const int grid = (int)std::max<long long>(1, std::min<long long>(sm_count * kCtasPerSm, want));
   const float scale_log2 = scale * 1.4426950408889634f;
   cudaStream_t s = (cudaStream_t)stream;
-  const bool scalar = (variant & 1) != 0;
-  const int fused = (variant & 2) ? 0 : 1;
   const int early = ((variant & 4) && fused) ? 1 : 0;  // the separate reduction kernel's prefix array is written before the wait
-  const size_t smem = main_smem_bytes(B, scalar);
+  const size_t smem = main_smem_bytes(scalar);
+  auto pick = [&](auto planned) {
+    constexpr bool kPlanned = decltype(planned)::value;
+    return few ? (scalar ? decode_attn_kernel<true, true, kPlanned> : decode_attn_kernel<false, true, kPlanned>)
+               : (scalar ? decode_attn_kernel<true, false, kPlanned> : decode_attn_kernel<false, false, kPlanned>);
+  };
+  auto* kernel = plan ? pick(std::true_type{}) : pick(std::false_type{});
   // the opt-in to more than 48 KB of dynamic shared memory is per function AND per device: set on every call
-  cudaError_t e = scalar ? cudaFuncSetAttribute(decode_attn_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                         : cudaFuncSetAttribute(decode_attn_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return B200KV_E_LAUNCH;
+  if (!allow_smem(kernel, smem)) return B200KV_E_LAUNCH;
   if (clear_bytes && cudaMemsetAsync(workspace, 0, clear_bytes, s) != cudaSuccess) return B200KV_E_LAUNCH;
   CacheView view = make_view(cache, table);
   cudaLaunchConfig_t cfg = {};
@@ -1346,8 +1468,7 @@ static int launch_decode(const void* q, int64_t q_sb, int64_t q_sh, const b200kv
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = early ? 1 : 0;
-  cudaError_t le = cudaLaunchKernelEx(&cfg, scalar ? decode_attn_kernel<true> : decode_attn_kernel<false>,
-                                      (const uint16_t*)q, (long long)q_sb, (long long)q_sh, view, cached_lens, num_decoding,
+  cudaError_t le = cudaLaunchKernelEx(&cfg, kernel, (const uint16_t*)q, (long long)q_sb, (long long)q_sh, view, cached_lens, num_decoding,
                                       scale_log2, (uint16_t*)out, (long long)o_sb, (long long)o_sh, (uint8_t*)workspace,
                                       (int)B, G, W, fused, early, (const int*)plan, status);
   if (le != cudaSuccess) return B200KV_E_LAUNCH;
@@ -1386,7 +1507,8 @@ extern "C" int b200kv_decode_plan(const b200kv_table* table, const int32_t* cach
   if (!aligned(plan, 16)) return B200KV_E_ALIGN;
   if (plan_bytes_given < b200kv_decode_plan_bytes(sm_count)) return B200KV_E_WORKSPACE;
   const int W = sm_count * kCtasPerSm * kWarps;
-  decode_plan_kernel<<<(W + kPlanThreads - 1) / kPlanThreads, kPlanThreads, 0, (cudaStream_t)stream>>>(
+  auto* kernel = few_pairs(B, Hkv, sm_count) ? decode_plan_kernel<true> : decode_plan_kernel<false>;
+  kernel<<<(W + kPlanThreads - 1) / kPlanThreads, kPlanThreads, 0, (cudaStream_t)stream>>>(
       cached_lens, num_decoding, table->ids, table->stride, table->max_pages, page_size, B, Hkv, W, (int*)plan);
   return cudaGetLastError() == cudaSuccess ? B200KV_OK : B200KV_E_LAUNCH;
 }

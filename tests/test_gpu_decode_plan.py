@@ -43,6 +43,14 @@ CASES = {
     "many short": [128] * 256,
     "ragged": [int(x) for x in np.random.default_rng(5).integers(1, 3000, 37)],
     "more entries than the shared-memory length table": [20] * 700,
+    # few (entry, head) pairs, whose split may start each at a CTA of its own: alone in it with one to four of its warps, at the line
+    # to several CTAs, several for each, the last batch that is few and the first that is not
+    "one of three tiles": [47],
+    "one of nineteen tiles": [300],
+    "alone beside short ones": [1, 64, 65, 129, 300, 511, 16],
+    "several each": [700, 40, 1500, 64, 2300],
+    "as many pairs as multiprocessors": [200 + 7 * i for i in range(18)],
+    "one entry more": [200 + 7 * i for i in range(19)],
 }
 
 
