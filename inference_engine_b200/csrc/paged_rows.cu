@@ -1023,7 +1023,7 @@ extern "C" int b200dec_rope_write(const void* qkv, int64_t qkv_stride, const b20
   };
   const bool eights = cache->k_dim % 8 == 0 && cache->v_dim % 8 == 0 && half % 8 == 0 && qkv_stride % 8 == 0 && aligned(qkv, 16) &&
                       aligned(cos_sin, 16) && cache->k_row <= 128 && cache->v_row <= 128;
-  if (eights) {
+  if (eights && rows->num_rows >= 128) {  // (fewer rows: 60 of 16 + 2 x 8 heads 4.4 us by rows, 3.8 by warps; one entry decoding 14.4 and 12.4 with its attention)
     const int lanes = cache->k_row <= 64 && cache->v_row <= 64 ? 8 : 16, per_row = heads + (write_kv ? 2 * cache->kv_heads : 0);
     const int threads = row_threads(rows->num_rows, per_row * lanes, 4);
     auto by_rows = [&](auto* kernel, auto* in, auto* q) {
