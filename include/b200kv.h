@@ -241,6 +241,17 @@ int b200kv_skinny_linear(const void* x, int64_t ldx, const void* w, int64_t ldw,
 void b200kv_set_chained_launch(int enabled);
 int b200kv_get_chained_launch(void);
 
+/* Calls that do not need one another, side by side in a graph that `stream` records: what is enqueued between _begin and
+ * _next, between one _next and another, and between the last of them and _end forms a branch each.  All start behind what the stream held
+ * before, and what follows _end waits for all.  May be nested; every _begin needs its _end, on the same thread.  Not recording (or
+ * waiting for more nodes than 16): _begin returns NULL, with which the other two do nothing, and the calls run in order.
+ * The first launch of a branch and the first behind _end are not chained.  Memory that a branch allocates in stream order must not be given back before _end. */
+void* b200kv_branches_begin(void* stream);
+int b200kv_branches_next(void* branches);
+int b200kv_branches_end(void* branches);
+/* This thread's next launch is not chained: for a library whose kernel may be the first behind branches of another one. */
+void b200kv_plain_launch(void);
+
 /* Bytes of fp32 workspace b200kv_decode_attn needs for a batch of B entries on a device with
  * `sm_count` SMs (replaces the three partial buffers of kernels.py:305-311).
  * Contract: the workspace must be ZERO-filled once when it is allocated.  It holds, besides the

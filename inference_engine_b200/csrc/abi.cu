@@ -1,15 +1,87 @@
 // Version and error-string entry points of the b200kv C ABI.
 #include "b200kv.h"
 
+#include <cuda_runtime.h>
+
 #include <atomic>
+#include <new>
 
 namespace b200kv {
 static std::atomic<int> g_chained{0};
-bool chained_launch_enabled() { return g_chained.load(std::memory_order_relaxed) != 0; }
+static thread_local bool t_plain = false;  // this thread's next launch stands behind a fork or a join of branches
+bool take_plain_launch() {
+  const bool plain = t_plain;
+  t_plain = false;
+  return plain;
+}
+static bool chained() { return g_chained.load(std::memory_order_relaxed) != 0; }
+bool take_chained_launch() { return !take_plain_launch() && chained(); }
+
+// A recording stream's place in its graph is the set of nodes that the next one will wait for.
+constexpr int kBranchNodes = 16;
+struct Branches {
+  cudaStream_t stream;
+  int num_from = 0, num_ends = 0;
+  cudaGraphNode_t from[kBranchNodes], ends[kBranchNodes];
+
+  // The stream's place: up to `room` nodes to `to`; -1: not recording, or more than that.
+  int place(cudaGraphNode_t* to, int room) {
+    cudaStreamCaptureStatus status;
+    const cudaGraphNode_t* nodes = nullptr;
+    size_t num = 0;
+    if (cudaStreamGetCaptureInfo_v2(stream, &status, nullptr, nullptr, &nodes, &num) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return -1;
+    }
+    if (status != cudaStreamCaptureStatusActive || num > (size_t)room) return -1;
+    for (size_t i = 0; i < num; ++i) to[i] = nodes[i];
+    return (int)num;
+  }
+  bool move_to(cudaGraphNode_t* nodes, int num) {
+    t_plain = true;
+    return cudaStreamUpdateCaptureDependencies(stream, nodes, num, cudaStreamSetCaptureDependencies) == cudaSuccess;
+  }
+  // The end of the branch at hand joins `ends`.
+  bool keep_end() {
+    const int n = place(ends + num_ends, kBranchNodes - num_ends);
+    if (n < 0) return false;
+    num_ends += n;
+    return true;
+  }
+};
 }  // namespace b200kv
 
+// One kernel after the other leaves the multiprocessors half empty where one is short of blocks and the next of bandwidth.
+// Branches need no second stream, whose tensors' lifetimes would have to be told to the allocator, and no events.
+extern "C" void* b200kv_branches_begin(void* stream) {
+  b200kv::Branches* b = new (std::nothrow) b200kv::Branches;
+  if (!b) return nullptr;
+  b->stream = (cudaStream_t)stream;
+  b->num_from = b->place(b->from, b200kv::kBranchNodes);
+  if (b->num_from < 0) {
+    delete b;
+    return nullptr;
+  }
+  b200kv::t_plain = true;
+  return b;
+}
+extern "C" int b200kv_branches_next(void* branches) {
+  b200kv::Branches* b = (b200kv::Branches*)branches;
+  if (!b) return B200KV_OK;
+  return b->keep_end() && b->move_to(b->from, b->num_from) ? B200KV_OK : B200KV_E_LAUNCH;
+}
+extern "C" int b200kv_branches_end(void* branches) {
+  b200kv::Branches* b = (b200kv::Branches*)branches;
+  if (!b) return B200KV_OK;
+  const bool ok = b->keep_end() && b->move_to(b->ends, b->num_ends);
+  delete b;
+  return ok ? B200KV_OK : B200KV_E_LAUNCH;
+}
+
 extern "C" void b200kv_set_chained_launch(int enabled) { b200kv::g_chained.store(enabled ? 1 : 0, std::memory_order_relaxed); }
-extern "C" int b200kv_get_chained_launch(void) { return b200kv::chained_launch_enabled() ? 1 : 0; }
+extern "C" int b200kv_get_chained_launch(void) { return b200kv::chained() ? 1 : 0; }
+
+extern "C" void b200kv_plain_launch(void) { b200kv::t_plain = true; }
 
 extern "C" int b200kv_version(void) { return B200KV_VERSION; }
 

@@ -97,6 +97,48 @@ def set_early_start(enabled: bool) -> None:
         _lib._decoder_lib.b200kv_set_chained_launch(1 if enabled else 0)
 
 
+def recording() -> bool:
+    return torch.cuda.is_current_stream_capturing()
+
+
+class Branches:
+    """Calls that do not need one another, side by side in a CUDA graph under recording():
+
+        with Branches(lib) as b:
+            ...
+            b.next()
+            ...
+
+    Both parts start behind what the current stream holds, and what comes after waits for both.  Where nothing is recorded the
+    calls run in order.  Tensors that a part allocates have to live until the end of the block: to the allocator the stream's
+    calls are ordered."""
+
+    def __init__(self, lib):
+        self.lib = lib
+
+    def __enter__(self):
+        self.handle = self.lib.b200kv_branches_begin(_stream())
+        return self
+
+    def next(self) -> None:
+        if self.handle is not None:
+            _lib.check(self.lib.b200kv_branches_next(self.handle), "branches")
+
+    def __exit__(self, kind, value, trace):
+        if self.handle is not None:
+            rc = self.lib.b200kv_branches_end(self.handle)
+            self.handle = None
+            for other in (_lib._lib, _lib._decoder_lib):
+                if other is not None:
+                    other.b200kv_plain_launch()
+            if kind is None:
+                _lib.check(rc, "branches")
+
+
+def early_start() -> bool:
+    return _early_start
+
+
 _workspaces: dict[tuple, torch.Tensor] = {}
 
 

@@ -316,9 +316,19 @@ def paged_attention(q: torch.Tensor, cache: PagedKV, rows: Rows, scale: float, o
         return attention_rows(q, cache, rows, scale, opt, out)
     if out is None:
         out = torch.empty(q.shape[0], q.shape[1], cache.v_dim, device=q.device, dtype=q.dtype)
-    if rows.seq_ids is not None:
+    if rows.seq_ids is None:
+        paged_decode_attention(q, cache, rows, scale, out, True, opt)
+        return out
+    if not K.recording():
         paged_prefill_attention(q, cache, rows, scale, out, opt)
-    paged_decode_attention(q, cache, rows, scale, out, rows.seq_ids is None, opt)
+        paged_decode_attention(q, cache, rows, scale, out, False, opt)
+        return out
+    # Rows of portions and of decoding entries: neither reads what the other writes.  us with the row writes, 16 heads in bf16: 32 entries
+    # beside 992 rows on 3072 100 -> 84, 8 beside 2 x 50 rows on 300 32.8 -> 18.7, five prompts of 1000 rows 34.9 -> 22.6.
+    with K.Branches(_lib_dec()) as both:
+        paged_prefill_attention(q, cache, rows, scale, out, opt)
+        both.next()
+        paged_decode_attention(q, cache, rows, scale, out, False, opt)
     return out
 
 

@@ -64,3 +64,48 @@ def test_argument_checks(K):
     big = torch.zeros(2, 8200, dtype=torch.bfloat16, device="cuda")
     with pytest.raises(ValueError):
         K.add_rms_norm(big, big, torch.ones(8200, dtype=torch.bfloat16, device="cuda"), 1e-6)
+
+
+@pytest.mark.parametrize("chained", [False, True])
+def test_branches_of_a_recorded_graph(K, chained):
+    """Calls side by side, one branch cut into two and one left empty: each starts behind what came before, what follows waits for all."""
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randn(3, 512, 4096, generator=g, device="cuda").to(torch.bfloat16)
+    from inference_engine_b200 import _lib
+
+    lib = _lib.load()
+
+    def call():
+        first = K.silu_mul(x[0])
+        with K.Branches(lib) as b:
+            kept = [torch.cat([first, first], dim=1)]  # what a branch allocates lives until the end
+            a = K.silu_mul(kept[0])
+            with K.Branches(lib) as c:
+                d = K.silu_mul(x[1])
+                c.next()
+                e = K.silu_mul(x[2])
+                c.next()
+            kept.append(torch.cat([d, e], dim=1))
+            f = K.silu_mul(kept[1])
+            b.next()
+            kept += [first + 1]
+            kept += [torch.cat([first, kept[2]], dim=1)]
+            h = K.silu_mul(kept[3])
+        return K.silu_mul(torch.cat([a + f, h], dim=1)), first
+
+    want = call()
+    s = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    K.set_early_start(chained)
+    try:
+        with torch.cuda.graph(graph, stream=s):
+            got = call()
+    finally:
+        K.set_early_start(False)
+    for _ in range(3):
+        graph.replay()
+        assert all(torch.equal(u, v) for u, v in zip(want, got))
+    x.mul_(0.5)
+    want = call()
+    graph.replay()
+    assert all(torch.equal(u, v) for u, v in zip(want, got))
