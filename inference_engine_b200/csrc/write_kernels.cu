@@ -466,7 +466,7 @@ prefill_rows_kernel(const uint16_t* __restrict__ q, long long q_sn, long long q_
 // another's 128 maxima through distributed shared memory between two cluster barriers, calibration =
 // max(1e-3, column max) (exact and order-independent, kernels.py:764-780) is stored by CTA 0, and every warp
 // quantizes its rows as k / calibration (kernels.py:786-811).
-constexpr int kFirstCtas = 8, kFirstWarps = 16, kFirstLanes = 4, kFirstTeams = 4, kKeepRows = 8;
+constexpr int kFirstCtas = 8, kFirstWarps = 16, kFirstLanes = 4, kFirstTeams = 4, kKeepRows = 8, kFirstFew = 192;
 // The kept rows lie in shared memory and the quantizing loop is not unrolled: two blocks share a multiprocessor without spills, and the
 // code that every call has to fetch is 27 KB instead of 69.  With the entries of a lane one after the other, 30 portions of 2000 rows in all
 // took 84 us, 59 now; 12 of 2000 65.6 and 60; one portion 7.55 and 7.4; five prompts of 1011 rows, with all else of two layers, 75.8
@@ -503,14 +503,19 @@ first_chunk_k_kernel(const uint16_t* __restrict__ k, long long k_sn, long long k
   };
   int total, unused;
   find(1 << 30, total);
-  const int mine = (total - y + kFirstLanes - 1) / kFirstLanes;  // entries of this cluster
+  // Four or more entries of few rows: as many clusters as fill their teams, and no more that a chained predecessor has to make room for.
+  // us of two chained layers with all else, four portions of 40 rows in all 38.2 -> 34.9, of 144 40.8 -> 38.6 (not chained 38.9 and 39.0); three of
+  // 144 35.0 and 39.0, four of 300 41.3 and 44.3 with the rule.
+  const bool few = N <= kFirstFew && total >= kFirstTeams;
+  const int lanes = few ? min(kFirstLanes, (total + kFirstTeams - 1) / kFirstTeams) : kFirstLanes;
+  const int mine = y < lanes ? (total - y + lanes - 1) / lanes : 0;  // entries of this cluster
   if (mine <= 0) return;
-  const int lg = mine >= 4 ? 2 : mine > 1 ? 1 : 0, teams = 1 << lg, per_team = kFirstWarps >> lg, team = warp >> (4 - lg);
+  const int lg = mine >= (few ? 3 : 4) ? 2 : mine > 1 ? 1 : 0, teams = 1 << lg, per_team = kFirstWarps >> lg, team = warp >> (4 - lg);
   static_assert(kFirstTeams == 4 && kFirstWarps == 16 && kKeepRows <= 32, "");
   const int wid = (int)crank * per_team + (warp & (per_team - 1)), nw = kFirstCtas * per_team;  // this warp among its team's
   pdl_wait();  // k comes from the kernel before this one
   for (int first = 0; first < mine; first += teams) {
-    const int b = first + team < mine ? find(y + kFirstLanes * (first + team), unused) : -1;
+    const int b = first + team < mine ? find(y + lanes * (first + team), unused) : -1;
     const int s0 = b < 0 ? 0 : cu[b], s1 = b < 0 ? 0 : min(cu[b + 1], N);
     const uint16_t* kcol = k + h * k_sh + 4 * lane;
     uint2 raw[kKeepRows];
