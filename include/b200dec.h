@@ -98,6 +98,10 @@ int b200dec_router(const float* x, const void* router_w, int32_t num_rows, int32
 int b200dec_dispatch(const void* xb, int32_t elem, const int32_t* ids, const float* scores, const int32_t* ranks, const int32_t* counts,
                      int32_t num_rows, int32_t width, int32_t experts, int32_t top, int32_t tile_rows, void* x_sorted,
                      float* score_sorted, int32_t* slots, int32_t* tiles, int32_t max_tiles, void* stream);
+/* The same for b200dec_expert_products: clears its counters, done int32 [max_tiles + 1]. */
+int b200dec_dispatch_counted(const void* xb, int32_t elem, const int32_t* ids, const float* scores, const int32_t* ranks, const int32_t* counts,
+                             int32_t num_rows, int32_t width, int32_t experts, int32_t top, int32_t tile_rows, void* x_sorted,
+                             float* score_sorted, int32_t* slots, int32_t* tiles, int32_t max_tiles, int32_t* done, void* stream);
 /* grouped product: y[row] = W_e x[row] for the rows of every tile; w [experts, out_rows, width].
  * act = 0: y [rows, out_rows].  act = 1: W_e's rows alternate gate, up; with the row's score s,
  *   g = min(s * gate . x, limit), u = clamp(s * up . x, -limit, limit), y = g * sigmoid(slope * g) * (u + 1),
@@ -106,6 +110,12 @@ int b200dec_dispatch(const void* xb, int32_t elem, const int32_t* ids, const flo
 int b200dec_grouped_linear(const void* x, const void* w, int32_t elem, const int32_t* tiles, int32_t max_tiles, int32_t tile_rows,
                            int32_t total_rows, int32_t experts, int32_t out_rows, int32_t width, const float* score_sorted,
                            int32_t act, float limit, float slope, void* y, int32_t sm_count, int32_t variant, int32_t* status, void* stream);
+/* Both products of the experts in one launch, bf16 on tcgen05: h [total_rows, ff] = the product of act = 1 with gate_up
+ * [experts, 2 * ff, width], y [total_rows, width] = that of act = 0 of h with down [experts, width, ff]; ff and width multiples of 8.
+ * done: as b200dec_dispatch_counted left it, used up by the call. */
+int b200dec_expert_products(const void* x, const void* gate_up, const void* down, const int32_t* tiles, int32_t max_tiles, int32_t tile_rows,
+                            int32_t total_rows, int32_t experts, int32_t ff, int32_t width, const float* score_sorted, float limit,
+                            float slope, void* h, void* y, int32_t* done, int32_t sm_count, int32_t* status, void* stream);
 
 /* ---- attention with a sliding window, a sink and an output gate: the three kernels above with options.
  * window > 0: the row at position i sees positions j with 0 <= i - j < window (0: all j <= i).

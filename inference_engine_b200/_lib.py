@@ -172,6 +172,10 @@ DECODER_SIGNATURES = {
                                  c_void_p]),
     "b200dec_dispatch": (c_int32, [c_void_p, c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32, c_int32, c_int32,
                                    c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_void_p]),
+    "b200dec_dispatch_counted": (c_int32, [c_void_p, c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32, c_int32,
+                                           c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_void_p, c_void_p]),
+    "b200dec_expert_products": (c_int32, [c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32, c_int32, c_int32, c_int32,
+                                          c_void_p, c_float, c_float, c_void_p, c_void_p, c_void_p, c_int32, c_void_p, c_void_p]),
     "b200dec_grouped_linear": (c_int32, [c_void_p, c_void_p, c_int32, c_void_p, c_int32, c_int32, c_int32, c_int32, c_int32, c_int32,
                                          c_void_p, c_int32, c_float, c_float, c_void_p, c_int32, c_int32, c_void_p, c_void_p]),
 }

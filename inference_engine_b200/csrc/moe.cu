@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(kDpThreads)
 dispatch_kernel(const T* __restrict__ xb, const int32_t* __restrict__ ids, const float* __restrict__ scores,
                 const int32_t* __restrict__ ranks, const int32_t* __restrict__ counts, int N, int width, int E, int top, int tile_rows,
                 T* __restrict__ x_sorted, float* __restrict__ score_sorted, int32_t* __restrict__ slots, int32_t* __restrict__ tiles,
-                int max_tiles) {
+                int max_tiles, int32_t* __restrict__ done) {
   __shared__ int first[kRtMaxExperts];
   __shared__ int red[kDpThreads / 32];
   pdl_enter();
@@ -176,10 +176,14 @@ dispatch_kernel(const T* __restrict__ xb, const int32_t* __restrict__ ids, const
         tiles[1 + 3 * t] = e;
         tiles[2 + 3 * t] = f + i * each;
         tiles[3 + 3 * t] = min(each, n - i * each);
+        if (done) done[t] = 0;
       }
     }
   }
-  if (blockIdx.x == 0 && tid == 0) tiles[0] = min(tbase, max_tiles);
+  if (blockIdx.x == 0 && tid == 0) {
+    tiles[0] = min(tbase, max_tiles);
+    if (done) done[max_tiles] = 0;
+  }
   __syncthreads();
   constexpr int kVec = 16 / sizeof(T);
   for (long long r = blockIdx.x; r < N; r += gridDim.x) {
@@ -266,6 +270,9 @@ grouped_linear_simt_kernel(const T* __restrict__ x, const T* __restrict__ w, con
 int launch_grouped_linear_tc5(const void* x, const void* w, const int32_t* tiles, int max_tiles, int tile_rows, int total_rows, int experts,
                               int out_rows, int width, const float* score_sorted, int act, float limit, float slope, void* y, int sms,
                               int32_t* status, cudaStream_t stream);
+int launch_expert_products_tc5(const void* x, const void* gate_up, const void* down, const int32_t* tiles, int max_tiles, int tile_rows,
+                               int total_rows, int experts, int ff, int width, const float* score_sorted, float limit, float slope, void* h,
+                               void* y, int32_t* done, int sms, int32_t* status, cudaStream_t stream);
 
 }  // namespace b200kv
 
@@ -304,6 +311,14 @@ extern "C" int b200dec_router(const float* x, const void* router_w, int32_t num_
 extern "C" int b200dec_dispatch(const void* xb, int32_t elem, const int32_t* ids, const float* scores, const int32_t* ranks,
                                 const int32_t* counts, int32_t num_rows, int32_t width, int32_t experts, int32_t top, int32_t tile_rows,
                                 void* x_sorted, float* score_sorted, int32_t* slots, int32_t* tiles, int32_t max_tiles, void* stream) {
+  return b200dec_dispatch_counted(xb, elem, ids, scores, ranks, counts, num_rows, width, experts, top, tile_rows, x_sorted, score_sorted, slots,
+                                  tiles, max_tiles, nullptr, stream);
+}
+
+extern "C" int b200dec_dispatch_counted(const void* xb, int32_t elem, const int32_t* ids, const float* scores, const int32_t* ranks,
+                                        const int32_t* counts, int32_t num_rows, int32_t width, int32_t experts, int32_t top,
+                                        int32_t tile_rows, void* x_sorted, float* score_sorted, int32_t* slots, int32_t* tiles,
+                                        int32_t max_tiles, int32_t* done, void* stream) {
   if (num_rows == 0) return B200KV_OK;
   if (!xb || !ids || !scores || !ranks || !counts || !x_sorted || !score_sorted || !slots || !tiles) return B200KV_E_NULL;
   if (num_rows < 0 || width < 1 || experts < 1 || experts > kRtMaxExperts || top < 1 || tile_rows < 1 || max_tiles < 1 || (elem != 2 && elem != 4))
@@ -313,9 +328,21 @@ extern "C" int b200dec_dispatch(const void* xb, int32_t elem, const int32_t* ids
   cudaStream_t s = (cudaStream_t)stream;
   if (elem == 2)
     return launch_result(launch_chained(dispatch_kernel<uint16_t>, grid, dim3(kDpThreads), 0, s, (const uint16_t*)xb, ids, scores, ranks, counts,
-                                        num_rows, width, experts, top, tile_rows, (uint16_t*)x_sorted, score_sorted, slots, tiles, max_tiles));
+                                        num_rows, width, experts, top, tile_rows, (uint16_t*)x_sorted, score_sorted, slots, tiles, max_tiles, done));
   return launch_result(launch_chained(dispatch_kernel<float>, grid, dim3(kDpThreads), 0, s, (const float*)xb, ids, scores, ranks, counts, num_rows,
-                                      width, experts, top, tile_rows, (float*)x_sorted, score_sorted, slots, tiles, max_tiles));
+                                      width, experts, top, tile_rows, (float*)x_sorted, score_sorted, slots, tiles, max_tiles, done));
+}
+
+extern "C" int b200dec_expert_products(const void* x, const void* gate_up, const void* down, const int32_t* tiles, int32_t max_tiles,
+                                       int32_t tile_rows, int32_t total_rows, int32_t experts, int32_t ff, int32_t width,
+                                       const float* score_sorted, float limit, float slope, void* h, void* y, int32_t* done, int32_t sm_count,
+                                       int32_t* status, void* stream) {
+  if (total_rows == 0) return B200KV_OK;
+  if (!x || !gate_up || !down || !tiles || !score_sorted || !h || !y || !done) return B200KV_E_NULL;
+  if (total_rows < 0 || max_tiles < 1 || tile_rows < 1 || experts < 1 || ff < 8 || ff % 8 || width < 8 || width % 8 || sm_count < 1) return B200KV_E_SHAPE;
+  if (!aligned(x, 16) || !aligned(gate_up, 16) || !aligned(down, 16) || !aligned(h, 16) || !aligned(y, 16)) return B200KV_E_ALIGN;
+  return launch_expert_products_tc5(x, gate_up, down, tiles, max_tiles, tile_rows, total_rows, experts, ff, width, score_sorted, limit, slope, h, y,
+                                    done, sm_count, status, (cudaStream_t)stream);
 }
 
 extern "C" int b200dec_grouped_linear(const void* x, const void* w, int32_t elem, const int32_t* tiles, int32_t max_tiles, int32_t tile_rows,

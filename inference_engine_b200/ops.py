@@ -369,8 +369,10 @@ def expert_tile_rows(num_rows: int, top: int, experts: int, dtype) -> int:
     weights are streamed and a narrow tile leaves shared memory for a deeper ring."""
     if dtype == torch.float32:
         return 32
-    total = num_rows * top
-    return 64 if total <= 512 or total <= 48 * experts else 256
+    # The line lies where some expert begins to have more than 64 rows, whose weights are then read twice; of many experts one does sooner.
+    # us, both products, tiles of 64 and 256: 8 experts of 3072, 2 a token, 192 rows 64.3 and 66.2 (a layer of 209 86.2 and 87.7), 224 85.8 and 66.6;
+    # a layer with 32 experts of 1536, 4 a token, 288 rows 137 and 137, 320 rows 143 and 137.5, 384 154 and 139.
+    return 64 if num_rows * top <= (52 if experts <= 16 else 39) * experts else 256
 
 
 def max_expert_tiles(total: int, experts: int, tile_rows: int) -> int:
@@ -407,16 +409,29 @@ def mixture(x: torch.Tensor, xb: torch.Tensor, ex: Experts, variant: int | None 
     max_tiles = max_expert_tiles(total, E, tile_rows)
     # separate allocations: no kernel of the chain reads a cache line that the next one's input shares
     ids, ranks, slots, scores = (torch.empty(total, dtype=torch.int32, device=dev) for _ in range(4))
-    tiles = torch.empty(1 + 3 * max_tiles, dtype=torch.int32, device=dev)
+    tiles = torch.empty(1 + 3 * max_tiles + max_tiles + 1, dtype=torch.int32, device=dev)  # and the counters of the products behind them
+    ff = ex.down.shape[2]
+    # Both products in one launch, unless the second one's items are the longer ones: as the last to be drawn they leave multiprocessors idle
+    # for longer than a start takes.  us a layer, two launches and one: 32 experts of 1536 (width 2048), 64 rows 135.3 and 123.0, 512 154.6
+    # and 145.4, 1024 175.2 and 165.7; 8 experts of 3072, 64 rows 79.5 and 82.3, 192 84.4 and 94.1, 700 106.8 and 113.8 (16 80.1 and 77.3, 1000 135 and 129).
+    both = variant is None and xb.dtype == torch.bfloat16 and W % 8 == 0 and ff % 8 == 0 and ff <= W
+    done = tiles.data_ptr() + 4 * (1 + 3 * max_tiles) if both else None
     score_sorted = torch.empty(total, dtype=torch.float32, device=dev)
     rc = lib.b200dec_router(x.data_ptr(), ex.router.data_ptr(), N, W, E, ex.top, ids.data_ptr(), scores.data_ptr(), ranks.data_ptr(),
                             ex.counts.data_ptr(), K._stream())
     _lib.check(rc, "router")
     xs = torch.empty(total, W, device=dev, dtype=xb.dtype)
-    rc = lib.b200dec_dispatch(xb.data_ptr(), xb.element_size(), ids.data_ptr(), scores.data_ptr(), ranks.data_ptr(), ex.counts.data_ptr(), N,
-                              W, E, ex.top, tile_rows, xs.data_ptr(), score_sorted.data_ptr(), slots.data_ptr(), tiles.data_ptr(), max_tiles,
-                              K._stream())
+    rc = lib.b200dec_dispatch_counted(xb.data_ptr(), xb.element_size(), ids.data_ptr(), scores.data_ptr(), ranks.data_ptr(), ex.counts.data_ptr(), N,
+                                      W, E, ex.top, tile_rows, xs.data_ptr(), score_sorted.data_ptr(), slots.data_ptr(), tiles.data_ptr(), max_tiles,
+                                      done, K._stream())
     _lib.check(rc, "dispatch")
+    if both:
+        h, y = (torch.empty(total, n, device=dev, dtype=xb.dtype) for n in (ff, W))
+        rc = lib.b200dec_expert_products(xs.data_ptr(), ex.gate_up.data_ptr(), ex.down.data_ptr(), tiles.data_ptr(), max_tiles, tile_rows, total, E,
+                                         ff, W, score_sorted.data_ptr(), float(ex.limit), float(ex.slope), h.data_ptr(), y.data_ptr(),
+                                         done, K.num_sms(dev), K.status_word(dev).data_ptr(), K._stream())
+        _lib.check(rc, "expert_products")
+        return y, slots.view(N, ex.top)
     h = grouped_linear(xs, ex.gate_up, tiles, max_tiles, tile_rows, score_sorted, ex.limit, ex.slope, variant)
     return grouped_linear(h, ex.down, tiles, max_tiles, tile_rows, variant=variant), slots.view(N, ex.top)
 

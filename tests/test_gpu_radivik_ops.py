@@ -363,6 +363,28 @@ def test_mixture(dtype, rows, width, ff, experts, top, limit):
     H.status_clear()
 
 
+@pytest.mark.parametrize("rows,width,ff,experts,top", [(1, 2048, 512, 8, 2), (70, 2048, 1536, 12, 4), (130, 1032, 520, 2, 1), (900, 1024, 776, 3, 2), (1000, 2048, 640, 16, 4)])
+def test_both_products_of_the_experts_in_one_launch(rows, width, ff, experts, top):
+    """More items than multiprocessors, one tile alone, weight blocks and steps with a remainder: the same bits as in two launches, again and again."""
+    from inference_engine_b200 import ops
+
+    g = torch.Generator(device=DEV).manual_seed(rows)
+    mat = lambda *s: torch.randn(*s, generator=g, device=DEV) * s[-1] ** -0.5
+    ex = ops.make_experts(mat(experts, width).to(torch.bfloat16), mat(experts, ff, width), mat(experts, ff, width), mat(experts, width, ff), top, 7.0, 1.702,
+                          torch.bfloat16, torch.device(DEV))
+    x = torch.randn(rows, width, generator=g, device=DEV)
+
+    def rows_of(variant):
+        ex.counts.zero_()
+        y, places = ops.mixture(x, x.to(torch.bfloat16), ex, variant)
+        return y[places.long()]
+
+    want = rows_of(0)
+    for _ in range(5):
+        assert torch.equal(rows_of(None), want)
+    H.status_clear()
+
+
 @pytest.mark.parametrize("rows,width,experts,top", [(600, 2052, 33, 3), (515, 4100, 5, 2), (700, 2052, 5, 2), (1190, 2052, 33, 4), (2060, 1028, 40, 2)])
 def test_router_of_prompt_steps(rows, width, experts, top):
     """The router's forms for many rows: eight steps of weights in flight with a remainder behind them, few experts whose
