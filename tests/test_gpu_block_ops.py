@@ -109,3 +109,21 @@ def test_branches_of_a_recorded_graph(K, chained):
     want = call()
     graph.replay()
     assert all(torch.equal(u, v) for u, v in zip(want, got))
+
+
+def test_branches_at_the_start_of_a_graph(K):
+    """Nothing stands in front of the fork, and the last branch is empty."""
+    from inference_engine_b200 import _lib
+
+    x = torch.randn(2, 64, 256, device="cuda").to(torch.bfloat16)
+    K.silu_mul(x[0])
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        with K.Branches(_lib.load()) as b:
+            a = K.silu_mul(x[0])
+            b.next()
+            c = K.silu_mul(x[1])
+            b.next()
+        d = K.silu_mul(torch.cat([a, c], dim=1))
+    graph.replay()
+    assert torch.equal(d, K.silu_mul(torch.cat([K.silu_mul(x[0]), K.silu_mul(x[1])], dim=1)))
