@@ -6,7 +6,8 @@
 // the block's writes solve a triangular system, u = (I + diag(beta) A)^-1 diag(beta) (v - S0^T kd), the outputs are
 // o = S0^T qd + B u, and the state behind is S = L_8 * S0 + sum_j kr_j u_j^T.
 //   prepare  one block of threads per (8 tokens, head), all independent: the vectors, the inverse T and B, to a workspace.
-//   scan     groups of lanes own four state columns each, block after block: two sums over the key channels per token on the
+//   scan     (rb_scan_kernel; rb_scan_split_kernel with the read-out in warps of its own)
+//            groups of lanes own four state columns each, block after block: two sums over the key channels per token on the
 //            same state, one exchange of the eight tokens' sums between the lanes, the eight writes in one pass.
 //            A block's vectors come by bulk copies into a ring; packed 32-bit arithmetic (two rows per instruction).
 // Every wait is bounded: when one runs out the block writes nothing more and sets B200KV_S_TIMEOUT.
@@ -249,6 +250,99 @@ __device__ __forceinline__ void rb_exchange(float (&v)[kRbCols * kRbTok], int la
   }
 }
 
+// What a lane does with its rows of the state, kR of kRbCols columns as pairs of rows: rows 4 kLanes j + 4 l + (0..3), j < kR / 4.
+template <int kLanes, int kR>
+__device__ __forceinline__ void rb_state_load(rb_pair (&S)[kRbCols][kR / 2], const float* state, bool some, int D, int P4, int p0, int l) {
+#pragma unroll
+  for (int i = 0; i < kR / 2; ++i) {
+    const int d = (i / 2) * 4 * kLanes + 4 * l + 2 * (i & 1);
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), c = a;
+    if (some) {
+      if (d < D) a = __ldcg(reinterpret_cast<const float4*>(state + (long long)d * P4 + p0));
+      if (d + 1 < D) c = __ldcg(reinterpret_cast<const float4*>(state + (long long)(d + 1) * P4 + p0));
+    }
+    S[0][i] = rb_pack(a.x, c.x);
+    S[1][i] = rb_pack(a.y, c.y);
+    S[2][i] = rb_pack(a.z, c.z);
+    S[3][i] = rb_pack(a.w, c.w);
+  }
+}
+template <int kLanes, int kR>
+__device__ __forceinline__ void rb_state_store(const rb_pair (&S)[kRbCols][kR / 2], float* state, int D, int P, int P4, int p0, int l) {
+#pragma unroll
+  for (int i = 0; i < kR / 2; ++i) {
+    const int d = (i / 2) * 4 * kLanes + 4 * l + 2 * (i & 1);
+    float a[kRbCols], c[kRbCols];
+#pragma unroll
+    for (int k = 0; k < kRbCols; ++k) {
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(a[k]), "=f"(c[k]) : "l"(S[k][i]));
+      if (p0 + k >= P) a[k] = c[k] = 0.f;
+    }
+    if (p0 < P4) {
+      if (d < D) st_elem4(state + (long long)d * P4 + p0, a);
+      if (d + 1 < D) st_elem4(state + (long long)(d + 1) * P4 + p0, c);
+    }
+  }
+}
+// its rows of a stage's eight vectors (of token i ^ swap in place i); mine: the stage, 16 l bytes on
+template <int kLanes, int kR>
+__device__ __forceinline__ void rb_rows(uint32_t mine, int vec, int swap, ulonglong2 (&k)[kRbTok][kR / 4]) {
+#pragma unroll
+  for (int i = 0; i < kRbTok; ++i)
+#pragma unroll
+    for (int j = 0; j < kR / 4; ++j) k[i][j] = rb_lds(mine + 4 * ((vec * kRbTok + (i ^ swap)) * kLanes * kR + 4 * kLanes * j));
+}
+// ... and their sums with the state
+template <int kR>
+__device__ __forceinline__ void rb_sums(const rb_pair (&S)[kRbCols][kR / 2], const ulonglong2 (&vec)[kRbTok][kR / 4], float (&r)[kRbCols * kRbTok]) {
+#pragma unroll
+  for (int i = 0; i < kRbTok; ++i) {
+    rb_pair acc[kRbCols];
+#pragma unroll
+    for (int j = 0; j < kR / 4; ++j) {
+      const ulonglong2 k = vec[i][j];
+#pragma unroll
+      for (int c = 0; c < kRbCols; ++c) {
+        acc[c] = j == 0 ? rb_mul(S[c][0], k.x) : rb_fma(S[c][2 * j], k.x, acc[c]);
+        acc[c] = rb_fma(S[c][2 * j + 1], k.y, acc[c]);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < kRbCols; ++c) r[kRbCols * i + c] = rb_both(acc[c]);
+  }
+}
+// S <- decay S + sum of k_i u_i^T
+template <int kR>
+__device__ __forceinline__ void rb_update(rb_pair (&S)[kRbCols][kR / 2], const ulonglong2 (&decay)[kR / 4], const ulonglong2 (&k)[kRbTok][kR / 4],
+                                          const float (&u)[kRbTok][kRbCols]) {
+#pragma unroll
+  for (int j = 0; j < kR / 4; ++j)
+#pragma unroll
+    for (int c = 0; c < kRbCols; ++c) {
+      S[c][2 * j] = rb_mul(S[c][2 * j], decay[j].x);
+      S[c][2 * j + 1] = rb_mul(S[c][2 * j + 1], decay[j].y);
+    }
+#pragma unroll
+  for (int i = 0; i < kRbTok; ++i) {
+    const float4 uu = *reinterpret_cast<const float4*>(u[i]);
+    const rb_pair up[kRbCols] = {rb_pack(uu.x, uu.x), rb_pack(uu.y, uu.y), rb_pack(uu.z, uu.z), rb_pack(uu.w, uu.w)};
+#pragma unroll
+    for (int j = 0; j < kR / 4; ++j) {
+#pragma unroll
+      for (int c = 0; c < kRbCols; ++c) {
+        S[c][2 * j] = rb_fma(k[i][j].x, up[c], S[c][2 * j]);
+        S[c][2 * j + 1] = rb_fma(k[i][j].y, up[c], S[c][2 * j + 1]);
+      }
+    }
+  }
+}
+// a token's row of T or B
+__device__ __forceinline__ void rb_row8(const float* p, float (&row)[kRbTok]) {
+  const float4 a = *reinterpret_cast<const float4*>(p), c = *reinterpret_cast<const float4*>(p + 4);
+  row[0] = a.x; row[1] = a.y; row[2] = a.z; row[3] = a.w;
+  row[4] = c.x; row[5] = c.y; row[6] = c.z; row[7] = c.w;
+}
+
 // kLanes lanes share kRbCols state columns; lane l owns rows 4 kLanes j + 4 l + (0..3), j < kR / 4, of all of them.
 // One block: kRbWarps warps, 32 kRbCols / kLanes columns each, of one head of one entry.
 template <typename T, int kLanes, int kR>
@@ -285,19 +379,7 @@ rb_scan_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, con
     for (int b = 0; b < min(kRbStages, blocks); ++b) fetch(b);
   float* state = rec.state + ((long long)x.slot * rec.heads + h) * D * P4;
   rb_pair S[kRbCols][kR / 2];  // [column][pair of rows]
-#pragma unroll
-  for (int i = 0; i < kR / 2; ++i) {
-    const int d = (i / 2) * 4 * kLanes + 4 * l + 2 * (i & 1);
-    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), c = a;
-    if (x.pos > 0 && p0 < P4) {
-      if (d < D) a = __ldcg(reinterpret_cast<const float4*>(state + (long long)d * P4 + p0));
-      if (d + 1 < D) c = __ldcg(reinterpret_cast<const float4*>(state + (long long)(d + 1) * P4 + p0));
-    }
-    S[0][i] = rb_pack(a.x, c.x);
-    S[1][i] = rb_pack(a.y, c.y);
-    S[2][i] = rb_pack(a.z, c.z);
-    S[3][i] = rb_pack(a.w, c.w);
-  }
+  rb_state_load<kLanes, kR>(S, state, x.pos > 0 && p0 < P4, D, P4, p0, l);
   // v of this lane's token and columns in block b; kept as loaded until it is used, so that nothing waits for it
   auto value = [&](int b, T (&v)[kC]) {
     const int t = b * kRbTok + tok;
@@ -315,51 +397,22 @@ rb_scan_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, con
     value(b + 1, v_next);
     if (!dt_mbar_wait(dt_smem(bars + b % kRbStages), (b / kRbStages) & 1)) dead = true;
     const float* st = rb_smem + (b % kRbStages) * kFloats;
-    // this lane's rows of eight vectors (of token i ^ swap in place i), and their sums with the state
     const uint32_t mine = dt_smem(st) + 16 * l;
-    auto rows = [&](int vec, int swap, ulonglong2 (&k)[kRbTok][kQuads]) {
-#pragma unroll
-      for (int i = 0; i < kRbTok; ++i)
-#pragma unroll
-        for (int j = 0; j < kQuads; ++j) k[i][j] = rb_lds(mine + 4 * ((vec * kRbTok + (i ^ swap)) * Dp + 4 * kLanes * j));
-    };
-    auto sums = [&](const ulonglong2 (&vec)[kRbTok][kQuads], float (&r)[kRbCols * kRbTok]) {
-#pragma unroll
-      for (int i = 0; i < kRbTok; ++i) {
-        rb_pair acc[kRbCols];
-#pragma unroll
-        for (int j = 0; j < kQuads; ++j) {
-          const ulonglong2 k = vec[i][j];
-#pragma unroll
-          for (int c = 0; c < kRbCols; ++c) {
-            acc[c] = j == 0 ? rb_mul(S[c][0], k.x) : rb_fma(S[c][2 * j], k.x, acc[c]);
-            acc[c] = rb_fma(S[c][2 * j + 1], k.y, acc[c]);
-          }
-        }
-#pragma unroll
-        for (int c = 0; c < kRbCols; ++c) r[kRbCols * i + c] = rb_both(acc[c]);
-      }
-    };
     ulonglong2 ka[kRbTok][kQuads], kb[kRbTok][kQuads], decay[kQuads];
     float r[kRbCols * kRbTok], o[kRbCols * kRbTok];
-    rows(0, tok, ka);
-    rows(1, tok, kb);
-    sums(ka, r);
-    rows(2, 0, ka);
+    rb_rows<kLanes, kR>(mine, 0, tok, ka);
+    rb_rows<kLanes, kR>(mine, 1, tok, kb);
+    rb_sums<kR>(S, ka, r);
+    rb_rows<kLanes, kR>(mine, 2, 0, ka);
     rb_exchange<kLanes>(r, l);
-    sums(kb, o);
+    rb_sums<kR>(S, kb, o);
 #pragma unroll
     for (int j = 0; j < kQuads; ++j) decay[j] = rb_lds(mine + 4 * (3 * kRbTok * Dp + 4 * kLanes * j));
     rb_exchange<kLanes>(o, l);
     const float* tb = st + 3 * kRbTok * Dp + Dp;
     float row[2][kRbTok];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const float4 a = *reinterpret_cast<const float4*>(tb + (i * kRbTok + tok) * kRbTok);
-      const float4 c = *reinterpret_cast<const float4*>(tb + (i * kRbTok + tok) * kRbTok + 4);
-      row[i][0] = a.x; row[i][1] = a.y; row[i][2] = a.z; row[i][3] = a.w;
-      row[i][4] = c.x; row[i][5] = c.y; row[i][6] = c.z; row[i][7] = c.w;
-    }
+    rb_row8(tb + tok * kRbTok, row[0]);
+    rb_row8(tb + (kRbTok + tok) * kRbTok, row[1]);
     float u[kC];
 #pragma unroll
     for (int c = 0; c < kC; ++c) {
@@ -385,29 +438,7 @@ rb_scan_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, con
       }
       if (t < x.n && pc + c < P && !dead) out[((long long)(x.first + t) * rec.heads + h) * P + pc + c] = even + odd;
     }
-#pragma unroll
-    for (int j = 0; j < kQuads; ++j) {
-      const ulonglong2 g = decay[j];
-#pragma unroll
-      for (int c = 0; c < kRbCols; ++c) {
-        S[c][2 * j] = rb_mul(S[c][2 * j], g.x);
-        S[c][2 * j + 1] = rb_mul(S[c][2 * j + 1], g.y);
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < kRbTok; ++i) {
-      const float4 uu = *reinterpret_cast<const float4*>(ubuf[warp][grp][i]);
-      const rb_pair up[kRbCols] = {rb_pack(uu.x, uu.x), rb_pack(uu.y, uu.y), rb_pack(uu.z, uu.z), rb_pack(uu.w, uu.w)};
-#pragma unroll
-      for (int j = 0; j < kQuads; ++j) {
-        const ulonglong2 k = ka[i][j];
-#pragma unroll
-        for (int c = 0; c < kRbCols; ++c) {
-          S[c][2 * j] = rb_fma(k.x, up[c], S[c][2 * j]);
-          S[c][2 * j + 1] = rb_fma(k.y, up[c], S[c][2 * j + 1]);
-        }
-      }
-    }
+    rb_update<kR>(S, decay, ka, ubuf[warp][grp]);
     if (__syncthreads_or(dead)) {  // (otherwise: the stage and ubuf are free)
       if (tid == 0) {
         if (status) atomicOr(status, B200KV_S_TIMEOUT);
@@ -418,21 +449,146 @@ rb_scan_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, con
     }
     if (tid == 0 && b + kRbStages < blocks) fetch(b + kRbStages);
   }
-#pragma unroll
-  for (int i = 0; i < kR / 2; ++i) {
-    const int d = (i / 2) * 4 * kLanes + 4 * l + 2 * (i & 1);
-    float a[kRbCols], c[kRbCols];
-#pragma unroll
-    for (int k = 0; k < kRbCols; ++k) {
-      asm("mov.b64 {%0, %1}, %2;" : "=f"(a[k]), "=f"(c[k]) : "l"(S[k][i]));
-      if (p0 + k >= P) a[k] = c[k] = 0.f;
+  rb_state_store<kLanes, kR>(S, state, D, P, P4, p0, l);
+  rec_keep_inputs<T>(rec, in, x, blockIdx.x, gridDim.x, 32 * kRbWarps);
+}
+
+// The same with two warps for the columns of one, for steps with so few portions that their blocks leave schedulers idle: the first finds
+// the writes (sums with k, u), the second reads out (sums with q, the outputs) on a copy of the state, which both advance.  The chain of a
+// block of eight tokens is then without the read-out, and nothing holds the warps together but what they hand on: u by a barrier, a stage's
+// end by another, which the fetching lane of a reading warp waits for.  The arithmetic is the same, bit for bit.
+template <typename T, int kLanes, int kR>
+__global__ void __launch_bounds__(64 * kRbWarps, 3)
+rb_scan_split_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, const T* __restrict__ conv, int conv_stride,
+                     const b200dec_entries ent, const float* __restrict__ ws, float* __restrict__ out, int slabs, int32_t* status) {
+  constexpr int Dp = kLanes * kR, kFloats = rb_floats(Dp), kQuads = kR / 4, kGroups = 32 / kLanes;
+  constexpr int kM = kLanes / 8, kC = kRbCols / kM;  // after the exchange a lane holds kC columns of one token
+  extern __shared__ __align__(128) float rb_smem[];  // [kRbStages][kFloats]
+  __shared__ __align__(16) float ubuf[kRbStages][kRbWarps][kGroups][kRbTok][kRbCols];
+  __shared__ __align__(8) uint64_t full[kRbStages], empty[kRbStages], written[kRbStages][kRbWarps];
+  pdl_enter();
+  const int e = blockIdx.y, h = blockIdx.x / slabs, slab = blockIdx.x - h * slabs, tid = threadIdx.x;
+  if (e < *ent.num_decoding) { pdl_wait(); return; }
+  const RecEntry x = rec_entry(ent, rec, e, status);
+  if (tid == 0) {
+    for (int i = 0; i < kRbStages; ++i) {
+      dt_mbar_init(dt_smem(full + i), 1);
+      dt_mbar_init(dt_smem(empty + i), 2 * kRbWarps);
+      for (int w = 0; w < kRbWarps; ++w) dt_mbar_init(dt_smem(&written[i][w]), 1);
     }
-    if (p0 < P4) {
-      if (d < D) st_elem4(state + (long long)d * P4 + p0, a);
-      if (d + 1 < D) st_elem4(state + (long long)(d + 1) * P4 + p0, c);
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  __syncthreads();
+  pdl_wait();
+  if (x.n == 0) return;
+  const int D = rec.dim, P = rec.vdim, P4 = rec_round4(P), blocks = (x.n + kRbTok - 1) / kRbTok;
+  const int lane = tid & 31, warp = (tid >> 5) % kRbWarps, grp = lane / kLanes, l = tid % kLanes;
+  const bool reads = tid >= 32 * kRbWarps;
+  const int p0 = ((slab * kRbWarps + warp) * kGroups + grp) * kRbCols;  // the first column
+  const int tok = l / kM, pc = p0 + kC * (l % kM);                  // what this lane holds after the exchange
+  const long long at0 = (long long)rb_first(ent, e) * rec.heads + h;
+  const bool fetches = tid == 32 * kRbWarps;
+  int sent = 0;
+  auto fetch = [&]() {
+    const uint32_t bar = dt_smem(full + sent % kRbStages);
+    dt_expect_tx(bar, kFloats * 4);
+    rb_bulk(dt_smem(rb_smem + (sent % kRbStages) * kFloats), ws + (at0 + (long long)sent * rec.heads) * kFloats, kFloats * 4, bar);
+    ++sent;
+  };
+  if (fetches)
+    while (sent < min(kRbStages, blocks)) fetch();
+  float* state = rec.state + ((long long)x.slot * rec.heads + h) * D * P4;
+  rb_pair S[kRbCols][kR / 2];  // [column][pair of rows]
+  rb_state_load<kLanes, kR>(S, state, x.pos > 0 && p0 < P4, D, P4, p0, l);
+  bool dead = false;
+  ulonglong2 ka[kRbTok][kQuads], decay[kQuads];
+  float r[kRbCols * kRbTok], row[kRbTok];
+  // block b's phase of a barrier of its stage, alike for all lanes of the warp
+  auto warp_wait = [&](const uint64_t* bar, int b) { return __all_sync(0xffffffffu, dt_mbar_wait(dt_smem(bar), (b / kRbStages) & 1)) != 0; };
+  // the sums of vectors `vec` with the state in front of block b; then what advances the state, and the token's row of T (0) or B (1)
+  auto look = [&](int b, int vec) {
+    const int s = b % kRbStages;
+    if (!warp_wait(full + s, b)) return false;
+    const float* st = rb_smem + s * kFloats;
+    const uint32_t mine = dt_smem(st) + 16 * l;
+    rb_rows<kLanes, kR>(mine, vec, tok, ka);
+    rb_sums<kR>(S, ka, r);
+    rb_rows<kLanes, kR>(mine, 2, 0, ka);
+    rb_exchange<kLanes>(r, l);
+#pragma unroll
+    for (int j = 0; j < kQuads; ++j) decay[j] = rb_lds(mine + 4 * (3 * kRbTok * Dp + 4 * kLanes * j));
+    rb_row8(st + 3 * kRbTok * Dp + Dp + (vec * kRbTok + tok) * kRbTok, row);
+    return true;
+  };
+  if (!reads) {
+    // v of this lane's token and columns in block b; kept as loaded until it is used, so that nothing waits for it
+    auto value = [&](int b, T (&v)[kC]) {
+      const int t = b * kRbTok + tok;
+      const T* src = conv + (long long)(x.first + t) * conv_stride + rec.off_v + h * P + pc;
+#pragma unroll
+      for (int c = 0; c < kC; ++c) v[c] = t < x.n && pc + c < P ? src[c] : T(0);
+    };
+    T v_next[kC];
+    value(0, v_next);
+    for (int b = 0; b < blocks; ++b) {
+      float w[kC];
+#pragma unroll
+      for (int c = 0; c < kC; ++c) w[c] = ld_elem(v_next + c);
+      value(b + 1, v_next);
+      if (!look(b, 0)) { dead = true; break; }
+      const int s = b % kRbStages;
+      float (&mine)[kRbTok][kRbCols] = ubuf[s][warp][grp];
+#pragma unroll
+      for (int c = 0; c < kC; ++c) {
+        w[c] -= r[c];
+        float even = 0.f, odd = 0.f;
+#pragma unroll
+        for (int j = 0; j < kRbTok; ++j) {
+          const float wj = __shfl_sync(0xffffffffu, w[c], j * kM + l % kM, kLanes);
+          if (j & 1) odd = fmaf(row[j], wj, odd); else even = fmaf(row[j], wj, even);
+        }
+        mine[tok][kC * (l % kM) + c] = even + odd;
+      }
+      __syncwarp();
+      if (lane == 0) dt_mbar_arrive(dt_smem(&written[s][warp]));
+      rb_update<kR>(S, decay, ka, mine);
+      __syncwarp();
+      if (lane == 0) dt_mbar_arrive(dt_smem(empty + s));
+    }
+  } else {
+    for (int b = 0; b < blocks; ++b) {
+      if (!look(b, 1)) { dead = true; break; }
+      const int s = b % kRbStages, t = b * kRbTok + tok;
+      if (!warp_wait(&written[s][warp], b)) { dead = true; break; }
+      const float (&theirs)[kRbTok][kRbCols] = ubuf[s][warp][grp];
+      rb_update<kR>(S, decay, ka, theirs);
+#pragma unroll
+      for (int c = 0; c < kC; ++c) {
+        float even = r[c], odd = 0.f;
+#pragma unroll
+        for (int j = 0; j < kRbTok; ++j) {
+          const float uj = theirs[j][kC * (l % kM) + c];
+          if (j & 1) odd = fmaf(row[j], uj, odd); else even = fmaf(row[j], uj, even);
+        }
+        if (t < x.n && pc + c < P) out[((long long)(x.first + t) * rec.heads + h) * P + pc + c] = even + odd;
+      }
+      __syncwarp();
+      if (lane == 0) dt_mbar_arrive(dt_smem(empty + s));
+      if (fetches && sent < blocks) {
+        if (dt_mbar_wait(dt_smem(empty + s), (b / kRbStages) & 1)) fetch(); else dead = true;
+      }
+      if (__any_sync(0xffffffffu, dead)) break;
     }
   }
-  rec_keep_inputs<T>(rec, in, x, blockIdx.x, gridDim.x, 32 * kRbWarps);
+  if (__syncthreads_or(dead)) {
+    if (fetches) {
+      if (status) atomicOr(status, B200KV_S_TIMEOUT);
+      for (int i = max(sent - kRbStages, 0); i < sent; ++i) dt_mbar_wait(dt_smem(full + i % kRbStages), (i / kRbStages) & 1);
+    }
+    return;
+  }
+  if (!reads) rb_state_store<kLanes, kR>(S, state, D, P, P4, p0, l);
+  rec_keep_inputs<T>(rec, in, x, blockIdx.x, gridDim.x, 64 * kRbWarps);
 }
 
 template <typename T, int kLanes, int kR>
@@ -446,11 +602,15 @@ static int rb_launch(const b200dec_recurrence& rec, const b200dec_recurrence_in&
                                               dim3(few ? 256 : 128), 0, s, rec, in, (const T*)conv, stride, ent, ws, status));
   if (rc != B200KV_OK) return rc;
   const size_t smem = (size_t)kRbStages * rb_floats(Dp) * 4;
-  if (cudaFuncSetAttribute(rb_scan_kernel<T, kLanes, kR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return B200KV_E_LAUNCH;
+  // All blocks of two warps' columns by four warps at once (three fit a multiprocessor), but for one entry, which a step's padding takes. us a
+  // layer: three portions of 1000 rows in all, 16 heads of 128 132.7 -> 125.1; one of 614 rows, 12 heads of 96 and 112 108.7 -> 100.5; of less than
+  // 200 rows the same. With more blocks than that the schedulers have work without it, and the second copy of the state is a third more.
+  const bool split = (long long)rec.heads * slabs * (ent.num_entries - 1) <= 3 * 148;
+  auto* scan = split ? rb_scan_split_kernel<T, kLanes, kR> : rb_scan_kernel<T, kLanes, kR>;
+  if (!allow_smem(scan, smem)) return B200KV_E_LAUNCH;
   // Not chained: brought up beside the kernel in front, its few long-running blocks would crowd on the multiprocessors that
   // come free first.
-  return launch_result(launch_kernel(false, rb_scan_kernel<T, kLanes, kR>, dim3(rec.heads * slabs, ent.num_entries), dim3(32 * kRbWarps), smem, s, rec, in,
+  return launch_result(launch_kernel(false, scan, dim3(rec.heads * slabs, ent.num_entries), dim3((split ? 64 : 32) * kRbWarps), smem, s, rec, in,
                                       (const T*)conv, stride, ent, (const float*)ws, out, slabs, status));
 }
 

@@ -318,6 +318,35 @@ def test_recurrence_with_two_states_in_the_ring(heads, groups, dim, vdim, kind, 
     test_recurrence_portions_and_decoding(heads, groups, dim, vdim, 4, kind, dtype, False, None)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads,groups,dim,vdim", [(4, 2, 32, 12), (3, 3, 60, 70), (4, 4, 128, 128), (2, 1, 200, 33)])
+def test_delta_rule_by_twice_the_warps(heads, groups, dim, vdim, dtype):
+    """Few portions have warps of their own for what is read out, many entries (here idle ones) do not: the same outputs and states."""
+    from inference_engine_b200 import ops
+
+    g = np.random.default_rng(dim)
+    rec, _ = make_rec(g, next(k for k in KINDS if "delta" in k), heads, groups, dim, vdim, 4)
+    chunks = [1, 7, 8, 9, 24, 100]
+    seqs = [rec_inputs(g, rec, n, dtype) for n in chunks]
+    x, step, beta = (torch.cat([q[i] for q in seqs]) for i in range(3))
+    first = torch.randn(6, heads, dim, vdim, device=DEV)
+
+    def run(idle):
+        st = ops.make_recurrent_state(rec, 6, dtype, DEV)
+        st.state[..., :vdim] = first
+        st.ring.copy_(torch.linspace(-1, 1, st.ring.numel(), device=DEV).view(st.ring.shape))
+        rows, _ = step_rows([3, 0, 5, 0, 2, 0] + [0] * idle, chunks + [0] * idle, 0, slots=[4, 1, 0, 2, 5, 3] + [-1] * idle)
+        out = torch.empty(rows.num_rows, heads * vdim, device=DEV)
+        ops.recurrence_prefill(rec, st, x, step, beta, rows, out, "blocked")
+        return out, st.state, st.ring
+
+    few, many = run(0), run(500)
+    for got, want in zip(few[:2], many[:2]):  # the preparation adds in another order: up to 200 terms in 32 bits, 200 * 2^-24
+        assert (got - want).norm().item() <= 2e-5 * want.norm().item()
+    assert torch.equal(few[2], many[2])
+    status_clear()
+
+
 @pytest.mark.parametrize("kind", KINDS)
 @pytest.mark.parametrize("heads,groups,dim,vdim", [(2, 1, 64, 64), (16, 4, 128, 72), (40, 8, 16, 16), (100, 4, 32, 8)])
 def test_long_portions_beside_others(kind, heads, groups, dim, vdim):
