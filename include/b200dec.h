@@ -112,7 +112,7 @@ int b200dec_grouped_linear(const void* x, const void* w, int32_t elem, const int
                            int32_t act, float limit, float slope, void* y, int32_t sm_count, int32_t variant, int32_t* status, void* stream);
 /* Both products of the experts in one launch, bf16 on tcgen05: h [total_rows, ff] = the product of act = 1 with gate_up
  * [experts, 2 * ff, width], y [total_rows, width] = that of act = 0 of h with down [experts, width, ff]; ff and width multiples of 8.
- * done: as b200dec_dispatch_counted left it, used up by the call. */
+ * done: as b200dec_dispatch_counted left it, used up by the call.  For up to about 192 rows an expert; with more two calls are faster. */
 int b200dec_expert_products(const void* x, const void* gate_up, const void* down, const int32_t* tiles, int32_t max_tiles, int32_t tile_rows,
                             int32_t total_rows, int32_t experts, int32_t ff, int32_t width, const float* score_sorted, float limit,
                             float slope, void* h, void* y, int32_t* done, int32_t sm_count, int32_t* status, void* stream);

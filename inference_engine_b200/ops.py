@@ -414,7 +414,10 @@ def mixture(x: torch.Tensor, xb: torch.Tensor, ex: Experts, variant: int | None 
     # Both products in one launch, unless the second one's items are the longer ones: as the last to be drawn they leave multiprocessors idle
     # for longer than a start takes.  us a layer, two launches and one: 32 experts of 1536 (width 2048), 64 rows 135.3 and 123.0, 512 154.6
     # and 145.4, 1024 175.2 and 165.7; 8 experts of 3072, 64 rows 79.5 and 82.3, 192 84.4 and 94.1, 700 106.8 and 113.8 (16 80.1 and 77.3, 1000 135 and 129).
-    both = variant is None and xb.dtype == torch.bfloat16 and W % 8 == 0 and ff % 8 == 0 and ff <= W
+    # Not where the first product has less than about two rounds of items (8 experts of 1024, 64 rows 39.1 and 41.8), nor where tiles are full and the
+    # tensor core is the bound (32 experts of 1536, router and dispatch included: 1536 rows 175.3 and 173.4, 2048 213.9 and 228.2, 4096 367 and 408).
+    both = (variant is None and xb.dtype == torch.bfloat16 and W % 8 == 0 and ff % 8 == 0 and ff <= W and total <= 192 * E
+            and 2 * ff * E >= 300 * 128)
     done = tiles.data_ptr() + 4 * (1 + 3 * max_tiles) if both else None
     score_sorted = torch.empty(total, dtype=torch.float32, device=dev)
     rc = lib.b200dec_router(x.data_ptr(), ex.router.data_ptr(), N, W, E, ex.top, ids.data_ptr(), scores.data_ptr(), ranks.data_ptr(),
