@@ -3,7 +3,7 @@
 //
 // Work: the unit is a block of 64 keys of one (entry, kv head, group of up to 16 query heads).  All units of the batch
 // lie end to end in (entry, head, block) order and are cut into equal ranges, one per CTA of a persistent grid (two
-// CTAs per SM), from cached_lens on the device: the grid depends on shapes only.
+// CTAs per SM, or four), from cached_lens on the device: the grid depends on shapes only.
 // One CTA: a producer warp fetches blocks by page with tensor-map copies into a ring of stages; four consumer warps own
 // 16 of a block's 64 keys each and run S = Q K^T and O += P V as bf16 mma.m16n8k16 with 32-bit scores, softmax state and
 // sums (query heads are the 16 rows of the product).  When the CTA's part of an (entry, head) ends, the four warps are
@@ -22,13 +22,20 @@ constexpr int kPdKeys = 64;      // keys per block
 constexpr int kPdWarps = 4;      // consumer warps
 constexpr int kPdThreads = 32 * (kPdWarps + 1);
 constexpr int kPdRows = 16;      // query heads per unit
-constexpr int kPdCtasPerSm = 2;
+// CTAs per multiprocessor: two, or four with half the stages for keys and values of up to 64 channels each. A narrow block takes its CTA about
+// as long as a wide one, which is a chain and not bytes; and with four, twice as many pairs of entry and head have a CTA of their own. Where there are no
+// more pairs than two per multiprocessor the deeper ring is better. us, two and four, 8 kv heads of 64 and 64: 64 entries of 500 22.0 and 13.8, of 200
+// to 4096 with a window of 512 23.5 and 14.4, 128 of 4000 to 4096 177.7 and 180.2 (heads of 32 and 64 173.9 and 137.7); 32 with the window 11.8 and
+// 12.9, one of 300 7.7 and 8.2.
+constexpr int kPdCtasPerSm = 2, kPdCtasNarrow = 4;
 constexpr int kPdMinBlocks = 4;  // smallest share of a CTA
 constexpr int kPdHandOff = 5;    // blocks that take one CTA as long as handing parts of an (entry, head) over through the workspace
 constexpr uint32_t kPdBlockBytes = kPdKeys * 128;  // 64 rows x 64 channels
 constexpr int kPdMaxB = 4096;
 
-__host__ __device__ constexpr int pd_stages(int kb, int vb) { return kb + vb == 4 ? 3 : (kb + vb == 3 ? 4 : 6); }
+__host__ __device__ constexpr int pd_stages(int kb, int vb, int ctas) {
+  return kb + vb == 4 || ctas == kPdCtasNarrow ? 3 : (kb + vb == 3 ? 4 : 6);
+}
 
 __device__ __forceinline__ void pd_ldsm(uint32_t (&r)[4], uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
@@ -97,14 +104,14 @@ struct PdCursor {
   }
 };
 
-template <int KB, int VB, bool kWide>
-__global__ void __launch_bounds__(kPdThreads, kPdCtasPerSm)
+template <int KB, int VB, bool kWide, int kCtas>
+__global__ void __launch_bounds__(kPdThreads, kCtas)
 paged_decode_kernel(const uint16_t* __restrict__ q, DecCache c, const int32_t* __restrict__ cached_lens,
                     const int32_t* __restrict__ num_decoding, int B, int heads, int groups, float scale_log2, DecAttnOpt opt,
                     uint16_t* __restrict__ out, int zero_idle, int* __restrict__ counters, float* __restrict__ parts, int box_rows, int32_t* status,
                     const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v) {
   extern __shared__ uint8_t pd_raw[];
-  constexpr int kStages = pd_stages(KB, VB);
+  constexpr int kStages = pd_stages(KB, VB, kCtas);
   constexpr uint32_t kStageBytes = (KB + VB) * kPdBlockBytes;
   constexpr int kTiles = 8 * VB;                        // 8-channel tiles of O
   constexpr int kPart = kPdRows * (64 * VB + 2);        // floats of one part: O rows, then m and l
@@ -478,14 +485,14 @@ paged_decode_kernel(const uint16_t* __restrict__ q, DecCache c, const int32_t* _
   }
 }
 
-template <int KB, int VB, bool kWide>
+template <int KB, int VB, bool kWide, int kCtas>
 static int pd_launch(const void* q, const DecCache& c, const int32_t* cached_lens, const int32_t* num_decoding, int B, int heads, int groups,
                      float scale_log2, const DecAttnOpt& opt, void* out, int zero_idle, int* counters, float* parts, int grid, int box_rows, int32_t* status,
                      const CUtensorMap& tm_k, const CUtensorMap& tm_v, cudaStream_t stream) {
-  constexpr size_t kRings = (size_t)pd_stages(KB, VB) * (KB + VB) * kPdBlockBytes + 1024;
+  constexpr size_t kRings = (size_t)pd_stages(KB, VB, kCtas) * (KB + VB) * kPdBlockBytes + 1024;
   const size_t smem = kRings + (size_t)(B + 1) * 4;
-  if (!allow_smem(paged_decode_kernel<KB, VB, kWide>, kRings + (size_t)(kPdMaxB + 1) * 4)) return B200KV_E_LAUNCH;
-  return launch_result(launch_chained(paged_decode_kernel<KB, VB, kWide>, dim3(grid), dim3(kPdThreads), smem, stream, (const uint16_t*)q, c,
+  if (!allow_smem(paged_decode_kernel<KB, VB, kWide, kCtas>, kRings + (size_t)(kPdMaxB + 1) * 4)) return B200KV_E_LAUNCH;
+  return launch_result(launch_chained(paged_decode_kernel<KB, VB, kWide, kCtas>, dim3(grid), dim3(kPdThreads), smem, stream, (const uint16_t*)q, c,
                                       cached_lens, num_decoding, B, heads, groups, scale_log2, opt, (uint16_t*)out, zero_idle, counters, parts,
                                       box_rows, status, tm_k, tm_v));
 }
@@ -500,7 +507,7 @@ extern "C" size_t b200dec_decode_attn_workspace(int32_t B, int32_t heads, int32_
   if (B < 1 || heads < 1 || kv_heads < 1 || v_dim < 1 || sm_count < 1) return 0;
   const int vb = v_dim <= 64 ? 1 : 2;
   // counters per (entry, head unit): there are never more units than query heads
-  return pd_counter_bytes(B, heads) + (size_t)sm_count * kPdCtasPerSm * 2 * kPdRows * (64 * vb + 2) * 4;
+  return pd_counter_bytes(B, heads) + (size_t)sm_count * (vb == 1 ? kPdCtasNarrow : kPdCtasPerSm) * 2 * kPdRows * (64 * vb + 2) * 4;
 }
 
 extern "C" int b200dec_decode_attn_opt(const void* q, const b200dec_cache* cache, const b200kv_table* table, const int32_t* cached_lens,
@@ -534,16 +541,18 @@ extern "C" int b200dec_decode_attn_opt(const void* q, const b200dec_cache* cache
   if (opt.window > 0 && entry_blocks > opt.window / kPdKeys + 2) entry_blocks = opt.window / kPdKeys + 2;
   const long long units = (long long)B * c.heads * groups * entry_blocks;
   const long long want = std::max((units + kPdMinBlocks - 1) / kPdMinBlocks, (long long)B * c.heads * groups);
-  const int grid = (int)(want < (long long)sm_count * kPdCtasPerSm ? want : (long long)sm_count * kPdCtasPerSm);
   const float sl = scale * 1.4426950408889634f;
   const int kb = c.k_dim > 64, vb = c.v_dim > 64, wide = G > 8;
+  const bool narrow = !kb && !vb && (long long)B * c.heads * groups > (long long)sm_count * kPdCtasPerSm;
+  const int grid = (int)std::min(want, (long long)sm_count * (narrow ? kPdCtasNarrow : kPdCtasPerSm));
   cudaStream_t s = (cudaStream_t)stream;
-#define PD_CASE(KB, VB, W)                                                                                                        \
-  if (kb == KB - 1 && vb == VB - 1 && wide == W)                                                                                  \
-    return pd_launch<KB, VB, W>(q, c, cached_lens, num_decoding, B, heads, groups, sl, opt, out, zero_idle, counters, parts, grid, box, \
+#define PD_CASE(KB, VB, W, CTAS)                                                                                                  \
+  if (kb == KB - 1 && vb == VB - 1 && wide == W && narrow == (CTAS == kPdCtasNarrow))                                             \
+    return pd_launch<KB, VB, W, CTAS>(q, c, cached_lens, num_decoding, B, heads, groups, sl, opt, out, zero_idle, counters, parts, grid, box, \
                                 status, tm_k, tm_v, s);
-  PD_CASE(1, 1, false) PD_CASE(1, 1, true) PD_CASE(1, 2, false) PD_CASE(1, 2, true)
-  PD_CASE(2, 1, false) PD_CASE(2, 1, true) PD_CASE(2, 2, false) PD_CASE(2, 2, true)
+  PD_CASE(1, 1, false, 2) PD_CASE(1, 1, true, 2) PD_CASE(1, 2, false, 2) PD_CASE(1, 2, true, 2)
+  PD_CASE(2, 1, false, 2) PD_CASE(2, 1, true, 2) PD_CASE(2, 2, false, 2) PD_CASE(2, 2, true, 2)
+  PD_CASE(1, 1, false, 4) PD_CASE(1, 1, true, 4)
 #undef PD_CASE
   return B200KV_E_SHAPE;
 }

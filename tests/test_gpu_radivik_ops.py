@@ -331,6 +331,33 @@ def test_decode_attention_splits_and_idle_rows():
         H.status_clear()
 
 
+@pytest.mark.parametrize("heads,kv,dim,vdim,window", [(16, 8, 64, 64, 0), (16, 8, 32, 48, 200), (72, 8, 64, 24, 0)])
+def test_decode_attention_of_many_narrow_heads(heads, kv, dim, vdim, window):
+    """More pairs of entry and kv head than two blocks per multiprocessor, keys and values of one block of channels, with and without
+    hand-offs: against the kernel for any size."""
+    from inference_engine_b200 import ops
+
+    g = np.random.default_rng(dim)
+    for lens in ([1, 63, 64, 65, 130] * 8, [3000] + [200] * 37 + [1, 2]):
+        B = len(lens) + 1  # one idle row
+        need = [(n + 63) // 64 for n in lens]
+        table = np.full((B, max(need)), -1, np.int32)
+        perm, at = g.permutation(sum(need)), 0
+        for b, n in enumerate(need):
+            table[b, :n] = perm[at : at + n]
+            at += n
+        cache = ops.make_paged_kv(sum(need), kv, 64, dim, vdim, torch.bfloat16, DEV)
+        cache.k[..., :dim] = torch.randn(cache.k.shape[:3] + (dim,), device=DEV)
+        cache.v[..., :vdim] = torch.randn(cache.v.shape[:3] + (vdim,), device=DEV)
+        rows = ops.Rows(B, i32([n - 1 for n in lens] + [7]), i32([len(lens)]), i32(table))
+        q = torch.randn(B, heads, dim, device=DEV).to(torch.bfloat16)
+        opt = ops.AttnOptions(window=window)
+        got = ops.paged_attention(q, cache, rows, 0.3, opt)
+        assert torch.equal(got, ops.paged_attention(q, cache, rows, 0.3, opt))
+        close(got, ops.attention_rows(q, cache, rows, 0.3, opt).float().cpu().numpy(), torch.bfloat16)
+        H.status_clear()
+
+
 MOE = [  # rows, width, ff, experts, top, limit
     (1, 64, 40, 4, 1, 2.0), (37, 64, 24, 5, 3, 0.5), (5, 72, 64, 8, 8, 1.0), (700, 136, 200, 3, 2, 7.0), (300, 64, 64, 40, 6, 1.5),
     (33, 30, 18, 3, 2, 1.0), (260, 520, 96, 2, 1, 2.0),
@@ -363,7 +390,7 @@ def test_mixture(dtype, rows, width, ff, experts, top, limit):
     H.status_clear()
 
 
-@pytest.mark.parametrize("rows,width,ff,experts,top", [(1, 2048, 512, 8, 2), (70, 2048, 1536, 12, 4), (130, 1032, 520, 2, 1), (900, 1024, 776, 3, 2), (1000, 2048, 640, 16, 4)])
+@pytest.mark.parametrize("rows,width,ff,experts,top", [(1, 2048, 512, 40, 2), (70, 2048, 1536, 13, 4), (130, 1032, 520, 40, 3), (900, 1024, 776, 25, 5), (1000, 2048, 1280, 16, 3)])
 def test_both_products_of_the_experts_in_one_launch(rows, width, ff, experts, top):
     """More items than multiprocessors, one tile alone, weight blocks and steps with a remainder: the same bits as in two launches, again and again."""
     from inference_engine_b200 import ops
