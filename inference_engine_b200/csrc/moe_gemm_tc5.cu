@@ -244,9 +244,10 @@ grouped_linear_tc5_kernel(const __grid_constant__ MgMaps<kMode> maps, const int3
     int n = 0;
     const int wl = warp & 3;  // tensor-memory lanes 32 wl ..
     for (int at = blockIdx.x;; at += gridDim.x) {
-      const int it = kMode == 2 ? take(n) : (at < items ? at : -1);
+      int it = kMode == 2 ? take(n) : (at < items ? at : -1);
       if (kMode == 2) {
-        __syncwarp();
+        // each lane has a limit of its own: where one's ran out the warp stops as a whole, as its lanes vote and load tensor memory together
+        if (__any_sync(0xffffffffu, it == kMgLost)) it = kMgLost;
         if (lane == 0 && it >= 0) dt_mbar_arrive(bar_taken(n % kMgQueue));
         if (it == kMgLost && lane == 0 && status) atomicOr(status, B200KV_S_TIMEOUT);
       }
