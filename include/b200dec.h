@@ -7,6 +7,9 @@
  * elements, no allocation and no synchronisation, grids from shape arguments only (every call can be captured in a CUDA
  * graph), B200KV_* return codes (negative: nothing was launched) and status bits (device-side inconsistencies: the
  * access is skipped).  `elem` is the element size of the model's precision: 2 = bf16, 4 = fp32.
+ *
+ * Chained launches (b200kv_set_chained_launch of this library): what a kernel may read before the one in front of it has
+ * completed is listed in b200kv.h, and no kernel in front of a call may write that.
  */
 #ifndef B200DEC_H
 #define B200DEC_H

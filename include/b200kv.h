@@ -233,10 +233,12 @@ int b200kv_skinny_linear(const void* x, int64_t ldx, const void* w, int64_t ldw,
  * (which is chained per call, through bit 2 of its `variant`) and b200kv_decode_plan (never chained) is launched
  * with programmatic stream serialization: it may be brought up while the kernel launched just before it on
  * the same stream is still running, reads only caller-provided metadata (cu_seqlens, cu_cached,
- * cached_lens, num_decoding, block table, tile_start, seq_ids) until that kernel has completed, and
- * touches everything else afterwards.  Enable it only if no kernel that precedes a call of this
- * library on its stream writes those metadata arrays - true for the reference engine, which uploads
- * them once per step before the first layer (engine.py:347-356).  Process-wide; has no counterpart
+ * cached_lens, num_decoding, block table, tile_start, seq_ids, positions, state slots, token ids) and
+ * the weights of b200kv_skinny_linear and of the recurrent layers' convolution until that kernel has
+ * completed, and touches everything else (norm weights and angles too) afterwards.  Enable it only if
+ * no kernel that precedes a call of this library on its stream, with chained launches alone in
+ * between, writes one of those arrays - true for the reference engine, which uploads
+ * the metadata once per step before the first layer (engine.py:347-356).  Process-wide; has no counterpart
  * in the reference. */
 void b200kv_set_chained_launch(int enabled);
 int b200kv_get_chained_launch(void);

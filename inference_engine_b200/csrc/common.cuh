@@ -44,7 +44,7 @@ inline CacheView make_view(const b200kv_cache* c, const b200kv_table* t) {
 
 // Chained launches (programmatic dependent launch).  Every kernel of the path (a) waits for the kernel launched
 // before it on the stream (pdl_wait) before it reads anything that kernel may have written or writes global
-// memory itself, having read at most caller-provided metadata by then, and (b) tells the stream when the next
+// memory itself, having read at most caller-provided metadata by then (and weights where b200kv_set_chained_launch says so), and (b) tells the stream when the next
 // kernel may be brought up (pdl_trigger).  Both are no-ops for a kernel launched the ordinary way; the launch
 // attribute is only set while b200kv_set_chained_launch(1) is in force.
 bool take_chained_launch();  // whether the launch at hand is chained: asked once for each, as the first one behind a fork or join of branches is not

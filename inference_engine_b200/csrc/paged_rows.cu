@@ -184,6 +184,7 @@ rope_rows_kernel(const T* __restrict__ qkv, long long qkv_stride, b200dec_rows r
   const int ch = 8 * gl;
   const bool turned = ch < 2 * half, low = ch < half;
   const int partner = (tid & 31) + (turned ? (low ? half / 8 : -(half / 8)) : 0);
+  pdl_wait();
   float cs[8], sn[8];
   if (turned) {
     const float* a = cos_sin + 2 * ((long long)pos * half + (low ? ch : ch - half));
@@ -198,7 +199,6 @@ rope_rows_kernel(const T* __restrict__ qkv, long long qkv_stride, b200dec_rows r
     }
   }
   const unsigned lanes = kLanes == 32 ? 0xffffffffu : ((1u << kLanes) - 1) << ((tid & 31) / kLanes * kLanes);
-  pdl_wait();
   const T* src = qkv + r * qkv_stride;
   long long at0 = 0;
   bool stored = false;
@@ -309,12 +309,12 @@ norm_rope_rows_kernel(const T* __restrict__ qkv, long long qkv_stride, b200dec_r
     ld_floats8(p < nq ? q_norm + 8 * p : k_norm + 8 * (p - nq), w);
     if (ch < 2 * half) ld_floats8(cs + ch, t);
   };
-  if (kVecs == 1 && tid < nqk) {  // they do not wait for the kernel in front
+  pdl_wait();
+  if (kVecs == 1 && tid < nqk) {
     int h, ch;
     locate(tid, h, ch);
     constants(tid, ch);
   }
-  pdl_wait();
   Raw8<T> raw[kVecs];
   const T* src = qkv + r * qkv_stride;
 #pragma unroll
@@ -448,8 +448,9 @@ norm_rope_write_kernel(const T* __restrict__ qkv, long long qkv_stride, b200dec_
   if constexpr (kKeep > 0) {
     const int qkp = (nq + nk) / 2, all = qkp + c.heads * c.v_dim / 2;
     float2 v[kKeep], w[kKeep], t[kKeep];
+    pdl_wait();
 #pragma unroll
-    for (int i = 0; i < kKeep; ++i) {  // nothing here waits for the kernel in front
+    for (int i = 0; i < kKeep; ++i) {
       const int p = tid + i * kNrThreads;
       if (p < qkp) {
         int h, pr;
@@ -458,7 +459,6 @@ norm_rope_write_kernel(const T* __restrict__ qkv, long long qkv_stride, b200dec_
         t[i] = pr < half ? cs[pr] : make_float2(1.f, 0.f);
       }
     }
-    pdl_wait();
 #pragma unroll
     for (int i = 0; i < kKeep; ++i) {
       const int p = tid + i * kNrThreads;

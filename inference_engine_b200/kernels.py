@@ -85,9 +85,11 @@ _early_start = False
 def set_early_start(enabled: bool) -> None:
     """Allow every kernel of this module to be brought up while the kernel enqueued just before it on
     the stream is still running (programmatic dependent launch).  A kernel reads only the step's
-    metadata (cu_seqlens, cu_cached, cached_lens, num_decoding, block table, tile_start, seq_ids)
-    before it waits for that kernel, and everything else afterwards.  Safe when no kernel that
-    directly precedes one of these ops on its stream writes those arrays, which holds for the engine:
+    metadata (cu_seqlens, cu_cached, cached_lens, num_decoding, block table, tile_start, seq_ids,
+    positions, state slots, token ids), the weights of the skinny matmul and those of the recurrent
+    layers' convolution before it waits for that kernel, and everything else (norm weights and angles
+    too) afterwards.  Safe when no kernel that precedes one of these ops on its stream, with ops of
+    this module alone in between, writes those arrays, which holds for the engine:
     it uploads them once per step, before the first layer (engine.py:347-356), and the ops are
     preceded by GEMMs or by one another (architecture.py:99-198).  Off by default."""
     global _early_start

@@ -434,3 +434,52 @@ def test_router_takes_rows_that_are_not_numbers():
     keep = [i for i in range(9) if i != 3]
     y2, places2 = ops.mixture(x[keep].contiguous(), x[keep].to(torch.bfloat16), ex)
     assert torch.equal(y[places[keep].long()].sum(1), y2[places2.long()].sum(1))
+
+
+@pytest.mark.parametrize("op", ["norm", "sum and norm", "rotation of many rows", "rotation of few rows", "whole norms by eights", "whole norms by pairs", "whole norms of any size"])
+def test_chained_launches_wait_for_weights_and_angles(op):
+    """The kernel in front writes the norm weights or the angle table of the one behind, which may be brought up meanwhile: it reads neither early."""
+    from inference_engine_b200 import kernels as K
+    from inference_engine_b200 import ops
+
+    g = torch.Generator(device=DEV).manual_seed(3)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    width = 5120 if op == "wide norm" else 2048
+    front, ones = rnd(2000, width), torch.ones(width, device=DEV)
+    made = front.clone()  # what the kernel in front writes, its last rows last
+    n, heads, kv = 300 if "many" in op else 40, 16, 8
+    dim = {"whole norms by pairs": 60, "whole norms of any size": 75}.get(op, 64)
+    cache = ops.make_paged_kv(n, kv, 16, dim, dim, torch.bfloat16, DEV)
+    rows = ops.Rows(n, i32(np.arange(n) % 16), i32([n]), i32(np.arange(n)[:, None]))
+    qkv = rnd(n, (heads + 2 * kv) * dim).to(torch.bfloat16)
+    x, delta = rnd(400, width), rnd(1600, width).to(torch.bfloat16)
+    places = torch.randperm(1600, generator=g, device=DEV).int().view(400, 4)
+
+    def behind(x):
+        w = made[-1]
+        if "norm" in op and "whole" not in op:
+            some = "sum" in op
+            return [ops.scaled_add_norm(x, delta if some else None, w, 1.5, 1e-5, torch.bfloat16, places if some else None)[1]]
+        angles = made[-4:].view(-1)[: 16 * 32 * 2].view(16, 32, 2) if dim == 64 else made[-4:].view(-1)[: 16 * 20 * 2].view(16, 20, 2)
+        if "whole" in op:
+            q = ops.norm_rope_write(qkv, rows, cache, made[-3:].view(-1)[: heads * dim], made[-1, : kv * dim], 1e-5, angles, heads)
+        else:
+            q = ops.rope_write(qkv, rows, cache, angles, heads, True, True, 1e-5)
+        return [q, cache.k.clone()]
+
+    def run():
+        mine = x.clone()
+        made.copy_(front)
+        ops.scaled_add_norm(made, None, ones, 1.0, 1e-5, torch.bfloat16)
+        return behind(mine)  # nothing stands between the two
+
+    want = run()
+    K.set_early_start(True)
+    try:
+        for _ in range(10):
+            made.fill_(float("nan"))
+            for got, w in zip(run(), want):
+                assert torch.equal(got, w)
+    finally:
+        K.set_early_start(False)
+    H.status_clear()
