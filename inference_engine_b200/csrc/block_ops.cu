@@ -27,7 +27,7 @@ __device__ __forceinline__ uint4 bo_pack(const float (&f)[8]) {
 
 // grid (N, ceil(D / 2048)): out[row, d] = bf16((gate * sigmoid(gate)) * up), gate = in[row, d], up = in[row, D + d]
 __global__ void __launch_bounds__(kBoThreads)
-silu_mul_kernel(const uint16_t* __restrict__ in, long long in_stride, uint16_t* __restrict__ out, long long out_stride,
+silu_mul_kernel(const uint16_t* in, long long in_stride, uint16_t* __restrict__ out, long long out_stride,
                 int D) {
   pdl_enter();
   const int col = (blockIdx.y * kBoThreads + threadIdx.x) * kBoVec;
@@ -45,8 +45,8 @@ silu_mul_kernel(const uint16_t* __restrict__ in, long long in_stride, uint16_t* 
 // grid (N), one CTA per row: new_residual = bf16(residual + delta); normed = bf16((new_residual * inv_rms) * w)
 // with inv_rms = 1 / sqrt(sum(new_residual^2) / D + eps) over the bf16-rounded new residual.
 __global__ void __launch_bounds__(kBoThreads)
-add_rms_norm_kernel(const uint16_t* __restrict__ residual, long long r_stride, const uint16_t* __restrict__ delta,
-                    long long d_stride, const uint16_t* __restrict__ weight, uint16_t* __restrict__ new_residual,
+add_rms_norm_kernel(const uint16_t* residual, long long r_stride, const uint16_t* delta,
+                    long long d_stride, const uint16_t* weight, uint16_t* __restrict__ new_residual,
                     long long nr_stride, uint16_t* __restrict__ normed, long long nn_stride, int D, float eps) {
   __shared__ float part[kBoThreads / 32];
   pdl_enter();

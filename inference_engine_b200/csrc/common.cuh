@@ -49,6 +49,8 @@ inline CacheView make_view(const b200kv_cache* c, const b200kv_table* t) {
 // attribute is only set while b200kv_set_chained_launch(1) is in force.
 bool take_chained_launch();  // whether the launch at hand is chained: asked once for each, as the first one behind a fork or join of branches is not
 bool take_plain_launch();    // whether it is such a first one
+// What a kernel may not read before the wait is not declared `const ... __restrict__`: the compiler takes such memory to be constant while
+// the kernel runs and moves its loads in front of the wait (the norm weights of rows of 5120 channels were read that way).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // First statement of every kernel.  The trigger may come this early: the next kernel cannot be brought up before

@@ -1011,7 +1011,7 @@ __device__ __forceinline__ unsigned long long gtime() {
 // 73 KB instead of 96; twelve layers of one entry of 128 tokens 110.6 -> 108.6 us).
 template <bool kScalar, bool kAlign, bool kPlanned>
 __global__ void __launch_bounds__(kWarps * 32, kCtasPerSm)
-decode_attn_kernel(const uint16_t* __restrict__ q, long long q_sb, long long q_sh, CacheView c,
+decode_attn_kernel(const uint16_t* q, long long q_sb, long long q_sh, CacheView c,
                    const int32_t* __restrict__ cached_lens, const int32_t* __restrict__ num_decoding, float scale_log2,
                    uint16_t* __restrict__ out, long long o_sb, long long o_sh, uint8_t* __restrict__ workspace, int B,
                    int G, int W, int fused, int early, const int* __restrict__ plan, int32_t* status) {
@@ -1315,7 +1315,7 @@ decode_attn_kernel(const uint16_t* __restrict__ q, long long q_sb, long long q_s
 // sums are added through shared memory - so even a sequence cut into 64 pieces costs a few rounds
 // of memory latency, not 64.
 __global__ void __launch_bounds__(kD)
-decode_combine_kernel(const uint8_t* __restrict__ workspace, const int32_t* __restrict__ num_decoding,
+decode_combine_kernel(const uint8_t* workspace, const int32_t* __restrict__ num_decoding,
                       uint16_t* __restrict__ out, long long o_sb, long long o_sh, int B, int Hkv, int G, int W) {
   __shared__ float wgt_s[kD];
   __shared__ float red_s[4];

@@ -16,7 +16,7 @@ constexpr int kRtMaxExperts = 1024;
 // kSteps: steps of weights in flight, which are its chain; eight take the registers of half the blocks.
 template <int kR, int kSteps>
 __global__ void __launch_bounds__(kRtWarps * 32, kSteps > 2 ? 2 : 4)
-router_kernel(const float* __restrict__ x, const uint16_t* __restrict__ w, int N, int width, int E, int top, int slices,
+router_kernel(const float* x, const uint16_t* w, int N, int width, int E, int top, int slices,
               int32_t* __restrict__ ids, float* __restrict__ scores, int32_t* __restrict__ ranks, int32_t* __restrict__ counts) {
   extern __shared__ __align__(16) float rt_smem[];
   const int pitch = (width + 3) & ~3;
@@ -149,8 +149,8 @@ __device__ __forceinline__ int dp_scan(int v, int* shared, int* sum) {
 // also writes the tile list.
 template <typename T>
 __global__ void __launch_bounds__(kDpThreads)
-dispatch_kernel(const T* __restrict__ xb, const int32_t* __restrict__ ids, const float* __restrict__ scores,
-                const int32_t* __restrict__ ranks, const int32_t* __restrict__ counts, int N, int width, int E, int top, int tile_rows,
+dispatch_kernel(const T* xb, const int32_t* ids, const float* scores,
+                const int32_t* ranks, const int32_t* counts, int N, int width, int E, int top, int tile_rows,
                 T* __restrict__ x_sorted, float* __restrict__ score_sorted, int32_t* __restrict__ slots, int32_t* __restrict__ tiles,
                 int max_tiles, int32_t* __restrict__ done) {
   __shared__ int first[kRtMaxExperts];
@@ -218,8 +218,8 @@ __device__ __forceinline__ float gated_unit(float g, float u, float limit, float
 
 template <typename T>
 __global__ void __launch_bounds__(kGsThreads)
-grouped_linear_simt_kernel(const T* __restrict__ x, const T* __restrict__ w, const int32_t* __restrict__ tiles, int out_rows, int width,
-                           const float* __restrict__ score_sorted, int act, float limit, float slope, T* __restrict__ y) {
+grouped_linear_simt_kernel(const T* x, const T* w, const int32_t* tiles, int out_rows, int width,
+                           const float* score_sorted, int act, float limit, float slope, T* __restrict__ y) {
   __shared__ float xs[kGsStep][kGsRows + 1];
   __shared__ float ws[kGsStep][kGsCols + 1];
   pdl_enter();

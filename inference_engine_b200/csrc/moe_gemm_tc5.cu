@@ -111,8 +111,8 @@ struct MgMaps {
 // kMode 0: a product; 1: one with the gated unit; 2: that, then the second product on what it wrote.
 template <int kN, int kMode>
 __global__ void __launch_bounds__(kMgThreads, 1)
-grouped_linear_tc5_kernel(const __grid_constant__ MgMaps<kMode> maps, const int32_t* __restrict__ tiles, int max_tiles, int experts, int total_rows,
-                          const MgProduct p1, const MgProduct p2, int32_t* done, const float* __restrict__ score_sorted, float limit, float slope,
+grouped_linear_tc5_kernel(const __grid_constant__ MgMaps<kMode> maps, const int32_t* tiles, int max_tiles, int experts, int total_rows,
+                          const MgProduct p1, const MgProduct p2, int32_t* done, const float* score_sorted, float limit, float slope,
                           int32_t* status) {
   using S = MgShape<kN>;
   extern __shared__ uint8_t mg_raw[];

@@ -106,7 +106,7 @@ struct PdCursor {
 
 template <int KB, int VB, bool kWide, int kCtas>
 __global__ void __launch_bounds__(kPdThreads, kCtas)
-paged_decode_kernel(const uint16_t* __restrict__ q, DecCache c, const int32_t* __restrict__ cached_lens,
+paged_decode_kernel(const uint16_t* q, DecCache c, const int32_t* __restrict__ cached_lens,
                     const int32_t* __restrict__ num_decoding, int B, int heads, int groups, float scale_log2, DecAttnOpt opt,
                     uint16_t* __restrict__ out, int zero_idle, int* __restrict__ counters, float* __restrict__ parts, int box_rows, int32_t* status,
                     const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v) {

@@ -21,7 +21,7 @@ __device__ __forceinline__ float2 rw_load2(const float* p) { return *reinterpret
 // kPairs: head sizes, half and the row stride are even, so both channels are loaded and rotated together.
 template <typename T, bool kPairs, int kMax>
 __global__ void __launch_bounds__(kRwWarps * 32)
-rope_write_kernel(const T* __restrict__ qkv, long long qkv_stride, b200dec_rows rows, DecCache c, const float* __restrict__ cos_sin,
+rope_write_kernel(const T* qkv, long long qkv_stride, b200dec_rows rows, DecCache c, const float* cos_sin,
                   int table_len, int half, int heads, int write_kv, int unit_norm, float eps, T* __restrict__ q_out, int32_t* status) {
   pdl_enter();
   const int hkv = write_kv ? c.heads : 0, per_row = heads + 2 * hkv;
@@ -155,7 +155,7 @@ __device__ __forceinline__ void ld_floats8(const float* p, float (&f)[8]) { ld_v
 // 1024 rows of 32 heads of 128 13.4 -> 7.5, 300 rows 6.1 -> 5.2, 60 rows 4.0 -> 4.4; 200 rows in fp32 7.7 -> 6.9.
 template <typename T, int kLanes>
 __global__ void __launch_bounds__(512)
-rope_rows_kernel(const T* __restrict__ qkv, long long qkv_stride, b200dec_rows rows, DecCache c, const float* __restrict__ cos_sin,
+rope_rows_kernel(const T* qkv, long long qkv_stride, b200dec_rows rows, DecCache c, const float* cos_sin,
                  int table_len, int half, int heads, int write_kv, int unit_norm, float eps, T* __restrict__ q_out, int32_t* status) {
   constexpr int kAtOnce = 2;  // heads of a group of lanes whose loads are in flight together
   pdl_enter();
@@ -268,8 +268,8 @@ rope_rows_kernel(const T* __restrict__ qkv, long long qkv_stride, b200dec_rows r
 // fit a multiprocessor.  1024 rows of 32 heads of 128 16.4 -> 7.1 us; of 48 heads of 64 15.4 -> 6.7, 64 rows of these 6.0 -> 4.1.
 template <typename T, int kVecs>
 __global__ void __launch_bounds__(512)
-norm_rope_rows_kernel(const T* __restrict__ qkv, long long qkv_stride, b200dec_rows rows, DecCache c, const float* __restrict__ q_norm,
-                      const float* __restrict__ k_norm, float eps, const float* __restrict__ cos_sin, int table_len, int half, int heads,
+norm_rope_rows_kernel(const T* qkv, long long qkv_stride, b200dec_rows rows, DecCache c, const float* q_norm,
+                      const float* k_norm, float eps, const float* cos_sin, int table_len, int half, int heads,
                       int k_shift, int v_shift, T* __restrict__ q_out, int32_t* status) {
   __shared__ float part[2][16];
   pdl_enter();
@@ -390,8 +390,8 @@ __device__ __forceinline__ void nr_split(int p, int pairs, int shift, int& head,
 // weights and angles are loaded beside them.  0: any sizes, the row is read twice.
 template <typename T, int kKeep>
 __global__ void __launch_bounds__(kNrThreads)
-norm_rope_write_kernel(const T* __restrict__ qkv, long long qkv_stride, b200dec_rows rows, DecCache c, const float* __restrict__ q_norm,
-                       const float* __restrict__ k_norm, float eps, const float* __restrict__ cos_sin, int table_len, int half, int heads,
+norm_rope_write_kernel(const T* qkv, long long qkv_stride, b200dec_rows rows, DecCache c, const float* q_norm,
+                       const float* k_norm, float eps, const float* cos_sin, int table_len, int half, int heads,
                        int k_shift, int v_shift, T* __restrict__ q_out, int32_t* status) {
   __shared__ float part[2][kNrThreads / 32];
   pdl_enter();
@@ -532,7 +532,7 @@ constexpr int kArPieces = 8;  // channels of the output per thread: v_dim up to 
 
 template <typename T>
 __global__ void __launch_bounds__(kArThreads)
-attn_rows_kernel(const T* __restrict__ q, DecCache c, b200dec_rows rows, int heads, float scale, DecAttnOpt opt, T* __restrict__ out,
+attn_rows_kernel(const T* q, DecCache c, b200dec_rows rows, int heads, float scale, DecAttnOpt opt, T* __restrict__ out,
                  int32_t* status) {
   extern __shared__ float ar_smem[];
   float* qs = ar_smem;                                                  // [k_dim]
@@ -680,7 +680,7 @@ __host__ __device__ constexpr size_t at_floats(int k_row, int v_row) {
 
 template <typename T, int kPieces>  // kPieces: output channels, in pieces of 128
 __global__ void __launch_bounds__(kAtThreads, 2)
-attn_tile_kernel(const T* __restrict__ q, DecCache c, b200dec_rows rows, const int32_t* __restrict__ cu_seqlens, int num_entries, int heads, int slice_heads, float scale, DecAttnOpt opt,
+attn_tile_kernel(const T* q, DecCache c, b200dec_rows rows, const int32_t* __restrict__ cu_seqlens, int num_entries, int heads, int slice_heads, float scale, DecAttnOpt opt,
                  T* __restrict__ out, int32_t* status) {
   extern __shared__ __align__(16) float at_smem[];
   const int splits = gridDim.z, part = blockIdx.z;  // of the cluster's blocks

@@ -63,11 +63,11 @@ __device__ __forceinline__ void load_tile(uint32_t dst, const uint16_t* src, lon
 }
 
 __global__ void __launch_bounds__(kPfWarps * 32)
-prefill_attn_kernel(const uint16_t* __restrict__ q, long long q_sn, long long q_sh, const uint16_t* __restrict__ k,
-                    long long k_sn, long long k_sh, const uint16_t* __restrict__ v, long long v_sn, long long v_sh,
+prefill_attn_kernel(const uint16_t* q, long long q_sn, long long q_sh, const uint16_t* k,
+                    long long k_sn, long long k_sh, const uint16_t* v, long long v_sn, long long v_sh,
                     const int32_t* __restrict__ seq_ids, const int32_t* __restrict__ cu_seqlens,
-                    const int32_t* __restrict__ tile_start, int block_m, int subs, const uint16_t* __restrict__ k_prefix,
-                    const uint16_t* __restrict__ v_prefix, long long p_sh, long long p_sn,
+                    const int32_t* __restrict__ tile_start, int block_m, int subs, const uint16_t* k_prefix,
+                    const uint16_t* v_prefix, long long p_sh, long long p_sn,
                     const int32_t* __restrict__ cu_cached, uint16_t* __restrict__ out, long long o_sn, long long o_sh,
                     int N, int G, float scale_log2) {
   extern __shared__ __align__(128) uint8_t pf_smem[];

@@ -358,7 +358,7 @@ constexpr int kRsTokens = 16;  // tokens prepared in shared memory at a time
 // columns of one head of one entry.
 template <typename T, int kRows, int kLanes>
 __global__ void __launch_bounds__(kRsThreads)
-recurrence_scan_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, const T* __restrict__ conv, int conv_stride,
+recurrence_scan_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, const T* conv, int conv_stride,
                        const b200dec_entries ent, float* __restrict__ out, int slabs, int32_t* status) {
   constexpr int kDim = kRows * kLanes, kCols = kRsThreads / kLanes;
   extern __shared__ __align__(16) float rs_smem[];

@@ -57,7 +57,7 @@ __device__ __forceinline__ float rp_exchange(float (&v)[16], int lane) {
 // slower where they are not (23.5).
 template <typename T, int Dp, int kParts>
 __global__ void __launch_bounds__(128 * kParts)
-rb_prepare_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, const T* __restrict__ conv, int conv_stride,
+rb_prepare_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, const T* conv, int conv_stride,
                   const b200dec_entries ent, float* __restrict__ ws, int32_t* status) {
   constexpr int kChannels = 128, kRpHalf = kRbTok / kParts, kLanes = 16 * kParts;
   constexpr bool kOne = Dp <= kChannels;  // a thread's channel stays in registers
@@ -347,8 +347,8 @@ __device__ __forceinline__ void rb_row8(const float* p, float (&row)[kRbTok]) {
 // One block: kRbWarps warps, 32 kRbCols / kLanes columns each, of one head of one entry.
 template <typename T, int kLanes, int kR>
 __global__ void __launch_bounds__(32 * kRbWarps)
-rb_scan_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, const T* __restrict__ conv, int conv_stride,
-               const b200dec_entries ent, const float* __restrict__ ws, float* __restrict__ out, int slabs, int32_t* status) {
+rb_scan_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, const T* conv, int conv_stride,
+               const b200dec_entries ent, const float* ws, float* __restrict__ out, int slabs, int32_t* status) {
   constexpr int Dp = kLanes * kR, kFloats = rb_floats(Dp), kQuads = kR / 4, kGroups = 32 / kLanes;
   constexpr int kM = kLanes / 8, kC = kRbCols / kM;  // after the exchange a lane holds kC columns of one token
   extern __shared__ __align__(128) float rb_smem[];  // [kRbStages][kFloats]
@@ -459,8 +459,8 @@ rb_scan_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, con
 // end by another, which the fetching lane of a reading warp waits for.  The arithmetic is the same, bit for bit.
 template <typename T, int kLanes, int kR>
 __global__ void __launch_bounds__(64 * kRbWarps, 3)
-rb_scan_split_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, const T* __restrict__ conv, int conv_stride,
-                     const b200dec_entries ent, const float* __restrict__ ws, float* __restrict__ out, int slabs, int32_t* status) {
+rb_scan_split_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, const T* conv, int conv_stride,
+                     const b200dec_entries ent, const float* ws, float* __restrict__ out, int slabs, int32_t* status) {
   constexpr int Dp = kLanes * kR, kFloats = rb_floats(Dp), kQuads = kR / 4, kGroups = 32 / kLanes;
   constexpr int kM = kLanes / 8, kC = kRbCols / kM;  // after the exchange a lane holds kC columns of one token
   extern __shared__ __align__(128) float rb_smem[];  // [kRbStages][kFloats]

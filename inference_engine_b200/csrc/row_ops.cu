@@ -22,7 +22,7 @@ __device__ __forceinline__ float row_sum(float v) {
 
 template <typename T>
 __global__ void __launch_bounds__(kRowThreads)
-embed_kernel(const T* __restrict__ table, const int32_t* __restrict__ ids, float* __restrict__ x, T* __restrict__ xb, int width,
+embed_kernel(const T* table, const int32_t* __restrict__ ids, float* __restrict__ x, T* __restrict__ xb, int width,
              int vocab, int32_t* status) {
   pdl_enter();
   const long long r = blockIdx.x;
@@ -59,8 +59,8 @@ struct __align__(4 * sizeof(T)) Raw4 {
 // delta each), us: 64 x 2048 (2) 6.1 -> 3.9, (1) 4.0 -> 2.6; 1024 x 2048 (4) 10.5 -> 9.1, (1) 7.5 -> 4.6.
 template <typename T, int kChunks, int kAtOnce>
 __global__ void __launch_bounds__(kRowThreads)
-scaled_add_norm_kernel(const float* x, const T* __restrict__ delta, const int32_t* __restrict__ index, int top,
-                       const float* __restrict__ weight, float alpha, float eps, float* x_out, T* __restrict__ xb_out,
+scaled_add_norm_kernel(const float* x, const T* delta, const int32_t* index, int top,
+                       const float* weight, float alpha, float eps, float* x_out, T* __restrict__ xb_out,
                        int width, int32_t* __restrict__ zero, int num_zero) {
   pdl_enter();
   pdl_wait();
@@ -128,8 +128,8 @@ scaled_add_norm_kernel(const float* x, const T* __restrict__ delta, const int32_
 // Any width: the sums are kept in dynamic shared memory.
 template <typename T>
 __global__ void __launch_bounds__(kRowThreads)
-scaled_add_norm_any_kernel(const float* x, const T* __restrict__ delta, const int32_t* __restrict__ index, int top,
-                           const float* __restrict__ weight, float alpha, float eps, float* x_out,
+scaled_add_norm_any_kernel(const float* x, const T* delta, const int32_t* index, int top,
+                           const float* weight, float alpha, float eps, float* x_out,
                            T* __restrict__ xb_out, int width, int32_t* __restrict__ zero, int num_zero) {
   extern __shared__ float srow[];
   pdl_enter();
@@ -157,7 +157,7 @@ scaled_add_norm_any_kernel(const float* x, const T* __restrict__ delta, const in
 // 0: any width, y is read twice.
 template <typename T, int kChunks>
 __global__ void __launch_bounds__(kRowThreads)
-norm_add_kernel(float* x, const T* __restrict__ y, const float* __restrict__ weight, float mult, float eps, T* __restrict__ xb, int width) {
+norm_add_kernel(float* x, const T* y, const float* weight, float mult, float eps, T* __restrict__ xb, int width) {
   pdl_enter();
   pdl_wait();
   const long long at = (long long)blockIdx.x * width;
@@ -204,7 +204,7 @@ norm_add_kernel(float* x, const T* __restrict__ y, const float* __restrict__ wei
 // kVec channels (8, or 1 for any size) of one row per thread.
 template <typename T, int kVec>
 __global__ void __launch_bounds__(kRowThreads)
-silu_mul_rows_kernel(const T* __restrict__ gu, long long stride, T* __restrict__ out, long long out_stride, int rows, int ff) {
+silu_mul_rows_kernel(const T* gu, long long stride, T* __restrict__ out, long long out_stride, int rows, int ff) {
   pdl_enter();
   pdl_wait();
   const long long r = blockIdx.x;
@@ -223,8 +223,8 @@ silu_mul_rows_kernel(const T* __restrict__ gu, long long stride, T* __restrict__
 // neighbouring channels at a time, kKeep such groups in registers per thread (0: read twice).
 template <typename T, int kThreads, int kVec, int kKeep>
 __global__ void __launch_bounds__(kRowThreads)
-gated_norm_kernel(const float* __restrict__ o, const T* __restrict__ gate, long long gate_stride, int gate_first,
-                  const float* __restrict__ weight, int weight_len, int weight_vec, float eps, float out_scale, T* __restrict__ out,
+gated_norm_kernel(const float* o, const T* gate, long long gate_stride, int gate_first,
+                  const float* weight, int weight_len, int weight_vec, float eps, float out_scale, T* __restrict__ out,
                   long long out_stride, int rows, int len, int parts) {
   pdl_enter();
   const int part = len / parts;

@@ -59,7 +59,7 @@ __device__ __forceinline__ void block_best(float& v, int& i) {
 
 // grid (B, ceil(V / 2048)).  logits bf16 (elem_bytes 2) or fp32 (4), row stride in elements.
 __global__ void __launch_bounds__(kSmThreads)
-sample_stage1_kernel(const void* __restrict__ logits, long long stride, int elem_bytes, const long long* __restrict__ seed,
+sample_stage1_kernel(const void* logits, long long stride, int elem_bytes, const long long* seed,
                      float tau, float* __restrict__ part_val, int* __restrict__ part_idx, int V) {
   pdl_enter();
   pdl_wait();  // the logits (and the seed, advanced by the previous call) come from the kernels before this one
@@ -85,7 +85,7 @@ sample_stage1_kernel(const void* __restrict__ logits, long long stride, int elem
 
 // grid (B).  The seed advances by one per call (kernels.py:1369), here, after every stage-1 CTA has read it.
 __global__ void __launch_bounds__(kSmThreads)
-sample_stage2_kernel(const float* __restrict__ part_val, const int* __restrict__ part_idx, int nblk, long long* __restrict__ out,
+sample_stage2_kernel(const float* part_val, const int* part_idx, int nblk, long long* __restrict__ out,
                      long long out_stride, long long* __restrict__ seed) {
   pdl_enter();
   pdl_wait();

@@ -109,7 +109,7 @@ __host__ __device__ constexpr int ss_blocks(int kn16, bool local, bool crowd) {
 // Workspace: 2 * kSsSegments places of [head][16 columns][8 channels][lane][4], then [kSsSegments][head] sums of log-decays.
 template <int kN16, bool kLocal, bool kCrowd>
 __global__ void __launch_bounds__(32 * kSsWarps, ss_blocks(kN16, kLocal, kCrowd))
-ssd_scan_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, const uint16_t* __restrict__ conv, int conv_stride,
+ssd_scan_kernel(const b200dec_recurrence rec, const b200dec_recurrence_in in, const uint16_t* conv, int conv_stride,
                 const b200dec_entries ent, float* __restrict__ out, int slabs, int max_segments, float* ws, int32_t* status) {
   constexpr int kN = 16 * kN16, kRow = kN + 8;  // bf16 per row of b and c in shared memory
   constexpr uint32_t kStage = kSsTok * (2 * kRow + kSsXRow) * 2;

@@ -170,12 +170,12 @@ __device__ __forceinline__ void quantize_store(const float (&x)[4], int8_t* code
 // grid (B, ceil((Hq + 2*Hkv) / 8)), 256 threads.  Warp job j: [0,Hq) q heads, [Hq,Hq+Hkv) k
 // heads, [Hq+Hkv, Hq+2Hkv) v heads.  kernels.py:364-480.
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
-write_decode_kernel(const uint16_t* __restrict__ q, long long q_sb, long long q_sh,
-                    const uint16_t* __restrict__ k, long long k_sb, long long k_sh,
-                    const uint16_t* __restrict__ v, long long v_sb, long long v_sh,
-                    const uint16_t* __restrict__ qw, const uint16_t* __restrict__ kw,
-                    const uint16_t* __restrict__ cosp, long long cos_sb,
-                    const uint16_t* __restrict__ sinp, long long sin_sb,
+write_decode_kernel(const uint16_t* q, long long q_sb, long long q_sh,
+                    const uint16_t* k, long long k_sb, long long k_sh,
+                    const uint16_t* v, long long v_sb, long long v_sh,
+                    const uint16_t* qw, const uint16_t* kw,
+                    const uint16_t* cosp, long long cos_sb,
+                    const uint16_t* sinp, long long sin_sb,
                     CacheView c, const int32_t* __restrict__ cached_lens, const int32_t* __restrict__ num_decoding,
                     uint16_t* __restrict__ q_out, long long o_sb, long long o_sh, int Hq, float eps, int32_t* status) {
   __shared__ __align__(16) float sq_all[kWarpsPerBlock][kD];
@@ -243,11 +243,11 @@ write_decode_kernel(const uint16_t* __restrict__ q, long long q_sb, long long q_
 // ------------------------------------------------------------------ prefill norm + rope
 // grid (N, ceil((Hq+Hkv)/8)); kernels.py:547-670.  Outputs rounded to bf16 (nearest even).
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
-norm_rope_prefill_kernel(const uint16_t* __restrict__ q, long long q_sn, long long q_sh,
-                         const uint16_t* __restrict__ k, long long k_sn, long long k_sh,
-                         const uint16_t* __restrict__ qw, const uint16_t* __restrict__ kw,
-                         const uint16_t* __restrict__ cosp, long long cos_sn,
-                         const uint16_t* __restrict__ sinp, long long sin_sn,
+norm_rope_prefill_kernel(const uint16_t* q, long long q_sn, long long q_sh,
+                         const uint16_t* k, long long k_sn, long long k_sh,
+                         const uint16_t* qw, const uint16_t* kw,
+                         const uint16_t* cosp, long long cos_sn,
+                         const uint16_t* sinp, long long sin_sn,
                          uint16_t* __restrict__ q_out, long long qo_sn, long long qo_sh,
                          uint16_t* __restrict__ k_out, long long ko_sn, long long ko_sh,
                          int Hq, int Hkv, float eps) {
@@ -340,11 +340,11 @@ __host__ __device__ constexpr int row_jobs(int heads, int per_warp) { return (he
 
 template <bool kFusedNorm, int kHeads, int kKv>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, kHeads == 1 ? 6 : 1)
-prefill_rows_kernel(const uint16_t* __restrict__ q, long long q_sn, long long q_sh,
-                    const uint16_t* __restrict__ k, long long k_sn, long long k_sh,
-                    const uint16_t* __restrict__ v, long long v_sn, long long v_sh,
-                    const uint16_t* __restrict__ qw, const uint16_t* __restrict__ kw,
-                    const uint16_t* __restrict__ cosp, long long cos_sn, const uint16_t* __restrict__ sinp, long long sin_sn,
+prefill_rows_kernel(const uint16_t* q, long long q_sn, long long q_sh,
+                    const uint16_t* k, long long k_sn, long long k_sh,
+                    const uint16_t* v, long long v_sn, long long v_sh,
+                    const uint16_t* qw, const uint16_t* kw,
+                    const uint16_t* cosp, long long cos_sn, const uint16_t* sinp, long long sin_sn,
                     uint16_t* __restrict__ q_out, long long qo_sn, long long qo_sh,
                     uint16_t* __restrict__ k_out, long long ko_sn, long long ko_sh,
                     CacheView c, const int32_t* __restrict__ cu, int num_entries, const int32_t* __restrict__ cached_lens,
@@ -472,7 +472,7 @@ constexpr int kFirstCtas = 8, kFirstWarps = 16, kFirstLanes = 4, kFirstTeams = 4
 // took 84 us, 59 now; 12 of 2000 65.6 and 60; one portion 7.55 and 7.4; five prompts of 1011 rows, with all else of two layers, 75.8
 // and 70.9.
 __global__ void __launch_bounds__(kFirstWarps * 32, 2)
-first_chunk_k_kernel(const uint16_t* __restrict__ k, long long k_sn, long long k_sh, CacheView c,
+first_chunk_k_kernel(const uint16_t* k, long long k_sn, long long k_sh, CacheView c,
                      const int32_t* __restrict__ cu, int num_entries, const int32_t* __restrict__ cached_lens,
                      const int32_t* __restrict__ num_decoding, int N, int32_t* status) {
   __shared__ __align__(16) float part[kFirstWarps][kD];

@@ -436,7 +436,7 @@ def test_router_takes_rows_that_are_not_numbers():
     assert torch.equal(y[places[keep].long()].sum(1), y2[places2.long()].sum(1))
 
 
-@pytest.mark.parametrize("op", ["norm", "sum and norm", "rotation of many rows", "rotation of few rows", "whole norms by eights", "whole norms by pairs", "whole norms of any size"])
+@pytest.mark.parametrize("op", ["norm", "sum and norm", "wide norm", "rotation of many rows", "rotation of few rows", "whole norms by eights", "whole norms by pairs", "whole norms of any size"])
 def test_chained_launches_wait_for_weights_and_angles(op):
     """The kernel in front writes the norm weights or the angle table of the one behind, which may be brought up meanwhile: it reads neither early."""
     from inference_engine_b200 import kernels as K
