@@ -247,12 +247,14 @@ int b200kv_get_chained_launch(void);
  * _next, between one _next and another, and between the last of them and _end forms a branch each.  All start behind what the stream held
  * before, and what follows _end waits for all.  May be nested; every _begin needs its _end, on the same thread.  Not recording (or
  * waiting for more nodes than 16): _begin returns NULL, with which the other two do nothing, and the calls run in order.
- * The first launch of a branch and the first behind _end are not chained.  Memory that a branch allocates in stream order must not be given back before _end. */
+ * The first launch of a branch and the first behind _end on `stream` are not chained, whatever the thread launches on other
+ * streams in between.  Memory that a branch allocates in stream order must not be given back before _end. */
 void* b200kv_branches_begin(void* stream);
 int b200kv_branches_next(void* branches);
 int b200kv_branches_end(void* branches);
-/* This thread's next launch is not chained: for a library whose kernel may be the first behind branches of another one. */
-void b200kv_plain_launch(void);
+/* This thread's next launch of this library on `stream` is not chained if nothing is recorded there before it: for a library whose kernel
+ * may be the first of a branch, or behind branches, of another one. */
+void b200kv_plain_next(void* stream);
 
 /* Bytes of fp32 workspace b200kv_decode_attn needs for a batch of B entries on a device with
  * `sm_count` SMs (replaces the three partial buffers of kernels.py:305-311).

@@ -114,7 +114,7 @@ SIGNATURES = {
                                        c_int32, c_void_p, c_void_p]),
     "b200kv_set_chained_launch": (None, [c_int32]),
     "b200kv_get_chained_launch": (c_int32, []),
-    "b200kv_plain_launch": (None, []),
+    "b200kv_plain_next": (None, [c_void_p]),
     "b200kv_branches_begin": (c_void_p, [c_void_p]),
     "b200kv_branches_next": (c_int32, [c_void_p]),
     "b200kv_branches_end": (c_int32, [c_void_p]),
@@ -180,7 +180,7 @@ DECODER_SIGNATURES = {
                                          c_void_p, c_int32, c_float, c_float, c_void_p, c_int32, c_int32, c_void_p, c_void_p]),
 }
 SHARED_SIGNATURES = ("b200kv_version", "b200kv_error_string", "b200kv_set_chained_launch", "b200kv_get_chained_launch",
-                     "b200kv_plain_launch", "b200kv_branches_begin", "b200kv_branches_next", "b200kv_branches_end", "b200kv_sample_workspace_bytes", "b200kv_sample")
+                     "b200kv_plain_next", "b200kv_branches_begin", "b200kv_branches_next", "b200kv_branches_end", "b200kv_sample_workspace_bytes", "b200kv_sample")
 
 _lib = None
 _decoder_lib = None

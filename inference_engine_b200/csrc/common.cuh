@@ -47,8 +47,8 @@ inline CacheView make_view(const b200kv_cache* c, const b200kv_table* t) {
 // memory itself, having read at most caller-provided metadata by then (and weights where b200kv_set_chained_launch says so), and (b) tells the stream when the next
 // kernel may be brought up (pdl_trigger).  Both are no-ops for a kernel launched the ordinary way; the launch
 // attribute is only set while b200kv_set_chained_launch(1) is in force.
-bool take_chained_launch();  // whether the launch at hand is chained: asked once for each, as the first one behind a fork or join of branches is not
-bool take_plain_launch();    // whether it is such a first one
+bool take_chained_launch(cudaStream_t stream);  // whether the launch at hand is chained: asked once for each, as the first one behind a fork or join of branches is not
+bool take_plain_launch(cudaStream_t stream);    // whether it is such a first one
 // What a kernel may not read before the wait is not declared `const ... __restrict__`: the compiler takes such memory to be constant while
 // the kernel runs and moves its loads in front of the wait (the norm weights of rows of 5120 channels were read that way).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -79,7 +79,7 @@ inline cudaError_t launch_kernel(bool chained, void (*kernel)(KArgs...), dim3 gr
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                                   Args... args) {
-  return launch_kernel(take_chained_launch(), kernel, grid, block, smem, stream, args...);
+  return launch_kernel(take_chained_launch(stream), kernel, grid, block, smem, stream, args...);
 }
 
 // Opts a kernel in to `most` bytes of dynamic shared memory (per function and device, so on every call): the most that any

@@ -1446,7 +1446,7 @@ static int launch_decode(const void* q, int64_t q_sb, int64_t q_sh, const b200kv
   const int grid = (int)std::max<long long>(1, std::min<long long>(sm_count * kCtasPerSm, want));
   const float scale_log2 = scale * 1.4426950408889634f;
   cudaStream_t s = (cudaStream_t)stream;
-  const int early = (!take_plain_launch() && (variant & 4) && fused) ? 1 : 0;  // the separate reduction kernel's prefix array is written before the wait
+  const int early = (!take_plain_launch(s) && (variant & 4) && fused) ? 1 : 0;  // the separate reduction kernel's prefix array is written before the wait
   const size_t smem = main_smem_bytes(scalar);
   auto pick = [&](auto planned) {
     constexpr bool kPlanned = decltype(planned)::value;

@@ -977,7 +977,7 @@ static cudaError_t launch_clusters(void (*kernel)(KArgs...), dim3 grid, dim3 blo
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = take_chained_launch() ? 2 : 1;
+  cfg.numAttrs = take_chained_launch(stream) ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 

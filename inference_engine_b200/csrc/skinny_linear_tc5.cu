@@ -297,7 +297,7 @@ static int sk_launch(const CUtensorMap& tm_w, const CUtensorMap& tm_x, uint16_t*
     attr[na].val.clusterDim.z = 1;
     ++na;
   }
-  if (take_chained_launch()) {
+  if (take_chained_launch(stream)) {
     attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[na].val.programmaticStreamSerializationAllowed = 1;
     ++na;

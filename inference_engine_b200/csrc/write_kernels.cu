@@ -784,7 +784,7 @@ static cudaError_t launch_first_chunk(const uint16_t* k, long long k_sn, long lo
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = take_chained_launch() ? 2 : 1;
+  cfg.numAttrs = take_chained_launch(s) ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, first_chunk_k_kernel, k, k_sn, k_sh, view, cu, num_entries, cached_lens, num_decoding, N,
                             status);
 }

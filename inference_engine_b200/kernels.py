@@ -119,20 +119,26 @@ class Branches:
         self.lib = lib
 
     def __enter__(self):
-        self.handle = self.lib.b200kv_branches_begin(_stream())
+        self.stream = _stream()
+        self.handle = self.lib.b200kv_branches_begin(self.stream)
+        self._tell_the_other()
         return self
+
+    def _tell_the_other(self) -> None:
+        for other in (_lib._lib, _lib._decoder_lib):
+            if self.handle is not None and other is not None and other is not self.lib:
+                other.b200kv_plain_next(self.stream)
 
     def next(self) -> None:
         if self.handle is not None:
             _lib.check(self.lib.b200kv_branches_next(self.handle), "branches")
+            self._tell_the_other()
 
     def __exit__(self, kind, value, trace):
         if self.handle is not None:
             rc = self.lib.b200kv_branches_end(self.handle)
+            self._tell_the_other()
             self.handle = None
-            for other in (_lib._lib, _lib._decoder_lib):
-                if other is not None:
-                    other.b200kv_plain_launch()
             if kind is None:
                 _lib.check(rc, "branches")
 

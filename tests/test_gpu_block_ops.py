@@ -127,3 +127,76 @@ def test_branches_at_the_start_of_a_graph(K):
         d = K.silu_mul(torch.cat([a, c], dim=1))
     graph.replay()
     assert torch.equal(d, K.silu_mul(torch.cat([K.silu_mul(x[0]), K.silu_mul(x[1])], dim=1)))
+
+
+def edges_of(body, *streams):
+    """What `body` records on each of the streams: (edges, chained ones among them)."""
+    import ctypes
+
+    from cuda.bindings import runtime as rt
+
+    driver = ctypes.CDLL("libcuda.so.1")
+
+    def ok(r):
+        assert r[0] == rt.cudaError_t.cudaSuccess, r
+        return r[1:]
+
+    for s in streams:
+        ok(rt.cudaStreamBeginCapture(s.cuda_stream, rt.cudaStreamCaptureMode.cudaStreamCaptureModeRelaxed))
+    try:
+        body()
+    finally:
+        graphs = [rt.cudaStreamEndCapture(s.cuda_stream) for s in streams]
+    out = []
+    for r in graphs:
+        (g,) = ok(r)
+        count = ctypes.c_size_t(64)
+        ends, data = (ctypes.c_void_p * 64)(), (ctypes.c_uint8 * 8 * 64)()  # data: from port, to port, type, reserved
+        assert driver.cuGraphGetEdges_v2(ctypes.c_void_p(int(g)), ends, (ctypes.c_void_p * 64)(), data, ctypes.byref(count)) == 0
+        out.append((count.value, sum(d[2] == 1 for d in data[: count.value])))
+        ok(rt.cudaGraphDestroy(g))
+    return out
+
+
+def test_first_launches_of_branches_and_behind_them_are_plain_on_their_stream_alone(K):
+    """Chained launches: neither launches on another stream in between nor branches of the other library change which ones are plain."""
+    from inference_engine_b200 import _lib
+
+    lib, dec = _lib.load(), _lib.load_decoder()
+    s, other = torch.cuda.Stream(), torch.cuda.Stream()
+    x, y = (torch.zeros(4, n, dtype=torch.bfloat16, device="cuda") for n in (128, 64))
+    silu = lambda on: _lib.check(lib.b200kv_silu_mul(x.data_ptr(), 128, y.data_ptr(), 64, 4, 64, on.cuda_stream), "silu_mul")
+    silu_dec = lambda on: _lib.check(dec.b200dec_silu_mul(x.data_ptr(), 128, 2, y.data_ptr(), 64, 4, 64, on.cuda_stream), "silu_mul")
+
+    def elsewhere():
+        silu(s)
+        b = lib.b200kv_branches_begin(s.cuda_stream)
+        silu(other)
+        silu(s)
+        assert lib.b200kv_branches_next(b) == 0
+        silu(other)
+        silu(s)
+        assert lib.b200kv_branches_end(b) == 0
+        silu(other)
+        silu(s)
+        silu(s)
+
+    def two_libraries():
+        silu_dec(s)
+        with torch.cuda.stream(s), K.Branches(lib) as b:
+            silu_dec(s)  # the first of its branch, though of the other library
+            b.next()
+            silu(s)
+        silu(s)  # behind the join: plain; from here on nothing is
+        silu_dec(s)
+        silu(s)
+
+    silu(s), silu_dec(s), torch.cuda.synchronize()
+    K.set_early_start(True)
+    try:
+        # 0 -> 1, 0 -> 2, 1 -> 3, 2 -> 3 plain, 3 -> 4 chained; the other stream's three launches a chain
+        assert edges_of(elsewhere, s, other) == [(5, 1), (2, 2)]
+        # 0 -> 1, 0 -> 2, 1 -> 3, 2 -> 3 plain, 3 -> 4 -> 5 chained
+        assert edges_of(two_libraries, s) == [(6, 2)]
+    finally:
+        K.set_early_start(False)
