@@ -136,8 +136,9 @@ typedef struct b200dec_attn_options {
 
 int b200dec_attn_rows_opt(const void* q, const b200dec_cache* cache, const b200kv_table* table, const b200dec_rows* rows, int32_t heads,
                           float scale, const b200dec_attn_options* opt, void* out, int32_t* status, void* stream);
-/* The same with the entries' first rows, cu_seqlens int32 [num_entries + 1]: entry e brings rows cu_seqlens[e] to cu_seqlens[e + 1] - 1 at
- * consecutive positions, and all rows belong to one.  No more blocks are launched than the rows need then.  NULL: as above. */
+/* The same with the entries' first rows, cu_seqlens int32 [num_entries + 1], ascending: entry e brings rows cu_seqlens[e] to cu_seqlens[e + 1] - 1.
+ * No more blocks are launched than the rows need then.  It says how the rows are shared out and no more: what a row is stands in seq_ids and
+ * positions, and rows that no entry brings are done as well.  NULL: as above. */
 int b200dec_attn_rows_entries(const void* q, const b200dec_cache* cache, const b200kv_table* table, const b200dec_rows* rows,
                               const int32_t* cu_seqlens, int32_t num_entries, int32_t heads, float scale, const b200dec_attn_options* opt, void* out,
                               int32_t* status, void* stream);

@@ -695,254 +695,265 @@ attn_tile_kernel(const T* q, DecCache c, b200dec_rows rows, const int32_t* __res
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int G = heads / c.heads, slices = (G + kAtSlots - 1) / kAtSlots;
   const int hk = blockIdx.x / slices, g0 = blockIdx.x % slices * slice_heads, gs = min(slice_heads, G - g0);
+  // Rows r0 to r0 + n - 1, of entry seq at the positions from pos on.
+  auto run = [&](const int r0, const int n, const int seq, const int pos) {
+    const int slots = n * gs;
+    for (int s = warp; s < kAtSlots; s += kWarps) {
+      const T* src = q + ((long long)(r0 + s / gs) * heads + hk * G + g0 + s % gs) * c.k_row;
+      for (int ch = lane; ch < c.k_row; ch += 32) qs[s * c.k_row + ch] = s < slots && ch < c.k_dim ? ld_elem(src + ch) * scale : 0.f;
+    }
+    // what this warp keeps: query rows kAtOwn warp + i
+    float m[kAtOwn], l[kAtOwn], o[kAtOwn][kPieces][4];
+    int last[kAtOwn], low[kAtOwn];  // the keys each of them sees
+#pragma unroll
+    for (int i = 0; i < kAtOwn; ++i) {
+      const int s = kAtOwn * warp + i, h = hk * G + g0 + s % gs;
+      last[i] = s < slots ? pos + s / gs : -1;
+      low[i] = s < slots && opt.window > 0 ? max(0, last[i] - opt.window + 1) : 0;
+      m[i] = opt.sink && s < slots && part == 0 ? opt.sink[h] : -INFINITY;
+      l[i] = opt.sink && part == 0 ? 1.f : 0.f;
+#pragma unroll
+      for (int j = 0; j < kPieces; ++j)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) o[i][j][k] = 0.f;
+    }
+    const bool mine = kAtOwn * warp < slots;
+    // Keys [all_low, all_last] are seen by every query row of the tile; the others are looked at one by one, so that what a row
+    // does not see (a later token, perhaps not a number) never meets it.
+    const int all_last = pos, all_low = opt.window > 0 ? max(0, pos + n - opt.window) : 0;
+    int first = opt.window > 0 ? max(0, pos - opt.window + 1) : 0, end = pos + n;
+    if (splits > 1) {  // this block's steps
+      const int share = ((end - first + kAtKeys - 1) / kAtKeys + splits - 1) / splits * kAtKeys;
+      first += part * share;
+      end = min(end, first + share);
+    }
+    // the rows of the keys from j0 on
+    auto look_up = [&](int j0, long long* at_rows) {
+      if (tid < kAtKeys) {
+        const int page = j0 + tid < end ? dec_page(c, seq, j0 + tid, status) : -1;
+        at_rows[tid] = page < 0 ? -1 : dec_row(c, page, hk, (j0 + tid) % c.P);
+      }
+    };
+    // their keys or values to shared memory, zero where there is none and behind `dim`
+    auto fetch = [&](const long long* at_rows, const void* cache, int row, int dim, float* to, int pitch) {
+      for (int k0 = warp; k0 < kAtKeys; k0 += 4 * kWarps) {
+        long long src[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) src[u] = at_rows[k0 + u * kWarps] * row;
+        for (int ch = 4 * lane; ch < row; ch += 128) {
+          float* d = to + k0 * pitch + ch;
+          if constexpr (sizeof(T) == 4) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              at_copy16(d + u * kWarps * pitch, (const float*)cache + max(src[u], 0ll) + ch, src[u] < 0 ? 0 : min(16, 4 * (dim - ch)));
+          } else {
+            float f[4][4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) ld_elem4((const T*)cache + max(src[u], 0ll) + ch, f[u]);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                if (src[u] < 0 || ch + e >= dim) f[u][e] = 0.f;
+              st_elem4(d + u * kWarps * pitch, f[u]);
+            }
+          }
+        }
+      }
+      at_commit();
+    };
+    // The keys of a step are fetched while the values of the one before are used, its values while its scores are made.
+    if (first < end) {
+      look_up(first, at[0]);
+      __syncthreads();
+      fetch(at[0], c.k, c.k_row, c.k_dim, ks, kp);
+      fetch(at[0], c.v, c.v_row, c.v_dim, vs, c.v_row);
+    }
+    for (int j0 = first, turn = 0; j0 < end; j0 += kAtKeys, turn ^= 1) {
+      const int count = min(kAtKeys, end - j0);
+      const bool more = j0 + kAtKeys < end;
+      look_up(j0 + kAtKeys, at[turn ^ 1]);
+      at_wait<1>();
+      __syncthreads();  // the keys are there, the scores of the step before are used
+      const int key = tid & (kAtKeys - 1), s0 = tid / kAtKeys * kAtDots;
+      if (s0 < slots) {
+        const float *kr = ks + key * kp, *qr = qs + s0 * c.k_row;
+        float acc[kAtDots];
+#pragma unroll
+        for (int i = 0; i < kAtDots; ++i) acc[i] = 0.f;
+        auto dots = [&](auto rows_at_once) {
+          constexpr int kN = decltype(rows_at_once)::value;
+#pragma unroll 2
+          for (int ch = 0; ch < c.k_row; ch += 4) {
+            const float4 kv = *reinterpret_cast<const float4*>(kr + ch);
+#pragma unroll
+            for (int i = 0; i < kN; ++i) {
+              const float4 x = *reinterpret_cast<const float4*>(qr + i * c.k_row + ch);
+              acc[i] = fmaf(x.w, kv.w, fmaf(x.z, kv.z, fmaf(x.y, kv.y, fmaf(x.x, kv.x, acc[i]))));
+            }
+          }
+        };
+        if (slots - s0 <= 2) dots(std::integral_constant<int, 2>{}); else dots(std::integral_constant<int, kAtDots>{});
+#pragma unroll
+        for (int i = 0; i < kAtDots; i += 4)
+          *reinterpret_cast<float4*>(ps + key * kAtPitch + s0 + i) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
+      }
+      __syncthreads();  // the keys are used
+      if (more) fetch(at[turn ^ 1], c.k, c.k_row, c.k_dim, ks, kp); else at_commit();
+      at_wait<1>();
+      __syncthreads();  // every thread's part of the values is there
+      if (mine) {
+        // softmax of the warp's query rows, keys lane and lane + 32
+        float p[2][kAtOwn];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int k = lane + 32 * u, j = j0 + k;
+          at_read(ps + k * kAtPitch + kAtOwn * warp, p[u]);
+          const bool some = at[turn][k] >= 0;
+#pragma unroll
+          for (int i = 0; i < kAtOwn; ++i)
+            if (!some || j > last[i] || j < low[i]) p[u][i] = -INFINITY;
+        }
+#pragma unroll
+        for (int i = 0; i < kAtOwn; ++i) {
+          float mx = fmaxf(p[0][i], p[1][i]);
+#pragma unroll
+          for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+          const float mn = fmaxf(m[i], mx), base = mn == -INFINITY ? 0.f : mn, alpha = expf(m[i] - base);
+          m[i] = mn;
+#pragma unroll
+          for (int u = 0; u < 2; ++u) p[u][i] = expf(p[u][i] - base);
+          l[i] = l[i] * alpha + warp_sum(p[0][i] + p[1][i]);
+#pragma unroll
+          for (int a = 0; a < kPieces; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) o[i][a][b] *= alpha;
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+          for (int i = 0; i < kAtOwn; i += 2)
+            *reinterpret_cast<float2*>(ps + (lane + 32 * u) * kAtPitch + kAtOwn * warp + i) = make_float2(p[u][i], p[u][i + 1]);
+        __syncwarp();
+        auto add = [&](int k, bool every) {
+          float w[kAtOwn];
+          at_read(ps + k * kAtPitch + kAtOwn * warp, w);
+#pragma unroll
+          for (int a = 0; a < kPieces; ++a) {
+            const int ch = 4 * lane + 128 * a;
+            if (ch >= c.v_row) break;
+            const float4 v = *reinterpret_cast<const float4*>(vs + k * c.v_row + ch);
+#pragma unroll
+            for (int i = 0; i < kAtOwn; ++i) {
+              if (!every && (j0 + k > last[i] || j0 + k < low[i])) continue;
+              o[i][a][0] = fmaf(w[i], v.x, o[i][a][0]);
+              o[i][a][1] = fmaf(w[i], v.y, o[i][a][1]);
+              o[i][a][2] = fmaf(w[i], v.z, o[i][a][2]);
+              o[i][a][3] = fmaf(w[i], v.w, o[i][a][3]);
+            }
+          }
+        };
+        // (a key without a page has a weight and a value of zero)
+        const int e0 = min(max(all_low - j0, 0), count), e1 = max(e0, min(all_last + 1 - j0, count));
+        for (int k = 0; k < e0; ++k) add(k, false);
+#pragma unroll 4
+        for (int k = e0; k < e1; ++k) add(k, true);
+        for (int k = e1; k < count; ++k) add(k, false);
+      }
+      __syncthreads();  // the values are used
+      if (more) fetch(at[turn ^ 1], c.v, c.v_row, c.v_dim, vs, c.v_row); else at_commit();
+    }
+    auto store = [&](int s, float sum, const float (&v)[kPieces][4]) {
+      const int r = r0 + s / gs, h = hk * G + g0 + s % gs;
+      const float inv = (sum > 0.f ? 1.f / sum : 0.f) * opt.factor<T>(r, h);
+#pragma unroll
+      for (int a = 0; a < kPieces; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          const int ch = 4 * lane + 128 * a + b;
+          if (ch < c.v_dim) st_elem(out + r * opt.out_stride + (long long)h * c.v_dim + ch, v[a][b] * inv);
+        }
+    };
+    if (splits == 1) {
+#pragma unroll
+      for (int i = 0; i < kAtOwn; ++i)
+        if (kAtOwn * warp + i < slots) store(kAtOwn * warp + i, l[i], o[i]);
+      return;
+    }
+    // the cluster's parts meet in its shared memory: outputs where the values were, maxima and sums where the scores were
+#pragma unroll
+    for (int i = 0; i < kAtOwn; ++i) {
+      const int s = kAtOwn * warp + i;
+      if (lane == 0) *reinterpret_cast<float2*>(ps + 2 * s) = make_float2(m[i], l[i]);
+#pragma unroll
+      for (int a = 0; a < kPieces; ++a)
+        if (4 * lane + 128 * a < c.v_row) st_elem4(vs + s * c.v_row + 4 * lane + 128 * a, o[i][a]);
+    }
+    at_cluster_sync();
+    for (int s = part + splits * warp; s < slots; s += splits * kWarps) {
+      float top = -INFINITY, sum = 0.f, v[kPieces][4] = {};
+      for (int j = 0; j < splits; ++j) top = fmaxf(top, at_peer2(ps + 2 * s, j).x);
+      const float base = top == -INFINITY ? 0.f : top;
+      for (int j = 0; j < splits; ++j) {
+        const float2 ml = at_peer2(ps + 2 * s, j);
+        const float w = expf(ml.x - base);
+        sum = fmaf(ml.y, w, sum);
+#pragma unroll
+        for (int a = 0; a < kPieces; ++a) {
+          if (4 * lane + 128 * a >= c.v_row) break;
+          const float4 x = at_peer4(vs + s * c.v_row + 4 * lane + 128 * a, j);
+          v[a][0] = fmaf(x.x, w, v[a][0]);
+          v[a][1] = fmaf(x.y, w, v[a][1]);
+          v[a][2] = fmaf(x.z, w, v[a][2]);
+          v[a][3] = fmaf(x.w, w, v[a][3]);
+        }
+      }
+      store(s, sum, v);
+    }
+    at_cluster_sync();  // a block's shared memory stays until its peers have read it
+  };
   // A tile starts at the first row of an entry and then every `most` rows.  With the entries' first rows a block finds its tile, of a list with
-  // a few places too many; without, there is a block for every row, and those that start nothing leave.
+  // a few places too many (the rows behind the last entry are one entry more); without, there is a block for every row, and those that start
+  // nothing leave.  What a row is stands in seq_ids and positions alone: the rows of a tile are done in runs of one entry's consecutive
+  // positions, as a rule one run.
   const int most = kAtSlots / slice_heads;
-  int r0 = blockIdx.y, seq = r0, pos, n = 1;
+  int r0 = blockIdx.y, left = 1, seq = r0, pos, n = 1;
   if (rows.seq_ids) {
+    left = min(most, rows.num_rows - r0);
     if (cu_seqlens) {
-      int lo = 0, hi = num_entries;  // the last entry whose first place is not behind this block's
+      int lo = 0, hi = num_entries + 1;  // the last entry whose first place is not behind this block's
       while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
         if (cu_seqlens[mid] / most + mid <= r0) lo = mid; else hi = mid;
       }
-      const int first = cu_seqlens[lo], end = min(cu_seqlens[lo + 1], rows.num_rows), tile = r0 - (first / most + lo);
-      r0 = first + tile * most;
+      const int first = lo > 0 ? cu_seqlens[lo] : 0, end = lo < num_entries ? min(cu_seqlens[lo + 1], rows.num_rows) : rows.num_rows;
+      r0 = first + (r0 - (lo > 0 ? first / most + lo : 0)) * most;
       if (r0 < 0 || r0 >= end) return;
-      n = min(most, end - r0);
+      left = min(most, end - r0);
+    } else if (r0 > 0) {
+      pos = rows.positions[r0];
+      if (pos >= 0 && pos % most != 0 && rows.seq_ids[r0 - 1] == rows.seq_ids[r0] && rows.positions[r0 - 1] == pos - 1) return;
     }
-    seq = rows.seq_ids[r0];
-    pos = rows.positions[r0];
-    if (!cu_seqlens) {
-      if (r0 > 0 && pos >= 0 && pos % most != 0 && rows.seq_ids[r0 - 1] == seq && rows.positions[r0 - 1] == pos - 1) return;
-      while (pos >= 0 && n < most && r0 + n < rows.num_rows && (pos + n) % most != 0 && rows.seq_ids[r0 + n] == seq &&
-             rows.positions[r0 + n] == pos + n)
-        ++n;
-    }
-  } else {
-    pos = r0 < *rows.num_decoding ? rows.cached_lens[r0] : -1;
   }
   pdl_wait();
-  const int slots = n * gs;
-  if (pos < 0) {  // idle row
-    if (part == 0)
-      for (int r = r0; r < r0 + n; ++r)
-        for (int i = tid; i < gs * c.v_dim; i += kAtThreads) st_elem(out + r * opt.out_stride + (hk * G + g0) * c.v_dim + i, 0.f);
-    return;
-  }
-  for (int s = warp; s < kAtSlots; s += kWarps) {
-    const T* src = q + ((long long)(r0 + s / gs) * heads + hk * G + g0 + s % gs) * c.k_row;
-    for (int ch = lane; ch < c.k_row; ch += 32) qs[s * c.k_row + ch] = s < slots && ch < c.k_dim ? ld_elem(src + ch) * scale : 0.f;
-  }
-  // what this warp keeps: query rows kAtOwn warp + i
-  float m[kAtOwn], l[kAtOwn], o[kAtOwn][kPieces][4];
-  int last[kAtOwn], low[kAtOwn];  // the keys each of them sees
-#pragma unroll
-  for (int i = 0; i < kAtOwn; ++i) {
-    const int s = kAtOwn * warp + i, h = hk * G + g0 + s % gs;
-    last[i] = s < slots ? pos + s / gs : -1;
-    low[i] = s < slots && opt.window > 0 ? max(0, last[i] - opt.window + 1) : 0;
-    m[i] = opt.sink && s < slots && part == 0 ? opt.sink[h] : -INFINITY;
-    l[i] = opt.sink && part == 0 ? 1.f : 0.f;
-#pragma unroll
-    for (int j = 0; j < kPieces; ++j)
-#pragma unroll
-      for (int k = 0; k < 4; ++k) o[i][j][k] = 0.f;
-  }
-  const bool mine = kAtOwn * warp < slots;
-  // Keys [all_low, all_last] are seen by every query row of the tile; the others are looked at one by one, so that what a row
-  // does not see (a later token, perhaps not a number) never meets it.
-  const int all_last = pos, all_low = opt.window > 0 ? max(0, pos + n - opt.window) : 0;
-  int first = opt.window > 0 ? max(0, pos - opt.window + 1) : 0, end = pos + n;
-  if (splits > 1) {  // this block's steps
-    const int share = ((end - first + kAtKeys - 1) / kAtKeys + splits - 1) / splits * kAtKeys;
-    first += part * share;
-    end = min(end, first + share);
-  }
-  // the rows of the keys from j0 on
-  auto look_up = [&](int j0, long long* at_rows) {
-    if (tid < kAtKeys) {
-      const int page = j0 + tid < end ? dec_page(c, seq, j0 + tid, status) : -1;
-      at_rows[tid] = page < 0 ? -1 : dec_row(c, page, hk, (j0 + tid) % c.P);
+  for (; left > 0; r0 += n, left -= n) {
+    if (rows.seq_ids) {  // the run from r0 on: lane i looks at row r0 + i
+      static_assert(kAtSlots < 32, "a warp sees where a run ends");
+      const int s = lane < left ? rows.seq_ids[r0 + lane] : 0, p = lane < left ? rows.positions[r0 + lane] : -1;
+      seq = __shfl_sync(0xffffffffu, s, 0);
+      pos = __shfl_sync(0xffffffffu, p, 0);
+      const bool same = p >= 0 && s == seq && p == pos + lane && (lane == 0 || cu_seqlens || p % most != 0);
+      n = max(1, __ffs(~__ballot_sync(0xffffffffu, same)) - 1);
+      if (!cu_seqlens) left = n;
+    } else {
+      pos = r0 < *rows.num_decoding ? rows.cached_lens[r0] : -1;
     }
-  };
-  // their keys or values to shared memory, zero where there is none and behind `dim`
-  auto fetch = [&](const long long* at_rows, const void* cache, int row, int dim, float* to, int pitch) {
-    for (int k0 = warp; k0 < kAtKeys; k0 += 4 * kWarps) {
-      long long src[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) src[u] = at_rows[k0 + u * kWarps] * row;
-      for (int ch = 4 * lane; ch < row; ch += 128) {
-        float* d = to + k0 * pitch + ch;
-        if constexpr (sizeof(T) == 4) {
-#pragma unroll
-          for (int u = 0; u < 4; ++u)
-            at_copy16(d + u * kWarps * pitch, (const float*)cache + max(src[u], 0ll) + ch, src[u] < 0 ? 0 : min(16, 4 * (dim - ch)));
-        } else {
-          float f[4][4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) ld_elem4((const T*)cache + max(src[u], 0ll) + ch, f[u]);
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-              if (src[u] < 0 || ch + e >= dim) f[u][e] = 0.f;
-            st_elem4(d + u * kWarps * pitch, f[u]);
-          }
-        }
-      }
+    if (pos >= 0) {
+      run(r0, n, seq, pos);
+    } else if (part == 0) {  // idle row
+      for (int i = tid; i < gs * c.v_dim; i += kAtThreads) st_elem(out + r0 * opt.out_stride + (hk * G + g0) * c.v_dim + i, 0.f);
     }
-    at_commit();
-  };
-  // The keys of a step are fetched while the values of the one before are used, its values while its scores are made.
-  if (first < end) {
-    look_up(first, at[0]);
-    __syncthreads();
-    fetch(at[0], c.k, c.k_row, c.k_dim, ks, kp);
-    fetch(at[0], c.v, c.v_row, c.v_dim, vs, c.v_row);
   }
-  for (int j0 = first, turn = 0; j0 < end; j0 += kAtKeys, turn ^= 1) {
-    const int count = min(kAtKeys, end - j0);
-    const bool more = j0 + kAtKeys < end;
-    look_up(j0 + kAtKeys, at[turn ^ 1]);
-    at_wait<1>();
-    __syncthreads();  // the keys are there, the scores of the step before are used
-    const int key = tid & (kAtKeys - 1), s0 = tid / kAtKeys * kAtDots;
-    if (s0 < slots) {
-      const float *kr = ks + key * kp, *qr = qs + s0 * c.k_row;
-      float acc[kAtDots];
-#pragma unroll
-      for (int i = 0; i < kAtDots; ++i) acc[i] = 0.f;
-      auto dots = [&](auto rows_at_once) {
-        constexpr int kN = decltype(rows_at_once)::value;
-#pragma unroll 2
-        for (int ch = 0; ch < c.k_row; ch += 4) {
-          const float4 kv = *reinterpret_cast<const float4*>(kr + ch);
-#pragma unroll
-          for (int i = 0; i < kN; ++i) {
-            const float4 x = *reinterpret_cast<const float4*>(qr + i * c.k_row + ch);
-            acc[i] = fmaf(x.w, kv.w, fmaf(x.z, kv.z, fmaf(x.y, kv.y, fmaf(x.x, kv.x, acc[i]))));
-          }
-        }
-      };
-      if (slots - s0 <= 2) dots(std::integral_constant<int, 2>{}); else dots(std::integral_constant<int, kAtDots>{});
-#pragma unroll
-      for (int i = 0; i < kAtDots; i += 4)
-        *reinterpret_cast<float4*>(ps + key * kAtPitch + s0 + i) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
-    }
-    __syncthreads();  // the keys are used
-    if (more) fetch(at[turn ^ 1], c.k, c.k_row, c.k_dim, ks, kp); else at_commit();
-    at_wait<1>();
-    __syncthreads();  // every thread's part of the values is there
-    if (mine) {
-      // softmax of the warp's query rows, keys lane and lane + 32
-      float p[2][kAtOwn];
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int k = lane + 32 * u, j = j0 + k;
-        at_read(ps + k * kAtPitch + kAtOwn * warp, p[u]);
-        const bool some = at[turn][k] >= 0;
-#pragma unroll
-        for (int i = 0; i < kAtOwn; ++i)
-          if (!some || j > last[i] || j < low[i]) p[u][i] = -INFINITY;
-      }
-#pragma unroll
-      for (int i = 0; i < kAtOwn; ++i) {
-        float mx = fmaxf(p[0][i], p[1][i]);
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-        const float mn = fmaxf(m[i], mx), base = mn == -INFINITY ? 0.f : mn, alpha = expf(m[i] - base);
-        m[i] = mn;
-#pragma unroll
-        for (int u = 0; u < 2; ++u) p[u][i] = expf(p[u][i] - base);
-        l[i] = l[i] * alpha + warp_sum(p[0][i] + p[1][i]);
-#pragma unroll
-        for (int a = 0; a < kPieces; ++a)
-#pragma unroll
-          for (int b = 0; b < 4; ++b) o[i][a][b] *= alpha;
-      }
-#pragma unroll
-      for (int u = 0; u < 2; ++u)
-#pragma unroll
-        for (int i = 0; i < kAtOwn; i += 2)
-          *reinterpret_cast<float2*>(ps + (lane + 32 * u) * kAtPitch + kAtOwn * warp + i) = make_float2(p[u][i], p[u][i + 1]);
-      __syncwarp();
-      auto add = [&](int k, bool every) {
-        float w[kAtOwn];
-        at_read(ps + k * kAtPitch + kAtOwn * warp, w);
-#pragma unroll
-        for (int a = 0; a < kPieces; ++a) {
-          const int ch = 4 * lane + 128 * a;
-          if (ch >= c.v_row) break;
-          const float4 v = *reinterpret_cast<const float4*>(vs + k * c.v_row + ch);
-#pragma unroll
-          for (int i = 0; i < kAtOwn; ++i) {
-            if (!every && (j0 + k > last[i] || j0 + k < low[i])) continue;
-            o[i][a][0] = fmaf(w[i], v.x, o[i][a][0]);
-            o[i][a][1] = fmaf(w[i], v.y, o[i][a][1]);
-            o[i][a][2] = fmaf(w[i], v.z, o[i][a][2]);
-            o[i][a][3] = fmaf(w[i], v.w, o[i][a][3]);
-          }
-        }
-      };
-      // (a key without a page has a weight and a value of zero)
-      const int e0 = min(max(all_low - j0, 0), count), e1 = max(e0, min(all_last + 1 - j0, count));
-      for (int k = 0; k < e0; ++k) add(k, false);
-#pragma unroll 4
-      for (int k = e0; k < e1; ++k) add(k, true);
-      for (int k = e1; k < count; ++k) add(k, false);
-    }
-    __syncthreads();  // the values are used
-    if (more) fetch(at[turn ^ 1], c.v, c.v_row, c.v_dim, vs, c.v_row); else at_commit();
-  }
-  auto store = [&](int s, float sum, const float (&v)[kPieces][4]) {
-    const int r = r0 + s / gs, h = hk * G + g0 + s % gs;
-    const float inv = (sum > 0.f ? 1.f / sum : 0.f) * opt.factor<T>(r, h);
-#pragma unroll
-    for (int a = 0; a < kPieces; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const int ch = 4 * lane + 128 * a + b;
-        if (ch < c.v_dim) st_elem(out + r * opt.out_stride + (long long)h * c.v_dim + ch, v[a][b] * inv);
-      }
-  };
-  if (splits == 1) {
-#pragma unroll
-    for (int i = 0; i < kAtOwn; ++i)
-      if (kAtOwn * warp + i < slots) store(kAtOwn * warp + i, l[i], o[i]);
-    return;
-  }
-  // the cluster's parts meet in its shared memory: outputs where the values were, maxima and sums where the scores were
-#pragma unroll
-  for (int i = 0; i < kAtOwn; ++i) {
-    const int s = kAtOwn * warp + i;
-    if (lane == 0) *reinterpret_cast<float2*>(ps + 2 * s) = make_float2(m[i], l[i]);
-#pragma unroll
-    for (int a = 0; a < kPieces; ++a)
-      if (4 * lane + 128 * a < c.v_row) st_elem4(vs + s * c.v_row + 4 * lane + 128 * a, o[i][a]);
-  }
-  at_cluster_sync();
-  for (int s = part + splits * warp; s < slots; s += splits * kWarps) {
-    float top = -INFINITY, sum = 0.f, v[kPieces][4] = {};
-    for (int j = 0; j < splits; ++j) top = fmaxf(top, at_peer2(ps + 2 * s, j).x);
-    const float base = top == -INFINITY ? 0.f : top;
-    for (int j = 0; j < splits; ++j) {
-      const float2 ml = at_peer2(ps + 2 * s, j);
-      const float w = expf(ml.x - base);
-      sum = fmaf(ml.y, w, sum);
-#pragma unroll
-      for (int a = 0; a < kPieces; ++a) {
-        if (4 * lane + 128 * a >= c.v_row) break;
-        const float4 x = at_peer4(vs + s * c.v_row + 4 * lane + 128 * a, j);
-        v[a][0] = fmaf(x.x, w, v[a][0]);
-        v[a][1] = fmaf(x.y, w, v[a][1]);
-        v[a][2] = fmaf(x.z, w, v[a][2]);
-        v[a][3] = fmaf(x.w, w, v[a][3]);
-      }
-    }
-    store(s, sum, v);
-  }
-  at_cluster_sync();  // a block's shared memory stays until its peers have read it
 }
 
 }  // namespace b200kv
@@ -1123,8 +1134,8 @@ extern "C" int b200dec_attn_rows_entries(const void* q, const b200dec_cache* cac
   if (tile_smem <= kAtMostSmem && cache->v_row <= 256) {
     const int G = heads / cache->kv_heads, slices = (G + kAtSlots - 1) / kAtSlots, slice_heads = (G + slices - 1) / slices;
     const int most = kAtSlots / slice_heads;
-    const bool listed = rows->seq_ids && cu_seqlens && num_entries > 0 && rows->num_rows / most + (long long)num_entries <= 65535;
-    const int blocks = listed ? rows->num_rows / most + num_entries : rows->num_rows;
+    const bool listed = rows->seq_ids && cu_seqlens && num_entries > 0 && rows->num_rows / most + (long long)num_entries < 65535;
+    const int blocks = listed ? rows->num_rows / most + num_entries + 1 : rows->num_rows;
     const int splits = at_splits((long long)cache->kv_heads * slices * (listed || !rows->seq_ids ? blocks : blocks / most + 1), most, (long long)table->max_pages * cache->page_size, opt.window);
     auto tiles = [&](auto* kernel, auto* in, auto* o) -> int {
       if (!allow_smem(kernel, kAtMostSmem)) return B200KV_E_LAUNCH;

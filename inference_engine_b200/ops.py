@@ -273,8 +273,10 @@ def attention_rows(q: torch.Tensor, cache: PagedKV, rows: Rows, scale: float, op
         out = torch.empty(q.shape[0], q.shape[1], cache.v_dim, device=q.device, dtype=q.dtype)
     cs, ts, rs = cache.struct(), K._table_struct(rows.block_table), rows.struct()
     cu = rows.cu_seqlens
+    if cu is not None and (cu.dtype != torch.int32 or not cu.is_contiguous() or cu.device != q.device or cu.numel() < 2):
+        cu = None  # it only says how the rows are shared out
     rc = _lib_dec().b200dec_attn_rows_entries(q.data_ptr(), ctypes.byref(cs), ctypes.byref(ts), ctypes.byref(rs),
-                                              None if cu is None else K._i32(cu), 0 if cu is None else cu.shape[0] - 1, q.shape[1], float(scale),
+                                              _ptr(cu), 0 if cu is None else cu.numel() - 1, q.shape[1], float(scale),
                                               _opt(opt, out), out.data_ptr(), K.status_word(q.device).data_ptr(), K._stream())
     _lib.check(rc, "attention_rows")
     return out

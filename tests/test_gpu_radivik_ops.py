@@ -483,3 +483,39 @@ def test_chained_launches_wait_for_weights_and_angles(op):
     finally:
         K.set_early_start(False)
     H.status_clear()
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads,kv,dim,vdim,window", [(4, 2, 48, 40, 0), (16, 8, 112, 96, 70), (3, 3, 128, 200, 0)])
+def test_attention_rows_go_by_their_own_entry_and_position(heads, kv, dim, vdim, window, dtype):
+    """The entries' first rows only say how rows are shared out: positions that jump, go back or stay, idle rows, rows of other entries and rows
+    behind the last entry are done as without the list.  The table has room for many more keys than there are."""
+    from inference_engine_b200 import ops
+
+    g = np.random.default_rng(dim)
+    at = [(0, p) for p in [10, 11, 12, 40, 41, 7, 7, -1, *range(90, 115), 149]]
+    at += [(1, p) for p in (149, 148, 147, 0, 1)] + [(0, 60), (2, 61), (2, 62), (1, 63)]
+    listed = [0, 34, 34, len(at)]
+    at += [(2, p) for p in (*range(20, 45), 149)] + [(0, -1), (0, 0), (1, 64)]  # of no entry in the list
+    n, keys, page = len(at), 150, 16
+    per = -(-keys // page)
+    perm = g.permutation(3 * per + 2)
+    table = np.full((3, 64), -1, np.int32)
+    table[:, :per] = perm[: 3 * per].reshape(3, per)
+    cache = ops.make_paged_kv(3 * per + 2, kv, page, dim, vdim, dtype, DEV)
+    k, v = H.bf16(g.standard_normal((3, keys, kv, dim))), H.bf16(g.standard_normal((3, keys, kv, vdim)))
+    for b in range(3):
+        fill(cache, table, b, t(k[b], dtype), t(v[b], dtype))
+    q, want = H.bf16(g.standard_normal((n, heads, dim))), np.zeros((n, heads, vdim))
+    for r, (b, p) in enumerate(at):
+        lo = max(0, p - window + 1) if window else 0
+        if p >= 0:
+            want[r : r + 1] = R.causal_attention(q[r : r + 1], k[b, lo : p + 1], v[b, lo : p + 1], dim ** -0.5, p - lo)
+    qd = torch.zeros(n, heads, cache.k.shape[3], device=DEV, dtype=dtype)
+    qd[..., :dim] = t(q, dtype)
+    for cu in (None, i32(listed), torch.tensor(listed, device=DEV), i32([0] * 40 + [n]), i32([0, n])):
+        rows = ops.Rows(n, i32([0] * 3), i32([0]), i32(table), i32([b for b, _ in at]), i32([p for _, p in at]), cu)
+        out = torch.full((n, heads, vdim), float("nan"), device=DEV, dtype=dtype)
+        ops.attention_rows(qd, cache, rows, dim ** -0.5, ops.AttnOptions(window=window), out)
+        close(out, want, dtype)
+    H.status_clear()
