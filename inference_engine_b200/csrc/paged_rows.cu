@@ -698,6 +698,21 @@ attn_tile_kernel(const T* q, DecCache c, b200dec_rows rows, const int32_t* __res
   // Rows r0 to r0 + n - 1, of entry seq at the positions from pos on.
   auto run = [&](const int r0, const int n, const int seq, const int pos) {
     const int slots = n * gs;
+    // The block's steps.  Where the table has room for more keys than there are, only the first `parts` blocks of the cluster have some.
+    int first = opt.window > 0 ? max(0, pos - opt.window + 1) : 0, end = pos + n, parts = 1;
+    if (splits > 1) {
+      const int steps = (end - first + kAtKeys - 1) / kAtKeys, share = (steps + splits - 1) / splits;
+      parts = (steps + share - 1) / share;
+      if (part >= parts) {
+        if (parts > 1) {  // the others meet
+          at_cluster_sync();
+          at_cluster_sync();
+        }
+        return;
+      }
+      first += part * share * kAtKeys;
+      end = min(end, first + share * kAtKeys);
+    }
     for (int s = warp; s < kAtSlots; s += kWarps) {
       const T* src = q + ((long long)(r0 + s / gs) * heads + hk * G + g0 + s % gs) * c.k_row;
       for (int ch = lane; ch < c.k_row; ch += 32) qs[s * c.k_row + ch] = s < slots && ch < c.k_dim ? ld_elem(src + ch) * scale : 0.f;
@@ -721,12 +736,6 @@ attn_tile_kernel(const T* q, DecCache c, b200dec_rows rows, const int32_t* __res
     // Keys [all_low, all_last] are seen by every query row of the tile; the others are looked at one by one, so that what a row
     // does not see (a later token, perhaps not a number) never meets it.
     const int all_last = pos, all_low = opt.window > 0 ? max(0, pos + n - opt.window) : 0;
-    int first = opt.window > 0 ? max(0, pos - opt.window + 1) : 0, end = pos + n;
-    if (splits > 1) {  // this block's steps
-      const int share = ((end - first + kAtKeys - 1) / kAtKeys + splits - 1) / splits * kAtKeys;
-      first += part * share;
-      end = min(end, first + share);
-    }
     // the rows of the keys from j0 on
     auto look_up = [&](int j0, long long* at_rows) {
       if (tid < kAtKeys) {
@@ -874,7 +883,7 @@ attn_tile_kernel(const T* q, DecCache c, b200dec_rows rows, const int32_t* __res
           if (ch < c.v_dim) st_elem(out + r * opt.out_stride + (long long)h * c.v_dim + ch, v[a][b] * inv);
         }
     };
-    if (splits == 1) {
+    if (parts == 1) {
 #pragma unroll
       for (int i = 0; i < kAtOwn; ++i)
         if (kAtOwn * warp + i < slots) store(kAtOwn * warp + i, l[i], o[i]);
@@ -890,11 +899,11 @@ attn_tile_kernel(const T* q, DecCache c, b200dec_rows rows, const int32_t* __res
         if (4 * lane + 128 * a < c.v_row) st_elem4(vs + s * c.v_row + 4 * lane + 128 * a, o[i][a]);
     }
     at_cluster_sync();
-    for (int s = part + splits * warp; s < slots; s += splits * kWarps) {
+    for (int s = part + parts * warp; s < slots; s += parts * kWarps) {
       float top = -INFINITY, sum = 0.f, v[kPieces][4] = {};
-      for (int j = 0; j < splits; ++j) top = fmaxf(top, at_peer2(ps + 2 * s, j).x);
+      for (int j = 0; j < parts; ++j) top = fmaxf(top, at_peer2(ps + 2 * s, j).x);
       const float base = top == -INFINITY ? 0.f : top;
-      for (int j = 0; j < splits; ++j) {
+      for (int j = 0; j < parts; ++j) {
         const float2 ml = at_peer2(ps + 2 * s, j);
         const float w = expf(ml.x - base);
         sum = fmaf(ml.y, w, sum);
@@ -960,7 +969,8 @@ attn_tile_kernel(const T* q, DecCache c, b200dec_rows rows, const int32_t* __res
 
 using namespace b200kv;
 
-// Blocks that share a tile's keys: as many as are resident at a time (two per multiprocessor), but no more than a tile has steps.  A block's
+// Blocks that share a tile's keys: as many as are resident at a time (two per multiprocessor), but no more than the steps that the table has
+// room for; what a tile has is known on the device only, where blocks without a step leave the others to it.  A block's
 // fixed cost is about two steps, so that with more than a round of blocks sharing only adds work.  us with 1 / 2 / 4 / 8, 16 heads of
 // 128 over 8: an entry of 550 decoding 51.3 / 34.9 / 24.7 / 20.6, of 4000 314 / 166 / 89 / 51; 8 of 550 55.4 / 34.9 / 26.7 / 37.0, 64 of
 // 550 118 / 133 / 164 / 240; 200 rows of a prompt 41.0 / 41.7 / 49.1 / 90.
