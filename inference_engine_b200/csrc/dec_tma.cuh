@@ -12,7 +12,8 @@ __device__ __forceinline__ uint32_t dt_smem(const void* p) { return (uint32_t)__
 __device__ __forceinline__ void dt_mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count) : "memory");
 }
-// Bounded wait for the phase with the given parity; false when the limit ran out.
+// Bounded wait for the phase with the given parity; false when the limit ran out.  Each lane has a limit of its own, so a warp whose lanes go on
+// to do something together votes on the outcome.
 __device__ __forceinline__ bool dt_mbar_wait(uint32_t bar, uint32_t parity, uint32_t limit = kDtSpin) {
   for (uint32_t spin = 0; spin < limit; ++spin) {
     uint32_t done;

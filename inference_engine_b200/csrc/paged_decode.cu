@@ -271,7 +271,7 @@ paged_decode_kernel(const uint16_t* q, DecCache c, const int32_t* __restrict__ c
     float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
     for (int k = 0; k < nblk; ++k, ++i) {
       const int s = i % kStages;
-      if (!dead && !dt_mbar_wait(full(s), (i / kStages) & 1)) dead = true;
+      if (!dead && !__all_sync(0xffffffffu, dt_mbar_wait(full(s), (i / kStages) & 1))) dead = true;
       const int nvalid = cur.n - (blk0 + k) * kPdKeys - warp * 16;  // keys of this warp's tile
       const int nskip = lo - (blk0 + k) * kPdKeys - warp * 16;      // ... and those in front of the window
       if (nvalid > 0 && nskip < 16 && !dead) {

@@ -83,7 +83,8 @@ __device__ __forceinline__ void t5_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void t5_mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count) : "memory");
 }
-// Bounded wait for the phase with the given parity; false when the limit ran out.
+// Bounded wait for the phase with the given parity; false when the limit ran out.  Each lane has a limit of its own, so a warp whose lanes go on
+// to do something together votes on the outcome.
 __device__ __forceinline__ bool t5_mbar_wait(uint32_t bar, uint32_t parity, uint32_t limit) {
   for (uint32_t spin = 0; spin < limit; ++spin) {
     uint32_t done;
@@ -381,7 +382,7 @@ prefill_attn_tc5_kernel(const uint16_t* q, long long q_sn, long long q_sh, const
             k_ph[x] = __shfl_sync(0xffffffffu, my_ph, ((step << lg) + x) & 31);
             k_row[x] = __shfl_sync(0xffffffffu, my_row, ((step << lg) + x) & 31);
           }
-          if (step >= ring && !t5_mbar_wait(bar_ke(w, k_sl), k_par, spin)) { live = false; break; }
+          if (step >= ring && !__all_sync(0xffffffffu, t5_mbar_wait(bar_ke(w, k_sl), k_par, spin))) { live = false; break; }
           if (lane == 0) {
             // keys behind the last one may be anything: their scores are never looked at
             const int count = min(kT5Keys, own_keys - (block_of(w, step) + skipped) * kT5Keys);
@@ -401,7 +402,7 @@ prefill_attn_tc5_kernel(const uint16_t* q, long long q_sn, long long q_sh, const
         if (step > 0) {
           const int j0 = (block_of(w, step - 1) + skipped) * kT5Keys, count = min(kT5Keys, own_keys - j0);
           const uint32_t dst = ring_v(w) + v_sl * kT5KvBytes, full = bar_vf(w, v_sl);
-          if (step > ring && !t5_mbar_wait(bar_ve(w, v_sl), v_par, spin)) { live = false; break; }
+          if (step > ring && !__all_sync(0xffffffffu, t5_mbar_wait(bar_ve(w, v_sl), v_par, spin))) { live = false; break; }
           if (count == kT5Keys) {
             if (lane == 0) {
               t5_mbar_expect_tx(full, (uint32_t)(kT5Keys * 128 * v_blocks));
@@ -455,7 +456,7 @@ prefill_attn_tc5_kernel(const uint16_t* q, long long q_sn, long long q_sh, const
           const uint32_t dst = (is_v ? ring_v(w) : ring_k(w)) + sl * kT5KvBytes;
           const uint32_t full = is_v ? bar_vf(w, sl) : bar_kf(w, sl), empty = is_v ? bar_ve(w, sl) : bar_ke(w, sl);
           // the product that read this slot a ring of blocks ago has completed
-          if (h >= ring && !t5_mbar_wait(empty, par, spin)) { live = false; break; }
+          if (h >= ring && !__all_sync(0xffffffffu, t5_mbar_wait(empty, par, spin))) { live = false; break; }
           if (tma) {
             if (lane == 0) {
               t5_mbar_expect_tx(full, kT5KvBytes);
@@ -625,6 +626,7 @@ prefill_attn_tc5_kernel(const uint16_t* q, long long q_sn, long long q_sh, const
       t5_st32(tS + 64 * (h & 1), pk);  // P over the first 32 columns of this S buffer
       asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
       t5_fence_before();
+      ok = __all_sync(0xffffffffu, ok);  // the warp goes on or stops as a whole
       if (ok) t5_mbar_arrive(bar_r(wg, h & 1));  // hand P(h) to the issuing warp
     }
     pdl_trigger();
