@@ -90,6 +90,14 @@ inline bool allow_smem(void (*kernel)(KArgs...), size_t most) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) == cudaSuccess;
 }
 
+// A multiprocessor changes the share of shared memory in its 256 KB only when it is empty: a chained kernel that needs shared memory cannot be
+// brought up beside one in front that runs on all L1.  So the one in front asks for half of it.
+template <typename... KArgs>
+inline void leave_shared_memory(void (*kernel)(KArgs...)) {
+  // (a wish: nothing is lost where it fails)
+  (void)cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, b200kv_get_chained_launch() ? 50 : cudaSharedmemCarveoutDefault);
+}
+
 inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 
 // Host-side validation shared by the entry points.  Returns B200KV_OK or an error code.
