@@ -90,6 +90,14 @@ inline bool allow_smem(void (*kernel)(KArgs...), size_t most) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) == cudaSuccess;
 }
 
+// Multiprocessors of the current device, for rules of a dispatch at entry points that are not given them.
+inline int device_sms() {
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0) return n;
+  (void)cudaGetLastError();
+  return 148;
+}
+
 // A multiprocessor changes the share of shared memory in its 256 KB only when it is empty: a chained kernel that needs shared memory cannot be
 // brought up beside one in front that runs on all L1.  So the one in front asks for half of it.
 template <typename... KArgs>

@@ -11,6 +11,8 @@
 //            same state, one exchange of the eight tokens' sums between the lanes, the eight writes in one pass.
 //            A block's vectors come by bulk copies into a ring; packed 32-bit arithmetic (two rows per instruction).
 // Every wait is bounded: when one runs out the block writes nothing more and sets B200KV_S_TIMEOUT.
+#include <algorithm>
+
 #include "dec_tma.cuh"
 #include "recurrence.cuh"
 
@@ -599,15 +601,21 @@ static int rb_launch(const b200dec_recurrence& rec, const b200dec_recurrence_in&
   const int list = ent.num_rows / kRbTok + ent.num_entries;
   // Blocks of 256 threads in one round; those of the list that have a decoding entry's place leave at once and do not
   // count: 185 rows, 16 heads of 128 beside 16 decoding entries, with the convolution and the scan 45.2 -> 42.5 us.
-  const bool few = (long long)(ent.num_rows / kRbTok + 1) * rec.heads <= 148 * 4;
+  const bool few = (long long)(ent.num_rows / kRbTok + 1) * rec.heads <= 4 * device_sms();
   const int rc = launch_result(launch_chained(few ? rb_prepare_kernel<T, Dp, 2> : rb_prepare_kernel<T, Dp, 1>, dim3(list, rec.heads),
                                               dim3(few ? 256 : 128), 0, s, rec, in, (const T*)conv, stride, ent, ws, status));
   if (rc != B200KV_OK) return rc;
   const size_t smem = (size_t)kRbStages * rb_floats(Dp) * 4;
-  // All blocks of two warps' columns by four warps at once (three fit a multiprocessor), but for one entry, which a step's padding takes. us a
-  // layer: three portions of 1000 rows in all, 16 heads of 128 132.7 -> 125.1; one of 614 rows, 12 heads of 96 and 112 108.7 -> 100.5; of less than
-  // 200 rows the same. With more blocks than that the schedulers have work without it, and the second copy of the state is a third more.
-  const bool split = (long long)rec.heads * slabs * (ent.num_entries - 1) <= 3 * 148;
+  // Warps of their own for the read-out where a portion's blocks have a multiprocessor each and all portions' blocks are one round; or, where three fit a
+  // multiprocessor, two portions', or nearly three rounds.  us a layer, without and with, blocks of all portions in brackets: one of 614 rows [64] 106.6 and 100.0, [96] 110.7 and
+  // 104.5, [128] 114.8 and 106.7, [160] 131.8 and 137.4, [192] 135.8 and 142.7; several of 1000 rows in all [96] 75.9 and 69.8, [128] 73.8 and
+  // 67.7, [168] 88.7 and 90.7, [192] 90.2 and 93.3 (of two portions 134.2 and 133.2), [256] of two 142.4 and 141.4, [336] 92.3 and 98.7 (129.2 and 129.1), [384] 129.3 and
+  // 122.0, [420] 138.3 and 129.1, [512] 114.8 and 131.1.  A step's entries are counted but for the padding one; entries that bring nothing are known on the
+  // device only, and with many of them the form with fewer warps is taken, as with many portions.
+  const int portions = std::max(1, ent.num_entries - 1);
+  const long long sms = device_sms(), portion = (long long)rec.heads * slabs, all = portion * portions;
+  const bool three = 3 * (smem + 4096) <= 227 * 1024;  // (with the static part and the reserved kilobyte)
+  const bool split = portion <= sms && (all <= sms || (three && (portions == 2 || (2 * all > 5 * sms && all <= 3 * sms))));
   auto* scan = split ? rb_scan_split_kernel<T, kLanes, kR> : rb_scan_kernel<T, kLanes, kR>;
   if (!allow_smem(scan, smem)) return B200KV_E_LAUNCH;
   // Not chained: brought up beside the kernel in front, its few long-running blocks would crowd on the multiprocessors that

@@ -347,6 +347,34 @@ def test_delta_rule_by_twice_the_warps(heads, groups, dim, vdim, dtype):
     status_clear()
 
 
+@pytest.mark.parametrize("chunks", [[17], [50, 33], [40, 9, 70]])
+@pytest.mark.parametrize("heads,groups,dim,vdim", [(4, 4, 128, 128), (16, 16, 128, 120), (19, 19, 100, 128), (3, 1, 200, 33), (18, 18, 256, 72), (16, 16, 130, 128)])
+def test_delta_rule_by_the_number_of_blocks(heads, groups, dim, vdim, chunks):
+    """One to three portions, from part of a round of blocks to more than three, in a table that fits them and in one with room for many more:
+    whichever form each takes, the same outputs and states, bit for bit (the preparation is the same)."""
+    from inference_engine_b200 import ops
+
+    g = np.random.default_rng(dim)
+    rec, _ = make_rec(g, next(k for k in KINDS if "delta" in k), heads, groups, dim, vdim, 4)
+    x, step, beta = (torch.cat(t) for t in zip(*(rec_inputs(g, rec, n, torch.bfloat16) for n in chunks)))
+    first = torch.randn(len(chunks), heads, dim, vdim, device=DEV)
+
+    def run(idle):
+        st = ops.make_recurrent_state(rec, len(chunks), torch.bfloat16, DEV)
+        st.state[..., :vdim] = first
+        n = len(chunks)
+        rows, _ = step_rows([3] * n + [0] * idle, chunks + [0] * idle, 0, slots=list(range(n)) + [-1] * idle)
+        out = torch.empty(rows.num_rows, heads * vdim, device=DEV)
+        ops.recurrence_prefill(rec, st, x, step, beta, rows, out, "blocked")
+        return out, st.state, st.ring
+
+    want = run(64)
+    for idle in (0, 1):
+        for got, w in zip(run(idle), want):
+            assert torch.equal(got, w)
+    status_clear()
+
+
 @pytest.mark.parametrize("kind", KINDS)
 @pytest.mark.parametrize("heads,groups,dim,vdim", [(2, 1, 64, 64), (16, 4, 128, 72), (40, 8, 16, 16), (100, 4, 32, 8)])
 def test_long_portions_beside_others(kind, heads, groups, dim, vdim):
