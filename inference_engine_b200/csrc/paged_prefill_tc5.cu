@@ -40,7 +40,7 @@ extern "C" int b200dec_prefill_attn_opt(const void* q, const b200dec_cache* cach
       kernel, dim3(heads, num_tiles * subs), dim3(kT5Threads), kT5Smem, (cudaStream_t)stream, (const uint16_t*)q,
       (long long)heads * pg.c.k_row, (long long)pg.c.k_row, none, 0LL, 0LL, none, 0LL, 0LL, seq_ids, cu_seqlens, tile_start, block_m, subs, none,
       none, 0LL, 0LL, no_lens, (uint16_t*)out, pg.opt.out_stride, (long long)pg.c.v_dim, num_rows, heads / pg.c.heads,
-      scale * 1.4426950408889634f, status, tm_k, tm_v, tm_k, tm_v, 0, 0, pg));
+      scale * 1.4426950408889634f, status, tm_k, tm_v, tm_k, tm_v, 0, 0, device_sms() / heads / subs, pg));
 }
 
 extern "C" int b200dec_prefill_attn(const void* q, const b200dec_cache* cache, const b200kv_table* table, const int32_t* seq_ids,

@@ -977,7 +977,8 @@ using namespace b200kv;
 static int at_splits(long long blocks, int tile_rows, long long most_keys, int window) {
   if (window > 0 && window + tile_rows < most_keys) most_keys = window + tile_rows;
   int splits = 1;
-  while (splits < 8 && 2 * splits * blocks <= 2 * 148 && splits * kAtKeys < most_keys) splits *= 2;
+  const int resident = 2 * device_sms();
+  while (splits < 8 && 2 * splits * blocks <= resident && splits * kAtKeys < most_keys) splits *= 2;
   return splits;
 }
 
@@ -1015,8 +1016,9 @@ static int check_rows(const b200dec_rows* r) {
 // Rotation, attention and all, us with 64 / 128 / 256 / 512 threads: 1000 rows 30.8 / 28.8 / 30.8 / 34.9, 300 rows 22.6 / 21.2 / 20.6 / 22.6,
 // 64 rows 45.6 / 43.2 / 42.3 / 42.2.
 static int row_threads(int num_rows, int items, int most) {
+  const long long round = 1024ll * device_sms();
   int threads = 512;
-  while (threads > 64 && (threads / 2 >= items || (2 * items <= most * threads && (long long)num_rows * threads > 148ll * 1024))) threads /= 2;
+  while (threads > 64 && (threads / 2 >= items || (2 * items <= most * threads && (long long)num_rows * threads > round))) threads /= 2;
   return threads;
 }
 

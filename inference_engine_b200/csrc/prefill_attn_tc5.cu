@@ -55,7 +55,7 @@ int launch_prefill_attn_tc5(const uint16_t* q, long long q_sn, long long q_sh, c
   const cudaError_t le = launch_chained(prefill_attn_tc5_kernel<false>, dim3(Hq, num_tiles * subs), dim3(kT5Threads), kT5Smem, stream,
                                         q, q_sn, q_sh, k, k_sn, k_sh, v, v_sn, v_sh, seq_ids, cu_seqlens, tile_start, block_m, subs,
                                         k_prefix, v_prefix, p_sh, p_sn, cu_cached, out, o_sn, o_sh, N, Hq / Hkv, scale_log2, status,
-                                        tm_k, tm_v, tm_kp, tm_vp, prefix_tma, idle_issuers, T5Paged{});
+                                        tm_k, tm_v, tm_kp, tm_vp, prefix_tma, idle_issuers, device_sms() / Hq / subs, T5Paged{});
   return le == cudaSuccess && cudaGetLastError() == cudaSuccess ? B200KV_OK : B200KV_E_LAUNCH;
 }
 

@@ -211,7 +211,6 @@ struct T5Paged {
 // of 1000 rows 34.9 -> 25.0, and on 2000 cached keys 53.3 -> 37.0; two portions on 4000 114 -> 90.  With
 // tiles of up to 6 blocks only that second one took 53.4, with 10 41.1 and with 16 as long, and the first 27.9 and 28.7 (before the loops
 // behind the products were rolled up).
-constexpr int kT5Sms = 148;
 constexpr int kT5PairBlocks = 10;
 
 template <bool kPaged, int kKeyBlocks = 2, bool kOptions = false>  // kKeyBlocks: 64-channel blocks of a key (2 covers up to 128 channels)
@@ -225,7 +224,7 @@ prefill_attn_tc5_kernel(const uint16_t* q, long long q_sn, long long q_sh, const
                         long long o_sh, int N, int G, float scale_log2, int32_t* status,
                         const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                         const __grid_constant__ CUtensorMap tm_kp, const __grid_constant__ CUtensorMap tm_vp, int prefix_tma,
-                        int idle_issuers, const __grid_constant__ T5Paged pg) {
+                        int idle_issuers, int full_tiles, const __grid_constant__ T5Paged pg) {
   extern __shared__ uint8_t t5_raw[];
   // idle_issuers (a test mode): the issuing warps do nothing and every wait gives up after a few thousand polls,
   // so that all bounded waits of the kernel run out and the time-out path is exercised without a fault
@@ -237,8 +236,8 @@ prefill_attn_tc5_kernel(const uint16_t* q, long long q_sn, long long q_sh, const
   // heads run fastest in the grid: the caller's real tiles come first in tile_start, so every CTA with work
   // is dispatched before the idle ones behind them
   const int tile = blockIdx.y / subs, sub = blockIdx.y - tile * subs, Hq = gridDim.x;
-  // the last tile with which every CTA of one head and tile has a multiprocessor of its own (the real tiles come first)
-  const int full = kT5Sms / Hq / subs, past = full * subs < (int)gridDim.y ? tile_start[full] : -1;
+  // full_tiles: the tiles with which every CTA of one head and tile has a multiprocessor of its own (the real tiles come first)
+  const int past = full_tiles * subs < (int)gridDim.y ? tile_start[full_tiles] : -1;
   const int tile_row = tile_start[tile];
   if (tile_row < 0 || tile_row >= N) return;
   const int seq = seq_ids[tile_row];
