@@ -372,13 +372,27 @@ def expert_tile_rows(num_rows: int, top: int, experts: int, dtype) -> int:
     if dtype == torch.float32:
         return 32
     # The line lies where some expert begins to have more than 64 rows, whose weights are then read twice; of many experts one does sooner.
-    # us, both products, tiles of 64 and 256: 8 experts of 3072, 2 a token, 192 rows 64.3 and 66.2 (a layer of 209 86.2 and 87.7), 224 85.8 and 66.6;
-    # a layer with 32 experts of 1536, 4 a token, 288 rows 137 and 137, 320 rows 143 and 137.5, 384 154 and 139.
-    return 64 if num_rows * top <= (52 if experts <= 16 else 39) * experts else 256
+    # us a layer with tiles of 64 and 256, rows an expert in brackets: 8 experts of 3072 [53.2] 83.2 and 86.1, [54] 103.0 and 86.2; 12 of 2048
+    # [41.7] 85.9 and 84.2, [46.7] 92.7 and 84.9; 16 of 2048 [37.5] 104.3 and 104.5, [42.5] 106.6 and 103.9, [47.5] 116.9 and 104.9; 20 of 1536 [36]
+    # 101.1 and 100.5; 24 [33.3] 114.2 and 112.8, [39] 120.9 and 114.3; 32 [36] 138.6 and 137.2, [37.5] 147.1 and 137.4; 64 of 1024 [31.2] 184.2 and 179.7.
+    return 64 if num_rows * top <= min(54 * experts, 28 * experts + 200) else 256
 
 
 def max_expert_tiles(total: int, experts: int, tile_rows: int) -> int:
     return total // tile_rows + min(experts, total)
+
+
+def one_launch(total: int, experts: int, width: int, ff: int, sms: int) -> bool:
+    """Whether both products of the experts are one launch."""
+    # Unless the second one's items are the longer ones: as the last to be drawn they leave multiprocessors idle
+    # for longer than a start takes.  us a layer, two launches and one: 32 experts of 1536 (width 2048), 64 rows 135.3 and 123.0, 512 154.6
+    # and 145.4, 1024 175.2 and 165.7; 8 experts of 3072, 64 rows 79.5 and 82.3, 192 84.4 and 94.1, 700 106.8 and 113.8 (16 80.1 and 77.3, 1000 135 and 129).
+    # Not where the first product of all experts is less than two rounds of items (8 experts of 2048, 32 rows 62.3 and 66.4), nor where that of the
+    # experts that a few rows can reach is less than one, since the second one's would only wait (1 row, 4 of 32 experts 45.2 and 46.9, 2 rows 63.6
+    # and 63.4, 3 rows 72.0 and 66.0; 2 rows, 4 of 64 experts of 1024 45.8 and 46.9, 3 rows 71.6 and 66.5), nor where tiles are full and the
+    # tensor core is the bound (32 experts of 1536, router and dispatch included: 1536 rows 175.3 and 173.4, 2048 213.9 and 228.2, 4096 367 and 408).
+    items = (2 * ff + 127) // 128  # of an expert with one tile
+    return ff <= width and total <= 192 * experts and items * experts >= 2 * sms and items * min(experts, total) >= sms
 
 
 def grouped_linear(x, w, tiles, max_tiles, tile_rows, scores=None, limit=0.0, slope=0.0, variant: int | None = None):
@@ -413,13 +427,7 @@ def mixture(x: torch.Tensor, xb: torch.Tensor, ex: Experts, variant: int | None 
     ids, ranks, slots, scores = (torch.empty(total, dtype=torch.int32, device=dev) for _ in range(4))
     tiles = torch.empty(1 + 3 * max_tiles + max_tiles + 1, dtype=torch.int32, device=dev)  # and the counters of the products behind them
     ff = ex.down.shape[2]
-    # Both products in one launch, unless the second one's items are the longer ones: as the last to be drawn they leave multiprocessors idle
-    # for longer than a start takes.  us a layer, two launches and one: 32 experts of 1536 (width 2048), 64 rows 135.3 and 123.0, 512 154.6
-    # and 145.4, 1024 175.2 and 165.7; 8 experts of 3072, 64 rows 79.5 and 82.3, 192 84.4 and 94.1, 700 106.8 and 113.8 (16 80.1 and 77.3, 1000 135 and 129).
-    # Not where the first product has less than about two rounds of items (8 experts of 1024, 64 rows 39.1 and 41.8), nor where tiles are full and the
-    # tensor core is the bound (32 experts of 1536, router and dispatch included: 1536 rows 175.3 and 173.4, 2048 213.9 and 228.2, 4096 367 and 408).
-    both = (variant is None and xb.dtype == torch.bfloat16 and W % 8 == 0 and ff % 8 == 0 and ff <= W and total <= 192 * E
-            and 2 * ff * E >= 300 * 128)
+    both = variant is None and xb.dtype == torch.bfloat16 and W % 8 == 0 and ff % 8 == 0 and one_launch(total, E, W, ff, K.num_sms(dev))
     done = tiles.data_ptr() + 4 * (1 + 3 * max_tiles) if both else None
     score_sorted = torch.empty(total, dtype=torch.float32, device=dev)
     rc = lib.b200dec_router(x.data_ptr(), ex.router.data_ptr(), N, W, E, ex.top, ids.data_ptr(), scores.data_ptr(), ranks.data_ptr(),

@@ -228,3 +228,26 @@ def test_trace_reader_feeds_the_engine(tmp_path):
     trace.run(eng, lines, str(tmp_path), done.append)
     assert done == [0, 1] and os.listdir(tmp_path) == ["0.f32"] and (eng.opened, eng.closed) == (1, 1)
     assert np.fromfile(tmp_path / "0.f32", "<f4").tolist() == [5.0, 5.0]
+
+
+def test_rules_of_the_experts_products():
+    """One launch only where the experts that the rows can reach give every multiprocessor an item of the first product; tiles of 256 rows from where
+    the busiest expert outgrows 64, which comes at fewer rows an expert the more of them there are, without a step between two numbers."""
+    import torch
+
+    from inference_engine_b200 import ops
+
+    assert not ops.one_launch(1 * 4, 32, 2048, 1536, 148) and ops.one_launch(3 * 4, 32, 2048, 1536, 148)
+    assert not ops.one_launch(2 * 4, 64, 2048, 1024, 148) and ops.one_launch(3 * 4, 64, 2048, 1024, 148)
+    assert not ops.one_launch(64 * 2, 8, 2048, 2048, 148) and not ops.one_launch(64 * 2, 8, 2048, 3072, 148)
+    assert ops.one_launch(1024 * 4, 32, 2048, 1536, 148) and not ops.one_launch(2048 * 4, 32, 2048, 1536, 148)
+    lines = []
+    for experts in range(1, 129):
+        rows = [n for n in range(1, 64 * experts) if ops.expert_tile_rows(n, 1, experts, torch.bfloat16) == 64]
+        assert rows == list(range(1, len(rows) + 1))
+        lines.append(len(rows))
+        assert ops.expert_tile_rows(10 ** 6, 1, experts, torch.bfloat16) == 256 and ops.expert_tile_rows(10 ** 6, 1, experts, torch.float32) == 32
+    assert all(0 < b - a <= 54 for a, b in zip(lines, lines[1:]))  # the line rises with the experts ...
+    assert all(a / (i + 1) >= b / (i + 2) for i, (a, b) in enumerate(zip(lines, lines[1:])))  # ... by less and less an expert
+    assert ops.expert_tile_rows(209, 2, 8, torch.bfloat16) == 64 and ops.expert_tile_rows(220, 2, 8, torch.bfloat16) == 256
+    assert ops.expert_tile_rows(340, 2, 16, torch.bfloat16) == 256 and ops.expert_tile_rows(300, 4, 32, torch.bfloat16) == 256
