@@ -344,11 +344,19 @@ class Engine:
         self.rows.pop(r.id, None)
 
     # ------------------------------------------------------------------ input buffers
-    def mixed_layout(self, n_tokens: int) -> list[int]:
+    def step_entries(self, n_tokens: int, live: int | None = None) -> int:
+        """Entries of a step with prefill, the padding one included: for a bucket as many as its tokens can belong to, for a step
+        that is not recorded those it has (`live`; above eight in steps of eight, since decode attention keeps a workspace
+        for each number).  The kernels choose their forms, and lay out their grids, by this number."""
+        if live is None:
+            return min(self.num_entries, n_tokens + 1)
+        return min(self.num_entries, live + 1 if live < 8 else -(-(live + 1) // 8) * 8)
+
+    def mixed_layout(self, n_tokens: int, live: int | None = None) -> list[int]:
         """Field lengths of a step with prefill padded to n_tokens: ids, positions, seq_ids, cu_seqlens,
-        cached_lens, cu_cached, tile_start, num_decoding, block table, state slots.  The same n_tokens always gives the
-        same layout, so a bucket's fields always sit at the same addresses."""
-        E = self.num_entries
+        cached_lens, cu_cached, tile_start, num_decoding, block table, state slots.  The same n_tokens always gives a bucket the
+        same layout, so its fields always sit at the same addresses."""
+        E = self.step_entries(n_tokens, live)
         return [n_tokens, n_tokens, n_tokens, E + 1, E, E + 1, math.ceil(n_tokens / self.block_m) + E, 1, E * self.max_pages, E]
 
     def decode_layout(self) -> list[int]:
@@ -367,12 +375,12 @@ class Engine:
             self.rows[r.id] = (len(r.pages), row)
         return row
 
-    def fill_mixed(self, step: Step, n_pad: int):
+    def fill_mixed(self, step: Step, n_pad: int, live: int | None = None):
         """Build the step's metadata on the host (scaffold.plan_step = the reference's fill_inputs), one copy."""
-        nd = step.num_decoding
+        nd, num_entries = step.num_decoding, self.step_entries(n_pad, live)
         plan = self.S.plan_step([r.cached_len for r, _ in step.entries[:nd]],
-                           [(r.cached_len, len(t)) for r, t in step.entries[nd:]], n_pad, self.num_entries, self.block_m)
-        sizes = self.mixed_layout(n_pad)
+                           [(r.cached_len, len(t)) for r, t in step.entries[nd:]], n_pad, num_entries, self.block_m)
+        sizes = self.mixed_layout(n_pad, live)
         buf = self.np_mixed[: sum(sizes)]
         offs = [0]
         for n in sizes:
@@ -383,7 +391,7 @@ class Engine:
         for i, key in enumerate(("positions", "seq_ids", "cu_seqlens", "cached", "cu_cached", "tile_start", "num_decoding"), 1):
             assert len(plan[key]) == sizes[i]
             buf[offs[i] : offs[i + 1]] = plan[key]
-        table = buf[offs[8] : offs[9]].reshape(self.num_entries, self.max_pages)
+        table = buf[offs[8] : offs[9]].reshape(num_entries, self.max_pages)
         for i, (r, _) in enumerate(step.entries):
             table[i] = self.table_row(r)
         table[len(step.entries)] = self.scratch_row  # the padding entry lives on the scratch run
@@ -394,11 +402,11 @@ class Engine:
         self.dev_mixed[: len(buf)].copy_(self.host_mixed[: len(buf)], non_blocking=True)
         return plan["cu_cached"][-1]
 
-    def mixed_views(self, n_pad: int, prefix_tokens: int = 0):
-        S = self.S
-        v = self.dev_mixed[: sum(self.mixed_layout(n_pad))].split(self.mixed_layout(n_pad))
+    def mixed_views(self, n_pad: int, prefix_tokens: int = 0, live: int | None = None):
+        S, sizes = self.S, self.mixed_layout(n_pad, live)
+        v = self.dev_mixed[: sum(sizes)].split(sizes)
         inp = S.StepInputs(ids=v[0], positions=v[1], seq_ids=v[2], cu_seqlens=v[3], cached_lens=v[4], cu_cached=v[5],
-                           tile_start=v[6], num_decoding=v[7], block_table=v[8].view(self.num_entries, self.max_pages),
+                           tile_start=v[6], num_decoding=v[7], block_table=v[8].view(-1, self.max_pages),
                            prefix_tokens=prefix_tokens, block_m=self.block_m, slots=v[9])
         if self.prefix is None:
             return inp, None
@@ -412,8 +420,8 @@ class Engine:
         return ids[:b], cached[:b], nd, table.view(B, self.max_pages)[:b], slots[:b]
 
     # ------------------------------------------------------------------ execution
-    def forward_mixed(self, n_pad: int, prefix_tokens: int = 0):
-        inp, prefix = self.mixed_views(n_pad, prefix_tokens)
+    def forward_mixed(self, n_pad: int, prefix_tokens: int = 0, live: int | None = None):
+        inp, prefix = self.mixed_views(n_pad, prefix_tokens, live)
         state = {} if self.slots is None else {"slots": inp.slots}
         return self.model.step(self.caches, inp, inp.ids, inp.cached_lens, inp.block_table, inp.num_decoding, prefix, **state)
 
@@ -490,8 +498,9 @@ class Engine:
         torch = self.torch
         N = step.num_tokens
         n_pad = next((x for x in self.token_buckets if x >= N), N)
+        live = None if n_pad in self.mixed_graphs else len(step.entries)
         t_in = time.perf_counter()
-        prefix_tokens = self.fill_mixed(step, n_pad)
+        prefix_tokens = self.fill_mixed(step, n_pad, live)
         self.seconds["inputs"] += time.perf_counter() - t_in
         if n_pad in self.mixed_graphs and (self.prefix is None or prefix_tokens <= self.prefix_capacity):
             g, out = self.mixed_graphs[n_pad]
@@ -499,6 +508,6 @@ class Engine:
             self.steps_run["mixed_graph"] += 1
         else:
             with torch.inference_mode():
-                out = self.forward_mixed(n_pad, prefix_tokens)
+                out = self.forward_mixed(n_pad, prefix_tokens, live)
             self.steps_run["eager"] += 1
         return out

@@ -52,6 +52,26 @@ def test_steps_beyond_the_largest_bucket_run_eagerly_with_the_same_result():
     assert [r.output for r in ra] == [r.output for r in rb]
 
 
+def test_steps_do_not_depend_on_the_room_for_requests():
+    """The kernels choose their forms by a step's entries, and so those are what the step has or its bucket can hold, not what the engine can: the
+    same steps in engines for three and for forty requests, recorded and not."""
+    outs = []
+    for use_graphs, most in ((False, 3), (False, 40), (True, 40)):
+        eng = build(use_graphs, max_batch_size=most, max_tokens_per_step=100, max_graph_tokens=96, max_len=256)
+        seen, fill = [], eng.fill_mixed
+        eng.fill_mixed = lambda step, n_pad, live=None: seen.append((n_pad, len(step.entries), eng.mixed_layout(n_pad, live)[4])) or fill(step, n_pad, live)
+        reqs = eng.generate(prompts()[:3], max_new_tokens=4)
+        outs.append([r.output for r in reqs])
+        for n_pad, live, entries in seen:
+            assert live < entries <= (min(most, n_pad) if n_pad in eng.mixed_graphs else live) + 1
+        if use_graphs:
+            assert eng.steps_run["eager"] > 0 and eng.steps_run["mixed_graph"] > 0
+    assert outs[0] == outs[1] == outs[2]
+    eng = build(False, max_batch_size=40)
+    assert [eng.step_entries(10, n) for n in (0, 1, 7, 8, 15, 16, 39, 40)] == [1, 2, 8, 16, 16, 24, 40, 41]
+    assert [eng.step_entries(n) for n in (1, 16, 40, 96)] == [2, 17, 41, 41]
+
+
 def test_requests_arriving_while_others_decode():
     eng = build(True)
     p = prompts()
