@@ -194,7 +194,10 @@ __host__ __device__ __forceinline__ Partition make_partition(int total_tiles_one
 }
 
 // At most one (entry, head) per multiprocessor: above that even shares keep the grid busy and hand-offs are hidden behind other
-// CTAs' tiles, while the longer code of an aligned split costs its fetch (nineteen entries of 512: the same either way).
+// CTAs' tiles, while the longer code of an aligned split costs its fetch (nineteen entries of 512: the same either way).  By the table's entries, not
+// those that decode: the kernel that could look would cost every large batch that code (us, two to four layers: 64 entries of 4096 208.4 and
+// 209.4, 32 of 128 41.1 and 43.1, 32 beside 992 rows 85.4 and 87.0), against a gain for steps with few decoding entries in a long table (16 beside
+// 50 rows in one of 65 49.0 and 42.1).
 __host__ __device__ __forceinline__ bool few_pairs(long long B, int Hkv, int sm_count) { return B * Hkv <= sm_count; }
 
 __host__ __device__ constexpr int scan_ints(int threads) { return threads + 1 + 2 * (threads / 32); }  // shared: prefix, warps' sums and maxima

@@ -26,7 +26,9 @@ constexpr int kPdRows = 16;      // query heads per unit
 // as long as a wide one, which is a chain and not bytes; and with four, twice as many pairs of entry and head have a CTA of their own. Where there are no
 // more pairs than two per multiprocessor the deeper ring is better. us, two and four, 8 kv heads of 64 and 64: 64 entries of 500 22.0 and 13.8, of 200
 // to 4096 with a window of 512 23.5 and 14.4, 128 of 4000 to 4096 177.7 and 180.2 (heads of 32 and 64 173.9 and 137.7); 32 with the window 11.8 and
-// 12.9, one of 300 7.7 and 8.2.
+// 12.9, one of 300 7.7 and 8.2.  Pairs are counted by the table's entries, since the grid and the rings are fixed before the device knows how many
+// decode.  With a table of 65 that costs a step with few of them up to 10 % (one of 300 7.7 and 8.0, 8 of 300 7.8 and 8.2, 37 of 500 10.5 and 11.7; but
+// 8 of 2000 16.8 and 14.1) and saves one with many more than that (44 of 500 18.2 and 11.8, 64 of 500 21.5 and 13.3).
 constexpr int kPdCtasPerSm = 2, kPdCtasNarrow = 4;
 constexpr int kPdMinBlocks = 4;  // smallest share of a CTA
 constexpr int kPdHandOff = 5;    // blocks that take one CTA as long as handing parts of an (entry, head) over through the workspace

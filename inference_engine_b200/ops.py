@@ -74,7 +74,8 @@ def make_paged_kv(num_pages: int, kv_heads: int, page_size: int, k_dim: int, v_d
 @dataclass
 class Rows:
     """Which (entry, position) each packed row of a step is.  seq_ids / positions None: pure decode, row = entry at
-    position cached_lens[row], rows from num_decoding on idle."""
+    position cached_lens[row], rows from num_decoding on idle.  cu_seqlens and tile_start (the entries' and tiles' first rows) are what recurrent layers
+    and the tensor cores' attention go by, whose rows lie entry after entry at consecutive positions; 32-bit attention goes by seq_ids and positions."""
 
     num_rows: int
     cached_lens: torch.Tensor
