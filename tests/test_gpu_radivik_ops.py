@@ -390,9 +390,10 @@ def test_mixture(dtype, rows, width, ff, experts, top, limit):
     H.status_clear()
 
 
-@pytest.mark.parametrize("rows,width,ff,experts,top", [(1, 2048, 512, 40, 2), (70, 2048, 1536, 13, 4), (130, 1032, 520, 40, 3), (900, 1024, 776, 25, 5), (1000, 2048, 1280, 16, 3)])
+@pytest.mark.parametrize("rows,width,ff,experts,top", [(1, 2048, 512, 40, 2), (4, 2048, 1536, 40, 2), (70, 2048, 1536, 13, 4), (130, 1032, 520, 40, 3), (900, 1024, 776, 25, 5), (1000, 2048, 1280, 16, 3)])
 def test_both_products_of_the_experts_in_one_launch(rows, width, ff, experts, top):
-    """More items than multiprocessors, one tile alone, weight blocks and steps with a remainder: the same bits as in two launches, again and again."""
+    """More items than multiprocessors, one tile alone and a few tiles of one or two rows (one row goes in two launches itself), weight blocks and
+    steps with a remainder: the same bits as in two launches, again and again."""
     from inference_engine_b200 import ops
 
     g = torch.Generator(device=DEV).manual_seed(rows)
