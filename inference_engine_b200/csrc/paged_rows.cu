@@ -678,7 +678,7 @@ __host__ __device__ constexpr size_t at_floats(int k_row, int v_row) {
   return (size_t)kAtSlots * k_row + (size_t)kAtKeys * (k_row + 4) + (size_t)kAtKeys * v_row + kAtKeys * kAtPitch;
 }
 
-template <typename T, int kPieces>  // kPieces: output channels, in pieces of 128
+template <typename T, int kPieces, bool kListed>  // kPieces: output channels, in pieces of 128; kListed: with the entries' first rows
 __global__ void __launch_bounds__(kAtThreads, 2)
 attn_tile_kernel(const T* q, DecCache c, b200dec_rows rows, const int32_t* __restrict__ cu_seqlens, int num_entries, int heads, int slice_heads, float scale, DecAttnOpt opt,
                  T* __restrict__ out, int32_t* status) {
@@ -929,7 +929,7 @@ attn_tile_kernel(const T* q, DecCache c, b200dec_rows rows, const int32_t* __res
   int r0 = blockIdx.y, left = 1, seq = r0, pos, n = 1;
   if (rows.seq_ids) {
     left = min(most, rows.num_rows - r0);
-    if (cu_seqlens) {
+    if (kListed) {
       int lo = 0, hi = num_entries + 1;  // the last entry whose first place is not behind this block's
       while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
@@ -945,15 +945,14 @@ attn_tile_kernel(const T* q, DecCache c, b200dec_rows rows, const int32_t* __res
     }
   }
   pdl_wait();
-  for (; left > 0; r0 += n, left -= n) {
+  for (; left > 0; r0 += n, left -= n) {  // (not listed: once)
     if (rows.seq_ids) {  // the run from r0 on: lane i looks at row r0 + i
       static_assert(kAtSlots < 32, "a warp sees where a run ends");
       const int s = lane < left ? rows.seq_ids[r0 + lane] : 0, p = lane < left ? rows.positions[r0 + lane] : -1;
       seq = __shfl_sync(0xffffffffu, s, 0);
       pos = __shfl_sync(0xffffffffu, p, 0);
-      const bool same = p >= 0 && s == seq && p == pos + lane && (lane == 0 || cu_seqlens || p % most != 0);
+      const bool same = p >= 0 && s == seq && p == pos + lane && (lane == 0 || kListed || p % most != 0);
       n = max(1, __ffs(~__ballot_sync(0xffffffffu, same)) - 1);
-      if (!cu_seqlens) left = n;
     } else {
       pos = r0 < *rows.num_decoding ? rows.cached_lens[r0] : -1;
     }
@@ -962,6 +961,7 @@ attn_tile_kernel(const T* q, DecCache c, b200dec_rows rows, const int32_t* __res
     } else if (part == 0) {  // idle row
       for (int i = tid; i < gs * c.v_dim; i += kAtThreads) st_elem(out + r0 * opt.out_stride + (hk * G + g0) * c.v_dim + i, 0.f);
     }
+    if (!kListed) break;
   }
 }
 
@@ -1154,9 +1154,14 @@ extern "C" int b200dec_attn_rows_entries(const void* q, const b200dec_cache* cac
       return launch_result(launch_clusters(kernel, dim3(cache->kv_heads * slices, blocks, splits), dim3(kAtThreads), tile_smem, s, in, c,
                                            *rows, listed ? cu_seqlens : nullptr, (int)num_entries, heads, slice_heads, scale, opt, o, status));
     };
-    if (cache->elem == 2)
-      return tiles(cache->v_row <= 128 ? attn_tile_kernel<uint16_t, 1> : attn_tile_kernel<uint16_t, 2>, (const uint16_t*)q, (uint16_t*)out);
-    return tiles(cache->v_row <= 128 ? attn_tile_kernel<float, 1> : attn_tile_kernel<float, 2>, (const float*)q, (float*)out);
+    auto by_list = [&](auto some) {
+      constexpr bool kListed = decltype(some)::value;
+      if (cache->elem == 2)
+        return tiles(cache->v_row <= 128 ? attn_tile_kernel<uint16_t, 1, kListed> : attn_tile_kernel<uint16_t, 2, kListed>, (const uint16_t*)q,
+                     (uint16_t*)out);
+      return tiles(cache->v_row <= 128 ? attn_tile_kernel<float, 1, kListed> : attn_tile_kernel<float, 2, kListed>, (const float*)q, (float*)out);
+    };
+    return listed ? by_list(std::true_type{}) : by_list(std::false_type{});
   }
   const size_t smem = (size_t)((cache->k_dim + 3) / 4 * 4 + 2 * kArKeys) * 4;
   if (cache->elem == 2)
